@@ -34,25 +34,27 @@ __device__ __forceinline__ int find_seg(const uint32_t *__restrict__ pre, int n,
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 5) k_first_multi(const Inst<T> *__restrict__ inst,
                                                             const uint32_t *__restrict__ tpre, int n) {
-    __shared__ TileOf<T, kFirst, false> sm;
+    extern __shared__ __align__(128) unsigned char march_smem[];
+    CopyMarch<T, kFirst> &sm = *reinterpret_cast<CopyMarch<T, kFirst> *>(march_smem);
     const int i = find_seg(tpre, n, blockIdx.x);
     const Inst<T> &I = inst[i];
     if (!I.first) return;  // uniform: only fields that start now
     const uint32_t lt = blockIdx.x - __ldg(tpre + i);
     const uint32_t bx = lt % I.tiles_x, rest = lt / I.tiles_x;
     const uint32_t by = rest % I.tiles_y, bz = rest / I.tiles_y;
-    // fp32 blocks whose tile, halo and planes zb-1 .. ze lie inside their
-    // field run the check-free body, as in k_tiled (21.8 against 21.97 ms on
-    // the 64-field batch; for fp64 the second body raises the spills)
-    const int x0 = static_cast<int>(bx) * kTX, y0 = static_cast<int>(by) * kTY, zb = static_cast<int>(bz) * I.g.zc;
-    const bool inside = x0 >= 1 && x0 + kTX + 1 <= I.g.nx && y0 >= 1 && y0 + kTY + 1 <= I.g.ny && zb >= 1 &&
-                        zb + I.g.zc + 1 <= I.g.nz;
-    if (sizeof(T) == 4 && inside)
-        tiled_body<T, kFirst, false, true>(sm, I.f, I.fh, I.codes, I.hp, I.req, I.act1, I.slots, I.g,
-                                           static_cast<int>(bx), static_cast<int>(by), static_cast<int>(bz));
+    const MarchArgs<T> a{I.f, I.fh, I.codes, I.hp, I.req, nullptr, I.act1, I.slots, nullptr};
+    const int x = static_cast<int>(bx), y = static_cast<int>(by), z = static_cast<int>(bz);
+    if (march_inside(I.g, x, y, z))
+        march_copies<T, kFirst, false>(sm, a, I.g, x, y, z);
     else
-        tiled_body<T, kFirst>(sm, I.f, I.fh, I.codes, I.hp, I.req, I.act1, I.slots, I.g, static_cast<int>(bx),
-                              static_cast<int>(by), static_cast<int>(bz));
+        march_copies<T, kFirst, true>(sm, a, I.g, x, y, z);
+}
+template <typename T>
+static int launch_first_multi(const Inst<T> *inst, const uint32_t *tpre, int n, uint32_t tiles, cudaStream_t s) {
+    PMSZ_CUDA(allow_smem(k_first_multi<T>, sizeof(CopyMarch<T, kFirst>)));
+    k_first_multi<T><<<tiles, dim3(kTX, kThreads / kTX, 1), sizeof(CopyMarch<T, kFirst>), s>>>(inst, tpre, n);
+    PMSZ_CUDA(cudaGetLastError());
+    return PMSZ_OK;
 }
 
 template <typename T>
@@ -166,7 +168,10 @@ int MultiRun<T>::setup(const std::vector<FieldSpec<T>> &specs, int64_t max_sweep
     uint64_t tiles = 0, rounds = 0;
     voxels = 0;
     for (const FieldSpec<T> &sp : specs) voxels += sp.nx * sp.ny * sp.nz;
-    const int zc = tuned_batch_zchunk(voxels, n, sizeof(T));  // one first-pass launch covers the batch
+    uint64_t columns = 0;
+    for (const FieldSpec<T> &sp : specs) columns += column_planes(sp.nx, sp.ny, sp.nz);
+    const int zc = batch_tune_known(voxels, n, sizeof(T)) ? march_depth(tuned_batch_zchunk(voxels, n, sizeof(T)))
+                                                          : default_depth(columns);  // one first-pass launch covers the batch
     for (int i = 0; i < n; ++i) {
         Geom g = make_geom(specs[i].nx, specs[i].ny, specs[i].nz);
         g.zc = zc;
@@ -189,7 +194,7 @@ int MultiRun<T>::setup(const std::vector<FieldSpec<T>> &specs, int64_t max_sweep
         I.first = 1;
         I.stride = n;
         I.tiles_x = static_cast<uint32_t>(g.wpr);
-        I.tiles_y = static_cast<uint32_t>((g.ny + kTY - 1) / kTY);
+        I.tiles_y = static_cast<uint32_t>((g.ny + kMY - 1) / kMY);
         const uint64_t tz = static_cast<uint64_t>((g.nz + g.zc - 1) / g.zc);
         tpre[i] = static_cast<uint32_t>(tiles);
         rpre[i] = static_cast<uint32_t>(rounds);
@@ -268,6 +273,7 @@ int MultiRun<T>::push_table() {
 template <typename T>
 int MultiRun<T>::set_zchunk(int zc) {
     uint64_t tiles = 0;
+    zc = march_depth(zc);
     for (int i = 0; i < n; ++i) {
         Inst<T> &I = host[i];
         I.g.zc = zc;
@@ -305,8 +311,7 @@ int MultiRun<T>::tune_zchunk() {
         for (int rep = 0; rep < 3; ++rep) {  // the first run of each candidate is a warm-up
             PMSZ_CUDA(cudaMemsetAsync(zero_base, 0, zero_total, s));
             PMSZ_CUDA(cudaEventRecord(et.ev[0], s));
-            k_first_multi<T><<<total_tiles, dim3(kTX, kTY, 1), 0, s>>>(dinst, dtpre, n);
-            PMSZ_CUDA(cudaGetLastError());
+            if ((rc = launch_first_multi<T>(dinst, dtpre, n, total_tiles, s))) return rc;
             PMSZ_CUDA(cudaEventRecord(et.ev[1], s));
             PMSZ_CUDA(cudaEventSynchronize(et.ev[1]));
             float t = 0.f;
@@ -354,7 +359,10 @@ template <typename T>
 int launch_generation(const Inst<T> *dinst, const uint32_t *dtpre, const uint32_t *drpre, int n,
                       uint32_t total_tiles, uint32_t total_rounds, bool any_first, cudaStream_t s,
                       const MultiLists *ml) {
-    if (any_first) k_first_multi<T><<<total_tiles, dim3(kTX, kTY, 1), 0, s>>>(dinst, dtpre, n);
+    if (any_first) {
+        const int rc = launch_first_multi<T>(dinst, dtpre, n, total_tiles, s);
+        if (rc) return rc;
+    }
     if (ml) return launch_list_sweep<T>(dinst, n, *ml, s);
     const unsigned grid = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(total_rounds, 152 * 16)));
     k_phase_multi<T, 0><<<grid, kListBlock, 0, s>>>(dinst, drpre, n, total_rounds);

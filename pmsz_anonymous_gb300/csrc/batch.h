@@ -2,7 +2,7 @@
 // kernels read, and the host driver shared by pmsz_correct_batch (batch.cu)
 // and the continuous-batching server (server.cpp).
 #pragma once
-#include "tiled.cuh"
+#include "march.cuh"
 #include "internal.h"
 
 #include <string>

@@ -164,10 +164,27 @@ struct Geom {
     size_t nwords;    // wpr * ny * nz (< 2^32)
     size_t n;         // nx * ny * nz
     FastDiv div_wpr, div_ny, div_nx;  // div_nx: for flat indices below 2^32
-    int zc;           // planes per tile column of the tiled passes (tile 32 x 8 x zc)
+    int zc;           // planes per tile column of the full-field passes (tile 32 x 8 x zc)
 };
 
 constexpr int kZChunkDefault = 32;  // zc when no tuned value is recorded for the shape
+// Tiles of the full-field passes (march.cuh): 32 x 8 columns, one block each,
+// two voxels of a plane per thread.
+constexpr int kTX = 32, kMY = 8;
+constexpr int kMarchMaxDepth = 128;  // deeper columns run as this (the passes queue 7-bit depths)
+inline int march_depth(int zc) { return zc < kMarchMaxDepth ? zc : kMarchMaxDepth; }
+// Depth without a tuned value: the default, halved while the launch has fewer
+// columns than six blocks per SM (152 SMs hold six), down to 4 -- a 64^3 field
+// has 16 columns of 32 x 8, and 32 planes deep they leave most SMs idle and
+// every block a long serial march (first pass 75 us at depth 32, 33 us at 4);
+// below 4 the two halo planes of a column cost more than the extra blocks gain.
+inline int default_depth(uint64_t columns_planes, int zc = kZChunkDefault) {  // sum over fields of columns * nz
+    while (zc > 4 && columns_planes / static_cast<uint64_t>(zc) < 152u * 6u) zc /= 2;
+    return zc;
+}
+inline uint64_t column_planes(size_t nx, size_t ny, size_t nz) {
+    return static_cast<uint64_t>((nx + kTX - 1) / kTX) * ((ny + kMY - 1) / kMY) * nz;
+}
 
 inline Geom make_geom(size_t nx, size_t ny, size_t nz) {
     Geom g;

@@ -235,7 +235,7 @@ static FirstMaps first_maps(const T *f, const T *fh, const Geom &g) {
                                 static_cast<cuuint64_t>(g.nz)};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(g.nx) * sizeof(T),
                                    static_cast<cuuint64_t>(g.nx) * g.ny * sizeof(T)};
-    const cuuint32_t box[3] = {static_cast<cuuint32_t>(RawBox<T>::kX), static_cast<cuuint32_t>(kHY), 1u};
+    const cuuint32_t box[3] = {static_cast<cuuint32_t>(RawBox<T>::kX), static_cast<cuuint32_t>(kMHY), 1u};
     const cuuint32_t es[3] = {1u, 1u, 1u};
     const CUtensorMapDataType dt = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     for (int k = 0; k < 2; ++k)
@@ -247,18 +247,24 @@ static FirstMaps first_maps(const T *f, const T *fh, const Geom &g) {
     return m;
 }
 
-// The deferring first pass over the z-chunks bz0 .. bz0+grid.z-1: TMA-fed
-// interior blocks when the maps exist; *err is set if a plane's copy did not
-// arrive within the bounded wait.
+constexpr char kCopyMissing[] = "first pass: a tile plane's tensor copy did not arrive within the bounded wait";
+
+// The fused first pass over the z-chunks bz0 .. bz0+grid.z-1: TMA-fed when the
+// maps exist; *err is set if a plane's copy did not arrive within the bounded
+// wait, *xc += the voxels decided on full keys.
 template <typename T>
-static void launch_first_pass(const FirstMaps &m, dim3 grid, cudaStream_t s, const T *f, T *fh, uint8_t *codes,
-                              uint32_t *hp, uint32_t *req, uint32_t *act, SweepSlot *slot, const Geom &g, int bz0,
-                              uint32_t *xl, uint32_t *xc, uint32_t *err) {
-    const dim3 blk(kTX, kTY, 1);
-    if (m.ok)
-        k_first_tma<T><<<grid, blk, 0, s>>>(m.f, m.fh, f, fh, codes, hp, req, act, slot, g, bz0, xl, xc, err);
-    else
-        k_tiled<T, kFirst, true><<<grid, blk, 0, s>>>(f, fh, codes, hp, req, act, slot, g, bz0, xl, xc);
+static int launch_first_pass(const FirstMaps &m, dim3 grid, cudaStream_t s, const T *f, T *fh, uint8_t *codes,
+                             uint32_t *hp, uint32_t *req, uint32_t *act, SweepSlot *slot, const Geom &g, int bz0,
+                             uint32_t *xc, uint32_t *err) {
+    const MarchArgs<T> a{f, fh, codes, hp, req, nullptr, act, slot, xc};
+    if (m.ok) {
+        PMSZ_CUDA(allow_smem(k_first_tma<T>, sizeof(TmaMarch<T>)));
+        k_first_tma<T><<<grid, dim3(kTX, kThreads / kTX, 1), sizeof(TmaMarch<T>), s>>>(m.f, m.fh, a, g, bz0, err);
+        PMSZ_CUDA(cudaGetLastError());
+    } else {
+        PMSZ_CUDA((launch_march<T, kFirst>(grid, s, a, g, bz0)));
+    }
+    return PMSZ_OK;
 }
 
 // Runs sweeps first.. in one cooperative launch of k_tail_loop (grid = the
@@ -396,7 +402,7 @@ int enqueue_ingest(const T *hf, const T *hfh, T *df, T *dfh, T *dprev, size_t nx
     int rc = check_geom(nx, ny, nz);
     if (rc) return rc;
     Geom g = make_geom(nx, ny, nz);
-    g.zc = tuned_zchunk(nx, ny, nz, sizeof(T));  // the tile depth correct_impl will use
+    g.zc = first_depth(nx, ny, nz, sizeof(T));  // the tile depth correct_impl will use
     const IngestSlabs sl = ingest_slabs(g, sizeof(T));
     c.cps = sl.cps;
     c.nchunks = sl.nchunks;
@@ -440,20 +446,17 @@ int enqueue_ingest(const T *hf, const T *hfh, T *df, T *dfh, T *dprev, size_t nx
 template <typename T>
 int first_pass_ingest(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes, uint32_t *hp, uint32_t *req,
                       uint32_t *a_next, SweepSlot *slot, const Geom &g, cudaStream_t s, int64_t *launches,
-                      uint32_t *xlist, uint32_t *xcount, const FirstMaps *maps = nullptr, uint32_t *err = nullptr) {
+                      uint32_t *xcount, const FirstMaps &maps, uint32_t *err) {
     if (in.df != f || !in.copies || in.copies->zc != g.zc)
         return set_error(PMSZ_ERR_ARG, "ingest copies do not match the field");
     const IngestCopies &r = *in.copies;
     const int cps = r.cps, nchunks = r.nchunks, nslabs = r.nslabs;
-    const dim3 blk3(kTX, kTY, 1);
+    int rc;
     for (int j = 0; j < nslabs; ++j) {
         PMSZ_CUDA(cudaStreamWaitEvent(s, r.ev[j], 0));
         dim3 grid = tiled_grid(g);
         grid.z = static_cast<unsigned>(std::min(cps, nchunks - j * cps));
-        if (xlist)  // deferring first pass (see k_first_exact)
-            launch_first_pass<T>(*maps, grid, s, f, fh, codes, hp, req, a_next, slot, g, j * cps, xlist, xcount, err);
-        else
-            k_tiled<T, kFirst><<<grid, blk3, 0, s>>>(f, fh, codes, hp, req, a_next, slot, g, j * cps);
+        if ((rc = launch_first_pass<T>(maps, grid, s, f, fh, codes, hp, req, a_next, slot, g, j * cps, xcount, err))) return rc;
         PMSZ_CUDA(cudaGetLastError());
         ++*launches;
     }
@@ -473,12 +476,9 @@ constexpr int kWaveSweeps = 6;
 constexpr int kWaveAt8[] = {4, 8, 12, 14, 16};
 constexpr int kWaveAt4[] = {4, 8, 12, 16};
 
-// One-thread bookkeeping between the pieces of the wavefront (kernels rather
-// than small copies or memsets: a device-to-device copy may queue behind the
-// host copies on the copy engine).
-static __global__ void k_wave_mark(LoopState *ls) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) ls->xdone = ls->lc[3];
-}
+// One-thread bookkeeping between the pieces of the wavefront (a kernel rather
+// than a small memset, which may queue behind the host copies on the copy
+// engine).
 static __global__ void k_wave_clear_spills(LoopState *ls) {
     if (threadIdx.x == 0 && blockIdx.x == 0) ls->lc[2] = 0;
 }
@@ -502,13 +502,14 @@ static __global__ void k_wave_clear_spills(LoopState *ls) {
 template <typename T>
 static int first_pass_waves(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes, uint8_t *cnt, uint32_t *hp,
                             uint32_t *req, uint32_t *const act[2], SweepSlot *slots, LoopState *ls, const Geom &g,
-                            const FirstMaps &maps, uint32_t *list, uint32_t *xlist, uint32_t *slist, uint32_t *bcnt,
+                            const FirstMaps &maps, uint32_t *list, uint32_t *slist, uint32_t *bcnt,
                             const FastDiv &div_nx, T eps, T delta, int q, int K, cudaStream_t s, int64_t *launches) {
     if (in.df != f || !in.copies || in.copies->zc != g.zc)
         return set_error(PMSZ_ERR_ARG, "ingest copies do not match the field");
     const IngestCopies &r = *in.copies;
     const int cps = r.cps, nchunks = r.nchunks, nslabs = r.nslabs;
     const unsigned lb = 152 * 8;
+    int rc;
     std::vector<int> Dp(static_cast<size_t>(K) + 1, 0), Ap(static_cast<size_t>(K) + 1, 0);  // fronts so far
     std::vector<char> wave_after(static_cast<size_t>(nslabs), 0);
     auto mark = [&](int e) { wave_after[static_cast<size_t>(std::max(1, (nslabs * e + 15) / 16) - 1)] = 1; };
@@ -521,16 +522,11 @@ static int first_pass_waves(const HostIngest<T> &in, const T *f, T *fh, uint8_t 
         PMSZ_CUDA(cudaStreamWaitEvent(s, r.ev[j], 0));
         dim3 grid = tiled_grid(g);
         grid.z = static_cast<unsigned>(std::min(cps, nchunks - j * cps));
-        launch_first_pass<T>(maps, grid, s, f, fh, codes, hp, req, act[1], &slots[0], g, j * cps, xlist, &ls->lc[3],
-                             &ls->err);
+        if ((rc = launch_first_pass<T>(maps, grid, s, f, fh, codes, hp, req, act[1], &slots[0], g, j * cps, &ls->lc[3],
+                             &ls->err))) return rc;
         ++*launches;
         if (!wave_after[static_cast<size_t>(j)]) continue;
-        // the first pass's deferred voxels so far (all below Z), then mark them done
-        k_first_exact<T><<<lb, 256, 0, s>>>(xlist, &ls->lc[3], f, fh, codes, req, act[1], &slots[0], g, div_nx,
-                                            &ls->xdone);
-        k_wave_mark<<<1, 32, 0, s>>>(ls);
         PMSZ_CUDA(cudaGetLastError());
-        *launches += 2;
         PMSZ_CUDA(cudaStreamWaitEvent(s, r.evp[j], 0));  // fhat's pre-correction copy of slabs 0 .. j
         const int Z = last ? g.nz : std::min(g.nz, (j + 1) * cps * g.zc);
         for (int k = 0; k <= K; ++k) {
@@ -580,7 +576,7 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         (rc = autotune_impl<T>(f, fh, nx, ny, nz, nullptr, s)))
         return rc;
     Geom g = make_geom(nx, ny, nz);
-    g.zc = tuned_zchunk(nx, ny, nz, sizeof(T));
+    g.zc = first_depth(nx, ny, nz, sizeof(T));
     const T eps = static_cast<T>(eb);
     const T delta = static_cast<T>(eb / static_cast<double>(q));  // pMSz.cu:2814
 
@@ -600,12 +596,11 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
     const size_t o_xlist = ws.reserve<uint32_t>(use_list ? g.n : 0);
     const size_t o_bcnt = ws.reserve<uint32_t>(use_list ? kCompactBlocks : 0);
     const size_t o_ls = ws.reserve<LoopState>(use_list ? 1 : 0);
+    const size_t o_err = ws.reserve<uint32_t>(1);
     // host-buffer calls of several slabs run sweeps 1 .. K behind the copy
-    // (first_pass_waves; K even, below max_sweeps); their detection spills go
-    // to a list of their own (xlist still collects the first pass's deferrals)
+    // (first_pass_waves; K even, below max_sweeps)
     const int wave_k = static_cast<int>(std::min<int64_t>(kWaveSweeps, max_sweeps - 1)) & ~1;
     const bool waves = ingest && use_list && wave_k >= 2 && ingest->copies && ingest->copies->nslabs >= 2;
-    const size_t o_slist = ws.reserve<uint32_t>(waves ? g.n : 0);
     if ((rc = ws.commit())) return rc;
     uint32_t *hp = ws.at<uint32_t>(o_hp);
     uint8_t *codes = ws.at<uint8_t>(o_codes);
@@ -617,10 +612,10 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
     uint32_t *xlist = use_list ? ws.at<uint32_t>(o_xlist) : nullptr;
     uint32_t *bcnt = use_list ? ws.at<uint32_t>(o_bcnt) : nullptr;  // per-block counts of a compaction
     LoopState *ls = use_list ? ws.at<LoopState>(o_ls) : nullptr;
-    uint32_t *slist = waves ? ws.at<uint32_t>(o_slist) : nullptr;
+    uint32_t *ferr = use_list ? &ls->err : ws.at<uint32_t>(o_err);  // set by a first pass whose copies did not arrive
     const FastDiv div_nx = make_fastdiv(static_cast<uint32_t>(g.nx));
     const unsigned list_blocks = 152 * 8;
-    const FirstMaps maps = use_list ? first_maps<T>(f, fh, g) : FirstMaps{};
+    const FirstMaps maps = first_maps<T>(f, fh, g);
     EventTimer et;
     if ((rc = et.init())) return rc;
     PMSZ_CUDA(cudaEventRecord(et.ev[3], s));  // start of the loop's device window
@@ -633,10 +628,13 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
     if (use_list) {
         PMSZ_CUDA(cudaMemsetAsync(ls, 0, sizeof(LoopState), s));
         PMSZ_CUDA(cudaMemsetAsync(&ls->go, 1, 1, s));  // sweep 0 runs (little-endian int 1)
+    } else {
+        PMSZ_CUDA(cudaMemsetAsync(ferr, 0, sizeof(uint32_t), s));
     }
 
-    SweepSlot *hslot = static_cast<SweepSlot *>(host_pinned(sizeof(SweepSlot)));
+    SweepSlot *hslot = static_cast<SweepSlot *>(host_pinned(sizeof(SweepSlot) + 64));
     if (!hslot) return set_error(PMSZ_ERR_OOM, "pinned host allocation failed");
+    uint32_t *herr = reinterpret_cast<uint32_t *>(hslot + 1);
     const bool timing = (flags & PMSZ_FLAG_TIMING) != 0;
     double ms_first = 0, ms_detect = 0, ms_apply = 0;
     int64_t launches = 0;
@@ -668,7 +666,7 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         }
         if (waves) {  // sweeps 0 .. wave_k behind the host copy, then the state after them
             if ((rc = first_pass_waves<T>(*ingest, f, fh, codes, cnt, hp, req, act, slots, ls, g, maps, list, xlist,
-                                          slist, bcnt, div_nx, eps, delta, q, wave_k, s, &launches)))
+                                          bcnt, div_nx, eps, delta, q, wave_k, s, &launches)))
                 return rc;
             if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[1], s));
             k_wave_gate<<<1, 32, 0, s>>>(ls, slots, wave_k, max_sweeps, tail_at, static_cast<unsigned long long>(g.n),
@@ -679,16 +677,13 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         } else {
             if (ingest) {
                 if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, act[1], &ls->cur, g, s, &launches,
-                                               xlist, &ls->lc[3], &maps, &ls->err)))
+                                               &ls->lc[3], maps, &ls->err)))
                     return rc;
             } else {
-                launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, act[1], &ls->cur, g, 0, xlist,
-                                     &ls->lc[3], &ls->err);
+                if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, act[1], &ls->cur, g, 0,
+                                     &ls->lc[3], &ls->err))) return rc;
                 ++launches;
             }
-            k_first_exact<T><<<list_blocks, 256, 0, s>>>(xlist, &ls->lc[3], f, fh, codes, req, act[1], &ls->cur, g,
-                                                         div_nx);
-            ++launches;
             if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[1], s));
             compact_bitmap(req, g, bcnt, list, &ls->lc[1], &ls->go, s);
             k_apply_list<T><<<list_blocks, 256, 0, s>>>(list, &ls->lc[1], f, fh, cnt, hp, act[1], &ls->cur, g, div_nx,
@@ -806,7 +801,7 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         }
         PMSZ_CUDA(cudaStreamSynchronize(s));
         if (hls->err)
-            return set_error(PMSZ_ERR_CUDA, "first pass: a tile plane's tensor copy did not arrive within the bounded wait");
+            return set_error(PMSZ_ERR_CUDA, kCopyMissing);
         const int64_t gdone = hls->k;  // sweeps 0 .. gdone-1 ran before the tail
         const int64_t done = std::max<int64_t>(*hdone, gdone);  // and 0 .. done-1 in all
         const int64_t nloop = std::max<int64_t>(gdone - (waves ? wave_k + 1 : 1), 0);  // sweeps of the loop
@@ -853,14 +848,15 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         uint32_t *a_next = act[cur ^ 1];
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[0], s));
         if (sweeps == 0 && ingest) {
-            if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, a_next, slot, g, s, &launches, nullptr,
-                                           nullptr)))
+            if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, a_next, slot, g, s, &launches, nullptr, maps,
+                                           ferr)))
                 return rc;
         } else if (sweeps == 0) {
-            k_tiled<T, kFirst><<<tiled_grid(g), blk3, 0, s>>>(f, fh, codes, hp, req, a_next, slot, g, 0);
+            if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, a_next, slot, g, 0, nullptr, ferr))) return rc;
             ++launches;
         } else if (flags & PMSZ_FLAG_FULL_SWEEPS) {
-            k_tiled<T, kDetect><<<tiled_grid(g), blk3, 0, s>>>(fh, nullptr, codes, nullptr, req, a_next, slot, g, 0);
+            PMSZ_CUDA((launch_march<T, kDetect>(
+                tiled_grid(g), s, MarchArgs<T>{nullptr, fh, codes, hp, req, nullptr, a_next, slot, nullptr}, g, 0)));
             ++launches;
         } else {
             k_sparse_px<T><<<list_grid(g), kListBlock, 0, s>>>(fh, hp, codes, act[cur], a_next, req, slot, g);
@@ -872,7 +868,9 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[2], s));
         PMSZ_CUDA(cudaGetLastError());
         PMSZ_CUDA(cudaMemcpyAsync(hslot, slot, sizeof(SweepSlot), cudaMemcpyDeviceToHost, s));
+        if (sweeps == 0) PMSZ_CUDA(cudaMemcpyAsync(herr, ferr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         PMSZ_CUDA(cudaStreamSynchronize(s));
+        if (sweeps == 0 && *herr) return set_error(PMSZ_ERR_CUDA, kCopyMissing);
         if (timing) {
             float a = 0, b = 0;
             PMSZ_CUDA(cudaEventElapsedTime(&a, et.ev[0], et.ev[1]));
@@ -951,50 +949,45 @@ int codes_impl(const T *v, size_t nx, size_t ny, size_t nz, uint8_t *codes, cuda
     if (!v || !codes) return set_error(PMSZ_ERR_ARG, "null pointer");
     int rc = check_geom(nx, ny, nz);
     if (rc) return rc;
-    const Geom g = make_geom(nx, ny, nz);
-    k_tiled<T, kCodes><<<tiled_grid(g), dim3(kTX, kTY, 1), 0, s>>>(v, nullptr, codes, nullptr, nullptr, nullptr, nullptr, g, 0);
+    Geom g = make_geom(nx, ny, nz);
+    g.zc = first_depth(nx, ny, nz, sizeof(T));
+    PMSZ_CUDA((launch_march<T, kCodes>(
+        tiled_grid(g), s, MarchArgs<T>{v, nullptr, codes, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr}, g, 0)));
     PMSZ_CUDA(cudaGetLastError());
     return PMSZ_OK;
 }
 
-// The tuner's first-pass timing: the fused first pass (deferring form) of
-// f / fhat at each tile depth zcs[k] on scratch of its own; ms[k] is the best
-// of two timed launches after a warm-up.  The code bytes (independent of the
-// depth) go to the caller's buffer, completed by k_first_exact for the voxels
-// the last run deferred, so every byte is a valid pair of ranks.
+// The tuner's first-pass timing: the fused first pass of f / fhat at each
+// tile depth zcs[k] on scratch of its own; ms[k] is the best of two timed
+// launches after a warm-up.  The code bytes (independent of the depth) go to
+// the caller's buffer.
 template <typename T>
 int time_first_pass(const T *f, const T *fh, size_t nx, size_t ny, size_t nz, uint8_t *codes, const int *zcs, int m,
                     float *ms, cudaStream_t s) {
     Geom g = make_geom(nx, ny, nz);
-    const bool defer = g.n < (static_cast<size_t>(1) << 32);
     Workspace ws(s);
     const size_t o_hp = ws.reserve<uint32_t>(g.n), o_req = ws.reserve<uint32_t>(g.nwords),
                  o_act = ws.reserve<uint32_t>(g.nwords), o_slot = ws.reserve<SweepSlot>(1),
-                 o_x = ws.reserve<uint32_t>(defer ? g.n : 0), o_xc = ws.reserve<uint32_t>(2);
+                 o_err = ws.reserve<uint32_t>(1);
     int rc = ws.commit();
     if (rc) return rc;
-    const FirstMaps maps = defer ? first_maps<T>(f, fh, g) : FirstMaps{};
+    const FirstMaps maps = first_maps<T>(f, fh, g);
     uint32_t *hp = ws.at<uint32_t>(o_hp), *req = ws.at<uint32_t>(o_req), *act = ws.at<uint32_t>(o_act);
-    uint32_t *xl = ws.at<uint32_t>(o_x), *xc = ws.at<uint32_t>(o_xc), *err = xc + 1;
+    uint32_t *err = ws.at<uint32_t>(o_err);
     SweepSlot *slot = ws.at<SweepSlot>(o_slot);
     PMSZ_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), s));
     EventTimer et;
     if ((rc = et.init())) return rc;
-    const dim3 blk3(kTX, kTY, 1);
     for (int k = 0; k < m; ++k) {
-        g.zc = zcs[k];
+        g.zc = march_depth(zcs[k]);
         float best = 0.f;
         for (int rep = 0; rep < 3; ++rep) {  // the first run of each candidate is a warm-up
             PMSZ_CUDA(cudaMemsetAsync(req, 0, g.nwords * 4, s));
             PMSZ_CUDA(cudaMemsetAsync(act, 0, g.nwords * 4, s));
             PMSZ_CUDA(cudaMemsetAsync(slot, 0, sizeof(SweepSlot), s));
-            PMSZ_CUDA(cudaMemsetAsync(xc, 0, sizeof(uint32_t), s));
             PMSZ_CUDA(cudaEventRecord(et.ev[0], s));
-            if (defer)
-                launch_first_pass<T>(maps, tiled_grid(g), s, f, const_cast<T *>(fh), codes, hp, req, act, slot, g, 0, xl,
-                                     xc, err);
-            else
-                k_tiled<T, kFirst><<<tiled_grid(g), blk3, 0, s>>>(f, fh, codes, hp, req, act, slot, g, 0);
+            if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, const_cast<T *>(fh), codes, hp, req, act, slot, g, 0,
+                                 nullptr, err))) return rc;
             PMSZ_CUDA(cudaGetLastError());
             PMSZ_CUDA(cudaEventRecord(et.ev[1], s));
             PMSZ_CUDA(cudaEventSynchronize(et.ev[1]));
@@ -1004,17 +997,10 @@ int time_first_pass(const T *f, const T *fh, size_t nx, size_t ny, size_t nz, ui
         }
         ms[k] = best;
     }
-    if (defer) {
-        uint32_t herr = 0;
-        PMSZ_CUDA(cudaMemcpyAsync(&herr, err, sizeof(herr), cudaMemcpyDeviceToHost, s));
-        PMSZ_CUDA(cudaStreamSynchronize(s));
-        if (herr)
-            return set_error(PMSZ_ERR_CUDA, "first pass: a tile plane's tensor copy did not arrive within the bounded wait");
-    }
-    if (defer) {  // the deferred voxels' code bytes: codes is complete for the caller
-        k_first_exact<T><<<152 * 8, 256, 0, s>>>(xl, xc, f, fh, codes, req, act, slot, g, g.div_nx);
-        PMSZ_CUDA(cudaGetLastError());
-    }
+    uint32_t herr = 0;
+    PMSZ_CUDA(cudaMemcpyAsync(&herr, err, sizeof(herr), cudaMemcpyDeviceToHost, s));
+    PMSZ_CUDA(cudaStreamSynchronize(s));
+    if (herr) return set_error(PMSZ_ERR_CUDA, kCopyMissing);
     return ws.release();
 }
 

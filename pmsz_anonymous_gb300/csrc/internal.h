@@ -156,6 +156,8 @@ int labels_impl(const uint8_t *codes, size_t nx, size_t ny, size_t nz, uint32_t 
 // pointer-jumping rounds per launch recorded for a shape class, or the
 // defaults; tune_known says whether the class has an entry.
 int tuned_zchunk(size_t nx, size_t ny, size_t nz, size_t elem);
+// The depth the full-field passes run a field at: the tuned one, or by size.
+int first_depth(size_t nx, size_t ny, size_t nz, size_t elem);
 int tuned_jump_rounds(size_t nx, size_t ny, size_t nz);
 bool tune_known(size_t nx, size_t ny, size_t nz, size_t elem);
 // The batch tile depth of a batch's size class (voxels, field count, element

@@ -1,0 +1,720 @@
+// march.cuh -- full-field passes: the fused labelling + first detection, the
+// full detection sweeps and the direction codes, included by list.cuh after
+// tiled.cuh.
+//
+// One block of 32 x 4 threads owns a 32 x 8 column of the field (two voxels
+// per thread and plane, one above the other in y) and marches it through g.zc
+// planes.  What bounds these passes is instruction issue and the ALU pipe, not
+// HBM, so the design counts instructions per voxel:
+//
+//  * Tagged proxies.  A cell's 32-bit value in shared memory is the high 28
+//    bits of its key (proxy_of) and, in the low 4 bits, the tag
+//    (7x + y + 2z) mod 16 of its ABSOLUTE coordinates.  The 15 stencil points
+//    have 15 different tags around any voxel ((7dx + dy + 2dz) mod 16 takes
+//    every value but 8), so the packed maximum names the winning cell and no
+//    chain adds a rank to its candidates.
+//  * Certificates.  A second chain over the values with the tag bits flipped
+//    picks, among cells that share the 28 value bits, the lowest tag instead
+//    of the highest: both chains name the same cell exactly when the winner is
+//    unique.  Otherwise the voxel goes to the block's exact queue.
+//  * Plane blocks.  In one plane the stencil uses the 2x2 blocks
+//      U = {(x,y-1), (x+1,y-1), (x,y), (x+1,y)}
+//      V = {(x-1,y), (x,y), (x-1,y+1), (x,y+1)}
+//    and the whole stencil of a voxel of plane z is U(z-1), U(z), V(z) and
+//    V(z+1).  A thread reads the 10 cells that a plane contributes to its two
+//    voxels once, keeps U and G = U(z-1) + U(z) + V(z) in registers, and
+//    finishes a voxel when the next plane brings V.  The two voxels share the
+//    row pairs of their blocks, so a chain takes 8 min/max and 5 shared-memory
+//    loads per voxel instead of 14 (plus the rank adds) and 15.
+//  * Cells outside the domain are never read: a thread on an x or y face reads
+//    another cell of the same 2x2 block instead (the same value and tag twice
+//    changes no winner and no certificate), and a plane outside in z
+//    contributes the chains' identities.
+//  * Planes arrive in a ring of raw stages several planes ahead, by TMA or by
+//    cp.async, so no register holds a value in flight.
+//
+// Exact decisions.  A voxel whose certificate fails (ties in the truncated
+// proxies) is queued in shared memory and decided on full keys, gathered from
+// global memory (recently loaded, so mostly L2 hits), by the whole block: full
+// warps instead of one lane per warp, no second kernel and no global list.
+// The same holds for voxels whose two codes differ and that need the rules,
+// and for values that may be NaN or the sentinel.  The queues are emptied when
+// one could overflow in the next plane, and at the end.
+//
+#pragma once
+#include "tiled.cuh"
+
+namespace pmsz {
+
+enum MarchMode { kFirst = 0, kDetect = 1, kCodes = 2 };
+
+__host__ __device__ constexpr uint32_t stencil_tag(int x, int y, int z) {
+    return (7u * static_cast<uint32_t>(x) + static_cast<uint32_t>(y) + 2u * static_cast<uint32_t>(z)) & 15u;
+}
+// Stencil rank of a tag difference (winner - voxel) mod 16; difference 8 does
+// not occur.
+constexpr uint64_t tag_rank_table() {
+    uint64_t t = 0;
+    for (int r = 0; r < 15; ++r)
+        t |= static_cast<uint64_t>(r) << (4 * stencil_tag(rank_dx(r), rank_dy(r), rank_dz(r)));
+    return t;
+}
+constexpr bool tags_distinct() {
+    uint32_t seen = 0;
+    for (int r = 0; r < 15; ++r) {
+        const uint32_t b = 1u << stencil_tag(rank_dx(r), rank_dy(r), rank_dz(r));
+        if (seen & b) return false;
+        seen |= b;
+    }
+    return true;
+}
+static_assert(tags_distinct(), "the 15 stencil points must carry 15 different tags");
+
+__device__ __forceinline__ uint8_t tag_pair_code(uint32_t d) {  // two tag differences -> code byte
+    constexpr uint64_t t = tag_rank_table();
+    return static_cast<uint8_t>(((t >> (4 * (d & 15u))) & 15u) | (((t >> (4 * ((d >> 4) & 15u))) & 15u) << 4));
+}
+
+// Maximum and minimum of a set of tagged values.
+struct Ext2 {
+    uint32_t hi, lo;
+};
+__device__ __forceinline__ Ext2 ext2(uint32_t a, uint32_t b) { return Ext2{max(a, b), min(a, b)}; }
+__device__ __forceinline__ Ext2 join(const Ext2 &a, const Ext2 &b) { return Ext2{max(a.hi, b.hi), min(a.lo, b.lo)}; }
+__device__ __forceinline__ Ext2 join(const Ext2 &a, const Ext2 &b, const Ext2 &c) {
+    return Ext2{__vimax3_u32(a.hi, b.hi, c.hi), __vimin3_u32(a.lo, b.lo, c.lo)};
+}
+__device__ __forceinline__ Ext2 join(uint32_t a, uint32_t b, const Ext2 &c) {
+    return Ext2{__vimax3_u32(a, b, c.hi), __vimin3_u32(a, b, c.lo)};
+}
+__device__ __forceinline__ Ext2 ext2_identity() { return Ext2{0u, 0xFFFFFFFFu}; }
+
+// Steepest ranks of one voxel on the full keys of v, gathered from global
+// memory five at a time (arg_ext's rule: ties by rank).
+template <typename T>
+__device__ __forceinline__ void exact_ranks(const T *__restrict__ v, size_t i, const Geom &g, uint32_t valid,
+                                            int &asc, int &desc) {
+    using K = typename KeyOf<T>::type;
+    const ptrdiff_t sy = g.nx, sz = static_cast<ptrdiff_t>(g.nx) * g.ny;
+    K bmax = 0, bmin = ~K(0);
+    asc = desc = kSelf;
+#pragma unroll
+    for (int r0 = 0; r0 < 15; r0 += 5) {
+        K k[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            const int r = r0 + j;
+            const ptrdiff_t off = rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz;
+            k[j] = ((valid >> r) & 1u) ? okey(__ldg(v + (static_cast<ptrdiff_t>(i) + off))) : K(0);
+        }
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            const int r = r0 + j;
+            if ((valid >> r) & 1u) {
+                if (k[j] >= bmax) { bmax = k[j]; asc = r; }
+                if (k[j] < bmin) { bmin = k[j]; desc = r; }
+            }
+        }
+    }
+}
+
+// What a march reads and writes.  kFirst: f and fhat in, codes, the proxies
+// hp, requests and mismatch bits out.  kDetect: the proxies hp (fhat for the
+// exact decisions) and the codes in; act_cur (or null: every voxel) is the
+// active set, consumed.  kCodes: f in, codes out.
+template <typename T>
+struct MarchArgs {
+    const T *f, *fh;
+    uint8_t *codes;
+    uint32_t *hp, *req, *act_cur, *act_next;
+    SweepSlot *slot;
+    uint32_t *xcount;  // += voxels decided on full keys (kFirst; may be null)
+};
+
+constexpr int kMHY = kMY + 2;        // rows of a tile, and with the halo
+constexpr int kMCells = kHX * kMHY;            // cells of a tile's plane
+constexpr int kPerThread = (kMCells + kThreads - 1) / kThreads;
+constexpr int kRawStages = 3;                  // planes in flight
+constexpr int kMarchRing = 4;                  // planes of proxies: k-2, k-1 (state), k and k+1
+static_assert(kMarchMaxDepth <= 128 && kMY <= 16, "queue entries hold 7 bits of depth and 4 of the row");
+constexpr uint32_t kQueueFlush = 512;          // a queue longer than this is emptied after the plane
+constexpr uint32_t kQueueCap = kQueueFlush + 2 * kThreads;
+
+// Queue entries: tx | row << 5 | (z - zb) << 9 | b << 16 | c << 24 with c the
+// code byte of the original.  Rules: b = the current field's tag differences.
+// Exact: b = 1 if c is known.
+template <typename T, int NF>
+struct MarchSmem {
+    uint32_t p[kMarchRing][NF][kMCells];  // tagged proxies
+    uint32_t xq[kQueueCap], rq[kQueueCap];
+    uint32_t qn;                           // queue lengths: rules, exact << 16
+    uint32_t cnt[3];                       // fmax, fmin, fdir
+    uint32_t active, bad, deferred;
+    uint8_t lut[256];                      // tag differences of the steepest pair -> code byte
+    MarchArgs<T> a;                        // for march_queues
+    Geom g;
+    int x0, y0, zb;
+};
+template <typename T, int MODE>
+using MarchSmemOf = MarchSmem<T, MODE == kFirst ? 2 : 1>;
+
+// Decides the queued voxels of the block (every thread calls it, behind a
+// barrier).  Not inlined: its registers stay out of the plane loop, whose
+// state lives across the rare calls from inside it.
+template <typename T, int MODE>
+__device__ __noinline__ void march_queues(MarchSmemOf<T, MODE> &sm) {
+    const int tid = threadIdx.y * kTX + threadIdx.x;
+    const MarchArgs<T> &a = sm.a;
+    const Geom &g = sm.g;
+    const int x0 = sm.x0, y0 = sm.y0, zb = sm.zb;
+    uint32_t cmax = 0, cmin = 0, cdir = 0;
+    auto outcome = [&](int x, int y, int z, uint32_t asc, uint32_t desc, uint32_t c) {
+        const uint32_t tm = detect_rules(static_cast<int>(asc), static_cast<int>(desc), static_cast<int>(c & 15u),
+                                         static_cast<int>(c >> 4), cmax, cmin, cdir);
+        if (tm) {
+            request_targets(a.req, g, x, y, z, tm);
+            atomicOr(a.act_next + word_of(g, x, y, z), 1u << (x & 31));
+        }
+    };
+    const uint32_t nx = sm.qn >> 16, nr = sm.qn & 0xFFFFu;
+    for (uint32_t j = tid; j < nx; j += kThreads) {
+        const uint32_t e = sm.xq[j];
+        const int x = x0 + static_cast<int>(e & 31u), y = y0 + static_cast<int>((e >> 5) & 15u),
+                  z = zb + static_cast<int>((e >> 9) & 127u);
+        const size_t i = flat(g, x, y, z);
+        const uint32_t valid = valid_mask(x, y, z, g.nx, g.ny, g.nz);
+        uint32_t c = e >> 24;
+        int asc, desc;
+        if (MODE == kFirst && (bad_value(__ldg(a.f + i)) || bad_value(__ldg(a.fh + i)))) atomicAdd(&sm.bad, 1u);
+        if (MODE == kCodes || (MODE == kFirst && !((e >> 16) & 1u))) {
+            exact_ranks(a.f, i, g, valid, asc, desc);
+            c = static_cast<uint32_t>(asc | (desc << 4));
+            a.codes[i] = static_cast<uint8_t>(c);
+        }
+        if (MODE != kCodes) {
+            exact_ranks(a.fh, i, g, valid, asc, desc);
+            outcome(x, y, z, static_cast<uint32_t>(asc), static_cast<uint32_t>(desc), c);
+        }
+    }
+    if (MODE == kCodes) return;
+    for (uint32_t j = tid; j < nr; j += kThreads) {
+        const uint32_t e = sm.rq[j];
+        const uint32_t now = sm.lut[(e >> 16) & 0xFFu];
+        outcome(x0 + static_cast<int>(e & 31u), y0 + static_cast<int>((e >> 5) & 15u),
+                zb + static_cast<int>((e >> 9) & 127u), now & 15u, now >> 4, e >> 24);
+    }
+    const uint32_t v[3] = {cmax, cmin, cdir};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const uint32_t t = warp_sum_u32(v[c]);
+        if (threadIdx.x == 0 && t) atomicAdd(&sm.cnt[c], t);
+    }
+    if (tid == 0) sm.deferred += nx;
+}
+
+__device__ __forceinline__ uint32_t march_proxy(double v) { return proxy_of(v); }
+__device__ __forceinline__ uint32_t march_proxy(float v) { return proxy_of(v); }
+__device__ __forceinline__ uint32_t march_proxy(uint32_t p) { return p; }  // a stored proxy
+// Proxies outside [lo, hi) may belong to a NaN or to the sentinel 1e30 (fp64).
+template <typename T> struct PlainRange;
+template <> struct PlainRange<double> {
+    static constexpr uint32_t lo = 0x00100000u, hi = (0x80000000u + 0x46293E59u) & ~15u;  // 1e30 = 0x46293E59...
+};
+template <> struct PlainRange<float> {
+    static constexpr uint32_t lo = 0x00800000u, hi = 0xFF800000u;
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// FACE: a block on a domain face, or one whose tile crosses the domain's far
+// end; the other blocks' tile, halo and planes zb-1 .. ze lie inside.
+template <typename T, int MODE, bool FACE, class SRC>
+__device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, const MarchArgs<T> &a,
+                                           const Geom &g, int bx, int by, int bz) {
+    constexpr int NF = MODE == kFirst ? 2 : 1;
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTX + tx;
+    const int x0 = bx * kTX, y0 = by * kMY, zb = bz * g.zc;
+    const int ze = FACE ? min(g.nz, zb + g.zc) : zb + g.zc;
+    const int x = x0 + tx, y = y0 + 2 * ty;
+    const bool vin0 = !FACE || (x < g.nx && y < g.ny), vin1 = !FACE || (x < g.nx && y + 1 < g.ny);
+    const size_t plane = static_cast<size_t>(g.nx) * g.ny;
+    const int nplanes = ze - zb + 2;  // zb-1 .. ze
+
+    // tags of this thread's cells (tid + 256 j of the 34 x 18 halo tile) in
+    // plane zb-1, 4 bits each
+    uint32_t ctags = 0;
+#pragma unroll
+    for (int j = 0; j < kPerThread; ++j) {
+        const int c = tid + j * kThreads;
+        const int cy = c / kHX, cx = c - cy * kHX;
+        ctags |= stencil_tag(x0 - 1 + cx, y0 - 1 + cy, zb - 1) << (8 * j);
+    }
+    auto plane_in = [&](int k) { return !FACE || (zb - 1 + k >= 0 && zb - 1 + k < g.nz); };
+    auto convert = [&](int k) {
+        src.wait(k);
+        if (!plane_in(k)) return;
+        uint32_t *dst = &sm.p[k % kMarchRing][0][tid];
+        const uint32_t tags = ctags + 0x020202u * (static_cast<uint32_t>(k) & 7u);
+#pragma unroll
+        for (int j = 0; j < kPerThread; ++j) {
+            if (j == kPerThread - 1 && tid + j * kThreads >= kMCells) break;
+            const uint32_t tag = (tags >> (8 * j)) & 15u;
+#pragma unroll
+            for (int F = 0; F < NF; ++F) dst[F * kMCells + j * kThreads] = march_proxy(src.cell(k, j, F)) | tag;
+        }
+    };
+    // The cells a plane contributes, from the centre cell of the lower voxel.
+    // On a face the step outside the domain is left out, which reads another
+    // cell of the same block a second time.
+    const int ctr = (2 * ty + 1) * kHX + tx + 1;
+    const int xm = FACE && x == 0 ? 0 : -1, xp = FACE && x + 1 >= g.nx ? 0 : 1;
+    const int ra = FACE && y == 0 ? 0 : -kHX, rc = FACE && y + 1 >= g.ny ? 0 : kHX,
+              rd = FACE && y + 2 >= g.ny ? rc : 2 * kHX;
+    // the blocks U and V of the two voxels in a plane, on the values with
+    // their tags flipped by `flip`
+    struct Blocks {
+        Ext2 u0, u1, v0, v1;
+    };
+    auto blocks = [&](const uint32_t *t, uint32_t flip) {
+        const uint32_t a0 = t[ra] ^ flip, a1 = t[ra + xp] ^ flip;
+        const uint32_t bm = t[xm] ^ flip, b0 = t[0] ^ flip, b1 = t[xp] ^ flip;
+        const uint32_t cm = t[rc + xm] ^ flip, c0 = t[rc] ^ flip, c1 = t[rc + xp] ^ flip;
+        const uint32_t dm = t[rd + xm] ^ flip, d0 = t[rd] ^ flip;
+        const Ext2 p1 = ext2(b0, b1), q1 = ext2(cm, c0);
+        return Blocks{join(a0, a1, p1), join(c0, c1, p1), join(bm, b0, q1), join(dm, d0, q1)};
+    };
+
+    if (tid == 0) {
+        sm.qn = 0;
+        sm.cnt[0] = sm.cnt[1] = sm.cnt[2] = 0;
+        sm.active = sm.bad = sm.deferred = 0;
+        sm.a = a;
+        sm.g = g;
+        sm.x0 = x0;
+        sm.y0 = y0;
+        sm.zb = zb;
+    }
+    for (int e = tid; e < 256; e += kThreads) sm.lut[e] = tag_pair_code(static_cast<uint32_t>(e));
+#pragma unroll 1
+    for (int k = 0; k < 3; ++k) {  // at least 3 planes
+        convert(k);
+        if (k == 0) src.prefetch(kRawStages);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < 3; ++k) src.release(k);
+    uint32_t active = 0;
+    size_t i = static_cast<size_t>(x) + static_cast<size_t>(y) * g.nx + static_cast<size_t>(zb) * plane;
+    const uint32_t stag0 = stencil_tag(x, y, zb - 2);
+    int k = 2;  // the next plane; it completes the voxels of plane k-1, z = zb + k - 2
+#pragma unroll 1
+    while (true) {
+        // the state before plane k, from the planes still in the ring (also
+        // after the queues were emptied, so that nothing lives across that
+        // call): [field][tags plain / flipped][voxel]
+        Ext2 G[NF][2][2], U[NF][2][2];
+#pragma unroll
+        for (int F = 0; F < NF; ++F)
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const Blocks w = blocks(&sm.p[(k - 1) % kMarchRing][F][ctr], p ? 15u : 0u);
+                U[F][p][0] = w.u0;
+                U[F][p][1] = w.u1;
+                G[F][p][0] = join(w.u0, w.v0);
+                G[F][p][1] = join(w.u1, w.v1);
+                if (plane_in(k - 2)) {
+                    const Blocks o = blocks(&sm.p[(k - 2) % kMarchRing][F][ctr], p ? 15u : 0u);
+                    G[F][p][0] = join(G[F][p][0], o.u0);
+                    G[F][p][1] = join(G[F][p][1], o.u1);
+                }
+            }
+        bool over = false;
+#pragma unroll 1
+        while (!over && k < nplanes) {
+            src.prefetch(k + kRawStages - 1);
+            const int zrel = k - 2;
+            uint32_t word[2] = {0xFFFFFFFFu, 0xFFFFFFFFu}, was[2] = {0u, 0u};
+            if (MODE == kDetect) {
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    if (a.act_cur) word[r] = (!FACE || y + r < g.ny) ? a.act_cur[word_of(g, x0, y + r, zb + zrel)] : 0u;
+                    if ((r ? vin1 : vin0) && word[r]) was[r] = a.codes[i + (r ? g.nx : 0)];
+                }
+            }
+            Ext2 S[NF][2][2];
+            if (plane_in(k)) {
+#pragma unroll
+                for (int F = 0; F < NF; ++F) {
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) {
+                        const Blocks w = blocks(&sm.p[k % kMarchRing][F][ctr], p ? 15u : 0u);
+                        S[F][p][0] = join(G[F][p][0], w.v0);
+                        S[F][p][1] = join(G[F][p][1], w.v1);
+                        G[F][p][0] = join(U[F][p][0], w.u0, w.v0);
+                        G[F][p][1] = join(U[F][p][1], w.u1, w.v1);
+                        U[F][p][0] = w.u0;
+                        U[F][p][1] = w.u1;
+                    }
+                }
+            } else {  // the plane beyond the domain, the last one
+#pragma unroll
+                for (int F = 0; F < NF; ++F)
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) {
+                        S[F][p][0] = G[F][p][0];
+                        S[F][p][1] = G[F][p][1];
+                    }
+            }
+            const uint32_t stag = stag0 + 2u * static_cast<uint32_t>(k);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const bool vin = r ? vin1 : vin0;
+                const size_t ir = i + (r ? static_cast<size_t>(g.nx) : 0);
+                if (MODE == kFirst && vin)  // fhat's proxies
+                    a.hp[ir] = sm.p[(k - 1) % kMarchRing][NF - 1][ctr + (r ? (FACE ? rc : kHX) : 0)] & ~15u;
+                const uint32_t cert0 = (S[0][0][r].hi ^ S[0][1][r].hi) & (S[0][0][r].lo ^ S[0][1][r].lo);
+                uint32_t cert = cert0;
+                if (NF == 2)
+                    cert &= (S[NF - 1][0][r].hi ^ S[NF - 1][1][r].hi) & (S[NF - 1][0][r].lo ^ S[NF - 1][1][r].lo);
+                const bool ok0 = (cert0 & 15u) == 15u;
+                bool ok = (cert & 15u) == 15u;
+                if (MODE == kFirst)
+                    ok = ok && max(S[0][0][r].hi, S[NF - 1][0][r].hi) < PlainRange<T>::hi &&
+                         min(S[0][0][r].lo, S[NF - 1][0][r].lo) >= PlainRange<T>::lo;
+                const uint32_t st = stag + static_cast<uint32_t>(r);
+                const uint32_t c0 = sm.lut[((S[0][0][r].hi - st) & 15u) | (((S[0][0][r].lo - st) & 15u) << 4)];
+                bool rule = false, ex = vin && !ok;
+                uint32_t c = c0;
+                if (MODE == kCodes) {
+                    if (vin && ok) a.codes[ir] = static_cast<uint8_t>(c0);
+                } else if (MODE == kFirst) {
+                    if (vin && ok0) a.codes[ir] = static_cast<uint8_t>(c0);
+                    // equal codes fire no rule unless the voxel is both maximum
+                    // and minimum of f, which a certified voxel is only without
+                    // neighbours (a field of one voxel)
+                    rule = vin && ok &&
+                           ((((S[0][0][r].hi ^ S[NF - 1][0][r].hi) | (S[0][0][r].lo ^ S[NF - 1][0][r].lo)) & 15u) != 0u ||
+                            (FACE && c0 == 0x77u));
+                } else {
+                    const bool on = vin && ((word[r] >> tx) & 1u);
+                    active += on ? 1u : 0u;
+                    c = was[r];
+                    ex = ex && on;
+                    rule = on && ok && (c0 != c || (FACE && c == 0x77u));
+                    if (a.act_cur && word[r] && tx == 0) a.act_cur[word_of(g, x0, y + r, zb + zrel)] = 0;
+                }
+                const uint32_t wq = __ballot_sync(0xFFFFFFFFu, rule || ex);
+                if (wq) {
+                    const uint32_t wx = __ballot_sync(0xFFFFFFFFu, ex), wr = wq & ~wx;
+                    const uint32_t lower = (1u << tx) - 1u;
+                    uint32_t base = 0;
+                    const uint32_t add = static_cast<uint32_t>(__popc(wr)) | (static_cast<uint32_t>(__popc(wx)) << 16);
+                    if (tx == 0) base = atomicAdd(&sm.qn, add);
+                    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                    const uint32_t here = static_cast<uint32_t>(tx) | (static_cast<uint32_t>(2 * ty + r) << 5) |
+                                          (static_cast<uint32_t>(zrel) << 9) | (c << 24);
+                    if (ex) {
+                        sm.xq[(base >> 16) + static_cast<uint32_t>(__popc(wx & lower))] =
+                            here | ((ok0 ? 1u : 0u) << 16);
+                    } else if (rule) {
+                        const uint32_t now = ((S[NF - 1][0][r].hi - st) & 15u) | (((S[NF - 1][0][r].lo - st) & 15u) << 4);
+                        sm.rq[(base & 0xFFFFu) + static_cast<uint32_t>(__popc(wr & lower))] = here | (now << 16);
+                    }
+                    const uint32_t end = base + add;
+                    over |= (end & 0xFFFFu) > kQueueFlush || (end >> 16) > kQueueFlush;
+                }
+            }
+            i += plane;
+            if (k + 1 < nplanes) convert(k + 1);
+            // the barrier that ends the plane also tells whether a queue could
+            // overflow in the next one (every appending warp knows its end)
+            over = __syncthreads_or(over) != 0;
+            src.release(k + 1);
+            ++k;
+        }
+        march_queues<T, MODE>(sm);
+        if (k >= nplanes) break;
+        __syncthreads();
+        if (tid == 0) sm.qn = 0;
+        __syncthreads();
+    }
+    if (MODE == kCodes) return;
+    if (MODE == kFirst) active = static_cast<uint32_t>(ze - zb) * ((vin0 ? 1u : 0u) + (vin1 ? 1u : 0u));
+    active = warp_sum_u32(active);
+    if (tx == 0 && active) atomicAdd(&sm.active, active);
+    __syncthreads();
+    // one atomic per non-zero counter and block
+    if (tid < 3 && sm.cnt[tid]) atomicAdd(reinterpret_cast<unsigned long long *>(a.slot) + tid, static_cast<unsigned long long>(sm.cnt[tid]));
+    if (tid == 3 && sm.active) atomicAdd(&a.slot->active, static_cast<unsigned long long>(sm.active));
+    if (tid == 4 && sm.bad) atomicAdd(&a.slot->bad, static_cast<unsigned long long>(sm.bad));
+    if (tid == 5 && a.xcount && sm.deferred) atomicAdd(a.xcount, sm.deferred);
+}
+
+__device__ __forceinline__ bool march_inside(const Geom &g, int bx, int by, int bz) {
+    const int x0 = bx * kTX, y0 = by * kMY, zb = bz * g.zc;
+    return x0 >= 1 && x0 + kTX + 1 <= g.nx && y0 >= 1 && y0 + kMY + 1 <= g.ny && zb >= 1 && zb + g.zc + 1 <= g.nz;
+}
+
+// ---------------------------------------------------------------------------
+// Plane sources.  cell(k, j, F): this thread's cell tid + 256 j of the halo
+// tile, of field F, in plane zb-1+k.
+//
+// CopySource: cp.async of single elements, any alignment and row length; every
+// thread copies and later converts its own cells, so a plane needs no barrier
+// between its arrival and its conversion.  prefetch(k) starts plane k into the
+// stage of plane k - kRawStages, whose conversion ended two planes ago.
+// ---------------------------------------------------------------------------
+template <typename R, int NF>
+struct CopyTile {
+    R raw[kRawStages][NF][kMCells];
+};
+
+template <typename R, int NF, bool FACE>
+struct CopySource {
+    CopyTile<R, NF> *ct;
+    const R *v0, *v1;
+    size_t plane;
+    size_t off[kPerThread];  // of this thread's cells in their plane
+    uint32_t in;             // bit j: cell j lies inside the domain
+    int zb, nz, nplanes;
+    __device__ __forceinline__ CopySource(CopyTile<R, NF> &t, const R *f0, const R *f1, const Geom &g, int bx, int by,
+                                          int bz)
+        : ct(&t), v0(f0), v1(f1), plane(static_cast<size_t>(g.nx) * g.ny), in(0), zb(bz * g.zc), nz(g.nz),
+          nplanes((FACE ? min(g.nz, bz * g.zc + g.zc) - bz * g.zc : g.zc) + 2) {
+        const int tid = threadIdx.y * kTX + threadIdx.x;
+#pragma unroll
+        for (int j = 0; j < kPerThread; ++j) {
+            const int c = tid + j * kThreads;
+            const int cy = c / kHX, cx = c - cy * kHX;
+            const int gx = bx * kTX - 1 + cx, gy = by * kMY - 1 + cy;
+            const bool ok = c < kMCells && (!FACE || (gx >= 0 && gx < g.nx && gy >= 0 && gy < g.ny));
+            if (ok) in |= 1u << j;
+            off[j] = ok ? static_cast<size_t>(gx) + static_cast<size_t>(gy) * g.nx : 0;
+        }
+#pragma unroll 1
+        for (int k = 0; k < kRawStages; ++k) prefetch(k);
+    }
+    __device__ __forceinline__ void prefetch(int k) {
+        if (k < nplanes && (!FACE || (zb - 1 + k >= 0 && zb - 1 + k < nz))) {
+            const size_t zo = static_cast<size_t>(zb - 1 + k) * plane;
+            const int s = k % kRawStages;
+            const int tid = threadIdx.y * kTX + threadIdx.x;
+#pragma unroll
+            for (int j = 0; j < kPerThread; ++j)
+                if ((in >> j) & 1u)
+#pragma unroll
+                    for (int F = 0; F < NF; ++F)
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                                         smem_u32(&ct->raw[s][F][tid + j * kThreads])),
+                                     "l"((F == 0 ? v0 : v1) + zo + off[j]), "n"(static_cast<int>(sizeof(R)))
+                                     : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");  // one group per plane, also when empty
+    }
+    // plane k has arrived: when it is converted, planes up to k + 2 have been started
+    __device__ __forceinline__ void wait(int) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRawStages - 2) : "memory");
+    }
+    __device__ __forceinline__ R cell(int k, int j, int F) const {
+        return ct->raw[k % kRawStages][F][threadIdx.y * kTX + threadIdx.x + j * kThreads];
+    }
+    __device__ __forceinline__ void release(int) {}
+};
+
+// The element type a march streams: the field itself, or the stored proxies.
+template <typename T, int MODE> struct MarchRaw { using type = T; };
+template <typename T> struct MarchRaw<T, kDetect> { using type = uint32_t; };
+
+template <typename T, int MODE>
+struct CopyMarch {  // shared memory of a copy-fed march
+    CopyTile<typename MarchRaw<T, MODE>::type, MODE == kFirst ? 2 : 1> raw;
+    MarchSmemOf<T, MODE> m;
+};
+
+template <typename T, int MODE, bool FACE>
+__device__ __forceinline__ void march_copies(CopyMarch<T, MODE> &sm, const MarchArgs<T> &a, const Geom &g, int bx,
+                                             int by, int bz) {
+    using R = typename MarchRaw<T, MODE>::type;
+    const R *v0, *v1 = nullptr;
+    if constexpr (MODE == kDetect) {
+        v0 = a.hp;
+    } else {
+        v0 = a.f;
+        v1 = a.fh;
+    }
+    CopySource<R, MODE == kFirst ? 2 : 1, FACE> s(sm.raw, v0, v1, g, bx, by, bz);
+    march_body<T, MODE, FACE>(sm.m, s, a, g, bx, by, bz);
+}
+
+// bz0: index of the first z-chunk the launch covers (a launch may cover a
+// z-range of chunks, e.g. the part of the field already copied in).
+template <typename T, int MODE>
+__global__ void __launch_bounds__(kThreads, 5) k_march(const __grid_constant__ MarchArgs<T> a,
+                                                       const __grid_constant__ Geom g, int bz0) {
+    extern __shared__ __align__(128) unsigned char march_smem[];
+    CopyMarch<T, MODE> &sm = *reinterpret_cast<CopyMarch<T, MODE> *>(march_smem);
+    const int bx = static_cast<int>(blockIdx.x), by = static_cast<int>(blockIdx.y),
+              bz = bz0 + static_cast<int>(blockIdx.z);
+    if (march_inside(g, bx, by, bz))
+        march_copies<T, MODE, false>(sm, a, g, bx, by, bz);
+    else
+        march_copies<T, MODE, true>(sm, a, g, bx, by, bz);
+}
+
+// ---------------------------------------------------------------------------
+// TmaSource (first pass): one thread issues, per plane, a
+// cp.async.bulk.tensor box of f and one of fhat (the tile with its one-voxel
+// halo, widened in x so that the box starts on a 16-byte boundary) into the
+// stage, guarded by an mbarrier that the copy engine completes with the box's
+// byte count; a stage is refilled with the plane kRawStages ahead after the
+// barrier that ends its conversion.  No thread computes a global address or
+// predicates a load for the tile.  Planes outside the domain are not copied:
+// their stage's barrier gets a plain arrive.
+//
+// Every mbarrier wait is bounded: a plane that does not arrive within the
+// limit sets *err (the host reports PMSZ_ERR_CUDA), and the block still waits,
+// again bounded, on every plane it issued before it exits.
+// ---------------------------------------------------------------------------
+template <typename T> struct RawBox;
+template <> struct RawBox<double> { static constexpr int kX = 36, kOff = 1; };  // x0-2 .. x0+33
+template <> struct RawBox<float> { static constexpr int kX = 40, kOff = 3; };   // x0-4 .. x0+35
+template <typename T>
+constexpr int kRawBytes = RawBox<T>::kX * kMHY * static_cast<int>(sizeof(T));  // one box of one field
+template <typename T>
+constexpr int kRawPitch = (kRawBytes<T> + 127) / 128 * 128;  // stages start on 128-byte boundaries
+
+template <typename T>
+struct __align__(128) TmaMarch {
+    // first: the copy engine writes the stages, which must start on 128-byte
+    // boundaries (the struct is 128-byte aligned, kRawPitch a multiple of 128)
+    alignas(128) unsigned char raw[kRawStages][2][kRawPitch<T>];  // boxes of f and fhat, rows of RawBox<T>::kX
+    MarchSmem<T, 2> m;
+    unsigned long long mbar[kRawStages];
+};
+static_assert(offsetof(TmaMarch<float>, raw) == 0 && offsetof(TmaMarch<double>, raw) == 0 &&
+                  kRawPitch<float> % 128 == 0 && kRawPitch<double> % 128 == 0,
+              "TMA stages must start on 128-byte boundaries");
+
+constexpr int kMbarTries = 1 << 22;  // try_wait suspends between tries: a bound of seconds, not a spin count
+
+__device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
+    for (int it = 0; it < kMbarTries; ++it) {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t mbar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 :: "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(mbar) : "memory");
+}
+
+template <typename T, bool FACE>
+struct TmaSource {
+    TmaMarch<T> *sm;
+    const CUtensorMap *tf, *tfh;
+    int x0, y0, zb, nz, nplanes;
+    int r[kPerThread];  // this thread's cells in a box
+    uint32_t failed;
+    __device__ __forceinline__ void issue(int k) {  // plane zb-1+k into stage k % kRawStages (one thread)
+        const int s = k % kRawStages;
+        const uint32_t mb = smem_u32(&sm->mbar[s]);
+        if (FACE && (zb - 1 + k < 0 || zb - 1 + k >= nz)) {  // nothing to copy: complete the phase
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(mb) : "memory");
+            return;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the stage's reads come first
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(mb), "r"(2 * kRawBytes<T>)
+                     : "memory");
+        tma_load_3d(smem_u32(sm->raw[s][0]), tf, x0 - RawBox<T>::kOff - 1, y0 - 1, zb - 1 + k, mb);
+        tma_load_3d(smem_u32(sm->raw[s][1]), tfh, x0 - RawBox<T>::kOff - 1, y0 - 1, zb - 1 + k, mb);
+    }
+    __device__ __forceinline__ void prefetch(int) {}
+    __device__ __forceinline__ void wait(int k) {
+        if (!mbar_wait(smem_u32(&sm->mbar[k % kRawStages]), static_cast<uint32_t>((k / kRawStages) & 1))) failed = 1;
+    }
+    __device__ __forceinline__ T cell(int k, int j, int F) const {
+        return reinterpret_cast<const T *>(sm->raw[k % kRawStages][F])[r[j]];
+    }
+    __device__ __forceinline__ void release(int k) {  // plane k is converted: its stage takes plane k + kRawStages
+        if (threadIdx.x == 0 && threadIdx.y == 0 && k + kRawStages < nplanes) issue(k + kRawStages);
+    }
+};
+
+template <typename T, bool FACE>
+__device__ __forceinline__ void first_tma_body(TmaMarch<T> &sm, const CUtensorMap *tf, const CUtensorMap *tfh,
+                                               const MarchArgs<T> &a, const Geom &g, int bx, int by, int bz,
+                                               uint32_t *err) {
+    TmaSource<T, FACE> s;
+    s.sm = &sm;
+    s.tf = tf;
+    s.tfh = tfh;
+    s.x0 = bx * kTX;
+    s.y0 = by * kMY;
+    s.zb = bz * g.zc;
+    s.nz = g.nz;
+    s.nplanes = (FACE ? min(g.nz, s.zb + g.zc) - s.zb : g.zc) + 2;
+    s.failed = 0;
+    const int tid = threadIdx.y * kTX + threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < kPerThread; ++j) {
+        const int c = min(tid + j * kThreads, kMCells - 1);
+        const int cy = c / kHX, cx = c - cy * kHX;
+        s.r[j] = cy * RawBox<T>::kX + cx + RawBox<T>::kOff;
+    }
+    if (tid == 0) {
+        for (int k = 0; k < kRawStages; ++k)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&sm.mbar[k])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (tid == 0)
+        for (int k = 0; k < kRawStages && k < s.nplanes; ++k) s.issue(k);
+    march_body<T, kFirst, FACE>(sm.m, s, a, g, bx, by, bz);
+    if (s.failed) atomicOr(err, 1u);
+}
+
+// tf / tfh map f / fhat as (nx, ny, nz) with a box of RawBox<T>::kX x kMHY x 1
+// (the caller takes k_march where no map can be made: rows whose byte length
+// is not a multiple of 16, or base pointers off a 16-byte boundary).
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 6) k_first_tma(const __grid_constant__ CUtensorMap tf,
+                                                           const __grid_constant__ CUtensorMap tfh,
+                                                           const __grid_constant__ MarchArgs<T> a,
+                                                           const __grid_constant__ Geom g, int bz0, uint32_t *err) {
+    extern __shared__ __align__(128) unsigned char march_smem[];
+    TmaMarch<T> &sm = *reinterpret_cast<TmaMarch<T> *>(march_smem);
+    const int bx = static_cast<int>(blockIdx.x), by = static_cast<int>(blockIdx.y),
+              bz = bz0 + static_cast<int>(blockIdx.z);
+    if (march_inside(g, bx, by, bz))
+        first_tma_body<T, false>(sm, &tf, &tfh, a, g, bx, by, bz, err);
+    else
+        first_tma_body<T, true>(sm, &tf, &tfh, a, g, bx, by, bz, err);
+}
+
+inline dim3 tiled_grid(const Geom &g) {
+    return dim3(static_cast<unsigned>(g.wpr), static_cast<unsigned>((g.ny + kMY - 1) / kMY),
+                static_cast<unsigned>((g.nz + g.zc - 1) / g.zc));
+}
+
+// A kernel above the 48 KB of static shared memory has to be allowed its size
+// on the current device before it is launched.
+template <class K>
+inline cudaError_t allow_smem(K kernel, size_t bytes) {
+    return cudaFuncSetAttribute(reinterpret_cast<const void *>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(bytes));
+}
+template <typename T, int MODE>
+inline cudaError_t launch_march(dim3 grid, cudaStream_t s, const MarchArgs<T> &a, const Geom &g, int bz0) {
+    const cudaError_t e = allow_smem(k_march<T, MODE>, sizeof(CopyMarch<T, MODE>));
+    if (e != cudaSuccess) return e;
+    k_march<T, MODE><<<grid, dim3(kTX, kThreads / kTX, 1), sizeof(CopyMarch<T, MODE>), s>>>(a, g, bz0);
+    return cudaGetLastError();
+}
+
+}  // namespace pmsz

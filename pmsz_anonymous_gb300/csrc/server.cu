@@ -77,7 +77,7 @@ static Inst<T> make_inst(Job &j, int q, int64_t max_sweeps) {
     I.active = 1;
     I.first = j.first ? 1 : 0;
     I.tiles_x = static_cast<uint32_t>(g.wpr);
-    I.tiles_y = static_cast<uint32_t>((g.ny + kTY - 1) / kTY);
+    I.tiles_y = static_cast<uint32_t>((g.ny + kMY - 1) / kMY);
     return I;
 }
 
@@ -121,7 +121,7 @@ public:
         auto j = std::make_unique<Job>();
         j->fd = fd;
         j->g = make_geom(fd.nx, fd.ny, fd.nz);
-        j->g.zc = tuned_zchunk(fd.nx, fd.ny, fd.nz, fd.elem_size);
+        j->g.zc = first_depth(fd.nx, fd.ny, fd.nz, fd.elem_size);
         j->scratch_bytes = field_scratch_bytes(j->g, cfg_.max_sweeps);
         // its fields, its scratch, and its share of the group's voxel lists
         j->bytes = j->scratch_bytes + 2 * j->g.n * fd.elem_size + 2 * sizeof(uint64_t) * j->g.n;

@@ -75,6 +75,11 @@ int tuned_zchunk(size_t nx, size_t ny, size_t nz, size_t elem) {
     return it == t.zc.end() ? kZChunkDefault : it->second;
 }
 
+int first_depth(size_t nx, size_t ny, size_t nz, size_t elem) {
+    return tune_known(nx, ny, nz, elem) ? march_depth(tuned_zchunk(nx, ny, nz, elem))
+                                        : default_depth(column_planes(nx, ny, nz));
+}
+
 int tuned_jump_rounds(size_t nx, size_t ny, size_t nz) {
     Table &t = table();
     std::lock_guard<std::mutex> lk(t.mu);
