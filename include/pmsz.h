@@ -291,6 +291,9 @@ int pmsz_rank_offset(int r, int *dx, int *dy, int *dz);
  */
 int pmsz_labels(const uint8_t *codes, size_t nx, size_t ny, size_t nz,
                 uint32_t *as_label, uint32_t *ds_label, void *stream);
+/* The same with 64-bit labels (device arrays of n int64). */
+int pmsz_labels_i64(const uint8_t *codes, size_t nx, size_t ny, size_t nz,
+                    int64_t *as_label, int64_t *ds_label, void *stream);
 
 /* pmsz_verify_{f32,f64}: re-verification of a corrected field fp against f. */
 int pmsz_verify_f32(const float *f, const float *fp, size_t nx, size_t ny, size_t nz,

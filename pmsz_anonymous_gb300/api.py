@@ -196,12 +196,12 @@ def labels(code: torch.Tensor, stream=None):
     if code.dtype != torch.uint8 or code.dim() != 3 or not code.is_cuda:
         raise TypeError("codes must be a (nz, ny, nx) uint8 CUDA tensor")
     nz, ny, nx = code.shape
-    a = torch.empty(code.shape, dtype=torch.int32, device=code.device)
-    d = torch.empty(code.shape, dtype=torch.int32, device=code.device)
+    a = torch.empty(code.shape, dtype=torch.int64, device=code.device)
+    d = torch.empty(code.shape, dtype=torch.int64, device=code.device)
     with torch.cuda.device(code.device):
-        capi.check(capi.load().pmsz_labels(code.data_ptr(), nx, ny, nz, a.data_ptr(), d.data_ptr(), _stream(stream)))
-    mask = (1 << 32) - 1
-    return a.to(torch.int64) & mask, d.to(torch.int64) & mask
+        capi.check(capi.load().pmsz_labels_i64(code.data_ptr(), nx, ny, nz, a.data_ptr(), d.data_ptr(),
+                                               _stream(stream)))
+    return a, d
 
 
 def verify(f: torch.Tensor, fp: torch.Tensor, eb: float, stream=None) -> dict:

@@ -81,6 +81,7 @@ SIGNATURES = {
     "pmsz_codes_f64": (c_int, [_P, c_size, c_size, c_size, _P, _P]),
     "pmsz_rank_offset": (c_int, [c_int, _P, _P, _P]),
     "pmsz_labels": (c_int, [_P, c_size, c_size, c_size, _P, _P, _P]),
+    "pmsz_labels_i64": (c_int, [_P, c_size, c_size, c_size, _P, _P, _P]),
     "pmsz_verify_f32": (c_int, [_P, _P, c_size, c_size, c_size, c_double, _P, _P]),
     "pmsz_verify_f64": (c_int, [_P, _P, c_size, c_size, c_size, c_double, _P, _P]),
     "pmsz_extract_edits_f32": (c_int, [_P, _P, _P, c_size, c_double, c_int, _P, _P, _P, _P, _P]),
