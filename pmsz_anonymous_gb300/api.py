@@ -90,9 +90,8 @@ def correct(f: torch.Tensor, fhat: torch.Tensor, eb: float, q: int = 5, max_swee
     (c_loops, pMSz.cu:1872-2074).  strategy="naive" runs the naive-MSz loop
     instead (naive_MSz.cu:1887-2220; full_sweeps and timing do not apply).
     autotune=True tunes the field's shape class on these inputs first when the
-    tuning table has no entry for it (PMSZ_FLAG_AUTOTUNE).  host_loop=True
-    enqueues the list sweeps from the host instead of a CUDA graph
-    (PMSZ_FLAG_HOST_LOOP; same results).
+    tuning table has no entry for it (PMSZ_FLAG_AUTOTUNE).  host_loop is
+    accepted without effect (PMSZ_FLAG_HOST_LOOP).
     Raises PmszError except for PMSZ_ERR_NOT_CONVERGED, which is reported in
     the result."""
     _check_field(f, "f")

@@ -153,6 +153,10 @@ __host__ __device__ __forceinline__ uint32_t fdiv(uint32_t n, const FastDiv &f) 
     return static_cast<uint32_t>((static_cast<uint64_t>(t) + n) >> f.s);
 }
 
+// Words per group of a bitmap (sweep.cuh keeps a flag byte per group): eight
+// words of four bytes, so that a warp has one byte of the group per lane.
+constexpr int kGroupWords = 8;
+
 // Blocks of the bitmap-compaction kernels (one contiguous word range each).
 constexpr int kCompactBlocks = 152 * 8;
 
@@ -171,12 +175,12 @@ constexpr int kZChunkDefault = 32;  // zc when no tuned value is recorded for th
 // Tiles of the full-field passes (march.cuh): 32 x 8 columns, one block each,
 // two voxels of a plane per thread.
 constexpr int kTX = 32, kMY = 8;
-constexpr int kMarchMaxDepth = 128;  // deeper columns run as this (the passes queue 7-bit depths)
+constexpr int kMarchMaxDepth = 64;  // deeper columns run as this (the passes keep bitmaps of a column)
 inline int march_depth(int zc) { return zc < kMarchMaxDepth ? zc : kMarchMaxDepth; }
 // Depth without a tuned value: the default, halved while the launch has fewer
 // columns than six blocks per SM (152 SMs hold six), down to 4 -- a 64^3 field
 // has 16 columns of 32 x 8, and 32 planes deep they leave most SMs idle and
-// every block a long serial march (first pass 75 us at depth 32, 33 us at 4);
+// every block a long serial march (first pass 75 us at depth 32, 19 us at 4);
 // below 4 the two halo planes of a column cost more than the extra blocks gain.
 inline int default_depth(uint64_t columns_planes, int zc = kZChunkDefault) {  // sum over fields of columns * nz
     while (zc > 4 && columns_planes / static_cast<uint64_t>(zc) < 152u * 6u) zc /= 2;

@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256) k_codes(const T *__restrict__ v, uint8_t 
 
 }  // namespace pmsz
 
-#include "tail.cuh"
+#include "sweep.cuh"
 
 namespace pmsz {
 
@@ -255,8 +255,8 @@ constexpr char kCopyMissing[] = "first pass: a tile plane's tensor copy did not 
 template <typename T>
 static int launch_first_pass(const FirstMaps &m, dim3 grid, cudaStream_t s, const T *f, T *fh, uint8_t *codes,
                              uint32_t *hp, uint32_t *req, uint32_t *act, SweepSlot *slot, const Geom &g, int bz0,
-                             uint32_t *xc, uint32_t *err) {
-    const MarchArgs<T> a{f, fh, codes, hp, req, nullptr, act, slot, xc};
+                             uint32_t *xc, uint32_t *err, uint8_t *freq = nullptr, uint8_t *fact = nullptr) {
+    const MarchArgs<T> a{f, fh, codes, hp, req, nullptr, act, slot, xc, freq, fact};
     if (m.ok) {
         PMSZ_CUDA(allow_smem(k_first_tma<T>, sizeof(TmaMarch<T>)));
         k_first_tma<T><<<grid, dim3(kTX, kThreads / kTX, 1), sizeof(TmaMarch<T>), s>>>(m.f, m.fh, a, g, bz0, err);
@@ -267,93 +267,42 @@ static int launch_first_pass(const FirstMaps &m, dim3 grid, cudaStream_t s, cons
     return PMSZ_OK;
 }
 
-// Runs sweeps first.. in one cooperative launch of k_tail_loop (grid = the
-// number of co-resident blocks) after summarising the active bitmap of sweep
-// `first`; *done receives the total number of sweeps.
+// The resident blocks of k_sweeps on the current device (queried once per
+// device: the queries cost more than a small field's sweep).
 template <typename T>
-static int run_sweep_loop(const T *f, T *fh, const uint8_t *codes, uint8_t *cnt, uint32_t *hp, uint32_t *req,
-                          uint32_t *const act[2], SweepSlot *slots, int64_t first, int64_t max_sweeps, const Geom &g,
-                          T eps, T delta, int q, cudaStream_t s, EventTimer *et, double *ms_acc, int64_t *done) {
-    int dev = 0, sms = 0, per_sm = 0, coop = 0;
+static int sweep_grid(unsigned *blocks) {
+    static std::mutex mu;
+    static std::vector<unsigned> known;
+    int dev = 0;
     PMSZ_CUDA(cudaGetDevice(&dev));
-    PMSZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    PMSZ_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if (!coop) return set_error(PMSZ_ERR_CUDA, "device does not support cooperative launches");
-    PMSZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tail_loop<T>, kTailBlock, 0));
-    if (per_sm < 1) return set_error(PMSZ_ERR_CUDA, "sweep loop kernel does not fit on an SM");
-    const size_t ns = summary_words(g);
-    const unsigned grid = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(ns, static_cast<size_t>(per_sm) * sms)));
-    long long *d_done = nullptr;
-    Workspace ws(s);
-    const size_t o_done = ws.reserve<long long>(1);
-    const size_t o_sum = ws.reserve<uint32_t>(3 * ns);
-    int rc = ws.commit();
-    if (rc) return rc;
-    d_done = ws.at<long long>(o_done);
-    uint32_t *sum = ws.at<uint32_t>(o_sum);  // summaries of act[0], act[1], req
-    if (et) PMSZ_CUDA(cudaEventRecord(et->ev[0], s));
-    PMSZ_CUDA(cudaMemsetAsync(sum, 0, 3 * ns * sizeof(uint32_t), s));
-    const int c = static_cast<int>(first & 1);
-    k_build_summary<<<static_cast<unsigned>(std::min<size_t>((ns + 7) / 8, 152 * 16)), 256, 0, s>>>(
-        act[c], g, sum + static_cast<size_t>(c) * ns);
-    PMSZ_CUDA(cudaGetLastError());
-    TailArgs<T> a{f,    fh,        codes, cnt, hp,    req, act[0], act[1], sum + 2 * ns, sum, sum + ns,
-                  slots, first, max_sweeps, d_done, g,  eps, delta,  q};
-    void *args[] = {&a};
-    PMSZ_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_tail_loop<T>), dim3(grid), dim3(kTailBlock),
-                                          args, 0, s));
-    if (et) PMSZ_CUDA(cudaEventRecord(et->ev[1], s));
-    long long h = 0;
-    PMSZ_CUDA(cudaMemcpyAsync(&h, d_done, sizeof(h), cudaMemcpyDeviceToHost, s));
-    PMSZ_CUDA(cudaStreamSynchronize(s));
-    if (et) {
-        float ms = 0;
-        PMSZ_CUDA(cudaEventElapsedTime(&ms, et->ev[0], et->ev[1]));
-        *ms_acc += ms;
+    std::lock_guard<std::mutex> lk(mu);
+    if (static_cast<size_t>(dev) >= known.size()) known.resize(static_cast<size_t>(dev) + 1, 0u);
+    if (!known[static_cast<size_t>(dev)]) {
+        int sms = 0, per_sm = 0, coop = 0;
+        PMSZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        PMSZ_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        if (!coop) return set_error(PMSZ_ERR_CUDA, "device does not support cooperative launches");
+        PMSZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweeps<T>, kSweepBlock, 0));
+        if (per_sm < 1) return set_error(PMSZ_ERR_CUDA, "sweep kernel does not fit on an SM");
+        known[static_cast<size_t>(dev)] = static_cast<unsigned>(per_sm * sms);
     }
-    *done = h;
-    return ws.release();
+    *blocks = known[static_cast<size_t>(dev)];
+    return PMSZ_OK;
 }
 
-// The cooperative tail behind the list sweeps, enqueued without waiting for
-// the host: it starts at sweep ls->k and runs only if the last gate handed
-// over to it (ls->tail); *hdone (pinned host memory) receives the total
-// number of sweeps once the stream gets there.
+// All remaining sweeps in one cooperative launch; a small field takes no more
+// blocks than it has groups of words.
 template <typename T>
-static int enqueue_gated_tail(const T *f, T *fh, const uint8_t *codes, uint8_t *cnt, uint32_t *hp, uint32_t *req,
-                              uint32_t *const act[2], SweepSlot *slots, const LoopState *ls, int64_t max_sweeps,
-                              const Geom &g, T eps, T delta, int q, cudaStream_t s, EventTimer *et, long long *hdone) {
-    int dev = 0, sms = 0, per_sm = 0, coop = 0;
-    PMSZ_CUDA(cudaGetDevice(&dev));
-    PMSZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    PMSZ_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if (!coop) return set_error(PMSZ_ERR_CUDA, "device does not support cooperative launches");
-    PMSZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tail_loop<T>, kTailBlock, 0));
-    if (per_sm < 1) return set_error(PMSZ_ERR_CUDA, "sweep loop kernel does not fit on an SM");
-    const size_t ns = summary_words(g);
-    const unsigned grid = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(ns, static_cast<size_t>(per_sm) * sms)));
-    Workspace ws(s);
-    const size_t o_done = ws.reserve<long long>(1);
-    const size_t o_sum = ws.reserve<uint32_t>(3 * ns);
-    int rc = ws.commit();
+static int launch_sweeps(SweepArgs<T> &a, cudaStream_t s) {
+    unsigned blocks = 0;
+    const int rc = sweep_grid<T>(&blocks);
     if (rc) return rc;
-    long long *d_done = ws.at<long long>(o_done);
-    uint32_t *sum = ws.at<uint32_t>(o_sum);  // summaries of act[0], act[1], req
-    if (et) PMSZ_CUDA(cudaEventRecord(et->ev[0], s));
-    PMSZ_CUDA(cudaMemsetAsync(sum, 0, 3 * ns * sizeof(uint32_t), s));
-    k_build_summary_at<<<static_cast<unsigned>(std::min<size_t>((ns + 7) / 8, 152 * 16)), 256, 0, s>>>(
-        act[0], act[1], g, sum, sum + ns, &ls->k, &ls->tail);
-    PMSZ_CUDA(cudaGetLastError());
-    TailArgs<T> a{f,    fh,        codes, cnt, hp,    req, act[0], act[1], sum + 2 * ns, sum, sum + ns,
-                  slots, 0, max_sweeps, d_done, g,  eps, delta,  q};
-    a.first_at = &ls->k;
-    a.run_if = &ls->tail;
+    const size_t want = (group_count(a.g) + kSweepWarps - 1) / kSweepWarps;
+    const unsigned grid = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(want, blocks)));
     void *args[] = {&a};
-    PMSZ_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_tail_loop<T>), dim3(grid), dim3(kTailBlock),
+    PMSZ_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_sweeps<T>), dim3(grid), dim3(kSweepBlock),
                                           args, 0, s));
-    if (et) PMSZ_CUDA(cudaEventRecord(et->ev[1], s));
-    PMSZ_CUDA(cudaMemcpyAsync(hdone, d_done, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    return ws.release();
+    return PMSZ_OK;
 }
 
 // Grid of the list-compaction kernels: one block per 2048-word round, at most
@@ -446,7 +395,7 @@ int enqueue_ingest(const T *hf, const T *hfh, T *df, T *dfh, T *dprev, size_t nx
 template <typename T>
 int first_pass_ingest(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes, uint32_t *hp, uint32_t *req,
                       uint32_t *a_next, SweepSlot *slot, const Geom &g, cudaStream_t s, int64_t *launches,
-                      uint32_t *xcount, const FirstMaps &maps, uint32_t *err) {
+                      uint32_t *xcount, const FirstMaps &maps, uint32_t *err, uint8_t *freq, uint8_t *fact) {
     if (in.df != f || !in.copies || in.copies->zc != g.zc)
         return set_error(PMSZ_ERR_ARG, "ingest copies do not match the field");
     const IngestCopies &r = *in.copies;
@@ -456,7 +405,7 @@ int first_pass_ingest(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes
         PMSZ_CUDA(cudaStreamWaitEvent(s, r.ev[j], 0));
         dim3 grid = tiled_grid(g);
         grid.z = static_cast<unsigned>(std::min(cps, nchunks - j * cps));
-        if ((rc = launch_first_pass<T>(maps, grid, s, f, fh, codes, hp, req, a_next, slot, g, j * cps, xcount, err))) return rc;
+        if ((rc = launch_first_pass<T>(maps, grid, s, f, fh, codes, hp, req, a_next, slot, g, j * cps, xcount, err, freq, fact))) return rc;
         PMSZ_CUDA(cudaGetLastError());
         ++*launches;
     }
@@ -464,8 +413,7 @@ int first_pass_ingest(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes
     return PMSZ_OK;
 }
 
-// Sweeps pipelined behind the host copy (even: the graph's two-sweep body
-// starts at an odd sweep), and the fractions of the slabs after which they
+// Sweeps pipelined behind the host copy, and the fractions of the slabs after which they
 // advance: every piece of a sweep costs two compaction kernels and five more
 // launches whatever its size, so the early waves are large and the late
 // ones, whose remainder is all that is left once the copy ends, small (a
@@ -535,9 +483,8 @@ static int first_pass_waves(const HostIngest<T> &in, const T *f, T *fh, uint8_t 
             if (k > 0 && D > Dp[k]) {
                 compact_bitmap_planes(act[k & 1], g, Dp[k], D, bcnt, list, &ls->lc[0], s);
                 k_detect_list<T><<<lb, 256, 0, s>>>(list, &ls->lc[0], fh, hp, codes, req, a_next, slist, &ls->lc[2],
-                                                    &slots[k], g, div_nx, nullptr, &ls->exact_keys, nullptr);
-                k_detect_exact<T><<<lb, 256, 0, s>>>(slist, &ls->lc[2], fh, codes, req, a_next, &slots[k], g, div_nx,
-                                                     nullptr);
+                                                    &slots[k], g, div_nx);
+                k_detect_exact<T><<<lb, 256, 0, s>>>(slist, &ls->lc[2], fh, codes, req, a_next, &slots[k], g, div_nx);
                 k_wave_clear_spills<<<1, 32, 0, s>>>(ls);
                 *launches += 5;
             }
@@ -546,7 +493,7 @@ static int first_pass_waves(const HostIngest<T> &in, const T *f, T *fh, uint8_t 
             if (A > Ap[k]) {
                 compact_bitmap_planes(req, g, Ap[k], A, bcnt, list, &ls->lc[1], s);
                 k_apply_list<T><<<lb, 256, 0, s>>>(list, &ls->lc[1], f, fh, cnt, hp, a_next, &slots[k], g, div_nx, eps,
-                                                   delta, q, nullptr);
+                                                   delta, q);
                 *launches += 3;
                 Ap[k] = A;
             }
@@ -580,245 +527,118 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
     const T eps = static_cast<T>(eb);
     const T delta = static_cast<T>(eb / static_cast<double>(q));  // pMSz.cu:2814
 
-    // Scratch: codes (n), counters (n), request + two active bitmaps, sweep slots.
+    // Scratch: what starts at zero first, in one piece (loop state and sweep
+    // slots, counters, request + two active bitmaps with their group flags),
+    // then codes and proxies.
+    const bool full = (flags & PMSZ_FLAG_FULL_SWEEPS) != 0;
+    const size_t groups = group_count(g);
     Workspace ws(s);
-    const size_t o_codes = ws.reserve<uint8_t>(g.n);
+    const size_t o_ls = ws.reserve<LoopState>(1);
+    const size_t o_slots = ws.reserve<SweepSlot>(static_cast<size_t>(max_sweeps));
     const bool own_cnt = !(ingest && ingest->cnt);
     const size_t o_cnt = ws.reserve<uint8_t>(own_cnt ? g.n : 0);
     const size_t o_req = ws.reserve<uint32_t>(g.nwords);
     const size_t o_a0 = ws.reserve<uint32_t>(g.nwords);
     const size_t o_a1 = ws.reserve<uint32_t>(g.nwords);
-    const size_t o_slots = ws.reserve<SweepSlot>(static_cast<size_t>(max_sweeps));
+    const size_t o_fr = ws.reserve<uint8_t>(groups), o_f0 = ws.reserve<uint8_t>(groups), o_f1 = ws.reserve<uint8_t>(groups);
+    const size_t zero_bytes = ws.reserve<uint8_t>(0);
+    const size_t o_codes = ws.reserve<uint8_t>(g.n);
     const size_t o_hp = ws.reserve<uint32_t>(g.n);
-    // voxel-list sweeps (list.cuh) for fields of fewer than 2^32 voxels
-    const bool use_list = !(flags & PMSZ_FLAG_FULL_SWEEPS) && g.n < (static_cast<size_t>(1) << 32);
-    const size_t o_list = ws.reserve<uint32_t>(use_list ? g.n : 0);
-    const size_t o_xlist = ws.reserve<uint32_t>(use_list ? g.n : 0);
-    const size_t o_bcnt = ws.reserve<uint32_t>(use_list ? kCompactBlocks : 0);
-    const size_t o_ls = ws.reserve<LoopState>(use_list ? 1 : 0);
-    const size_t o_err = ws.reserve<uint32_t>(1);
     // host-buffer calls of several slabs run sweeps 1 .. K behind the copy
-    // (first_pass_waves; K even, below max_sweeps)
-    const int wave_k = static_cast<int>(std::min<int64_t>(kWaveSweeps, max_sweeps - 1)) & ~1;
-    const bool waves = ingest && use_list && wave_k >= 2 && ingest->copies && ingest->copies->nslabs >= 2;
+    // (first_pass_waves; K below max_sweeps) on voxel lists
+    const int wave_k = static_cast<int>(std::min<int64_t>(kWaveSweeps, max_sweeps - 1));
+    const bool waves = ingest && !full && g.n < (static_cast<size_t>(1) << 32) && wave_k >= 1 && ingest->copies &&
+                       ingest->copies->nslabs >= 2;
+    const size_t o_list = ws.reserve<uint32_t>(waves ? g.n : 0);
+    const size_t o_xlist = ws.reserve<uint32_t>(waves ? g.n : 0);
+    const size_t o_bcnt = ws.reserve<uint32_t>(waves ? kCompactBlocks : 0);
     if ((rc = ws.commit())) return rc;
-    uint32_t *hp = ws.at<uint32_t>(o_hp);
-    uint8_t *codes = ws.at<uint8_t>(o_codes);
+    LoopState *ls = ws.at<LoopState>(o_ls);
+    SweepSlot *slots = ws.at<SweepSlot>(o_slots);
     uint8_t *cnt = own_cnt ? ws.at<uint8_t>(o_cnt) : ingest->cnt;
     uint32_t *req = ws.at<uint32_t>(o_req);
     uint32_t *act[2] = {ws.at<uint32_t>(o_a0), ws.at<uint32_t>(o_a1)};
-    SweepSlot *slots = ws.at<SweepSlot>(o_slots);
-    uint32_t *list = use_list ? ws.at<uint32_t>(o_list) : nullptr;
-    uint32_t *xlist = use_list ? ws.at<uint32_t>(o_xlist) : nullptr;
-    uint32_t *bcnt = use_list ? ws.at<uint32_t>(o_bcnt) : nullptr;  // per-block counts of a compaction
-    LoopState *ls = use_list ? ws.at<LoopState>(o_ls) : nullptr;
-    uint32_t *ferr = use_list ? &ls->err : ws.at<uint32_t>(o_err);  // set by a first pass whose copies did not arrive
-    const FastDiv div_nx = make_fastdiv(static_cast<uint32_t>(g.nx));
-    const unsigned list_blocks = 152 * 8;
+    uint8_t *freq = ws.at<uint8_t>(o_fr), *fact[2] = {ws.at<uint8_t>(o_f0), ws.at<uint8_t>(o_f1)};
+    uint8_t *codes = ws.at<uint8_t>(o_codes);
+    uint32_t *hp = ws.at<uint32_t>(o_hp);
     const FirstMaps maps = first_maps<T>(f, fh, g);
     EventTimer et;
     if ((rc = et.init())) return rc;
     PMSZ_CUDA(cudaEventRecord(et.ev[3], s));  // start of the loop's device window
 
-    PMSZ_CUDA(cudaMemsetAsync(cnt, 0, g.n, s));  // init_counter, pMSz.cu:1745-1749
-    PMSZ_CUDA(cudaMemsetAsync(req, 0, g.nwords * 4, s));
-    PMSZ_CUDA(cudaMemsetAsync(act[0], 0, g.nwords * 4, s));
-    PMSZ_CUDA(cudaMemsetAsync(act[1], 0, g.nwords * 4, s));
-    PMSZ_CUDA(cudaMemsetAsync(slots, 0, sizeof(SweepSlot) * static_cast<size_t>(max_sweeps), s));
-    if (use_list) {
-        PMSZ_CUDA(cudaMemsetAsync(ls, 0, sizeof(LoopState), s));
-        PMSZ_CUDA(cudaMemsetAsync(&ls->go, 1, 1, s));  // sweep 0 runs (little-endian int 1)
-    } else {
-        PMSZ_CUDA(cudaMemsetAsync(ferr, 0, sizeof(uint32_t), s));
-    }
+    PMSZ_CUDA(cudaMemsetAsync(ls, 0, zero_bytes, s));  // init_counter among them, pMSz.cu:1745-1749
+    if (!own_cnt) PMSZ_CUDA(cudaMemsetAsync(cnt, 0, g.n, s));
 
-    SweepSlot *hslot = static_cast<SweepSlot *>(host_pinned(sizeof(SweepSlot) + 64));
-    if (!hslot) return set_error(PMSZ_ERR_OOM, "pinned host allocation failed");
-    uint32_t *herr = reinterpret_cast<uint32_t *>(hslot + 1);
     const bool timing = (flags & PMSZ_FLAG_TIMING) != 0;
     double ms_first = 0, ms_detect = 0, ms_apply = 0;
     int64_t launches = 0;
-    const dim3 blk3(32, 8, 1);
-    int cur = 0;  // act[cur] = active set of the coming sweep; act[cur^1] receives the next one
     int64_t sweeps = 0;
     uint64_t edits = 0;
     int status = PMSZ_ERR_NOT_CONVERGED;
     bool end_recorded = false;  // et.ev[0] marks the end of the correction's device window
     std::vector<SweepSlot> log;
-    // The cooperative tail takes over once the next active set is estimated
-    // below N/32, but never above kTailCap voxels: its barrier-separated
-    // phases serve millions of active voxels worse than list sweeps do, and at
-    // 1536^3 N/32 is 113 M.
-    constexpr unsigned long long kTailCap = 1ull << 20;
-    const unsigned long long tail_at = std::max<unsigned long long>(std::min<unsigned long long>(g.n / 32, kTailCap), 1ull << 16);
-    if (use_list) {
-        // Sweep 0 (the fused first pass and its edits) on the stream; then the
-        // voxel-list sweeps as a CUDA graph whose while node repeats a body of
-        // two sweeps (odd: act[1] -> act[0], even: act[0] -> act[1]) for as
-        // long as k_loop_gate lets the next sweep run: no host round trip
-        // between sweeps.  The graph is built on the host while sweep 0 runs.
-        // What the gate leaves (a small active set) goes to the cooperative
-        // tail.
-        EventTimer lt;  // sweep 0 start, first pass done, sweep 0 done, list sweeps done
+    // The state and the first slots of the sweep log, in one read-back.
+    constexpr int64_t kLogAhead = 64;
+    static_assert(sizeof(LoopState) <= 256, "the slots follow the loop state at its 256-byte slot");
+    const int64_t pre = std::min<int64_t>(max_sweeps, kLogAhead);
+    const size_t head = 256 + static_cast<size_t>(pre) * sizeof(SweepSlot);
+    unsigned char *hb = static_cast<unsigned char *>(host_pinned(head));
+    if (!hb) return set_error(PMSZ_ERR_OOM, "pinned host allocation failed");
+    const LoopState *hls = reinterpret_cast<const LoopState *>(hb);
+    const SweepSlot *hlog = reinterpret_cast<const SweepSlot *>(hb + 256);
+    if (!full) {
+        // The fused first pass, then every sweep in one cooperative launch
+        // (k_sweeps), which starts with the edits of sweep 0 -- or, behind the
+        // host copy, where the wavefront left off.  One read-back at the end.
+        EventTimer lt;  // start, first pass done, sweeps done
         if (timing) {
             if ((rc = lt.init())) return rc;
             PMSZ_CUDA(cudaEventRecord(lt.ev[0], s));
         }
-        if (waves) {  // sweeps 0 .. wave_k behind the host copy, then the state after them
-            if ((rc = first_pass_waves<T>(*ingest, f, fh, codes, cnt, hp, req, act, slots, ls, g, maps, list, xlist,
-                                          bcnt, div_nx, eps, delta, q, wave_k, s, &launches)))
+        SweepArgs<T> a{f,  fh,         codes, cnt, hp,  req,   act[0], act[1], freq, fact[0], fact[1], slots,
+                       ls, max_sweeps, 1,     g,   eps, delta, q};
+        if (waves) {
+            if ((rc = first_pass_waves<T>(*ingest, f, fh, codes, cnt, hp, req, act, slots, ls, g, maps,
+                                          ws.at<uint32_t>(o_list), ws.at<uint32_t>(o_xlist), ws.at<uint32_t>(o_bcnt),
+                                          make_fastdiv(static_cast<uint32_t>(g.nx)), eps, delta, q, wave_k, s,
+                                          &launches)))
                 return rc;
-            if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[1], s));
-            k_wave_gate<<<1, 32, 0, s>>>(ls, slots, wave_k, max_sweeps, tail_at, static_cast<unsigned long long>(g.n),
-                                         list_blocks);
+            k_wave_gate<<<1, 32, 0, s>>>(ls, slots, wave_k, max_sweeps);
+            k_build_flags<<<static_cast<unsigned>(std::min<size_t>((groups + 7) / 8, 152 * 16)), 256, 0, s>>>(
+                act[0], act[1], g, fact[0], fact[1], &ls->k);
+            PMSZ_CUDA(cudaGetLastError());
+            launches += 2;
+            a.from_edits = 0;
+        } else if (ingest) {
+            if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, act[1], &slots[0], g, s, &launches,
+                                           &ls->lc[3], maps, &ls->err, freq, fact[1])))
+                return rc;
+        } else {
+            if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, act[1], &slots[0], g, 0,
+                                           &ls->lc[3], &ls->err, freq, fact[1])))
+                return rc;
             ++launches;
-            PMSZ_CUDA(cudaGetLastError());
-            if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[2], s));
-        } else {
-            if (ingest) {
-                if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, act[1], &ls->cur, g, s, &launches,
-                                               &ls->lc[3], maps, &ls->err)))
-                    return rc;
-            } else {
-                if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, act[1], &ls->cur, g, 0,
-                                     &ls->lc[3], &ls->err))) return rc;
-                ++launches;
-            }
-            if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[1], s));
-            compact_bitmap(req, g, bcnt, list, &ls->lc[1], &ls->go, s);
-            k_apply_list<T><<<list_blocks, 256, 0, s>>>(list, &ls->lc[1], f, fh, cnt, hp, act[1], &ls->cur, g, div_nx,
-                                                        eps, delta, q, &ls->go);
-            k_pick_detection<<<1, 32, 0, s>>>(ls, static_cast<unsigned long long>(g.n), list_blocks);
-            k_loop_gate<<<1, 32, 0, s>>>(ls, slots, max_sweeps, tail_at, cudaGraphConditionalHandle{}, 0);
-            launches += 5;
-            PMSZ_CUDA(cudaGetLastError());
-            if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[2], s));
         }
-
-        // One body: two list sweeps (odd: act[1] -> act[0], even: act[0] ->
-        // act[1]), each ending with k_loop_gate; with set_cond the second gate
-        // also sets the graph's while condition.
-        auto enqueue_body = [&](cudaStream_t bs, cudaGraphConditionalHandle cond, bool set_cond) {
-            for (int half = 0; half < 2; ++half) {
-                uint32_t *a_cur = act[half == 0 ? 1 : 0], *a_next = act[half == 0 ? 0 : 1];
-                compact_bitmap(a_cur, g, bcnt, list, &ls->lc[0], &ls->go, bs);
-                k_detect_list<T><<<list_blocks, 256, 0, bs>>>(list, &ls->lc[0], fh, hp, codes, req, a_next, xlist,
-                                                              &ls->lc[2], &ls->cur, g, div_nx, &ls->go,
-                                                              &ls->exact_keys, &ls->deferred);
-                k_detect_exact<T><<<list_blocks, 256, 0, bs>>>(xlist, &ls->lc[2], fh, codes, req, a_next, &ls->cur, g,
-                                                               div_nx, &ls->go);
-                compact_bitmap(req, g, bcnt, list, &ls->lc[1], &ls->go, bs);
-                k_apply_list<T><<<list_blocks, 256, 0, bs>>>(list, &ls->lc[1], f, fh, cnt, hp, a_next, &ls->cur, g,
-                                                             div_nx, eps, delta, q, &ls->go);
-                k_loop_gate<<<1, 32, 0, bs>>>(ls, slots, max_sweeps, tail_at, cond, set_cond && half == 1 ? 1 : 0);
-            }
-        };
-        int64_t bodies = 0;
-        if (flags & PMSZ_FLAG_HOST_LOOP) {
-            // the same sweeps enqueued from the host, two per round trip to the
-            // device gate (tools that cannot look into conditional graph nodes)
-            int *hgo = static_cast<int *>(host_pinned(sizeof(int)));
-            if (!hgo) return set_error(PMSZ_ERR_OOM, "pinned host allocation failed");
-            for (;;) {
-                PMSZ_CUDA(cudaMemcpyAsync(hgo, &ls->go, sizeof(int), cudaMemcpyDeviceToHost, s));
-                PMSZ_CUDA(cudaStreamSynchronize(s));
-                if (!*hgo) break;
-                enqueue_body(s, cudaGraphConditionalHandle{}, false);
-                PMSZ_CUDA(cudaGetLastError());
-                ++bodies;
-            }
-        } else {
-            // The graph: k_loop_enter, then one conditional while node whose
-            // body is enqueue_body, captured while sweep 0 runs; no host round
-            // trip between sweeps.
-            struct GraphGuard {
-                cudaGraph_t graph = nullptr;
-                cudaGraphExec_t exec = nullptr;
-                cudaStream_t cs = nullptr;
-                ~GraphGuard() {
-                    if (exec) cudaGraphExecDestroy(exec);
-                    if (graph) cudaGraphDestroy(graph);
-                    if (cs) cudaStreamDestroy(cs);
-                }
-            } gg;
-            PMSZ_CUDA(cudaGraphCreate(&gg.graph, 0));
-            cudaGraphConditionalHandle cond;
-            PMSZ_CUDA(cudaGraphConditionalHandleCreate(&cond, gg.graph, 1, cudaGraphCondAssignDefault));
-            cudaGraphNodeParams cp = {};
-            cp.type = cudaGraphNodeTypeConditional;
-            cp.conditional.handle = cond;
-            cp.conditional.type = cudaGraphCondTypeWhile;
-            cp.conditional.size = 1;
-            // k_loop_enter sets the condition before the while node is reached
-            const LoopState *cls = ls;
-            void *eargs[] = {&cls, &cond};
-            cudaGraphNodeParams ep = {};
-            ep.type = cudaGraphNodeTypeKernel;
-            ep.kernel.func = reinterpret_cast<void *>(k_loop_enter);
-            ep.kernel.gridDim = dim3(1);
-            ep.kernel.blockDim = dim3(32);
-            ep.kernel.kernelParams = eargs;
-            cudaGraphNode_t enode, wnode;
-            PMSZ_CUDA(cudaGraphAddNode(&enode, gg.graph, nullptr, nullptr, 0, &ep));
-            PMSZ_CUDA(cudaGraphAddNode(&wnode, gg.graph, &enode, nullptr, 1, &cp));
-            cudaGraph_t body = cp.conditional.phGraph_out[0];
-            PMSZ_CUDA(cudaStreamCreateWithFlags(&gg.cs, cudaStreamNonBlocking));
-            PMSZ_CUDA(cudaStreamBeginCaptureToGraph(gg.cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-            enqueue_body(gg.cs, cond, true);
-            PMSZ_CUDA(cudaStreamEndCapture(gg.cs, &body));
-            PMSZ_CUDA(cudaGraphInstantiate(&gg.exec, gg.graph, 0));
-            PMSZ_CUDA(cudaGraphLaunch(gg.exec, s));
-        }
-        if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[3], s));
-
-        // The cooperative tail follows without a host round trip (it reads
-        // the gate's decision), then the caller's work on the result; one
-        // read-back brings the loop state, the sweep count and the first
-        // slots of the sweep log.
-        constexpr int64_t kLogAhead = 64;
-        const int64_t pre = std::min<int64_t>(max_sweeps, kLogAhead);
-        const size_t ls_bytes = (sizeof(LoopState) + 63) / 64 * 64;
-        unsigned char *hb =
-            static_cast<unsigned char *>(host_pinned(ls_bytes + 64 + static_cast<size_t>(pre) * sizeof(SweepSlot)));
-        if (!hb) return set_error(PMSZ_ERR_OOM, "pinned host allocation failed");
-        LoopState *hls = reinterpret_cast<LoopState *>(hb);
-        long long *hdone = reinterpret_cast<long long *>(hb + ls_bytes);
-        const SweepSlot *hlog = reinterpret_cast<const SweepSlot *>(hb + ls_bytes + 64);
-        EventTimer tt;
-        if (timing && (rc = tt.init())) return rc;
-        if ((rc = enqueue_gated_tail<T>(f, fh, codes, cnt, hp, req, act, slots, ls, max_sweeps, g, eps, delta, q, s,
-                                        timing ? &tt : nullptr, hdone)))
-            return rc;
-        launches += 2;
+        if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[1], s));
+        if ((rc = launch_sweeps<T>(a, s))) return rc;
+        ++launches;
+        if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[2], s));
         PMSZ_CUDA(cudaEventRecord(et.ev[0], s));  // end of the correction's device window
         end_recorded = true;
-        PMSZ_CUDA(cudaMemcpyAsync(hls, ls, sizeof(LoopState), cudaMemcpyDeviceToHost, s));
-        PMSZ_CUDA(cudaMemcpyAsync(hb + ls_bytes + 64, slots, static_cast<size_t>(pre) * sizeof(SweepSlot),
-                                  cudaMemcpyDeviceToHost, s));
+        PMSZ_CUDA(cudaMemcpyAsync(hb, ls, head, cudaMemcpyDeviceToHost, s));
         if (ingest && ingest->after && ingest->after->fn) {
             ingest->after->done = true;
             if ((rc = ingest->after->fn(s))) return rc;
         }
         PMSZ_CUDA(cudaStreamSynchronize(s));
-        if (hls->err)
-            return set_error(PMSZ_ERR_CUDA, kCopyMissing);
-        const int64_t gdone = hls->k;  // sweeps 0 .. gdone-1 ran before the tail
-        const int64_t done = std::max<int64_t>(*hdone, gdone);  // and 0 .. done-1 in all
-        const int64_t nloop = std::max<int64_t>(gdone - (waves ? wave_k + 1 : 1), 0);  // sweeps of the loop
-        // graph: k_loop_enter and one body (16 kernels) per two sweeps that ran
-        launches += (flags & PMSZ_FLAG_HOST_LOOP) ? 16 * bodies : 1 + 16 * ((nloop + 1) / 2);
-        if (timing) {  // the list sweeps' edits run inside the graph and count as detection time
-            float a = 0, b = 0, c = 0;
-            PMSZ_CUDA(cudaEventElapsedTime(&a, lt.ev[0], lt.ev[1]));
-            PMSZ_CUDA(cudaEventElapsedTime(&b, lt.ev[1], lt.ev[2]));
-            PMSZ_CUDA(cudaEventElapsedTime(&c, lt.ev[2], lt.ev[3]));
-            ms_first += a;
-            ms_apply += b;
-            ms_detect += c;
-            if (hls->tail) {
-                PMSZ_CUDA(cudaEventElapsedTime(&a, tt.ev[0], tt.ev[1]));
-                ms_detect += a;
-            }
+        if (hls->err) return set_error(PMSZ_ERR_CUDA, kCopyMissing);
+        const int64_t done = hls->done;  // sweeps 0 .. done-1
+        if (timing) {  // sweep 0's edits run inside the launch and count as detection time
+            float x = 0, y = 0;
+            PMSZ_CUDA(cudaEventElapsedTime(&x, lt.ev[0], lt.ev[1]));
+            PMSZ_CUDA(cudaEventElapsedTime(&y, lt.ev[1], lt.ev[2]));
+            ms_first += x;
+            ms_detect += y;
         }
         log.assign(hlog, hlog + std::min(done, pre));
         if (done > pre) {
@@ -829,37 +649,32 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         }
         for (const SweepSlot &t : log) edits += t.requested;
         sweeps = done;
-        const SweepSlot h = log[static_cast<size_t>(gdone - 1)];  // the sweep the last gate decided on
-        if (gdone == 1 && h.bad) {
+        const SweepSlot &last = log.back();
+        if (done == 1 && last.bad) {
             status = set_error(PMSZ_ERR_ARG, "input contains NaN or the value 1e30 (the reference's halo sentinel)");
-        } else if (h.fmax == 0 && h.fmin == 0 && h.fdir == 0) {
+        } else if (last.fmax == 0 && last.fmin == 0 && last.fdir == 0) {
             status = PMSZ_OK;
-        } else if (h.progressed == 0) {
+        } else if (last.progressed == 0) {
             set_error(PMSZ_ERR_NOT_CONVERGED, "a sweep requested edits that changed nothing (all requested vertices clamped)");
-        } else if (done > gdone) {  // the cooperative tail ran sweeps gdone .. done-1
-            const SweepSlot &last = log.back();
-            if (last.fmax == 0 && last.fmin == 0 && last.fdir == 0) status = PMSZ_OK;
-            else if (last.progressed == 0)
-                set_error(PMSZ_ERR_NOT_CONVERGED, "a sweep requested edits that changed nothing (all requested vertices clamped)");
         }
     }
-    while (!use_list && sweeps < max_sweeps) {
+    // The reference's schedule: every sweep over the whole field, host-driven.
+    while (full && sweeps < max_sweeps) {
         SweepSlot *slot = slots + sweeps;
-        uint32_t *a_next = act[cur ^ 1];
+        uint32_t *a_next = act[(sweeps + 1) & 1];
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[0], s));
         if (sweeps == 0 && ingest) {
             if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, a_next, slot, g, s, &launches, nullptr, maps,
-                                           ferr)))
+                                           &ls->err, nullptr, nullptr)))
                 return rc;
         } else if (sweeps == 0) {
-            if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, a_next, slot, g, 0, nullptr, ferr))) return rc;
-            ++launches;
-        } else if (flags & PMSZ_FLAG_FULL_SWEEPS) {
-            PMSZ_CUDA((launch_march<T, kDetect>(
-                tiled_grid(g), s, MarchArgs<T>{nullptr, fh, codes, hp, req, nullptr, a_next, slot, nullptr}, g, 0)));
+            if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, a_next, slot, g, 0, nullptr,
+                                           &ls->err)))
+                return rc;
             ++launches;
         } else {
-            k_sparse_px<T><<<list_grid(g), kListBlock, 0, s>>>(fh, hp, codes, act[cur], a_next, req, slot, g);
+            PMSZ_CUDA((launch_march<T, kDetect>(
+                tiled_grid(g), s, MarchArgs<T>{nullptr, fh, codes, hp, req, nullptr, a_next, slot, nullptr}, g, 0)));
             ++launches;
         }
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[1], s));
@@ -867,16 +682,17 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         ++launches;
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[2], s));
         PMSZ_CUDA(cudaGetLastError());
+        SweepSlot *hslot = reinterpret_cast<SweepSlot *>(hb + 256);
         PMSZ_CUDA(cudaMemcpyAsync(hslot, slot, sizeof(SweepSlot), cudaMemcpyDeviceToHost, s));
-        if (sweeps == 0) PMSZ_CUDA(cudaMemcpyAsync(herr, ferr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        if (sweeps == 0) PMSZ_CUDA(cudaMemcpyAsync(hb, ls, sizeof(LoopState), cudaMemcpyDeviceToHost, s));
         PMSZ_CUDA(cudaStreamSynchronize(s));
-        if (sweeps == 0 && *herr) return set_error(PMSZ_ERR_CUDA, kCopyMissing);
+        if (sweeps == 0 && hls->err) return set_error(PMSZ_ERR_CUDA, kCopyMissing);
         if (timing) {
-            float a = 0, b = 0;
-            PMSZ_CUDA(cudaEventElapsedTime(&a, et.ev[0], et.ev[1]));
-            PMSZ_CUDA(cudaEventElapsedTime(&b, et.ev[1], et.ev[2]));
-            (sweeps == 0 ? ms_first : ms_detect) += a;
-            ms_apply += b;
+            float x = 0, y = 0;
+            PMSZ_CUDA(cudaEventElapsedTime(&x, et.ev[0], et.ev[1]));
+            PMSZ_CUDA(cudaEventElapsedTime(&y, et.ev[1], et.ev[2]));
+            (sweeps == 0 ? ms_first : ms_detect) += x;
+            ms_apply += y;
         }
         ++sweeps;
         const SweepSlot h = *hslot;
@@ -889,33 +705,6 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         if (h.fmax == 0 && h.fmin == 0 && h.fdir == 0) { status = PMSZ_OK; break; }
         if (h.progressed == 0) {
             set_error(PMSZ_ERR_NOT_CONVERGED, "a sweep requested edits that changed nothing (all requested vertices clamped)");
-            break;
-        }
-        cur ^= 1;
-        // Once the next active set is small, per-sweep launches and host round
-        // trips dominate: hand the remaining sweeps to one cooperative launch.
-        const unsigned long long est_next = 15ull * h.changed + h.fdir;
-        if (!(flags & PMSZ_FLAG_FULL_SWEEPS) && sweeps < max_sweeps && est_next <= tail_at) {
-            int64_t done = 0;
-            if ((rc = run_sweep_loop<T>(f, fh, codes, cnt, hp, req, act, slots, sweeps, max_sweeps, g, eps, delta, q,
-                                        s, timing ? &et : nullptr, &ms_detect, &done)))
-                return rc;
-            ++launches;
-            const size_t m = static_cast<size_t>(done - sweeps);
-            if (m) {
-                std::vector<SweepSlot> tail(m);
-                PMSZ_CUDA(cudaMemcpyAsync(tail.data(), slots + sweeps, m * sizeof(SweepSlot), cudaMemcpyDeviceToHost, s));
-                PMSZ_CUDA(cudaStreamSynchronize(s));
-                for (const SweepSlot &t : tail) {
-                    log.push_back(t);
-                    edits += t.requested;
-                }
-                const SweepSlot &last = tail.back();
-                if (last.fmax == 0 && last.fmin == 0 && last.fdir == 0) status = PMSZ_OK;
-                else if (last.progressed == 0)
-                    set_error(PMSZ_ERR_NOT_CONVERGED, "a sweep requested edits that changed nothing (all requested vertices clamped)");
-            }
-            sweeps = done;
             break;
         }
     }

@@ -1,10 +1,8 @@
-// list.cuh -- voxel-list sweeps for the host-driven part of the correction
-// loop, included by correct.cu after tiled.cuh.
+// list.cuh -- voxel-list sweeps over plane ranges: the sweeps that run behind
+// the host copy of pmsz_correct_host_* (first_pass_waves); included by
+// sweep.cuh and batch_list.cuh.
 //
-// The early sweeps of a large field touch millions of voxels each.  Instead
-// of compacting and processing a bitmap round by round inside one kernel
-// (which keeps the round state and the detection registers live together and
-// caps residency at a few blocks per SM), each sweep runs as
+// Each piece of a sweep runs as
 //   compaction      bitmap -> list of flat voxel indices in voxel order
 //                   (clears the bitmap); every consumer is order-free anyway
 //                   (requests and marks are bit ORs, counters sums)
@@ -16,9 +14,9 @@
 //   compaction      request bitmap -> list
 //   k_apply_list    one thread per requested voxel: the edit, the proxy
 //                   refresh, the closed-stencil marks of the next active set
-// The per-voxel kernels are light enough for full residency, so the 15
-// gathers of many voxels are in flight at once.  Flat indices are 32-bit:
-// the list form is used when the field has fewer than 2^32 voxels.
+// A sweep whose planes arrive piece by piece cannot wait at a grid barrier, so
+// these stay separate launches; once the copy has ended, k_sweeps (sweep.cuh)
+// takes over.  Flat indices are 32-bit: fields of fewer than 2^32 voxels.
 #pragma once
 #include "march.cuh"
 
@@ -56,10 +54,8 @@ __device__ __forceinline__ uint32_t block_sum_u32(uint32_t v, uint32_t *s_warp) 
 // cleared.  List entries are absolute voxel indices.  The block count is the
 // launch's (compact_per).
 static __global__ void __launch_bounds__(kCompactBlock) k_count_words(const uint32_t *__restrict__ bm, Geom g,
-                                                               uint32_t *__restrict__ counts, const int *run,
-                                                               uint32_t skip = 0) {
+                                                               uint32_t *__restrict__ counts, uint32_t skip) {
     __shared__ uint32_t s_warp[kCompactBlock / 32];
-    if (run && *run == 0) return;
     const size_t per = compact_per(g, gridDim.x);
     const size_t lo = static_cast<size_t>(blockIdx.x) * per, hi = min(g.nwords, lo + per);
     uint32_t c = 0;
@@ -139,11 +135,9 @@ __device__ __forceinline__ void write_step_entries(const uint32_t (&w)[4], uint3
 static __global__ void __launch_bounds__(kCompactBlock) k_write_list(uint32_t *__restrict__ bm, Geom g,
                                                               const uint32_t *__restrict__ counts,
                                                               uint32_t *__restrict__ list, uint32_t *total,
-                                                              const int *run, uint32_t wbase = 0,
-                                                              uint32_t skip = 0) {
+                                                              uint32_t wbase, uint32_t skip) {
     __shared__ uint32_t s_warp[kCompactBlock / 32];
     __shared__ __align__(16) unsigned char s_raw[kStageBytes];
-    if (run && *run == 0) return;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     uint32_t before = 0, all = 0;
     for (int b = t; b < static_cast<int>(gridDim.x); b += kCompactBlock) {
@@ -240,8 +234,7 @@ __device__ __forceinline__ void detect_outcome(const Geom &g, int x, int y, int 
 // array.  A voxel whose certificate fails (ties in the truncated proxies) is
 // buffered in shared memory and decided on full keys by the whole block after
 // its list loop, so the loop never runs a one-lane slow path; a full buffer
-// spills to a second list that k_detect_exact decides.  *deferred (or null)
-// counts the buffered and spilled voxels.
+// spills to a second list that k_detect_exact decides.
 constexpr uint32_t kExactCap = 2048;  // failed certificates buffered per block
 template <typename T>
 __global__ void __launch_bounds__(256, 5) k_detect_list(const uint32_t *__restrict__ list, const uint32_t *count,
@@ -249,15 +242,9 @@ __global__ void __launch_bounds__(256, 5) k_detect_list(const uint32_t *__restri
                                                      const uint32_t *__restrict__ hp, const uint8_t *__restrict__ codes,
                                                      uint32_t *__restrict__ req, uint32_t *__restrict__ act_next,
                                                      uint32_t *__restrict__ exact_list, uint32_t *exact_count,
-                                                     SweepSlot *slot, Geom g, FastDiv div_nx, const int *run,
-                                                     const int *exact_keys, uint32_t *deferred = nullptr) {
+                                                     SweepSlot *slot, Geom g, FastDiv div_nx) {
     __shared__ uint32_t s_exact[kExactCap];
     __shared__ uint32_t s_n;
-    if (run && *run == 0) return;
-    // fp32 with exact_keys set (k_pick_detection, k_loop_gate): the 4-byte keys
-    // of fhat, gathered as the proxies would be, decide every voxel (no
-    // certificates, nothing deferred)
-    const bool keys = sizeof(T) == 4 && exact_keys && *exact_keys;
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
     const uint32_t m = *count;
@@ -271,19 +258,6 @@ __global__ void __launch_bounds__(256, 5) k_detect_list(const uint32_t *__restri
         const uint32_t valid = interior ? kAllValid : valid_mask(x, y, z, g.nx, g.ny, g.nz);
         const uint8_t c = __ldg(codes + i);
         ++active;
-        if (keys) {
-            uint32_t kk[15];
-#pragma unroll
-            for (int r = 0; r < 15; ++r) {
-                const ptrdiff_t off = rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz;
-                kk[r] = ((valid >> r) & 1u) ? static_cast<uint32_t>(okey(__ldg(fh + (static_cast<ptrdiff_t>(i) + off))))
-                                            : 0u;
-            }
-            int asc, desc;
-            arg_ext(kk, valid, asc, desc);
-            detect_outcome(g, x, y, z, asc, desc, c, req, act_next, cmax, cmin, cdir);
-            continue;
-        }
         const uint32_t *c0 = hp + i;
         uint32_t t[15];
 #pragma unroll
@@ -301,8 +275,7 @@ __global__ void __launch_bounds__(256, 5) k_detect_list(const uint32_t *__restri
         }
     }
     __syncthreads();  // s_n is final
-    const uint32_t nd = s_n, nb = min(nd, kExactCap);
-    if (deferred && threadIdx.x == 0 && nd) atomicAdd(deferred, nd);
+    const uint32_t nb = min(s_n, kExactCap);
     // the buffered voxels on the 15 exact keys of fhat, one per thread; the
     // keys are scanned one at a time (rank order, arg_ext's rule) so that this
     // rare path adds no registers to the list loop
@@ -334,8 +307,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_detect_exact(const uint32_t *__restrict__ exact_list, const uint32_t *count,
                                                       const T *__restrict__ fh, const uint8_t *__restrict__ codes,
                                                       uint32_t *__restrict__ req, uint32_t *__restrict__ act_next,
-                                                      SweepSlot *slot, Geom g, FastDiv div_nx, const int *run) {
-    if (run && *run == 0) return;
+                                                      SweepSlot *slot, Geom g, FastDiv div_nx) {
     const uint32_t m = *count;
     uint32_t cmax = 0, cmin = 0, cdir = 0;
     const ptrdiff_t sy = g.nx, sz = static_cast<ptrdiff_t>(g.nx) * g.ny;
@@ -367,8 +339,7 @@ __global__ void __launch_bounds__(256) k_apply_list(const uint32_t *__restrict__
                                                     const T *__restrict__ f, T *__restrict__ fh,
                                                     uint8_t *__restrict__ cnt, uint32_t *__restrict__ hp,
                                                     uint32_t *__restrict__ act_next, SweepSlot *slot, Geom g,
-                                                    FastDiv div_nx, T eps, T delta, int q, const int *run) {
-    if (run && *run == 0) return;
+                                                    FastDiv div_nx, T eps, T delta, int q) {
     const uint32_t m = *count;
     uint32_t nreq = 0, nchg = 0, nprog = 0;
     const uint32_t lane = threadIdx.x & 31;
@@ -410,16 +381,9 @@ __global__ void __launch_bounds__(256) k_apply_list(const uint32_t *__restrict__
     block_flush_slot(slot, v);
 }
 
-// Bitmap -> list (k_count_words, k_write_list); counts: kCompactBlocks words of
-// scratch; *total receives the list length.  run (or null): the sweep's gate.
-inline void compact_bitmap(uint32_t *bm, const Geom &g, uint32_t *counts, uint32_t *list, uint32_t *total,
-                           const int *run, cudaStream_t s) {
-    k_count_words<<<kCompactBlocks, kCompactBlock, 0, s>>>(bm, g, counts, run);
-    k_write_list<<<kCompactBlocks, kCompactBlock, 0, s>>>(bm, g, counts, list, total, run);
-}
-
-// The same over the planes [z0, z1) of the bitmap (z0 < z1), with at most a
-// block per step of words (a z-range is often a small part of the bitmap).
+// The planes [z0, z1) of a bitmap -> list (k_count_words, k_write_list);
+// counts: kCompactBlocks words of scratch; *total receives the list length.  At
+// most a block per step of words (a z-range is often a small part of the bitmap).
 inline void compact_bitmap_planes(uint32_t *bm, const Geom &g, int z0, int z1, uint32_t *counts, uint32_t *list,
                                   uint32_t *total, cudaStream_t s) {
     const size_t wpp = static_cast<size_t>(g.wpr) * g.ny;  // words per plane
@@ -429,109 +393,37 @@ inline void compact_bitmap_planes(uint32_t *bm, const Geom &g, int z0, int z1, u
     const uint32_t skip = static_cast<uint32_t>(first - base);
     const unsigned blocks = static_cast<unsigned>(
         std::min<size_t>(kCompactBlocks, (r.nwords + kCompactWords - 1) / kCompactWords));
-    k_count_words<<<blocks, kCompactBlock, 0, s>>>(bm + base, r, counts, nullptr, skip);
-    k_write_list<<<blocks, kCompactBlock, 0, s>>>(bm + base, r, counts, list, total, nullptr,
-                                                   static_cast<uint32_t>(base), skip);
+    k_count_words<<<blocks, kCompactBlock, 0, s>>>(bm + base, r, counts, skip);
+    k_write_list<<<blocks, kCompactBlock, 0, s>>>(bm + base, r, counts, list, total, static_cast<uint32_t>(base), skip);
 }
 
-// State of the device-side sweep loop: the index of the sweep that runs
-// next, its gate, its list lengths and its counters (copied to the sweep's
-// slot by k_loop_gate).
+// State of the sweep loop (k_sweeps), ahead of the sweep slots in memory so
+// that one copy brings both to the host.
 struct LoopState {
-    long long k;
-    int go;
-    int tail;        // the loop stopped only because the next active set is small: the cooperative tail runs
-    int exact_keys;  // fp32 list detection on exact keys (k_pick_detection)
-    uint32_t lc[4];  // active list, request list, exact list (spills), first-pass deferrals
-    uint32_t deferred;  // voxels of the current list sweep decided on exact keys
-    uint32_t err;    // set by the first pass when a tensor copy did not arrive
-    SweepSlot cur;
+    long long k;          // the sweep it starts with (the host-buffer wavefront ran the ones before)
+    long long done;       // sweeps in all, once it ends
+    int go;               // that sweep runs
+    uint32_t lc[4];       // wavefront: active list, request list, spills; first-pass decisions on full keys
+    uint32_t deferred[2]; // voxels of a sweep decided on full keys, by the sweep's parity (fp32)
+    uint32_t err;         // set by the first pass when a tensor copy did not arrive
 };
 
-// Before the first list sweep (after sweep 0's edits): fp32 fields run the
-// list detection on exact keys when the first pass deferred more than a
-// tenth of the voxels (plateaus of quantised values: each such voxel would
-// be detected twice), or when the first list -- estimated as 15 * changed +
-// fdir of sweep 0 -- would defer, at the first pass's rate, more than half
-// of every detection block's buffer (a list of a billion voxels would
-// otherwise spill its deferrals through one global counter).  k_loop_gate
-// makes the first switch later when a list sweep defers more than a tenth.
-static __global__ void k_pick_detection(LoopState *ls, unsigned long long n, unsigned long long blocks) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const unsigned long long deferred = ls->lc[3];
-    const unsigned long long est = 15ull * ls->cur.changed + ls->cur.fdir;
-    const double spill = static_cast<double>(deferred) * static_cast<double>(est) / static_cast<double>(n);
-    if (10ull * deferred > n || spill > 0.5 * kExactCap * static_cast<double>(blocks)) ls->exact_keys = 1;
-}
-
-// After sweep ls->k: store its counters, decide whether the next sweep runs
-// (not converged, not stuck, no NaN input at sweep 0, sweeps left, and an
-// active set still too large for the cooperative tail: 15 * changed + fdir >
-// tail_at), advance k, clear the per-sweep state, and, in the loop body, set
-// the condition of the graph's while node.
-static __global__ void k_loop_gate(LoopState *ls, SweepSlot *slots, long long max_sweeps, unsigned long long tail_at,
-                            cudaGraphConditionalHandle cond, int set_cond) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (ls->go) {
-        const SweepSlot c = ls->cur;
-        const long long k = ls->k;
-        slots[k] = c;
-        // a list sweep that deferred more than a tenth of its voxels (failed
-        // certificates) switches the following ones to exact keys, for good
-        if (10ull * ls->deferred > ls->lc[0]) ls->exact_keys = 1;
-        const bool stop = (k == 0 && c.bad) || (c.fmax == 0 && c.fmin == 0 && c.fdir == 0) || c.progressed == 0 ||
-                          k + 1 >= max_sweeps;
-        const bool tail = 15ull * c.changed + c.fdir <= tail_at;
-        ls->go = (!stop && !tail) ? 1 : 0;
-        ls->tail = (!stop && tail) ? 1 : 0;
-        ls->k = k + 1;
-        ls->cur = SweepSlot{};
-        ls->lc[0] = ls->lc[1] = ls->lc[2] = ls->lc[3] = 0;
-        ls->deferred = 0;
-    }
-    if (set_cond) cudaGraphSetConditional(cond, ls->go ? 1u : 0u);
-}
-
-// The graph node ahead of the while node: the loop's first body runs only if
-// the gate before the graph let the next sweep run.
-static __global__ void k_loop_enter(const LoopState *ls, cudaGraphConditionalHandle cond) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) cudaGraphSetConditional(cond, ls->go ? 1u : 0u);
-}
-
-// After the host-buffer wavefront has run sweeps 0 .. K to the end: the loop
-// state that k_loop_gate would have left after sweep K, or after the first of
-// those sweeps that stops the loop (the sweeps after a stopping one changed
-// nothing: they found an empty active set, or repeated a sweep whose edits
-// changed no value and no counter, or follow a NaN input whose call fails),
-// and k_pick_detection's choice from sweep 0.
-static __global__ void k_wave_gate(LoopState *ls, const SweepSlot *slots, long long K, long long max_sweeps,
-                                   unsigned long long tail_at, unsigned long long n, unsigned long long blocks) {
+// After the host-buffer wavefront has run sweeps 0 .. K to the end: the state
+// after sweep K, or after the first of those sweeps that stops the loop (the
+// sweeps after a stopping one changed nothing: they found an empty active set,
+// or repeated a sweep whose edits changed no value and no counter, or follow a
+// NaN input whose call fails).
+static __global__ void k_wave_gate(LoopState *ls, const SweepSlot *slots, long long K, long long max_sweeps) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     long long k = 0;
     bool stop = false;
     for (; k <= K; ++k) {
         const SweepSlot c = slots[k];
-        stop = (k == 0 && c.bad) || (c.fmax == 0 && c.fmin == 0 && c.fdir == 0) || c.progressed == 0 ||
-               k + 1 >= max_sweeps;
+        stop = (k == 0 && c.bad) || sweep_stops(c.fmax, c.fmin, c.fdir, c.progressed, k + 1, max_sweeps);
         if (stop) break;
     }
-    if (stop) {
-        ls->k = k + 1;
-        ls->go = 0;
-        ls->tail = 0;
-    } else {
-        const SweepSlot c = slots[K];
-        ls->k = K + 1;
-        ls->go = 15ull * c.changed + c.fdir <= tail_at ? 0 : 1;
-        ls->tail = 1 - ls->go;
-    }
-    const unsigned long long deferred = ls->lc[3];
-    const unsigned long long est = 15ull * slots[0].changed + slots[0].fdir;
-    const double spill = static_cast<double>(deferred) * static_cast<double>(est) / static_cast<double>(n);
-    if (10ull * deferred > n || spill > 0.5 * kExactCap * static_cast<double>(blocks)) ls->exact_keys = 1;
-    ls->cur = SweepSlot{};
-    ls->lc[0] = ls->lc[1] = ls->lc[2] = ls->lc[3] = 0;
-    ls->deferred = 0;
+    ls->k = stop ? k + 1 : K + 1;
+    ls->go = stop ? 0 : 1;
 }
 
 }  // namespace pmsz

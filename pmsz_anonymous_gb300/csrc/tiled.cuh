@@ -309,17 +309,6 @@ struct DetectFlush {
     __device__ __forceinline__ void operator()(size_t w, uint32_t m) { act_next[w] = m; }
 };
 
-template <class L, typename T>
-__device__ __forceinline__ void sparse_detect_body(ListSmem &sm, const T *__restrict__ fh, const uint32_t *__restrict__ hp,
-                                                   const uint8_t *__restrict__ codes, uint32_t *__restrict__ act_cur,
-                                                   uint32_t *__restrict__ act_next, uint32_t *__restrict__ req,
-                                                   SweepSlot *slot, const Geom &g) {
-    DetectWork<L, T> work{fh, hp, codes, req, g};
-    DetectFlush flush{act_next};
-    for_each_set_bit<L>(sm, act_cur, g, work, flush);
-    work.flush_to(slot);
-}
-
 // ---------------------------------------------------------------------------
 // Apply with the proxy array: applyDeltaBuffer_local (pMSz.cu:623-645) on
 // every requested vertex, in T:
@@ -396,15 +385,6 @@ __device__ __forceinline__ void apply_body(ListSmem &sm, const T *__restrict__ f
     for_each_set_bit<L>(sm, req, g, work, flush);
     const uint32_t v[8] = {0u, 0u, 0u, work.nreq, flush.nchg, work.nprog, 0u, 0u};
     block_flush_slot(slot, v);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kListBlock, 3) k_sparse_px(const T *__restrict__ fh, const uint32_t *__restrict__ hp,
-                                                          const uint8_t *__restrict__ codes, uint32_t *__restrict__ act_cur,
-                                                          uint32_t *__restrict__ act_next, uint32_t *__restrict__ req,
-                                                          SweepSlot *slot, Geom g) {
-    __shared__ ListSmem sm;
-    sparse_detect_body<LdgLoads>(sm, fh, hp, codes, act_cur, act_next, req, slot, g);
 }
 
 template <typename T>
