@@ -10,45 +10,81 @@
 //  * A flag byte per GROUP of 8 bitmap words (plain stores of 1: no atomics)
 //    tells which groups hold anything, so a late sweep reads a byte per 256
 //    voxels.
-//  * Chunks of groups are dealt round-robin to all warps of the grid,
+//  * Chunks of groups are dealt round-robin to all threads of the grid,
 //    neighbouring chunks to different SMs, so a cluster of activity spreads over
-//    the chip.
-//  * A warp takes four flagged groups at a time, lists their set bits in shared
-//    memory (each lane the bits of its own word at its prefix), then visits them
-//    32 at a time: nearly full warps whatever the density, and no barrier wider
-//    than the warp.
+//    the chip.  A block lists its flagged groups in order and its warps take up
+//    to four of them at a time as they come free: the wait at the grid barrier
+//    was a quarter of the warps' time where each warp kept to its own chunks.
+//  * A warp lists the set bits of its four groups in shared memory (each lane
+//    the bits of its own word at its prefix) and visits them 32 at a time:
+//    nearly full warps whatever the density.
 //  * Loads are ordinary cached loads: a grid barrier orders them behind the
 //    other blocks' writes, and within a phase no array is both read at
 //    neighbours and written (detection reads proxies and codes and writes
 //    bitmaps, the edits touch their own voxel's values only), so the 15 gathers
 //    of neighbouring voxels share L1 lines.
-//  * Failed certificates collect in a per-warp buffer and are decided on full
-//    keys 32 at a time; fp32 fields with many (plateaus) detect on exact keys
+//  * Failed certificates wait in a per-warp buffer and are decided on full keys
+//    32 at a time; fp32 fields with many (plateaus) detect on full keys
 //    throughout.
+//  * Dense visits collect their result bits in shared memory (SweepBits).
 //
-// Bound by the latency of the gathers and, in small fields and late sweeps, of
-// the two grid barriers a sweep takes (about 2 us each).  Three blocks per SM:
-// with four (64 registers) fp64 detection is 2 % and dense fp32 sweeps on full
-// keys 5 % slower; blocks of 128 threads, five or six blocks per SM, groups of
-// 32 words and results merged in shared memory before the marks were all slower.
-// Whole corrections, list kernels in a conditional CUDA graph (before) -> this:
-//   64^3 fp32, 8 sweeps              358 -> 181 us
-//   173x141x203 fp32, 12 sweeps      560 -> 353 us
-//   512^3 fp64, 16 sparse sweeps    4134 -> 3654 us (first pass 1.50 -> 1.19 ms of it)
-//   256^3 fp32, 27 dense sweeps     4727 -> 4467 us (on full keys)
+// Bound by the latency of the gathers (issue slots 40 % used) and, in small
+// fields and late sweeps, of the two grid barriers a sweep takes (about 2 us
+// each).  Three blocks per SM: four (64 registers) are 0-10 % slower.  The code
+// is kept small and with one site per decision: with dense and sparse visits as
+// two copies the same work took 15-25 % longer.
+// Whole corrections: list kernels in a conditional CUDA graph -> warps on their
+// own chunks, every bit an atomic -> this:
+//   64^3 fp32, 8 sweeps              358 -> 181 -> 172 us
+//   173x141x203 fp32, 12 sweeps      560 -> 353 -> 335 us
+//   512^3 fp64, 16 sparse sweeps    3852 -> 3355 -> 3248 us
+//   256^3 fp32, 27 dense sweeps     4727 -> 4467 -> 3744 us (on full keys)
+//   160^3 fp64, 40 dense sweeps     2308 -> 2320 -> 2046 us
 #pragma once
 #include "list.cuh"
 
 namespace pmsz {
 
 constexpr int kSweepBlock = 256, kSweepWarps = kSweepBlock / 32;
-constexpr uint32_t kSweepDefer = 64;  // failed certificates buffered per warp (decided from 32 on)
 
 __host__ __device__ __forceinline__ size_t group_count(const Geom &g) {
     return (g.nwords + kGroupWords - 1) / kGroupWords;
 }
 
-// or_word / mark_stencil / request_targets that also set the group's flag.
+// The stencil's seven rows (dy, dz): (0,0) (1,0) (0,1) (1,1) (-1,0) (0,-1)
+// (-1,-1).  Row 0 holds dx = -1, 0, 1; rows 1-3 dx = 0, 1; rows 4-6 dx = -1, 0.
+constexpr int kSweepRows = 7;
+__host__ __device__ constexpr int step_row(int dy, int dz) {
+    return dy == 0 && dz == 0 ? 0 : (dy > 0 || dz > 0 ? 0 : 3) + (dy != 0 ? 1 : 0) + (dz != 0 ? 2 : 0);
+}
+__device__ __forceinline__ int row_dy(int row) { return row == 1 || row == 3 ? 1 : row == 4 || row == 6 ? -1 : 0; }
+__device__ __forceinline__ int row_dz(int row) { return row == 2 || row == 3 ? 1 : row == 5 || row == 6 ? -1 : 0; }
+__device__ __forceinline__ uint32_t row_words(const Geom &g, int row) {  // mod 2^32, as word indices are
+    return static_cast<uint32_t>(g.wpr) * (static_cast<uint32_t>(row_dy(row)) +
+                                           static_cast<uint32_t>(row_dz(row)) * static_cast<uint32_t>(g.ny));
+}
+// The target of a request by stencil rank (15 entries on 30 banks: no conflicts).
+struct SweepStep {
+    int dx;       // dx + 1 + 4 * row
+    uint32_t dw;  // row_words of the row
+};
+__device__ __forceinline__ void fill_steps(SweepStep *t, const Geom &g, int lane) {
+    if (lane < 15) {
+        const uint32_t r2 = 2u * static_cast<uint32_t>(lane);
+        const int row = step_row(static_cast<int>((kStepY >> r2) & 3u) - 1, static_cast<int>((kStepZ >> r2) & 3u) - 1);
+        t[lane] = {static_cast<int>((kStepX >> r2) & 3u) + 4 * row, row_words(g, row)};
+    }
+}
+
+// A warp's result bits for the 32 words it visits at a time: the words' own
+// (mismatches, changes) and the requests into their seven rows.  Collected
+// here they go out as one atomic per word instead of up to three per voxel
+// (L2 takes one atomic of an address at a time: 160^3 fp64, 40 dense sweeps,
+// 2393 us without, 2012 us with).
+struct SweepBits {
+    uint32_t own[32], row[kSweepRows][32];  // zero between visits
+};
+
 __device__ __forceinline__ void or_word_f(uint32_t *act, uint8_t *flag, const Geom &g, int wx, int y, int z, uint32_t m) {
     if (!m || wx < 0 || wx >= g.wpr || y < 0 || y >= g.ny || z < 0 || z >= g.nz) return;
     m &= row_tail_mask(g, wx);
@@ -72,44 +108,30 @@ __device__ __forceinline__ void mark_stencil_f(uint32_t *act, uint8_t *flag, con
     or_word_f(act, flag, g, wx, y - 1, z - 1, p); or_word_f(act, flag, g, wx + 1, y - 1, z - 1, hi);
 }
 
-// The same for the lanes of a warp that each hold a word's merged changed bits
-// (lead: this lane does; every lane calls it).  Few words -- runs of changed
-// voxels, as in dense sweeps -- take one word after the other, its 14 marks on
-// 14 lanes: 40 instructions a word, where one lane's 14 marks in a row are 350.
-__device__ __forceinline__ void mark_stencils(uint32_t *act, uint8_t *flag, const Geom &g, bool lead, int wx, int y, int z,
-                                              uint32_t c) {
-    uint32_t m = __ballot_sync(0xFFFFFFFFu, lead);
+// Marks the closed stencils of the changed bits c of the lanes' words (every
+// lane calls it).  Many words: each lane's own marks one after the other, 350
+// instructions for up to 32 words.  Few -- runs of changed voxels, as in dense
+// sweeps: one word after the other, its marks on 15 lanes, 40 instructions each.
+__device__ __forceinline__ void mark_stencils(uint32_t *act, uint8_t *flag, const Geom &g, int wx, int y, int z, uint32_t c) {
+    uint32_t m = __ballot_sync(0xFFFFFFFFu, c != 0);
     if (__popc(m) > 4) {
-        if (lead) mark_stencil_f(act, flag, g, wx, y, z, c);
+        if (c) mark_stencil_f(act, flag, g, wx, y, z, c);
         return;
     }
-    // lane l < 14: the row (dy, dz) of l / 2, and its own word (even) or the
-    // neighbouring one that the row's shifted bits reach (odd)
-    const int lane = threadIdx.x & 31, row = lane >> 1;
-    const int dy = row == 1 || row == 3 ? 1 : row == 4 || row == 6 ? -1 : 0;
-    const int dz = row == 2 || row == 3 ? 1 : row == 5 || row == 6 ? -1 : 0;
-    // rows 1-3 take x-1, x; rows 4-6 take x, x+1; row 0 takes all three (its
-    // second neighbour word is lane 14's)
-    const bool left = row == 0 || (row >= 1 && row <= 3), right = row == 0 || (row >= 4 && row <= 6) || lane == 14;
+    // lane l < 14: row l / 2, and its own word (even) or the neighbouring one
+    // that the row's shifted bits reach (odd); row 0's second one is lane 14's
+    const int lane = threadIdx.x & 31, row = lane == 14 ? 0 : lane >> 1;
+    const int dy = row_dy(row), dz = row_dz(row);
+    const bool left = row <= 3 && lane != 14, right = row == 0 || row >= 4;
     for (; m; m &= m - 1) {
         const int src = __ffs(m) - 1;
         const uint32_t cb = __shfl_sync(0xFFFFFFFFu, c, src);
         const int bx = __shfl_sync(0xFFFFFFFFu, wx, src), by = __shfl_sync(0xFFFFFFFFu, y, src),
                   bz = __shfl_sync(0xFFFFFFFFu, z, src);
         if (lane < 15) {
-            const uint32_t lo = (cb & 1u) << 31, hi = cb >> 31;
-            uint32_t bits;
-            int ox = 0;
-            if (lane == 14) {
-                bits = hi;
-                ox = 1;
-            } else if (lane & 1) {
-                bits = left ? lo : hi;
-                ox = left ? -1 : 1;
-            } else {
-                bits = cb | (left ? cb >> 1 : 0u) | (right ? cb << 1 : 0u);
-            }
-            or_word_f(act, flag, g, bx + ox, lane == 14 ? by : by + dy, lane == 14 ? bz : bz + dz, bits);
+            const bool side = lane == 14 || (lane & 1);
+            const uint32_t bits = side ? (left ? cb << 31 : cb >> 31) : cb | (left ? cb >> 1 : 0u) | (right ? cb << 1 : 0u);
+            or_word_f(act, flag, g, bx + (side ? (left ? -1 : 1) : 0), by + dy, bz + dz, bits);
         }
     }
 }
@@ -147,26 +169,337 @@ struct SweepArgs {
 };
 
 struct SweepSmem {
-    uint32_t group[kSweepWarps][256];     // flagged groups to visit
+    uint16_t group[kSweepBlock * 8];      // flagged groups to visit: thread of the chunk * 8 + group in it
+    uint32_t groups[kSweepWarps], next;   // listed by each warp, taken
     uint16_t list[kSweepWarps][1024];     // lane of the word << 5 | bit of four groups' set bits
     int4 at[kSweepWarps][32];             // x of bit 0, y, z of their words, and the word
-    uint2 defer[kSweepWarps][kSweepDefer];  // word, bit
+    SweepBits bits[kSweepWarps];
+    uint2 defer[kSweepWarps][64];         // word, bit
     uint32_t deferred;
+    SweepStep step[15];
 };
 
-// Calls visit(active, word, bit, x, y, z) for the set bits of every flagged
-// group of this warp, whole warps at a time (active: the lane has a voxel),
-// clearing bits and flags.  Chunks of `chunk` neighbouring groups are dealt to
-// the warps in turn: eight (2048 voxels, whose stencils share cache lines) where
-// the field has enough of them for every warp, fewer in small fields.
+// One voxel of a sweep, for A = SweepArgs<T> or Inst<T> (batch.h): the two hold
+// a field's pointers and parameters under the same names.
+//
+// Detection's outcome from the two ranks: detect_rules as two targets, so that
+// the lanes of a warp stay together (as a loop over the requested ranks this
+// was half of a dense sweep's instructions); the requests and the voxel's
+// mismatch bit of the next active set.
+template <class A>
+__device__ __forceinline__ void sweep_outcome(const A &a, const SweepStep *steps, SweepBits &bits, bool collect, uint32_t *nxt,
+                                              uint8_t *fnxt, uint32_t entry, uint32_t w, int asc, int desc, uint8_t c,
+                                              uint32_t &cmax, uint32_t &cmin, uint32_t &cdir) {
+    if ((asc | (desc << 4)) == static_cast<int>(c) && asc != desc) return;  // (a lone voxel is both: never settled)
+    const int oasc = c & 15, odesc = c >> 4;
+    const bool omax = oasc == kSelf, omin = !omax && odesc == kSelf;
+    const bool r1 = (asc == kSelf) != omax, r2 = (desc == kSelf) != omin, r = r1 || r2;
+    const bool v1 = r ? r1 : asc != oasc, v2 = r ? r2 : desc != odesc;
+    if (!v1 && !v2) return;
+    const uint32_t slot = entry >> 5;
+    const int bit = static_cast<int>(entry & 31u);
+    cmax += r1;
+    cmin += r2;
+    cdir += r ? 1u : static_cast<uint32_t>(v1) + static_cast<uint32_t>(v2);
+    if (collect) {
+        atomicOr(&bits.own[slot], 1u << bit);
+    } else {
+        atomicOr(nxt + w, 1u << bit);
+        fnxt[w / kGroupWords] = 1;
+    }
+    auto request = [&](int rank) {
+        const SweepStep st = steps[rank];
+        const int tx = bit + (st.dx & 3) - 1;
+        if (collect && static_cast<uint32_t>(tx) < 32u) {
+            atomicOr(&bits.row[st.dx >> 2][slot], 1u << tx);
+        } else {
+            const uint32_t wt = w + st.dw + static_cast<uint32_t>(tx >> 5);
+            atomicOr(a.req + wt, 1u << (tx & 31));
+            a.freq[wt / kGroupWords] = 1;
+        }
+    };
+    if (v1) request(r1 && !omax ? kSelf : asc);
+    if (v2) request(r2 && omin ? kSelf : odesc);
+}
+
+// The ranks on full keys (interior: of a warp whose voxels all are; fp32).
+template <typename T, class A>
+__device__ __forceinline__ void sweep_keys(const A &a, size_t i, int x, int y, int z, bool interior, int &asc, int &desc) {
+    const T *c0 = a.fh + i;
+    const ptrdiff_t sy = a.g.nx, sz = static_cast<ptrdiff_t>(a.g.nx) * a.g.ny;
+    asc = kSelf;
+    desc = kSelf;
+    if constexpr (sizeof(T) == 4) {
+        // The values themselves order fp32 fields (-0 and +0 are equal, a field
+        // with NaN ends before its first sweep): the extremes by max and min,
+        // NaN standing for a point outside the domain, then the last rank that
+        // holds the maximum and the first that holds the minimum.
+        T v[15];
+        if (interior) {
+#pragma unroll
+            for (int r = 0; r < 15; ++r) v[r] = c0[rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz];
+        } else {
+            const uint32_t valid = valid_mask(x, y, z, a.g.nx, a.g.ny, a.g.nz);
+#pragma unroll
+            for (int r = 0; r < 15; ++r)
+                v[r] = ((valid >> r) & 1u) ? c0[rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz] : __int_as_float(0x7FC00000);
+        }
+        T hi = v[0], lo = v[0];
+#pragma unroll
+        for (int r = 1; r < 15; r += 2) {
+            hi = fmaxf(fmaxf(hi, v[r]), v[r + 1]);
+            lo = fminf(fminf(lo, v[r]), v[r + 1]);
+        }
+#pragma unroll
+        for (int r = 0; r < 15; ++r) {
+            if (v[r] == hi) asc = r;
+            if (v[14 - r] == lo) desc = 14 - r;
+        }
+        return;
+    }
+    using K = typename KeyOf<T>::type;
+    constexpr int kKeyLoads = 5;  // in flight (fp64 keys are two registers each)
+    K hi = 0, lo = ~K(0);
+    const uint32_t valid = valid_mask(x, y, z, a.g.nx, a.g.ny, a.g.nz);
+#pragma unroll
+    for (int r0 = 0; r0 < 15; r0 += kKeyLoads) {
+        K kk[kKeyLoads];
+#pragma unroll
+        for (int j = 0; j < kKeyLoads; ++j) {
+            const int r = r0 + j;
+            kk[j] = ((valid >> r) & 1u) ? okey(c0[rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz]) : K(0);
+        }
+#pragma unroll
+        for (int j = 0; j < kKeyLoads; ++j)
+            if ((valid >> (r0 + j)) & 1u) {
+                if (kk[j] >= hi) { hi = kk[j]; asc = r0 + j; }
+                if (kk[j] < lo) { lo = kk[j]; desc = r0 + j; }
+            }
+    }
+}
+// The ranks on the proxies, with their certificate: of a warp whose voxels are
+// all interior (nearly every one: no test per gather), or not.
+template <class A>
+__device__ __forceinline__ Ext sweep_proxies(const A &a, size_t i) {
+    const uint32_t *c0 = a.hp + i;
+    const ptrdiff_t sy = a.g.nx, sz = static_cast<ptrdiff_t>(a.g.nx) * a.g.ny;
+    uint32_t t[15];
+#pragma unroll
+    for (int r = 0; r < 15; ++r) t[r] = c0[rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz];
+    return proxy_ext_interior<true>(t);
+}
+template <class A>
+__device__ __forceinline__ Ext sweep_proxies_face(const A &a, size_t i, int x, int y, int z) {
+    const uint32_t *c0 = a.hp + i;
+    const ptrdiff_t sy = a.g.nx, sz = static_cast<ptrdiff_t>(a.g.nx) * a.g.ny;
+    uint32_t t[15];
+    const uint32_t valid = valid_mask(x, y, z, a.g.nx, a.g.ny, a.g.nz);
+#pragma unroll
+    for (int r = 0; r < 15; ++r) t[r] = ((valid >> r) & 1u) ? c0[rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz] : 0u;
+    return proxy_ext<true>(t);
+}
+__device__ __forceinline__ bool sweep_interior(const Geom &g, int x, int y, int z) {
+    return x >= 1 && x <= g.nx - 2 && y >= 1 && y <= g.ny - 2 && z >= 1 && z <= g.nz - 2;
+}
+// The edit of one requested voxel (applyDeltaBuffer_local); true if its value changed.
+template <typename T, class A>
+__device__ __forceinline__ bool sweep_edit(const A &a, size_t v, uint32_t &nreq, uint32_t &nchg, uint32_t &nprog) {
+    const T old = a.fh[v];
+    const uint8_t oc = a.cnt[v];
+    const T fv = __ldg(a.f + v);
+    const T lowered = old - a.delta;
+    T nv;
+    uint8_t nc;
+    if (fabs(fv - lowered) <= a.eps && static_cast<int>(oc) < a.q - 1) {
+        nv = lowered;
+        nc = static_cast<uint8_t>(oc + 1);
+    } else {
+        nc = static_cast<uint8_t>(a.q);
+        nv = fv - a.eps;
+    }
+    a.fh[v] = nv;
+    a.cnt[v] = nc;
+    const bool chg = bits_of(old) != bits_of(nv);
+    ++nreq;
+    nprog += (chg || nc != oc) ? 1u : 0u;
+    if (chg) {
+        ++nchg;
+        a.hp[v] = proxy_of(nv);
+    }
+    return chg;
+}
+
+// A list entry's voxel.
+struct SweepVoxel {
+    bool on;
+    uint32_t entry, w;
+    int x, y, z;
+};
+__device__ __forceinline__ SweepVoxel sweep_voxel(const SweepSmem &sm, uint32_t j, uint32_t total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    SweepVoxel v;
+    v.on = j + lane < total;
+    v.entry = v.on ? sm.list[warp][j + lane] : 0u;
+    const int4 at = sm.at[warp][v.entry >> 5];
+    v.w = static_cast<uint32_t>(at.w);
+    v.x = at.x + static_cast<int>(v.entry & 31u);
+    v.y = at.y;
+    v.z = at.z;
+    return v;
+}
+
+// Four groups with this many set bits (of 1024) collect their result bits in
+// shared memory: below, sending the few that are left out one by one costs less
+// than the eight words per lane (from 64 on 160^3 fp64 takes 1949 us, from 192
+// on 2027 us; sparse fields are the same).
+constexpr uint32_t kSweepDense = 64;
+
+// Detection of the `total` listed voxels of a warp's 32 words (lane l holds
+// word w): on the proxies, failed certificates into the warp's buffer (ndefer
+// entries), or (keys) on full keys throughout.  The buffer is decided on full
+// keys 32 at a time, in the same place; `finish`: to the end.  v: fmax, fmin,
+// fdir, active; ndeferred += this lane's failed certificates.
+template <typename T, class A>
+__device__ __forceinline__ void detect_words(SweepSmem &sm, const A &a, const SweepStep *steps, uint32_t *nxt, uint8_t *fnxt,
+                                             uint32_t total, uint32_t w, bool keys, bool finish, uint32_t (&v)[4],
+                                             uint32_t &ndefer, uint32_t &ndeferred) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    SweepBits &bits = sm.bits[warp];
+    const bool dense = total >= kSweepDense;
+    v[3] += lane == 0 ? total : 0u;
+    for (uint32_t j = 0;;) {
+        const bool buffered = ndefer >= 32 || (finish && ndefer && j >= total);
+        if (!buffered && j >= total) break;
+        if (!buffered && !keys) {
+            const SweepVoxel p = sweep_voxel(sm, j, total);
+            const bool inside = p.on && sweep_interior(a.g, p.x, p.y, p.z);
+            bool open = p.on;
+            const bool all_inside = __all_sync(0xFFFFFFFFu, inside || !p.on);
+            if (p.on) {
+                const size_t i = flat(a.g, p.x, p.y, p.z);
+                const uint8_t c = __ldg(a.codes + i);
+                const Ext e = all_inside ? sweep_proxies(a, i) : sweep_proxies_face(a, i, p.x, p.y, p.z);
+                open = !e.exact;
+                if (!open)
+                    sweep_outcome(a, steps, bits, dense, nxt, fnxt, p.entry, p.w, e.asc, e.desc, c, v[0], v[1], v[2]);
+            }
+            const uint32_t md = __ballot_sync(0xFFFFFFFFu, open);
+            if (md) {
+                if (open)
+                    sm.defer[warp][ndefer + static_cast<uint32_t>(__popc(md & ((1u << lane) - 1u)))] =
+                        make_uint2(p.w, p.entry & 31u);
+                ndefer += static_cast<uint32_t>(__popc(md));
+                ndeferred += open;
+            }
+            j += 32;
+            continue;
+        }
+        SweepVoxel p;
+        if (buffered) {
+            __syncwarp();
+            const uint32_t from = ndefer > 32 ? ndefer - 32 : 0;
+            p.on = from + lane < ndefer;
+            const uint2 e = p.on ? sm.defer[warp][from + lane] : make_uint2(0u, 0u);
+            int wx;
+            word_coords(a.g, e.x, wx, p.y, p.z);
+            p.w = e.x;
+            p.entry = e.y;
+            p.x = wx * 32 + static_cast<int>(e.y);
+            ndefer = from;
+            __syncwarp();
+        } else {
+            p = sweep_voxel(sm, j, total);
+            j += 32;
+        }
+        const bool inside = __all_sync(0xFFFFFFFFu, !p.on || sweep_interior(a.g, p.x, p.y, p.z));
+        if (p.on) {
+            const size_t i = flat(a.g, p.x, p.y, p.z);
+            int asc, desc;
+            sweep_keys<T>(a, i, p.x, p.y, p.z, inside, asc, desc);
+            sweep_outcome(a, steps, bits, dense && !buffered, nxt, fnxt, p.entry, p.w, asc, desc, __ldg(a.codes + i), v[0],
+                          v[1], v[2]);
+        }
+    }
+    if (!dense) return;
+    __syncwarp();
+    const uint32_t own = bits.own[lane];
+    if (own) {
+        bits.own[lane] = 0;
+        atomicOr(nxt + w, own);
+        fnxt[w / kGroupWords] = 1;
+    }
+#pragma unroll
+    for (int r = 0; r < kSweepRows; ++r) {
+        const uint32_t m = bits.row[r][lane];
+        if (m) {
+            bits.row[r][lane] = 0;
+            const uint32_t wt = w + row_words(a.g, r);
+            atomicOr(a.req + wt, m);
+            a.freq[wt / kGroupWords] = 1;
+        }
+    }
+}
+
+// The edits of the listed voxels, and the closed stencils of those whose value
+// changed.  v: requested, changed, progressed.
+template <typename T, class A>
+__device__ __forceinline__ void edit_words(SweepSmem &sm, const A &a, uint32_t *nxt, uint8_t *fnxt, uint32_t total,
+                                           uint32_t (&v)[4]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint32_t j = 0; j < total; j += 32) {
+        const SweepVoxel p = sweep_voxel(sm, j, total);
+        uint32_t cb = 0;
+        if (p.on && sweep_edit<T>(a, flat(a.g, p.x, p.y, p.z), v[0], v[1], v[2])) cb = 1u << (p.entry & 31u);
+        const bool lead = warp_merge_word(p.on ? p.w : 0xFFFFFFFFu, cb);
+        mark_stencils(nxt, fnxt, a.g, p.x >> 5, p.y, p.z, lead ? cb : 0u);
+    }
+}
+
+__device__ __forceinline__ void clear_bits(SweepBits &b) {
+    const int lane = threadIdx.x & 31;
+    b.own[lane] = 0;
+    for (int r = 0; r < kSweepRows; ++r) b.row[r][lane] = 0;
+    __syncwarp();
+}
+
+// The set bits of this lane's word as entries of the warp's list, in order;
+// their coordinates into at.  Returns the warp's count.
+__device__ __forceinline__ uint32_t list_words(SweepSmem &sm, const Geom &g, uint64_t w, uint32_t word) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (word) {
+        int wx, y, z;
+        word_coords(g, w, wx, y, z);
+        sm.at[warp][lane] = make_int4(wx << 5, y, z, static_cast<int>(static_cast<uint32_t>(w)));
+    }
+    const uint32_t c = static_cast<uint32_t>(__popc(word));
+    uint32_t inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    for (uint32_t p = inc - c; word; word &= word - 1, ++p)
+        sm.list[warp][p] = static_cast<uint16_t>((lane << 5) | (__ffs(word) - 1));
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, inc, 31);
+    __syncwarp();
+    return total;
+}
+
+// Calls visit(total, word, last) on the listed set bits of every flagged group
+// of this block, up to four groups at a time (lane l holds word l), clearing
+// bits and flags; last: this warp's last call.  Chunks of `chunk` neighbouring
+// groups are dealt to the warps of the grid in turn: eight (2048 voxels, whose
+// stencils share cache lines) where the field has enough of them for every
+// thread, fewer in small fields.  The flagged groups of a block's chunks are
+// listed in order (blocks then move through the field together, and share its
+// cache lines), and its warps take them from the list as they come free.
 template <class Visit>
 __device__ __forceinline__ void for_each_group(SweepSmem &sm, uint32_t *bm, uint8_t *flag, const Geom &g, uint32_t chunk,
                                                Visit &&visit) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t W = gridDim.x * kSweepWarps, wid = static_cast<uint32_t>(warp) * gridDim.x + blockIdx.x;
     const uint64_t ng = group_count(g), nc = (ng + chunk - 1) / chunk;
-    for (uint64_t base = 0; base < nc; base += 32ull * W) {
-        const uint64_t mine = (base + static_cast<uint64_t>(lane) * W + wid) * chunk;  // this lane's chunk
+    for (uint64_t base = 0; base < nc; base += static_cast<uint64_t>(kSweepBlock) * gridDim.x) {
+        const uint64_t mine = (base + static_cast<uint64_t>(threadIdx.x) * gridDim.x + blockIdx.x) * chunk;  // this thread's chunk
         uint32_t fm = 0;
         if (mine < ng) {  // (the flags are padded to 256 bytes and start at a multiple of the chunk)
             if (chunk == 8) {
@@ -188,48 +521,46 @@ __device__ __forceinline__ void for_each_group(SweepSmem &sm, uint32_t *bm, uint
             const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
             if (lane >= o) inc += v;
         }
-        const uint32_t groups = __shfl_sync(0xFFFFFFFFu, inc, 31);
-        if (!groups) continue;
-        for (uint32_t p = inc - c; fm; fm &= fm - 1, ++p)
-            sm.group[warp][p] = static_cast<uint32_t>(mine) + static_cast<uint32_t>(__ffs(fm) - 1);
-        __syncwarp();
-        auto word_at = [&](uint32_t t) -> uint64_t {  // this lane's word of the four groups from t on
-            return t + (lane >> 3) < groups ? static_cast<uint64_t>(sm.group[warp][t + (lane >> 3)]) * kGroupWords + (lane & 7)
-                                            : ~0ull;
-        };
-        uint64_t w = word_at(0);
-        uint32_t word = w < g.nwords ? bm[w] : 0u;
-        for (uint32_t t = 0; t < groups; t += 4) {
-            const uint64_t w_next = word_at(t + 4);
-            const uint32_t next = w_next < g.nwords ? bm[w_next] : 0u;  // in flight while these groups are visited
-            if (word) {
-                bm[w] = 0;
-                int wx, y, z;
-                word_coords(g, w, wx, y, z);
-                sm.at[warp][lane] = make_int4(wx << 5, y, z, static_cast<int>(static_cast<uint32_t>(w)));
-            }
-            const uint32_t cw = static_cast<uint32_t>(__popc(word));
-            uint32_t iw = cw;
+        if (lane == 31) sm.groups[warp] = inc;
+        if (threadIdx.x == 0) sm.next = 0;
+        __syncthreads();
+        uint32_t first = inc - c, groups = 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, iw, o);
-                if (lane >= o) iw += v;
+        for (int k = 0; k < kSweepWarps; ++k) {
+            const uint32_t n = sm.groups[k];
+            first += k < warp ? n : 0u;
+            groups += n;
+        }
+        for (; fm; fm &= fm - 1, ++first) sm.group[first] = static_cast<uint16_t>(threadIdx.x * 8 + __ffs(fm) - 1);
+        __syncthreads();
+        // as few rounds of up to four as it takes, then as evenly as they come
+        const uint32_t rounds = (groups + 4 * kSweepWarps - 1) / (4 * kSweepWarps);
+        const uint32_t take = groups ? (groups + kSweepWarps * rounds - 1) / (kSweepWarps * rounds) : 1u;
+        auto next_words = [&](uint64_t &w) -> uint32_t {  // this lane's word of the next groups (none: w = ~0 in every lane)
+            uint32_t t = lane == 0 ? atomicAdd(&sm.next, take) : 0u;
+            t = __shfl_sync(0xFFFFFFFFu, t, 0);
+            w = ~0ull;
+            const uint32_t i = lane >> 3;
+            if (i < take && t + i < groups) {
+                const uint32_t e = sm.group[t + i];
+                w = ((base + static_cast<uint64_t>(e >> 3) * gridDim.x + blockIdx.x) * chunk + (e & 7u)) *
+                        kGroupWords + (lane & 7);
             }
-            const uint32_t total = __shfl_sync(0xFFFFFFFFu, iw, 31);
-            for (uint32_t p = iw - cw; word; word &= word - 1, ++p)
-                sm.list[warp][p] = static_cast<uint16_t>((lane << 5) | (__ffs(word) - 1));
-            __syncwarp();
-            for (uint32_t j = 0; j < total; j += 32) {
-                const bool on = j + lane < total;
-                const uint32_t e = on ? sm.list[warp][j + lane] : 0u;
-                const int4 at = on ? sm.at[warp][e >> 5] : make_int4(0, 0, 0, 0);
-                visit(on, static_cast<uint32_t>(at.w), static_cast<int>(e & 31u), at.x + static_cast<int>(e & 31u), at.y,
-                      at.z);
-            }
+            return w < g.nwords ? bm[w] : 0u;
+        };
+        uint64_t w;
+        uint32_t word = next_words(w);
+        while (__shfl_sync(0xFFFFFFFFu, w, 0) != ~0ull) {
+            uint64_t w_next;
+            const uint32_t next = next_words(w_next);  // in flight while these groups are visited
+            if (word) bm[w] = 0;
+            const uint32_t total = list_words(sm, g, w, word);
+            visit(total, static_cast<uint32_t>(w), __shfl_sync(0xFFFFFFFFu, w_next, 0) == ~0ull);
             __syncwarp();  // list and at are rewritten by the next groups
             w = w_next;
             word = next;
         }
+        __syncthreads();  // group, groups and next are rewritten by the next chunks
     }
 }
 
@@ -239,9 +570,11 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps(const __grid_constant
     cg::grid_group grid = cg::this_grid();
     const Geom &g = a.g;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const ptrdiff_t sy = g.nx, sz = static_cast<ptrdiff_t>(g.nx) * g.ny;
     uint32_t chunk = 8;
-    while (chunk > 1 && group_count(g) < static_cast<uint64_t>(chunk) * 8u * gridDim.x * kSweepWarps) chunk >>= 1;
+    while (chunk > 1 && group_count(g) < static_cast<uint64_t>(chunk) * gridDim.x * kSweepWarps) chunk >>= 1;
+    if (warp == 0) fill_steps(sm.step, g, lane);
+    clear_bits(sm.bits[warp]);
+    __syncthreads();
     int64_t k = 0;
     bool edits_only = a.from_edits != 0;
     if (!edits_only) {  // every block reads the same state: all return, or none
@@ -260,116 +593,15 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps(const __grid_constant
         if (!edits_only) {
             const SweepSlot *p = a.slots + (k - 1);
             if (sweep_stops(p->fmax, p->fmin, p->fdir, p->progressed, k, a.max_sweeps) || (k == 1 && p->bad)) break;
-            uint32_t cmax = 0, cmin = 0, cdir = 0, active = 0, ndefer = 0, ndeferred = 0;
+            uint32_t c[4] = {0u, 0u, 0u, 0u}, ndefer = 0, ndeferred = 0;
             if (threadIdx.x == 0) sm.deferred = 0;
-            auto outcome = [&](uint32_t w, int bit, int x, int y, int z, int asc, int desc, uint8_t c) {
-                uint32_t tm = detect_rules(asc, desc, c & 15, c >> 4, cmax, cmin, cdir);
-                if (!tm) return;
-                atomicOr(nxt + w, 1u << bit);
-                fnxt[w / kGroupWords] = 1;
-                for (; tm; tm &= tm - 1) {
-                    const uint32_t r2 = 2u * static_cast<uint32_t>(__ffs(tm) - 1);
-                    const int tx = x + static_cast<int>((kStepX >> r2) & 3u) - 1,
-                              ty = y + static_cast<int>((kStepY >> r2) & 3u) - 1,
-                              tz = z + static_cast<int>((kStepZ >> r2) & 3u) - 1;
-                    const size_t wt = word_of(g, tx, ty, tz);
-                    atomicOr(a.req + wt, 1u << (tx & 31));
-                    a.freq[wt / kGroupWords] = 1;
-                }
-            };
-            // Full keys of one voxel (interior: of a warp whose voxels all are).
-            auto on_keys = [&](uint32_t w, int bit, int x, int y, int z, bool interior) {
-                const size_t i = flat(g, x, y, z);
-                const T *c0 = a.fh + i;
-                using K = typename KeyOf<T>::type;
-                constexpr int kKeyLoads = 5;  // in flight (fp64 keys are two registers each; fp32 is no faster with 15)
-                K hi = 0, lo = ~K(0);
-                int asc = kSelf, desc = kSelf;
-                auto scan = [&](auto test) {
-#pragma unroll
-                    for (int r0 = 0; r0 < 15; r0 += kKeyLoads) {
-                        K kk[kKeyLoads];
-#pragma unroll
-                        for (int j = 0; j < kKeyLoads; ++j) {
-                            const int r = r0 + j;
-                            kk[j] = test(r) ? okey(c0[rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz]) : K(0);
-                        }
-#pragma unroll
-                        for (int j = 0; j < kKeyLoads; ++j)
-                            if (test(r0 + j)) {
-                                if (kk[j] >= hi) { hi = kk[j]; asc = r0 + j; }
-                                if (kk[j] < lo) { lo = kk[j]; desc = r0 + j; }
-                            }
-                    }
-                };
-                if (interior) {
-                    scan([](int) { return true; });
-                } else {
-                    const uint32_t valid = valid_mask(x, y, z, g.nx, g.ny, g.nz);
-                    scan([&](int r) { return ((valid >> r) & 1u) != 0; });
-                }
-                outcome(w, bit, x, y, z, asc, desc, __ldg(a.codes + i));
-            };
-            auto drain = [&](uint32_t from, uint32_t to) {  // buffered voxels, one per lane
-                __syncwarp();
-                if (from + lane < to) {
-                    const uint2 e = sm.defer[warp][from + lane];
-                    int wx, y, z;
-                    word_coords(g, e.x, wx, y, z);
-                    on_keys(e.x, static_cast<int>(e.y), wx * 32 + static_cast<int>(e.y), y, z, false);
-                }
-                __syncwarp();
-            };
-            for_each_group(sm, cur, fcur, g, chunk, [&](bool on, uint32_t w, int bit, int x, int y, int z) {
-                bool exact = true;
-                // nearly every warp has only interior voxels: no test per gather
-                const bool inside = x >= 1 && x <= g.nx - 2 && y >= 1 && y <= g.ny - 2 && z >= 1 && z <= g.nz - 2;
-                const bool all_inside = __all_sync(0xFFFFFFFFu, inside || !on);
-                if (on) {
-                    ++active;
-                    if (keys) {
-                        on_keys(w, bit, x, y, z, sizeof(T) == 4 && all_inside);
-                    } else {
-                        const size_t i = flat(g, x, y, z);
-                        const uint8_t c = __ldg(a.codes + i);
-                        const uint32_t *c0 = a.hp + i;
-                        uint32_t t[15];
-                        Ext e;
-                        if (all_inside) {
-#pragma unroll
-                            for (int r = 0; r < 15; ++r)
-                                t[r] = c0[rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz];
-                            e = proxy_ext_interior<true>(t);
-                        } else {
-                            const uint32_t valid = valid_mask(x, y, z, g.nx, g.ny, g.nz);
-#pragma unroll
-                            for (int r = 0; r < 15; ++r)
-                                t[r] = ((valid >> r) & 1u) ? c0[rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz] : 0u;
-                            e = proxy_ext<true>(t);
-                        }
-                        exact = e.exact;
-                        if (exact) outcome(w, bit, x, y, z, e.asc, e.desc, c);
-                    }
-                }
-                const uint32_t md = __ballot_sync(0xFFFFFFFFu, !exact);
-                if (md) {
-                    if (!exact)
-                        sm.defer[warp][ndefer + static_cast<uint32_t>(__popc(md & ((1u << lane) - 1u)))] =
-                            make_uint2(static_cast<uint32_t>(w), static_cast<uint32_t>(bit));
-                    ndefer += static_cast<uint32_t>(__popc(md));
-                    ndeferred += static_cast<uint32_t>(__popc(md));
-                    if (ndefer > kSweepDefer - 32) {
-                        drain(ndefer - 32, ndefer);
-                        ndefer -= 32;
-                    }
-                }
+            for_each_group(sm, cur, fcur, g, chunk, [&](uint32_t total, uint32_t w, bool last) {
+                detect_words<T>(sm, a, sm.step, nxt, fnxt, total, w, keys, last, c, ndefer, ndeferred);
             });
-            drain(0, min(ndefer, 32u));
-            if (ndefer > 32) drain(32, ndefer);
-            const uint32_t v[8] = {cmax, cmin, cdir, 0u, 0u, 0u, active, 0u};
+            const uint32_t v[8] = {c[0], c[1], c[2], 0u, 0u, 0u, c[3], 0u};
             block_flush_slot(a.slots + k, v);  // (contains a barrier: sm.deferred is zero before)
             if (sizeof(T) == 4) {
-                if (lane == 0 && ndeferred) atomicAdd(&sm.deferred, ndeferred);
+                if (ndeferred) atomicAdd(&sm.deferred, ndeferred);
                 __syncthreads();
                 if (threadIdx.x == 0 && sm.deferred) atomicAdd(&a.ls->deferred[k & 1], sm.deferred);
             }
@@ -381,39 +613,10 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps(const __grid_constant
         }
         edits_only = false;
         {
-            uint32_t nreq = 0, nchg = 0, nprog = 0;
-            for_each_group(sm, a.req, a.freq, g, chunk, [&](bool on, uint32_t w, int bit, int x, int y, int z) {
-                uint32_t cb = 0;
-                if (on) {
-                    const size_t v = flat(g, x, y, z);
-                    const T old = a.fh[v];
-                    const uint8_t oc = a.cnt[v];
-                    const T fv = __ldg(a.f + v);
-                    const T lowered = old - a.delta;
-                    T nv;
-                    uint8_t nc;
-                    if (fabs(fv - lowered) <= a.eps && static_cast<int>(oc) < a.q - 1) {
-                        nv = lowered;
-                        nc = static_cast<uint8_t>(oc + 1);
-                    } else {
-                        nc = static_cast<uint8_t>(a.q);
-                        nv = fv - a.eps;
-                    }
-                    a.fh[v] = nv;
-                    a.cnt[v] = nc;
-                    const bool chg = bits_of(old) != bits_of(nv);
-                    ++nreq;
-                    nprog += (chg || nc != oc) ? 1u : 0u;
-                    if (chg) {
-                        ++nchg;
-                        a.hp[v] = proxy_of(nv);
-                        cb = 1u << bit;
-                    }
-                }
-                const bool lead = warp_merge_word(on ? w : 0xFFFFFFFFu, cb);
-                mark_stencils(nxt, fnxt, g, lead, x >> 5, y, z, cb);
-            });
-            const uint32_t v[8] = {0u, 0u, 0u, nreq, nchg, nprog, 0u, 0u};
+            uint32_t c[4] = {0u, 0u, 0u, 0u};
+            for_each_group(sm, a.req, a.freq, g, chunk,
+                           [&](uint32_t total, uint32_t, bool) { edit_words<T>(sm, a, nxt, fnxt, total, c); });
+            const uint32_t v[8] = {0u, 0u, 0u, c[0], c[1], c[2], 0u, 0u};
             block_flush_slot(a.slots + k, v);
         }
         grid.sync();
