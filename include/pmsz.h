@@ -228,10 +228,10 @@ int pmsz_correct_batch(const pmsz_field *fields, int count, const pmsz_opts *opt
  * per program run; the server accepts jobs from any host thread and runs them
  * on the device current at pmsz_server_create.  A worker thread repeats
  * generations: admit queued jobs in arrival order while the HBM budget (the
- * job's two fields plus its scratch) and the running-job limit allow, run one
- * sweep of every running job in shared multi-field launches (the fused first
- * pass for jobs admitted now), and retire jobs whose correction stopped.  A
- * job's result is bit-identical to pmsz_correct_* on the same field alone.
+ * job's two fields plus its scratch) and the running-job limit allow, run
+ * the running jobs' sweeps in one launch (after the fused first pass of jobs
+ * admitted now) until a job stops or another is submitted, and retire jobs
+ * whose correction stopped.  A job's result is bit-identical to pmsz_correct_* on the same field alone.
  * Field pointers are device pointers the caller keeps alive, and whose
  * producing work the caller has completed (e.g. synchronised) before submit;
  * fhat is corrected in place.

@@ -1,6 +1,6 @@
 // batch.h -- multi-field correction: the per-field table the multi-field
-// kernels read, and the host driver shared by pmsz_correct_batch (batch.cu)
-// and the continuous-batching server (server.cpp).
+// kernels read, and the host side shared by pmsz_correct_batch (batch.cu) and
+// the continuous-batching server (server.cu).
 #pragma once
 #include "march.cuh"
 #include "internal.h"
@@ -19,6 +19,8 @@ struct Inst {
     T *fh;
     uint8_t *codes, *cnt;
     uint32_t *hp, *req, *act0, *act1;
+    uint8_t *freq, *f0, *f1;  // group flags of req, act0, act1, padded to whole chunks of eight groups
+    uint32_t *def;      // voxels decided on full keys: the first pass, even and odd sweeps; [3]: full keys for good
     SweepSlot *slots;   // this field's slot of sweep k is slots[k * stride]
     int64_t stride;
     Geom g;
@@ -45,51 +47,99 @@ struct BatchOutcome {
     std::vector<SweepSlot> log;
 };
 
-// Scratch of the voxel-list generations of a table of fields (batch_list.cuh).
-// State of the device-gated generations of pmsz_correct_batch (k_batch_gate).
-struct BatchState {
-    long long k;             // sweep index of the next generation
-    int go;                  // the next generation runs
-    int live;                // fields still running after the last gate
-    unsigned long long est;  // their next active sets, estimated (15 * changed + fdir)
+// Scratch of one field, at 256-byte offsets: first what starts at zero
+// (counters, bitmaps and their group flags, the full-key counts), then codes
+// and proxies.  The sweep slots are the caller's.
+struct FieldScratch {
+    size_t cnt, req, act0, act1, freq, f0, f1, def, zero, codes, hp, total;
+    explicit FieldScratch(const Geom &g) {
+        size_t at = 0;
+        auto take = [&](size_t bytes) {
+            const size_t off = at;
+            at += (bytes + 255) & ~static_cast<size_t>(255);
+            return off;
+        };
+        const size_t groups = (g.nwords + kGroupWords - 1) / kGroupWords;
+        cnt = take(g.n);
+        req = take(4 * g.nwords);
+        act0 = take(4 * g.nwords);
+        act1 = take(4 * g.nwords);
+        freq = take(groups);
+        f0 = take(groups);
+        f1 = take(groups);
+        def = take(4 * sizeof(uint32_t));
+        zero = at;
+        codes = take(g.n);
+        hp = take(4 * g.n);
+        total = at;
+    }
+    // The table row's scratch pointers: zeroed part at z, the rest at r
+    // (r = z where a field's scratch is one piece).
+    template <typename T>
+    void point(Inst<T> &I, unsigned char *z, unsigned char *r) const {
+        I.cnt = z + cnt;
+        I.req = reinterpret_cast<uint32_t *>(z + req);
+        I.act0 = reinterpret_cast<uint32_t *>(z + act0);
+        I.act1 = reinterpret_cast<uint32_t *>(z + act1);
+        I.freq = z + freq;
+        I.f0 = z + f0;
+        I.f1 = z + f1;
+        I.def = reinterpret_cast<uint32_t *>(z + def);
+        I.codes = r + codes;
+        I.hp = reinterpret_cast<uint32_t *>(r + hp);
+    }
 };
+// Chunks of eight groups (kGroupWords words each) of a field.
+inline uint64_t sweep_chunks(const Geom &g) {
+    const uint64_t groups = (g.nwords + kGroupWords - 1) / kGroupWords;
+    return (groups + 7) / 8;
+}
 
-struct MultiLists {
-    uint32_t *wpre = nullptr;   // n + 1 word prefixes (multiples of 4), device
-    uint64_t total_words = 0;
-    uint32_t *counts = nullptr; // one count per compaction block (kCompactBlocks)
-    uint64_t *list = nullptr, *xlist = nullptr;  // capacity: the fields' voxels
-    uint32_t *lc = nullptr;     // 4 list lengths
-    BatchState *state = nullptr;
+// One type's fields in a k_sweeps_multi launch.
+struct SweepReport {
+    SweepSlot last;  // of the last sweep run, where the field has stopped
+    unsigned long long edits;  // sum of its sweeps' requests, likewise
+    long long sweeps;          // run so far
+    long long running;
 };
+template <typename T>
+struct SweepTable {
+    const Inst<T> *inst = nullptr;
+    const uint32_t *cpre = nullptr;  // n + 1 prefixes of sweep_chunks
+    int n = 0;
+    uint32_t chunks = 0;             // their total
+    SweepReport *report = nullptr;   // n
+};
+struct SweepCtl {
+    long long iters;  // sweeps run by the launch
+    int yield[2];
+};
+struct MultiSweeps {
+    SweepTable<float> t32;
+    SweepTable<double> t64;
+    SweepCtl *ctl = nullptr;
+    const volatile int *yield = nullptr;  // mapped host memory, or null
+    int until_stop = 0;                   // end as soon as a field has stopped
+};
+// The sweeps of both tables: of fields with `first` set from the edits of
+// sweep 0 on, of the others from the detection of sweep k on.
+int launch_multi_sweeps(const MultiSweeps &a, cudaStream_t s);
+// The fused first pass of the fields whose tiles tpre counts (n + 1 prefixes).
+template <typename T>
+int launch_first_multi(const Inst<T> *inst, const uint32_t *tpre, int n, uint32_t tiles, cudaStream_t s);
 
-// Scratch and table of one multi-field run; slot rows are sweep-major
-// (row k holds the slot of sweep k of every field).
+// Scratch and table of one batch of same-type fields; slot rows are
+// sweep-major (row k holds the slot of sweep k of every field).
 template <typename T>
 struct MultiRun {
     explicit MultiRun(cudaStream_t st) : s(st), ws(st) {}
-    ~MultiRun() {
-        if (pin) cudaFreeHost(pin);
-    }
     MultiRun(const MultiRun &) = delete;
     MultiRun &operator=(const MultiRun &) = delete;
-    int setup(const std::vector<FieldSpec<T>> &specs, int64_t max_sweeps, int q, cudaStream_t s);
-    // One generation: the fused first pass of fields with `first` set, the
-    // detection of every other active field, then the edits of all active
-    // fields.  Clears `first` afterwards.
-    int generation();
-    // The remaining sweeps of all active fields in one cooperative launch.
-    int loop(int64_t *iters);
-    // The same launch on the device table as it stands when the stream gets
-    // there, without waiting: *hiters (pinned) receives the iteration count.
-    int enqueue_loop(long long *hiters);
-    int read_row(int64_t k, std::vector<SweepSlot> &row);
-    // rows k .. k+count-1 in one copy (row j at out[j * n])
-    int read_rows(int64_t k, int64_t count, std::vector<SweepSlot> &out);
-    // The host table goes up through one of two pinned copies in turn, with
-    // no wait: every generation ends in a read_row, which synchronises the
-    // stream before the same copy is written again.
-    int push_table();
+    int setup(const std::vector<FieldSpec<T>> &specs, int64_t max_sweeps, int q);
+    // Uploads the table and the prefixes and launches the first passes.
+    int start();
+    SweepTable<T> table() const;
+    int upload();
     // Sets every field's tile depth (and the tile prefixes) to zc.
     int set_zchunk(int zc);
     // Times the first-pass launch over the whole table at each candidate
@@ -101,59 +151,23 @@ struct MultiRun {
     Workspace ws;
     int n = 0;
     int64_t max_sweeps = 0;
-    int q = 5;
     std::vector<Inst<T>> host;
-    std::vector<uint32_t> tpre, rpre;
-    uint32_t total_tiles = 0, total_rounds = 0;
+    std::vector<uint32_t> tpre, cpre;
     Inst<T> *dinst = nullptr;
-    uint32_t *dtpre = nullptr, *drpre = nullptr;
-    long long *diters = nullptr;
+    uint32_t *dtpre = nullptr, *dcpre = nullptr;
+    SweepCtl *ctl = nullptr;
+    SweepReport *report = nullptr;
     SweepSlot *slots = nullptr;
-    MultiLists ml;
-    bool lists = false;
-    Inst<T> *pin = nullptr;  // 2 * n table entries, pinned
-    int pin_next = 0;
     unsigned char *zero_base = nullptr;  // the scratch that starts zeroed (counters, bitmaps, slots)
     size_t zero_total = 0;
-    size_t voxels = 0;  // voxel-list generations (all fields together below 2^32 voxels)
+    size_t voxels = 0;
 };
 
-// One generation over a device table of n fields (see MultiRun::generation),
-// and the gather of each field's current-sweep slot into out[0..n).
-// ml: the voxel-list scratch, or null for the round-based passes.
-template <typename T>
-int launch_generation(const Inst<T> *dinst, const uint32_t *dtpre, const uint32_t *drpre, int n,
-                      uint32_t total_tiles, uint32_t total_rounds, bool any_first, cudaStream_t s,
-                      const MultiLists *ml);
-
-// Word prefixes of a table (each field's bitmap words rounded up to a multiple
-// of 4) and their total; false if the list form does not apply (the fields'
-// voxels or words reach 2^32).
-inline bool list_prefixes(const std::vector<Geom> &geoms, std::vector<uint32_t> &wpre, uint64_t &total_words) {
-    wpre.assign(geoms.size() + 1, 0);
-    uint64_t words = 0, voxels = 0;
-    for (size_t i = 0; i < geoms.size(); ++i) {
-        wpre[i] = static_cast<uint32_t>(words);
-        words += (geoms[i].nwords + 3) & ~static_cast<size_t>(3);
-        voxels += geoms[i].n;
-        if (words >= (1ull << 32) || voxels >= (1ull << 32)) return false;
-    }
-    wpre[geoms.size()] = static_cast<uint32_t>(words);
-    total_words = words;
-    return true;
-}
-template <typename T>
-int launch_gather(const Inst<T> *dinst, int n, SweepSlot *out, cudaStream_t s);
-
-// Scratch bytes of one field (codes, counters, proxies, three bitmaps) and
-// its sweep slots.
+// Scratch bytes of one field and its sweep slots, as admission budgets count
+// them (codes, counters, proxies, three bitmaps).
 inline size_t field_scratch_bytes(const Geom &g, int64_t max_sweeps) {
     auto up = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
     return up(g.n) * 2 + up(4 * g.n) + 3 * up(4 * g.nwords) + up(sizeof(SweepSlot) * static_cast<size_t>(max_sweeps));
 }
-
-template <typename T>
-int batch_impl(const std::vector<FieldSpec<T>> &specs, const pmsz_opts *opts, std::vector<BatchOutcome> &out,
-               cudaStream_t s);
 
 }  // namespace pmsz

@@ -1,6 +1,6 @@
 // list.cuh -- voxel-list sweeps over plane ranges: the sweeps that run behind
 // the host copy of pmsz_correct_host_* (first_pass_waves); included by
-// sweep.cuh and batch_list.cuh.
+// sweep.cuh.
 //
 // Each piece of a sweep runs as
 //   compaction      bitmap -> list of flat voxel indices in voxel order

@@ -5,16 +5,21 @@
 // continuous batching: a worker thread repeats generations, and in each one
 //   1. admits queued jobs in arrival order while the HBM budget (the job's
 //      two fields plus its scratch) and the job-slot limit allow,
-//   2. runs ONE sweep of every running job in shared launches -- the fused
-//      first pass of the jobs admitted now, the detection of the others, the
-//      edits of all (the multi-field kernels of batch.cu),
-//   3. reads each job's sweep counters, applies the stop rule of the
-//      correction loop, and retires finished jobs (scratch freed, waiters
-//      woken).
-// A job that arrives while others run joins at the next generation, so its
-// work overlaps theirs on the device.  Every job keeps its own scratch, sweep
-// index and stop state: its corrected field is bit-identical to running it
-// alone through pmsz_correct_*.
+//   2. runs the fused first pass of the jobs admitted now, then sweeps of all
+//      running jobs of both types in one cooperative launch (the multi-field
+//      kernels of batch.cu), which ends after the sweep at which some job has
+//      stopped or a new job was submitted,
+//   3. reads where each job stands and retires finished jobs (waiters woken,
+//      scratch freed).
+// A job that arrives while others run joins at the next sweep, so its work
+// overlaps theirs on the device.  Every job keeps its own scratch, sweep index
+// and stop state: its corrected field is bit-identical to running it alone
+// through pmsz_correct_*.
+//
+// A generation used to be one sweep, with up to nine launches, two copies and a
+// read-back for each type: a burst of 24 mixed jobs (18 million voxels) took
+// 8.6 ms, now 4.0.  What is left is the depth of the longest job's sweeps and a
+// generation's fixed costs for every job that ends.
 #include "batch.h"
 
 #include <algorithm>
@@ -40,31 +45,28 @@ struct Job {
     unsigned char *scratch = nullptr;
     size_t scratch_bytes = 0;
     int64_t k = 0;
-    bool first = true, done = false;
+    bool first = true;
+    bool over = false;     // the worker's: no sweep left (done follows when the job is retired)
+    bool done = false;     // under the server's lock: its waiters may release it
     int status = PMSZ_ERR_NOT_CONVERGED;
-    std::vector<SweepSlot> log;
+    int64_t sweeps = 0;
+    uint64_t edits = 0;
     Clock::time_point t_submit, t_start, t_done;
 };
 
+// A job's scratch: the zeroed part of FieldScratch, its sweep slots (zeroed
+// too), then the rest.
+static size_t slot_bytes(int64_t max_sweeps) {
+    return (sizeof(SweepSlot) * static_cast<size_t>(max_sweeps) + 255) & ~static_cast<size_t>(255);
+}
+
 template <typename T>
-static Inst<T> make_inst(Job &j, int q, int64_t max_sweeps) {
+static Inst<T> make_inst(const Job &j, int q, int64_t max_sweeps) {
     Inst<T> I{};
     const Geom &g = j.g;
-    auto up = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
-    unsigned char *p = j.scratch;
-    I.cnt = p;
-    p += up(g.n);
-    I.req = reinterpret_cast<uint32_t *>(p);
-    p += up(4 * g.nwords);
-    I.act0 = reinterpret_cast<uint32_t *>(p);
-    p += up(4 * g.nwords);
-    I.act1 = reinterpret_cast<uint32_t *>(p);
-    p += up(4 * g.nwords);
-    I.slots = reinterpret_cast<SweepSlot *>(p);
-    p += up(sizeof(SweepSlot) * static_cast<size_t>(max_sweeps));
-    I.codes = p;
-    p += up(g.n);
-    I.hp = reinterpret_cast<uint32_t *>(p);
+    const FieldScratch fs(g);
+    fs.point(I, j.scratch, j.scratch + slot_bytes(max_sweeps));
+    I.slots = reinterpret_cast<SweepSlot *>(j.scratch + fs.zero);
     I.f = static_cast<const T *>(j.fd.f);
     I.fh = static_cast<T *>(j.fd.fhat);
     I.stride = 1;
@@ -79,12 +81,6 @@ static Inst<T> make_inst(Job &j, int q, int64_t max_sweeps) {
     I.tiles_x = static_cast<uint32_t>(g.wpr);
     I.tiles_y = static_cast<uint32_t>((g.ny + kMY - 1) / kMY);
     return I;
-}
-
-// Zero-initialised part of a job's scratch: counters, bitmaps, slots.
-static size_t zero_prefix(const Geom &g, int64_t max_sweeps) {
-    auto up = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
-    return up(g.n) + 3 * up(4 * g.nwords) + up(sizeof(SweepSlot) * static_cast<size_t>(max_sweeps));
 }
 
 class Server {
@@ -122,9 +118,10 @@ public:
         j->fd = fd;
         j->g = make_geom(fd.nx, fd.ny, fd.nz);
         j->g.zc = first_depth(fd.nx, fd.ny, fd.nz, fd.elem_size);
-        j->scratch_bytes = field_scratch_bytes(j->g, cfg_.max_sweeps);
-        // its fields, its scratch, and its share of the group's voxel lists
-        j->bytes = j->scratch_bytes + 2 * j->g.n * fd.elem_size + 2 * sizeof(uint64_t) * j->g.n;
+        j->scratch_bytes = FieldScratch(j->g).total + slot_bytes(cfg_.max_sweeps);
+        // its fields, its scratch, and 16 bytes a voxel for what the running
+        // set shares (a charge that budgets are sized by: more than is held now)
+        j->bytes = field_scratch_bytes(j->g, cfg_.max_sweeps) + 2 * j->g.n * fd.elem_size + 2 * sizeof(uint64_t) * j->g.n;
         if (cfg_.hbm_budget_bytes && j->bytes > cfg_.hbm_budget_bytes)
             return set_error(PMSZ_ERR_OOM, "job larger than the server's HBM budget");
         j->t_submit = Clock::now();
@@ -134,6 +131,7 @@ public:
         *id = j->id;
         pending_.push_back(j.get());
         jobs_[j->id] = std::move(j);
+        if (yield_) __atomic_store_n(yield_, 1, __ATOMIC_RELEASE);  // the running launch ends after its sweep
         cv_work_.notify_all();
         return PMSZ_OK;
     }
@@ -152,8 +150,8 @@ public:
         out->done = j->done ? 1 : 0;
         if (!j->done) return PMSZ_OK;
         out->status = j->status;
-        out->sweeps = static_cast<int64_t>(j->log.size());
-        for (const SweepSlot &h : j->log) out->edits += h.requested;
+        out->sweeps = j->sweeps;
+        out->edits = j->edits;
         out->queue_ms = std::chrono::duration<double, std::milli>(j->t_start - j->t_submit).count();
         out->run_ms = std::chrono::duration<double, std::milli>(j->t_done - j->t_start).count();
         out->latency_ms = std::chrono::duration<double, std::milli>(j->t_done - j->t_submit).count();
@@ -169,139 +167,133 @@ public:
     }
 
 private:
+    // The running jobs of one type, and where a generation's upload holds them.
     template <typename T>
     struct Group {
         std::vector<Job *> jobs;
-        std::vector<Inst<T>> host;
-        Inst<T> *dinst = nullptr;
-        uint32_t *dpre = nullptr;
-        SweepSlot *dslots = nullptr, *hslots = nullptr;
-        int cap = 0;
-        MultiLists ml;            // voxel-list scratch of the running set
-        uint32_t *dwpre = nullptr;
-        size_t list_cap = 0;      // entries of ml.list / ml.xlist
+        size_t inst = 0, tpre = 0, cpre = 0, report = 0;  // offsets
+        uint32_t tiles = 0, chunks = 0;
+    };
+    // One upload (tables and prefixes of both types) and one read-back
+    // (reports) a generation, through buffers that grow to the largest set.
+    struct Buffers {
+        unsigned char *up = nullptr, *dup = nullptr;    // pinned, device
+        unsigned char *rep = nullptr, *drep = nullptr;  // pinned, device: SweepCtl, then the reports
+        size_t up_cap = 0, rep_cap = 0;
     };
 
-    template <typename T>
-    int ensure(Group<T> &G, int n) {
-        if (n <= G.cap) return PMSZ_OK;
-        if (G.dinst) cudaFree(G.dinst);
-        if (G.dpre) cudaFree(G.dpre);
-        if (G.dslots) cudaFree(G.dslots);
-        if (G.hslots) cudaFreeHost(G.hslots);
-        G.cap = std::max(n, 64);
-        PMSZ_CUDA(cudaMalloc(&G.dinst, sizeof(Inst<T>) * G.cap));
-        PMSZ_CUDA(cudaMalloc(&G.dpre, sizeof(uint32_t) * 2 * (G.cap + 1)));
-        PMSZ_CUDA(cudaMalloc(&G.dslots, sizeof(SweepSlot) * G.cap));
-        PMSZ_CUDA(cudaMallocHost(&G.hslots, sizeof(SweepSlot) * G.cap));
-        if (G.dwpre) cudaFree(G.dwpre);
-        PMSZ_CUDA(cudaMalloc(&G.dwpre, sizeof(uint32_t) * (G.cap + 1)));
+    static int grow(unsigned char *&host, unsigned char *&dev, size_t &cap, size_t want) {
+        if (want <= cap) return PMSZ_OK;
+        if (host) cudaFreeHost(host);
+        if (dev) cudaFree(dev);
+        host = dev = nullptr;
+        cap = 0;
+        want = std::max<size_t>(2 * want, 64u << 10);
+        PMSZ_CUDA(cudaMallocHost(reinterpret_cast<void **>(&host), want));
+        PMSZ_CUDA(cudaMalloc(reinterpret_cast<void **>(&dev), want));
+        cap = want;
         return PMSZ_OK;
     }
 
-    // List buffers for `voxels` entries (grown, never shrunk while the server runs).
+    // Sizes a group's part of the two buffers.
     template <typename T>
-    int ensure_lists(Group<T> &G, size_t voxels) {
-        if (!G.ml.counts) {
-            PMSZ_CUDA(cudaMalloc(&G.ml.counts, sizeof(uint32_t) * kCompactBlocks));
-            PMSZ_CUDA(cudaMalloc(&G.ml.lc, sizeof(uint32_t) * 4));
-        }
-        if (voxels <= G.list_cap) return PMSZ_OK;
-        if (G.ml.list) cudaFree(G.ml.list);
-        if (G.ml.xlist) cudaFree(G.ml.xlist);
-        G.ml.list = G.ml.xlist = nullptr;
-        G.list_cap = 0;
-        const size_t cap = std::max<size_t>(voxels, 1 << 20);
-        PMSZ_CUDA(cudaMalloc(&G.ml.list, sizeof(uint64_t) * cap));
-        PMSZ_CUDA(cudaMalloc(&G.ml.xlist, sizeof(uint64_t) * cap));
-        G.list_cap = cap;
-        return PMSZ_OK;
+    void place(Group<T> &G, size_t &up, size_t &rep) {
+        const size_t n = G.jobs.size();
+        auto take = [](size_t &at, size_t bytes) {
+            const size_t off = at;
+            at += (bytes + 255) & ~static_cast<size_t>(255);
+            return off;
+        };
+        G.inst = take(up, n * sizeof(Inst<T>));
+        G.tpre = take(up, (n + 1) * sizeof(uint32_t));
+        G.cpre = take(up, (n + 1) * sizeof(uint32_t));
+        G.report = take(rep, n * sizeof(SweepReport));
     }
 
+    // Writes a group's table and prefixes; tiles are those of the jobs that start now.
     template <typename T>
-    void release_group(Group<T> &G) {
-        if (G.dinst) cudaFree(G.dinst);
-        if (G.dpre) cudaFree(G.dpre);
-        if (G.dslots) cudaFree(G.dslots);
-        if (G.hslots) cudaFreeHost(G.hslots);
-        if (G.dwpre) cudaFree(G.dwpre);
-        if (G.ml.counts) cudaFree(G.ml.counts);
-        if (G.ml.lc) cudaFree(G.ml.lc);
-        if (G.ml.list) cudaFree(G.ml.list);
-        if (G.ml.xlist) cudaFree(G.ml.xlist);
-        G = Group<T>{};
-    }
-
-    // One sweep of every running job of type T.
-    template <typename T>
-    int step(Group<T> &G) {
-        const int n = static_cast<int>(G.jobs.size());
-        if (!n) return PMSZ_OK;
-        int rc = ensure(G, n);
-        if (rc) return rc;
-        G.host.resize(n);
-        std::vector<uint32_t> pre(2 * (n + 1));
-        uint64_t tiles = 0, rounds = 0;
-        bool any_first = false;
-        for (int i = 0; i < n; ++i) {
-            Job &j = *G.jobs[i];
-            G.host[i] = make_inst<T>(j, cfg_.q, cfg_.max_sweeps);
-            any_first |= j.first;
-            pre[i] = static_cast<uint32_t>(tiles);
-            pre[n + 1 + i] = static_cast<uint32_t>(rounds);
-            tiles += static_cast<uint64_t>(G.host[i].tiles_x) * G.host[i].tiles_y * ((j.g.nz + j.g.zc - 1) / j.g.zc);
-            rounds += (j.g.nwords + kRoundWords - 1) / kRoundWords;
-        }
-        if (tiles >= (1ull << 31) || rounds >= (1ull << 31)) return set_error(PMSZ_ERR_ARG, "running set too large");
-        pre[n] = static_cast<uint32_t>(tiles);
-        pre[2 * n + 1] = static_cast<uint32_t>(rounds);
-        std::vector<Geom> geoms(n);
-        size_t voxels = 0;
-        for (int i = 0; i < n; ++i) {
-            geoms[i] = G.host[i].g;
-            voxels += geoms[i].n;
-        }
-        // Voxel-list generations pay off once the running set's next active
-        // sets are large (estimate: 15 * changed + fdir of the last sweep, a
-        // sixteenth of a joining field); small groups take the two round-based
-        // launches, which cost less than the list form's eight.
-        unsigned long long est = 0;
-        for (int i = 0; i < n; ++i) {
+    int fill(Group<T> &G) {
+        const size_t n = G.jobs.size();
+        Inst<T> *inst = reinterpret_cast<Inst<T> *>(buf_.up + G.inst);
+        uint32_t *tpre = reinterpret_cast<uint32_t *>(buf_.up + G.tpre), *cpre = reinterpret_cast<uint32_t *>(buf_.up + G.cpre);
+        uint64_t tiles = 0, chunks = 0;
+        for (size_t i = 0; i < n; ++i) {
             const Job &j = *G.jobs[i];
-            if (j.first || j.log.empty()) est += j.g.n / 16;
-            else est += 15ull * j.log.back().changed + j.log.back().fdir;
+            inst[i] = make_inst<T>(j, cfg_.q, cfg_.max_sweeps);
+            tpre[i] = static_cast<uint32_t>(tiles);
+            cpre[i] = static_cast<uint32_t>(chunks);
+            if (j.first)
+                tiles += static_cast<uint64_t>(inst[i].tiles_x) * inst[i].tiles_y * ((j.g.nz + j.g.zc - 1) / j.g.zc);
+            chunks += sweep_chunks(j.g);
+            if (tiles >= (1ull << 31) || chunks >= (1ull << 31)) return set_error(PMSZ_ERR_ARG, "running set too large");
         }
-        std::vector<uint32_t> wpre;
-        const bool lists = est >= std::max<unsigned long long>(1ull << 20, voxels / 32) &&
-                           list_prefixes(geoms, wpre, G.ml.total_words);
-        if (lists) {
-            if ((rc = ensure_lists(G, voxels))) return rc;
-            G.ml.wpre = G.dwpre;
-            PMSZ_CUDA(cudaMemcpyAsync(G.dwpre, wpre.data(), sizeof(uint32_t) * wpre.size(), cudaMemcpyHostToDevice, s_));
-        }
-        PMSZ_CUDA(cudaMemcpyAsync(G.dinst, G.host.data(), sizeof(Inst<T>) * n, cudaMemcpyHostToDevice, s_));
-        PMSZ_CUDA(cudaMemcpyAsync(G.dpre, pre.data(), sizeof(uint32_t) * pre.size(), cudaMemcpyHostToDevice, s_));
-        if ((rc = launch_generation<T>(G.dinst, G.dpre, G.dpre + n + 1, n, static_cast<uint32_t>(tiles),
-                                       static_cast<uint32_t>(rounds), any_first, s_, lists ? &G.ml : nullptr)))
-            return rc;
-        if ((rc = launch_gather<T>(G.dinst, n, G.dslots, s_))) return rc;
-        PMSZ_CUDA(cudaMemcpyAsync(G.hslots, G.dslots, sizeof(SweepSlot) * n, cudaMemcpyDeviceToHost, s_));
-        PMSZ_CUDA(cudaStreamSynchronize(s_));
-        for (int i = 0; i < n; ++i) {
+        tpre[n] = G.tiles = static_cast<uint32_t>(tiles);
+        cpre[n] = G.chunks = static_cast<uint32_t>(chunks);
+        return PMSZ_OK;
+    }
+
+    template <typename T>
+    int start_first(const Group<T> &G) {
+        if (!G.tiles) return PMSZ_OK;
+        return launch_first_multi<T>(reinterpret_cast<const Inst<T> *>(buf_.dup + G.inst),
+                                     reinterpret_cast<const uint32_t *>(buf_.dup + G.tpre), static_cast<int>(G.jobs.size()),
+                                     G.tiles, s_);
+    }
+
+    template <typename T>
+    SweepTable<T> table(const Group<T> &G) {
+        SweepTable<T> t;
+        t.inst = reinterpret_cast<const Inst<T> *>(buf_.dup + G.inst);
+        t.cpre = reinterpret_cast<const uint32_t *>(buf_.dup + G.cpre);
+        t.n = static_cast<int>(G.jobs.size());
+        t.chunks = G.chunks;
+        t.report = reinterpret_cast<SweepReport *>(buf_.drep + G.report);
+        return t;
+    }
+
+    template <typename T>
+    void read(const Group<T> &G) {
+        const SweepReport *rep = reinterpret_cast<const SweepReport *>(buf_.rep + G.report);
+        for (size_t i = 0; i < G.jobs.size(); ++i) {
             Job &j = *G.jobs[i];
-            const SweepSlot h = G.hslots[i];
-            j.log.push_back(h);
+            const SweepReport &r = rep[i];
             j.first = false;
-            if (j.k == 0 && h.bad) {
-                j.status = PMSZ_ERR_ARG;
-                j.done = true;
-            } else if (sweep_stops(h.fmax, h.fmin, h.fdir, h.progressed, j.k + 1, cfg_.max_sweeps)) {
-                j.status = (h.fmax == 0 && h.fmin == 0 && h.fdir == 0) ? PMSZ_OK : PMSZ_ERR_NOT_CONVERGED;
-                j.done = true;
-            } else {
-                ++j.k;
-            }
+            j.k = r.sweeps;
+            if (r.running) continue;
+            const SweepSlot &h = r.last;
+            j.sweeps = r.sweeps;
+            j.edits = r.edits;
+            j.status = r.sweeps == 1 && h.bad                          ? PMSZ_ERR_ARG
+                       : h.fmax == 0 && h.fmin == 0 && h.fdir == 0 ? PMSZ_OK
+                                                                   : PMSZ_ERR_NOT_CONVERGED;
+            j.over = true;
         }
+    }
+
+    // A generation of the running jobs.
+    int step(Group<float> &g32, Group<double> &g64) {
+        if (g32.jobs.empty() && g64.jobs.empty()) return PMSZ_OK;
+        size_t up = 0, rep = 256;
+        static_assert(sizeof(SweepCtl) <= 256, "the reports follow the control block");
+        place(g32, up, rep);
+        place(g64, up, rep);
+        int rc;
+        if ((rc = grow(buf_.up, buf_.dup, buf_.up_cap, up)) || (rc = grow(buf_.rep, buf_.drep, buf_.rep_cap, rep)) ||
+            (rc = fill(g32)) || (rc = fill(g64)))
+            return rc;
+        PMSZ_CUDA(cudaMemcpyAsync(buf_.dup, buf_.up, up, cudaMemcpyHostToDevice, s_));
+        if ((rc = start_first(g32)) || (rc = start_first(g64))) return rc;
+        MultiSweeps a;
+        if (!g32.jobs.empty()) a.t32 = table(g32);
+        if (!g64.jobs.empty()) a.t64 = table(g64);
+        a.ctl = reinterpret_cast<SweepCtl *>(buf_.drep);
+        a.yield = dyield_;
+        a.until_stop = 1;
+        if ((rc = launch_multi_sweeps(a, s_))) return rc;
+        PMSZ_CUDA(cudaMemcpyAsync(buf_.rep, buf_.drep, rep, cudaMemcpyDeviceToHost, s_));
+        PMSZ_CUDA(cudaStreamSynchronize(s_));
+        read(g32);
+        read(g64);
         return PMSZ_OK;
     }
 
@@ -318,9 +310,18 @@ private:
 
     void run() {
         cudaSetDevice(device_);
-        if (cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking) != cudaSuccess) {
+        int *flag = nullptr, *dflag = nullptr;
+        if (cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaHostAlloc(reinterpret_cast<void **>(&flag), sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer(reinterpret_cast<void **>(&dflag), flag, 0) != cudaSuccess) {
             fail_all(PMSZ_ERR_CUDA);
             return;
+        }
+        *flag = 0;
+        dyield_ = dflag;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            yield_ = flag;
         }
         retain_pool_once();
         Group<float> g32;
@@ -331,6 +332,7 @@ private:
                 std::unique_lock<std::mutex> lk(mu_);
                 cv_work_.wait(lk, [&] { return stopping_ || !pending_.empty() || !running_.empty(); });
                 if (stopping_ && pending_.empty() && running_.empty()) break;
+                __atomic_store_n(yield_, 0, __ATOMIC_RELEASE);  // what is pending is looked at now
                 while (!pending_.empty() && static_cast<int>(running_.size() + admitted.size()) < cfg_.max_jobs) {
                     Job *j = pending_.front();
                     if (cfg_.hbm_budget_bytes && used_ + j->bytes > cfg_.hbm_budget_bytes) break;  // FIFO admission
@@ -342,10 +344,10 @@ private:
             for (Job *j : admitted) {
                 j->t_start = Clock::now();
                 if (cudaMallocAsync(reinterpret_cast<void **>(&j->scratch), j->scratch_bytes, s_) != cudaSuccess ||
-                    cudaMemsetAsync(j->scratch, 0, zero_prefix(j->g, cfg_.max_sweeps), s_) != cudaSuccess) {
+                    cudaMemsetAsync(j->scratch, 0, FieldScratch(j->g).zero + slot_bytes(cfg_.max_sweeps), s_) != cudaSuccess) {
                     cudaGetLastError();
                     j->status = PMSZ_ERR_OOM;
-                    j->done = true;
+                    j->over = true;
                 }
             }
             {
@@ -355,23 +357,23 @@ private:
             g32.jobs.clear();
             g64.jobs.clear();
             for (Job *j : running_)
-                if (!j->done) (j->fd.elem_size == 4 ? (std::vector<Job *> &)g32.jobs : g64.jobs).push_back(j);
-            int rc = step(g32);
-            if (!rc) rc = step(g64);
-            if (rc) {
+                if (!j->over) (j->fd.elem_size == 4 ? (std::vector<Job *> &)g32.jobs : g64.jobs).push_back(j);
+            if (step(g32, g64) != PMSZ_OK) {
                 fail_all(PMSZ_ERR_CUDA);
                 continue;
             }
-            // retire finished jobs
+            // retire finished jobs (a waiter may release its job as soon as the lock is free)
             std::vector<Job *> keep;
+            std::vector<unsigned char *> done;
             {
                 std::lock_guard<std::mutex> lk(mu_);
                 for (Job *j : running_) {
-                    if (j->done) {
-                        if (j->scratch) cudaFreeAsync(j->scratch, s_);
+                    if (j->over) {
+                        if (j->scratch) done.push_back(j->scratch);
                         j->scratch = nullptr;
                         used_ -= j->bytes;
                         j->t_done = Clock::now();
+                        j->done = true;
                     } else {
                         keep.push_back(j);
                     }
@@ -379,16 +381,28 @@ private:
                 running_.swap(keep);
             }
             cv_done_.notify_all();
+            for (unsigned char *p : done) cudaFreeAsync(p, s_);
         }
         cudaStreamSynchronize(s_);
-        release_group(g32);
-        release_group(g64);
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            yield_ = nullptr;
+        }
+        cudaFreeHost(flag);
+        if (buf_.up) cudaFreeHost(buf_.up);
+        if (buf_.dup) cudaFree(buf_.dup);
+        if (buf_.rep) cudaFreeHost(buf_.rep);
+        if (buf_.drep) cudaFree(buf_.drep);
+        buf_ = Buffers{};
         cudaStreamDestroy(s_);
     }
 
     pmsz_server_config cfg_;
     int device_ = 0;
     cudaStream_t s_ = nullptr;
+    Buffers buf_;
+    int *yield_ = nullptr;               // mapped: set by a submission (under mu_)
+    const volatile int *dyield_ = nullptr;  // its device address
     std::thread worker_;
     std::mutex mu_;
     std::condition_variable cv_work_, cv_done_;

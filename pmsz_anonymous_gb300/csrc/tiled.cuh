@@ -110,22 +110,6 @@ __device__ __forceinline__ Ext proxy_ext_interior(const uint32_t (&t)[15]) {
 constexpr int kHX = kTX + 2;
 constexpr int kThreads = kTX * kMY / 2;
 // ---------------------------------------------------------------------------
-// Load policies.  Standalone sweep kernels read arrays that no thread of the
-// same launch writes through the read-only path (__ldg).  Persistent loop
-// kernels (the multi-field loop of batch.cu) write those arrays in one phase
-// and read them in the next, across grid-wide barriers, so they read them at
-// L2 (__ldcg), never from a possibly stale L1 line.
-// ---------------------------------------------------------------------------
-struct LdgLoads {
-    template <class P>
-    static __device__ __forceinline__ P ld(const P *p) { return __ldg(p); }
-};
-struct CgLoads {
-    template <class P>
-    static __device__ __forceinline__ P ld(const P *p) { return __ldcg(p); }
-};
-
-// ---------------------------------------------------------------------------
 // Block-local compaction of a bitmap.  A round covers 2048 consecutive words:
 // each of the 256 threads loads 8 of them with two 16-byte loads, and one
 // barrier skips the round when all are empty (late sweeps touch a few words of
@@ -151,18 +135,17 @@ struct ListSmem {
 // Loads the 8 words of this thread for the round starting at `base` (bitmaps
 // are 256-byte aligned and rounds start at multiples of 2048 words, so the
 // vector loads are aligned); returns whether any word of the block is set.
-template <class L>
 __device__ __forceinline__ bool load_round(const uint32_t *__restrict__ bm, size_t base, const Geom &g,
                                            uint32_t (&w8)[kWordsPerThread]) {
     const size_t w0 = base + static_cast<size_t>(threadIdx.x) * kWordsPerThread;
     if (w0 + kWordsPerThread <= g.nwords) {
-        const uint4 a = L::ld(reinterpret_cast<const uint4 *>(bm + w0));
-        const uint4 b = L::ld(reinterpret_cast<const uint4 *>(bm + w0 + 4));
+        const uint4 a = __ldg(reinterpret_cast<const uint4 *>(bm + w0));
+        const uint4 b = __ldg(reinterpret_cast<const uint4 *>(bm + w0 + 4));
         w8[0] = a.x; w8[1] = a.y; w8[2] = a.z; w8[3] = a.w;
         w8[4] = b.x; w8[5] = b.y; w8[6] = b.z; w8[7] = b.w;
     } else {
 #pragma unroll
-        for (int j = 0; j < kWordsPerThread; ++j) w8[j] = w0 + j < g.nwords ? L::ld(bm + w0 + j) : 0u;
+        for (int j = 0; j < kWordsPerThread; ++j) w8[j] = w0 + j < g.nwords ? __ldg(bm + w0 + j) : 0u;
     }
     uint32_t any = 0;
 #pragma unroll
@@ -175,13 +158,13 @@ __device__ __forceinline__ bool load_round(const uint32_t *__restrict__ bm, size
 // and flush(w, mask) is then called once per word with a non-zero mask, by the
 // thread that owns the word.  Every thread of the block must call this.
 // One round (2048 words from `base`) of for_each_set_bit.
-template <class L, class Work, class Flush>
+template <class Work, class Flush>
 __device__ __forceinline__ void process_round(ListSmem &sm, uint32_t *__restrict__ bm, const Geom &g, size_t base,
                                               Work &work, Flush &flush) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     {
         uint32_t w8[kWordsPerThread];
-        if (!load_round<L>(bm, base, g, w8)) return;  // uniform
+        if (!load_round(bm, base, g, w8)) return;  // uniform
         const size_t w0 = base + static_cast<size_t>(t) * kWordsPerThread;
         uint32_t c = 0;
 #pragma unroll
@@ -246,68 +229,13 @@ __device__ __forceinline__ void process_round(ListSmem &sm, uint32_t *__restrict
     }
 }
 
-template <class L, class Work, class Flush>
+template <class Work, class Flush>
 __device__ __forceinline__ void for_each_set_bit(ListSmem &sm, uint32_t *__restrict__ bm, const Geom &g, Work &work,
                                                  Flush &flush) {
     for (size_t base = static_cast<size_t>(blockIdx.x) * kRoundWords; base < g.nwords;
          base += static_cast<size_t>(gridDim.x) * kRoundWords)
-        process_round<L>(sm, bm, g, base, work, flush);
+        process_round(sm, bm, g, base, work, flush);
 }
-
-// ---------------------------------------------------------------------------
-// Sparse detection of one voxel of the active set, reading the proxy array of
-// fhat (exact keys on a failed certificate), with the reference rules; the
-// word's mismatch bits go to act_next through DetectFlush (one writer per
-// word).  Counters accumulate in the functor.
-// ---------------------------------------------------------------------------
-template <class L, typename T>
-struct DetectWork {
-    const T *fh;
-    const uint32_t *hp;
-    const uint8_t *codes;
-    uint32_t *req;
-    Geom g;
-    uint32_t cmax = 0, cmin = 0, cdir = 0, active = 0;
-    __device__ __forceinline__ bool operator()(int x, int y, int z, uint32_t) {
-        const ptrdiff_t sy = g.nx, sz = static_cast<ptrdiff_t>(g.nx) * g.ny;
-        const size_t i = flat(g, x, y, z);
-        const bool interior = x >= 1 && x <= g.nx - 2 && y >= 1 && y <= g.ny - 2 && z >= 1 && z <= g.nz - 2;
-        const uint32_t valid = interior ? kAllValid : valid_mask(x, y, z, g.nx, g.ny, g.nz);
-        const uint32_t *c0 = hp + i;
-        uint32_t t[15];
-#pragma unroll
-        for (int r = 0; r < 15; ++r) {
-            const ptrdiff_t off = rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz;
-            t[r] = ((valid >> r) & 1u) ? L::ld(c0 + off) : 0u;
-        }
-        Ext ex = interior ? proxy_ext_interior<true>(t) : proxy_ext<true>(t);
-        if (!ex.exact) {
-            typename KeyOf<T>::type kk[15];
-#pragma unroll
-            for (int r = 0; r < 15; ++r) {
-                const ptrdiff_t off = rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz;
-                kk[r] = ((valid >> r) & 1u) ? okey(L::ld(fh + (static_cast<ptrdiff_t>(i) + off)))
-                                            : typename KeyOf<T>::type(0);
-            }
-            arg_ext(kk, valid, ex.asc, ex.desc);
-        }
-        const uint8_t c = __ldg(codes + i);
-        const uint32_t tm = detect_rules(ex.asc, ex.desc, c & 15, c >> 4, cmax, cmin, cdir);
-        ++active;
-        if (tm) request_targets(req, g, x, y, z, tm);
-        return tm != 0;
-    }
-    __device__ __forceinline__ void flush_to(SweepSlot *slot) {  // every thread of the block
-        const uint32_t v[8] = {cmax, cmin, cdir, 0u, 0u, 0u, active, 0u};
-        block_flush_slot(slot, v);
-        cmax = cmin = cdir = active = 0;
-    }
-};
-
-struct DetectFlush {
-    uint32_t *act_next;
-    __device__ __forceinline__ void operator()(size_t w, uint32_t m) { act_next[w] = m; }
-};
 
 // ---------------------------------------------------------------------------
 // Apply with the proxy array: applyDeltaBuffer_local (pMSz.cu:623-645) on
@@ -317,7 +245,7 @@ struct DetectFlush {
 // the proxy of every changed value refreshed; ApplyFlush marks the closed
 // stencil of the changed vertices of a word in act_next (owner thread).
 // ---------------------------------------------------------------------------
-template <class L, typename T>
+template <typename T>
 struct ApplyWork {
     const T *f;
     T *fh;
@@ -329,8 +257,8 @@ struct ApplyWork {
     uint32_t nreq = 0, nprog = 0;
     __device__ __forceinline__ bool operator()(int x, int y, int z, uint32_t) {
         const size_t v = flat(g, x, y, z);
-        const T old = L::ld(fh + v);
-        const uint8_t oc = L::ld(cnt + v);
+        const T old = __ldg(fh + v);
+        const uint8_t oc = __ldg(cnt + v);
         const T fv = __ldg(f + v);
         const T lowered = old - delta;
         T nv;
@@ -375,14 +303,14 @@ __device__ __forceinline__ void flush_apply_counts(SweepSlot *slot, uint32_t nre
     }
 }
 
-template <class L, typename T>
+template <typename T>
 __device__ __forceinline__ void apply_body(ListSmem &sm, const T *__restrict__ f, T *__restrict__ fh,
                                            uint8_t *__restrict__ cnt, uint32_t *__restrict__ hp,
                                            uint32_t *__restrict__ req, uint32_t *__restrict__ act_next, SweepSlot *slot,
                                            const Geom &g, T eps, T delta, int q) {
-    ApplyWork<L, T> work{f, fh, cnt, hp, g, eps, delta, q};
+    ApplyWork<T> work{f, fh, cnt, hp, g, eps, delta, q};
     ApplyFlush flush{act_next, g};
-    for_each_set_bit<L>(sm, req, g, work, flush);
+    for_each_set_bit(sm, req, g, work, flush);
     const uint32_t v[8] = {0u, 0u, 0u, work.nreq, flush.nchg, work.nprog, 0u, 0u};
     block_flush_slot(slot, v);
 }
@@ -393,7 +321,7 @@ __global__ void __launch_bounds__(kListBlock) k_apply_px(const T *__restrict__ f
                                                          uint32_t *__restrict__ req, uint32_t *__restrict__ act_next,
                                                          SweepSlot *slot, Geom g, T eps, T delta, int q) {
     __shared__ ListSmem sm;
-    apply_body<LdgLoads>(sm, f, fh, cnt, hp, req, act_next, slot, g, eps, delta, q);
+    apply_body(sm, f, fh, cnt, hp, req, act_next, slot, g, eps, delta, q);
 }
 
 // Stop rule of the correction loop after a sweep (the slot of that sweep):
