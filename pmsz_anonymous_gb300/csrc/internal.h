@@ -152,6 +152,16 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
 // AS / DS labels (roots of the steepest-ascent / descent forests) of a code
 // array; n < 2^32.
 int labels_impl(const uint8_t *codes, size_t nx, size_t ny, size_t nz, uint32_t *as, uint32_t *ds, cudaStream_t s);
+// The same in pieces, without a synchronisation, both kinds in place:
+// labels_roots leaves a voxel's label at L[L[i]] (labels_finish then at L[i])
+// unless the stream sets *words; labels_complete is the general way from there
+// (it synchronises) and leaves the labels at L[i].  lists: label_list_words()
+// words; words: 2, set by labels_roots.
+size_t label_list_words(size_t nx, size_t ny, size_t nz);
+int labels_roots(const uint8_t *codes, size_t nx, size_t ny, size_t nz, uint32_t *as, uint32_t *ds, uint32_t *lists,
+                 unsigned int *words, cudaStream_t s);
+int labels_finish(size_t nx, size_t ny, size_t nz, uint32_t *as, uint32_t *ds, cudaStream_t s);
+int labels_complete(size_t nx, size_t ny, size_t nz, uint32_t *as, uint32_t *ds, unsigned int *words, cudaStream_t s);
 // Tuning table (tune.cu): the tile depth (planes per tile column) and the
 // pointer-jumping rounds per launch recorded for a shape class, or the
 // defaults; tune_known says whether the class has an entry.

@@ -84,7 +84,7 @@ static int jump_to_roots(uint32_t *L, size_t n, unsigned int *d_flag, cudaStream
 }
 
 constexpr int kLX = 32, kLY = 16, kLZ = 16, kLTile = kLX * kLY * kLZ;
-constexpr int kLThreads = 256;
+constexpr int kLWarps = 16, kLThreads = 32 * kLWarps;
 constexpr uint32_t kLShell = kLTile - (kLX - 2) * (kLY - 2) * (kLZ - 2);  // most exits a tile can have
 constexpr int kWalkHops = 64;  // hops of an exit per launch (two per tile crossed)
 
@@ -108,22 +108,24 @@ struct TileRootsSmem {
     uint32_t n[NL];
 };
 
-// One block per tile; thread (lane, w) owns the rows y = w and w + 8 of every
-// plane.  L[l][i] receives the label so far of nibble lo[l] (0: ascent, 4:
+// One block of 16 warps per tile; warp w owns the row y = w of every plane (with
+// 8 warps and two rows each the chase has half the chains in flight: both
+// labels of 32 M voxels 545 us, now 494).  L[l][i] receives the label so far of nibble lo[l] (0: ascent, 4:
 // descent), exits[l] the tile's exits (global indices) and count[l] their
 // number.  *flag is set if a chain does not end within the tile's voxel count
 // (a cycle: not the codes of a field).  Bound by shared-memory latency and
 // conflicts of the pointer chase (L1 78 % busy, issue 63 %): pointers are stored
 // as byte offsets, steps come from a shuffle, the in-tile test from rank masks,
-// and exits are handled by full warps behind the loop.  71.5 M voxels, one kind:
-// 250 us and 87 warp instructions per voxel (312 us and 152 with coordinates
-// decoded per voxel and exits handled in the loop).
+// and exits are handled by full warps behind the loop.  71.5 M voxels, one kind, with 8
+// warps: 250 us and 87 warp instructions per voxel (312 us and 152 with
+// coordinates decoded per voxel and exits handled in the loop).
 template <int NL>
 __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restrict__ codes, uint32_t *__restrict__ l0,
                                                           uint32_t *__restrict__ l1, int lo0, int lo1,
                                                           uint32_t *__restrict__ exits0, uint32_t *__restrict__ exits1,
                                                           uint32_t stride, uint32_t *__restrict__ count0,
                                                           uint32_t *__restrict__ count1, unsigned int *flag, Geom g) {
+    constexpr int NW = kLWarps, H = kLY / NW;  // rows of a plane per thread
     __shared__ TileRootsSmem<NL> sm;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int x0 = blockIdx.x * kLX, y0 = blockIdx.y * kLY, z0 = blockIdx.z * kLZ;
@@ -140,11 +142,11 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
     const int r16 = lane & 15;
     const int step = r16 < 15 ? 2 * (rank_dx(r16) + kLX * rank_dy(r16) + kLX * kLY * rank_dz(r16)) : 0;
     const uint32_t xmask = kAllValid & ~(lane == 0 ? kNegX : 0u) & ~(lane + 1 >= ex ? kPosX : 0u);
-    uint32_t ymask[2];
-    bool in_row[2];
+    uint32_t ymask[H];
+    bool in_row[H];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int y = w + 8 * h;
+    for (int h = 0; h < H; ++h) {
+        const int y = w + NW * h;
         ymask[h] = xmask & ~(y == 0 ? kNegY : 0u) & ~(y + 1 >= ey ? kPosY : 0u);
         in_row[h] = lane < ex && y < ey;
     }
@@ -154,9 +156,9 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
     for (int z = 0; z < kLZ; ++z) {
         const uint32_t zmask = kAllValid & ~(z == 0 ? kNegZ : 0u) & ~(z + 1 >= ez ? kPosZ : 0u);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t v = v0 + static_cast<uint32_t>(kLX * 8 * h + kLX * kLY * z);
-            const uint32_t c = in_row[h] && z < ez ? codes[i0 + sy * (8u * h) + sz * static_cast<uint32_t>(z)] : 0x77u;
+        for (int h = 0; h < H; ++h) {
+            const uint32_t v = v0 + static_cast<uint32_t>(kLX * NW * h + kLX * kLY * z);
+            const uint32_t c = in_row[h] && z < ez ? codes[i0 + sy * static_cast<uint32_t>(NW * h) + sz * static_cast<uint32_t>(z)] : 0x77u;
             const uint32_t mask = ymask[h] & zmask;
 #pragma unroll
             for (int l = 0; l < NL; ++l) {
@@ -174,8 +176,8 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
 #pragma unroll 1
     for (int round = 0; round < 2; ++round) {
 #pragma unroll 8
-        for (int k = 0; k < 2 * kLZ; ++k) {
-            const uint32_t off = 2 * v0 + static_cast<uint32_t>(2 * kLX * 8 * k);
+        for (int k = 0; k < H * kLZ; ++k) {
+            const uint32_t off = 2 * v0 + static_cast<uint32_t>(2 * kLX * NW * k);
 #pragma unroll
             for (int l = 0; l < NL; ++l) at(l, off) = at(l, at(l, at(l, off)));
         }
@@ -183,11 +185,11 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
     }
     bool stuck = false;
 #pragma unroll 2
-    for (int k = 0; k < 2 * kLZ; ++k) {
-        const int z = k >> 1;
-        const uint32_t off = 2 * v0 + static_cast<uint32_t>(2 * kLX * 8 * k);
-        const bool in = in_row[k & 1] && z < ez;
-        const uint32_t i = i0 + sy * (8u * static_cast<uint32_t>(k & 1)) + sz * static_cast<uint32_t>(z);
+    for (int k = 0; k < H * kLZ; ++k) {
+        const int z = k / H;
+        const uint32_t off = 2 * v0 + static_cast<uint32_t>(2 * kLX * NW * k);
+        const bool in = in_row[k % H] && z < ez;
+        const uint32_t i = i0 + sy * static_cast<uint32_t>(NW * (k % H)) + sz * static_cast<uint32_t>(z);
 #pragma unroll
         for (int l = 0; l < NL; ++l) {
             uint32_t p = at(l, off), q = at(l, p);
@@ -240,12 +242,15 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
     }
 }
 
-// Every exit of a tile (one block) walks to its root; *flag is set where the
-// hops run out.
-__global__ void __launch_bounds__(512) k_exit_walk(uint32_t *L, const uint32_t *__restrict__ exits, uint32_t stride,
-                                                   const uint32_t *__restrict__ count, unsigned int *flag) {
-    const uint32_t m = count[blockIdx.x];
-    const uint32_t *list = exits + static_cast<size_t>(blockIdx.x) * stride;
+// Every exit of a tile (one block for each kind of label, blockIdx.y) walks to
+// its root; *flag is set where the hops run out.
+__global__ void __launch_bounds__(512) k_exit_walk(uint32_t *l0, uint32_t *l1, const uint32_t *__restrict__ exits0,
+                                                   const uint32_t *__restrict__ exits1, uint32_t stride,
+                                                   const uint32_t *__restrict__ count0,
+                                                   const uint32_t *__restrict__ count1, unsigned int *flag) {
+    uint32_t *L = blockIdx.y ? l1 : l0;
+    const uint32_t m = (blockIdx.y ? count1 : count0)[blockIdx.x];
+    const uint32_t *list = (blockIdx.y ? exits1 : exits0) + static_cast<size_t>(blockIdx.x) * stride;
     bool open = false;
     for (uint32_t j = threadIdx.x; j < m; j += blockDim.x) {
         const uint32_t e = list[j];
@@ -300,8 +305,9 @@ struct LabelRun {
         else
             k_tile_roots<1><<<t.grid, kLThreads, 0, s>>>(codes, L[0], nullptr, lo[0], 0, exits(0), nullptr, t.stride,
                                                          counts(0), nullptr, words, g);
-        for (int l = 0; l < nl; ++l)
-            k_exit_walk<<<static_cast<unsigned>(t.tiles()), 512, 0, s>>>(L[l], exits(l), t.stride, counts(l), words);
+        const int last = nl - 1;
+        k_exit_walk<<<dim3(static_cast<unsigned>(t.tiles()), static_cast<unsigned>(nl)), 512, 0, s>>>(
+            L[0], L[last], exits(0), exits(last), t.stride, counts(0), counts(last), words);
         PMSZ_CUDA(cudaGetLastError());
         return PMSZ_OK;
     }
@@ -360,6 +366,34 @@ static int labels_run(const uint8_t *codes, size_t nx, size_t ny, size_t nz, OUT
 
 int labels_impl(const uint8_t *codes, size_t nx, size_t ny, size_t nz, uint32_t *as, uint32_t *ds, cudaStream_t s) {
     return labels_run<uint32_t>(codes, nx, ny, nz, as, ds, s);
+}
+
+static LabelRun both_kinds(size_t nx, size_t ny, size_t nz, uint32_t *as, uint32_t *ds, uint32_t *lists,
+                           unsigned int *words) {
+    LabelRun r;
+    r.g = make_geom(nx, ny, nz);
+    r.t = tile_grid(r.g);
+    r.L[0] = as;
+    r.L[1] = ds;
+    r.nl = 2;
+    r.lists = lists;
+    r.words = words;
+    return r;
+}
+size_t label_list_words(size_t nx, size_t ny, size_t nz) {
+    return 2 * LabelRun::list_words(tile_grid(make_geom(nx, ny, nz)));
+}
+int labels_roots(const uint8_t *codes, size_t nx, size_t ny, size_t nz, uint32_t *as, uint32_t *ds, uint32_t *lists,
+                 unsigned int *words, cudaStream_t s) {
+    return both_kinds(nx, ny, nz, as, ds, lists, words).roots(codes, s);
+}
+int labels_finish(size_t nx, size_t ny, size_t nz, uint32_t *as, uint32_t *ds, cudaStream_t s) {
+    LabelRun r = both_kinds(nx, ny, nz, as, ds, nullptr, nullptr);
+    const int rc = r.finish<uint32_t>(0, as, s);
+    return rc ? rc : r.finish<uint32_t>(1, ds, s);
+}
+int labels_complete(size_t nx, size_t ny, size_t nz, uint32_t *as, uint32_t *ds, unsigned int *words, cudaStream_t s) {
+    return both_kinds(nx, ny, nz, as, ds, nullptr, words).complete(s, tuned_jump_rounds(nx, ny, nz));
 }
 
 int time_jump_rounds(const uint8_t *codes, size_t nx, size_t ny, size_t nz, const int *rounds, int m, float *ms,
