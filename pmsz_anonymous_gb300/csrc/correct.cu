@@ -199,7 +199,7 @@ static inline unsigned stride_grid(size_t items) {
     return static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(want, 152 * 16)));
 }
 
-// Tensor maps of f and fhat for the TMA-fed first pass (k_first_tma): 3-D
+// Tensor maps of f and fhat for the TMA-fed first pass (k_pair_tma): 3-D
 // (nx, ny, nz) maps with a box of one tile plane.  The encoder is the driver's
 // cuTensorMapEncodeTiled, reached through the runtime (the library does not
 // link libcuda).  Not available (ok = false: the first pass loads its tiles
@@ -258,8 +258,8 @@ static int launch_first_pass(const FirstMaps &m, dim3 grid, cudaStream_t s, cons
                              uint32_t *xc, uint32_t *err, uint8_t *freq = nullptr, uint8_t *fact = nullptr) {
     const MarchArgs<T> a{f, fh, codes, hp, req, nullptr, act, slot, xc, freq, fact};
     if (m.ok) {
-        PMSZ_CUDA(allow_smem(k_first_tma<T>, sizeof(TmaMarch<T>)));
-        k_first_tma<T><<<grid, dim3(kTX, kThreads / kTX, 1), sizeof(TmaMarch<T>), s>>>(m.f, m.fh, a, g, bz0, err);
+        PMSZ_CUDA(allow_smem(k_pair_tma<T, kFirst>, sizeof(TmaMarch<T>)));
+        k_pair_tma<T, kFirst><<<grid, dim3(kTX, kThreads / kTX, 1), sizeof(TmaMarch<T>), s>>>(m.f, m.fh, a, g, bz0, err);
         PMSZ_CUDA(cudaGetLastError());
     } else {
         PMSZ_CUDA((launch_march<T, kFirst>(grid, s, a, g, bz0)));
@@ -745,6 +745,33 @@ int codes_impl(const T *v, size_t nx, size_t ny, size_t nz, uint8_t *codes, cuda
     PMSZ_CUDA(cudaGetLastError());
     return PMSZ_OK;
 }
+
+// Both fields' codes in one pass, their differences and the values' distances
+// counted (MarchArgs::pair); *err as in the first pass.
+template <typename T>
+int pair_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, T eps, uint64_t sure, uint8_t *c0, uint8_t *c1,
+              unsigned long long *counts, uint32_t *err, cudaStream_t s) {
+    Geom g = make_geom(nx, ny, nz);
+    g.zc = first_depth(nx, ny, nz, sizeof(T));
+    MarchArgs<T> a{f, fp, c0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    a.codes_h = c1;
+    a.eps = eps;
+    a.sure = sure;
+    a.pair = counts;
+    const FirstMaps m = first_maps<T>(f, fp, g);
+    if (m.ok) {
+        PMSZ_CUDA(allow_smem(k_pair_tma<T, kPair>, sizeof(TmaMarch<T>)));
+        k_pair_tma<T, kPair><<<tiled_grid(g), dim3(kTX, kThreads / kTX, 1), sizeof(TmaMarch<T>), s>>>(m.f, m.fh, a, g, 0, err);
+        PMSZ_CUDA(cudaGetLastError());
+    } else {
+        PMSZ_CUDA((launch_march<T, kPair>(tiled_grid(g), s, a, g, 0)));
+    }
+    return PMSZ_OK;
+}
+template int pair_impl<float>(const float *, const float *, size_t, size_t, size_t, float, uint64_t, uint8_t *, uint8_t *,
+                              unsigned long long *, uint32_t *, cudaStream_t);
+template int pair_impl<double>(const double *, const double *, size_t, size_t, size_t, double, uint64_t, uint8_t *,
+                               uint8_t *, unsigned long long *, uint32_t *, cudaStream_t);
 
 // The tuner's first-pass timing: the fused first pass of f / fhat at each
 // tile depth zcs[k] on scratch of its own; ms[k] is the best of two timed

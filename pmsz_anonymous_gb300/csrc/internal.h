@@ -191,6 +191,15 @@ int naive_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, co
                pmsz_result *res, cudaStream_t s);
 template <typename T>
 int codes_impl(const T *v, size_t nx, size_t ny, size_t nz, uint8_t *codes, cudaStream_t s);
+// The codes of f and fp (c0, c1) in one pass; counts (zeroed by the caller) +=
+// voxels whose codes differ, of those the ones whose extremum kind does, values
+// with |fp - f| > eps, values outside [f - eps, f + eps]; counts[4], [5] = 1 if
+// some ascending / descending direction differs.  sure: the magnitude bits of
+// eps, 0 unless it is positive and finite.  *err is set if a plane's copy did not
+// arrive within the bounded wait.
+template <typename T>
+int pair_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, T eps, uint64_t sure, uint8_t *c0, uint8_t *c1,
+              unsigned long long *counts, uint32_t *err, cudaStream_t s);
 template <typename T>
 int verify_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, double eb, pmsz_verify_result *out,
                 cudaStream_t s);

@@ -426,67 +426,6 @@ int time_jump_rounds(const uint8_t *codes, size_t nx, size_t ny, size_t nz, cons
     return ws.release();
 }
 
-__device__ __forceinline__ uint64_t bits_mag(double v) {
-    return static_cast<uint64_t>(__double_as_longlong(v)) & 0x7FFFFFFFFFFFFFFFull;
-}
-__device__ __forceinline__ uint64_t bits_mag(float v) { return __float_as_uint(v) & 0x7FFFFFFFu; }
-// Differences of the codes, and of the values against the bound.  GB300's
-// fp64 pipe runs two operations per SM and cycle, so the five fp64 operations
-// of the two bound tests are what an fp64 field would wait for (824 us for 71.5 M
-// voxels against 190 us of traffic): one subtraction per voxel decides nearly
-// all.  fl(p - f) rounds monotonically and eps is representable, so
-// |fl(p - f)| < eps means |p - f| < eps, and then p lies within
-// [fl(f - eps), fl(f + eps)] as well.  sure: the magnitude bits of eps, or 0
-// where eps is not a positive finite number.  Four voxels per thread and step, their
-// loads together.
-template <typename T>
-__global__ void __launch_bounds__(256) k_verify_cmp(const T *__restrict__ f, const T *__restrict__ fp,
-                                                    const uint8_t *__restrict__ c0, const uint8_t *__restrict__ c1,
-                                                    size_t n, T eps, uint64_t sure, unsigned long long *out) {
-    uint32_t dm = 0, em = 0, bs = 0, bc = 0, any = 0;
-    const size_t step = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (size_t i0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * step) {
-        T fv[4], pv[4];
-        uint32_t a[4], b[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const size_t i = i0 + j * step;
-            const bool in = i < n;
-            fv[j] = in ? f[i] : T(0);
-            pv[j] = in ? fp[i] : T(0);
-            a[j] = in ? c0[i] : 0u;
-            b[j] = in ? c1[i] : 0u;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            dm += a[j] != b[j];
-            any |= a[j] ^ b[j];
-            em += (((a[j] & 15u) == kSelf) != ((b[j] & 15u) == kSelf)) ||
-                  (((a[j] >> 4) == kSelf) != ((b[j] >> 4) == kSelf));
-            const T d = pv[j] - fv[j];
-            if (bits_mag(d) >= sure && i0 + j * step < n) {  // NaN included
-                bs += !(fabs(d) <= eps);
-                bc += !(pv[j] >= fv[j] - eps && pv[j] <= fv[j] + eps);
-            }
-        }
-    }
-    dm = warp_sum_u32(dm);
-    em = warp_sum_u32(em);
-    bs = warp_sum_u32(bs);
-    bc = warp_sum_u32(bc);
-    if ((threadIdx.x & 31) == 0) {
-        if (dm) atomicAdd(out + 0, (unsigned long long)dm);
-        if (em) atomicAdd(out + 1, (unsigned long long)em);
-        if (bs) atomicAdd(out + 4, (unsigned long long)bs);
-        if (bc) atomicAdd(out + 5, (unsigned long long)bc);
-    }
-    any = __reduce_or_sync(0xFFFFFFFFu, any);
-    if ((threadIdx.x & 31) == 0 && any) {
-        if (any & 15u) out[6] = 1;  // some ascending direction differs
-        if (any >> 4) out[7] = 1;   // some descending one
-    }
-}
-
 // Voxels whose labels differ, the labels of both fields finished on the way
 // (hop: L holds local roots as before k_finish; else the labels themselves).
 __global__ void __launch_bounds__(256) k_count_diff(const uint32_t *__restrict__ a, const uint32_t *__restrict__ b,
@@ -529,34 +468,35 @@ int verify_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, double
     const size_t o_c0 = ws.reserve<uint8_t>(g.n), o_c1 = ws.reserve<uint8_t>(g.n);
     const size_t o_l0 = ws.reserve<uint32_t>(with_labels ? g.n : 0), o_l1 = ws.reserve<uint32_t>(with_labels ? g.n : 0);
     const size_t o_e = ws.reserve<uint32_t>(with_labels ? LabelRun::list_words(tiles) : 0), o_w = ws.reserve<unsigned int>(8);
-    const size_t o_cnt = ws.reserve<unsigned long long>(8);
+    const size_t o_cnt = ws.reserve<unsigned long long>(9);
     if ((rc = ws.commit())) return rc;
     uint8_t *c0 = ws.at<uint8_t>(o_c0), *c1 = ws.at<uint8_t>(o_c1);
     unsigned long long *cnt = ws.at<unsigned long long>(o_cnt);
-    constexpr size_t kCounts = 8 * sizeof(unsigned long long);
+    constexpr size_t kCounts = 9 * sizeof(unsigned long long);
     unsigned long long *h = static_cast<unsigned long long *>(host_pinned(kCounts + 8 * sizeof(unsigned int)));
     if (!h) return set_error(PMSZ_ERR_OOM, "pinned host allocation failed");
     PMSZ_CUDA(cudaMemsetAsync(cnt, 0, kCounts, s));
-    if ((rc = codes_impl<T>(f, nx, ny, nz, c0, s))) return rc;
-    if ((rc = codes_impl<T>(fp, nx, ny, nz, c1, s))) return rc;
     const T eps = static_cast<T>(eb);
     uint64_t sure = 0;
     if (eps > T(0) && std::isfinite(eps)) {
         if (sizeof(T) == 8) std::memcpy(&sure, &eps, 8);
         else std::memcpy(&sure, &eps, 4);  // little-endian: the low word
     }
-    k_verify_cmp<T><<<grid_for((g.n + 3) / 4), 256, 0, s>>>(f, fp, c0, c1, g.n, eps, sure, cnt);
-    PMSZ_CUDA(cudaGetLastError());
+    // cnt: codes, extrema, beyond the bound, beyond the clamp, some ascent, some
+    // descent differ; then the label mismatches of either kind, and the copies' flag
+    if ((rc = pair_impl<T>(f, fp, nx, ny, nz, eps, sure, c0, c1, cnt, reinterpret_cast<uint32_t *>(cnt + 8), s))) return rc;
     PMSZ_CUDA(cudaMemcpyAsync(h, cnt, kCounts, cudaMemcpyDeviceToHost, s));
     PMSZ_CUDA(cudaStreamSynchronize(s));
-    unsigned long long got[8];  // what follows reads back through the same pinned block
+    unsigned long long got[9];  // what follows reads back through the same pinned block
     std::memcpy(got, h, kCounts);
+    if (got[8]) return set_error(PMSZ_ERR_CUDA, "verification: a tile plane's tensor copy did not arrive within the bounded wait");
     // A label is the end of a voxel's chain of steepest neighbours, so fields
     // whose directions agree at every voxel have the same labels: a kind is
     // labelled only if some direction of it differs.  A corrected field, the
     // usual one to be checked, agrees in all of them (71.5 M voxels fp64 2809 ->
-    // 1017 us); reading that back first costs the others 15 us.
-    const bool wanted[2] = {with_labels && got[6] != 0, with_labels && got[7] != 0};
+    // 1017 us, and 727 with both codes and the comparison in one pass); reading
+    // that back first costs the others 15 us.
+    const bool wanted[2] = {with_labels && got[4] != 0, with_labels && got[5] != 0};
     // AS, then DS labels of both fields in the same two arrays; the flags of
     // the runs are read once, at the end
     auto run_of = [&](int kind, int field) {
@@ -575,18 +515,18 @@ int verify_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, double
         for (int field = 0; field < 2; ++field)
             if ((rc = run_of(kind, field).roots(field ? c1 : c0, s))) return rc;
         k_count_diff<<<grid_for((g.n + 3) / 4), 256, 0, s>>>(ws.at<uint32_t>(o_l0), ws.at<uint32_t>(o_l1), g.n, 1,
-                                                             cnt + 2 + kind);
+                                                             cnt + 6 + kind);
         PMSZ_CUDA(cudaGetLastError());
     }
     unsigned int words[8] = {};
     if (wanted[0] || wanted[1]) {
-        unsigned int *hw = reinterpret_cast<unsigned int *>(h + 8);
+        unsigned int *hw = reinterpret_cast<unsigned int *>(h + 9);
         PMSZ_CUDA(cudaMemcpyAsync(h, cnt, kCounts, cudaMemcpyDeviceToHost, s));
         PMSZ_CUDA(cudaMemcpyAsync(hw, ws.at<unsigned int>(o_w), 8 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
         PMSZ_CUDA(cudaStreamSynchronize(s));
         std::memcpy(words, hw, sizeof(words));
-        got[2] = h[2];
-        got[3] = h[3];
+        got[6] = h[6];
+        got[7] = h[7];
     }
     const bool open[2] = {wanted[0] && (words[0] | words[2]) != 0, wanted[1] && (words[4] | words[6]) != 0};
     for (int kind = 0; kind < 2; ++kind) {
@@ -597,20 +537,20 @@ int verify_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, double
             LabelRun r = run_of(kind, field);
             if ((rc = r.roots(field ? c1 : c0, s)) || (rc = r.complete(s, rounds))) return rc;
         }
-        PMSZ_CUDA(cudaMemsetAsync(cnt + 2 + kind, 0, sizeof(unsigned long long), s));
+        PMSZ_CUDA(cudaMemsetAsync(cnt + 6 + kind, 0, sizeof(unsigned long long), s));
         k_count_diff<<<grid_for((g.n + 3) / 4), 256, 0, s>>>(ws.at<uint32_t>(o_l0), ws.at<uint32_t>(o_l1), g.n, 0,
-                                                             cnt + 2 + kind);
+                                                             cnt + 6 + kind);
         PMSZ_CUDA(cudaGetLastError());
-        PMSZ_CUDA(cudaMemcpyAsync(h, cnt + 2 + kind, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+        PMSZ_CUDA(cudaMemcpyAsync(h, cnt + 6 + kind, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
         PMSZ_CUDA(cudaStreamSynchronize(s));
-        got[2 + kind] = h[0];
+        got[6 + kind] = h[0];
     }
     out->dir_mismatch = got[0];
     out->ext_mismatch = got[1];
-    out->as_mismatch = with_labels ? got[2] : UINT64_MAX;
-    out->ds_mismatch = with_labels ? got[3] : UINT64_MAX;
-    out->bound_strict = got[4];
-    out->bound_beyond_clamp = got[5];
+    out->as_mismatch = with_labels ? got[6] : UINT64_MAX;
+    out->ds_mismatch = with_labels ? got[7] : UINT64_MAX;
+    out->bound_strict = got[2];
+    out->bound_beyond_clamp = got[3];
     return ws.release();
 }
 
