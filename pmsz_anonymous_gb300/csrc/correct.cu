@@ -267,41 +267,34 @@ static int launch_first_pass(const FirstMaps &m, dim3 grid, cudaStream_t s, cons
     return PMSZ_OK;
 }
 
-// The resident blocks of k_sweeps on the current device (queried once per
-// device: the queries cost more than a small field's sweep).
-template <typename T>
-static int sweep_grid(unsigned *blocks) {
+// A sweep kernel over all resident blocks of the current device (three per SM:
+// queried once per device, since the queries cost more than a small field's
+// sweep), or as many as `words` bitmap words keep busy.
+template <typename T, class Kernel, class... Args>
+static int launch_cooperative(Kernel kernel, size_t words, cudaStream_t s, const Args &...args) {
     static std::mutex mu;
     static std::vector<unsigned> known;
-    int dev = 0;
-    PMSZ_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lk(mu);
-    if (static_cast<size_t>(dev) >= known.size()) known.resize(static_cast<size_t>(dev) + 1, 0u);
-    if (!known[static_cast<size_t>(dev)]) {
-        int sms = 0, per_sm = 0, coop = 0;
-        PMSZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        PMSZ_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-        if (!coop) return set_error(PMSZ_ERR_CUDA, "device does not support cooperative launches");
-        PMSZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweeps<T>, kSweepBlock, 0));
-        if (per_sm < 1) return set_error(PMSZ_ERR_CUDA, "sweep kernel does not fit on an SM");
-        known[static_cast<size_t>(dev)] = static_cast<unsigned>(per_sm * sms);
-    }
-    *blocks = known[static_cast<size_t>(dev)];
-    return PMSZ_OK;
-}
-
-// All remaining sweeps in one cooperative launch; a small field takes no more
-// blocks than it has groups of words.
-template <typename T>
-static int launch_sweeps(SweepArgs<T> &a, cudaStream_t s) {
     unsigned blocks = 0;
-    const int rc = sweep_grid<T>(&blocks);
-    if (rc) return rc;
-    const size_t want = (group_count(a.g) + kSweepWarps - 1) / kSweepWarps;
+    {
+        int dev = 0;
+        PMSZ_CUDA(cudaGetDevice(&dev));
+        std::lock_guard<std::mutex> lk(mu);
+        if (static_cast<size_t>(dev) >= known.size()) known.resize(static_cast<size_t>(dev) + 1, 0u);
+        if (!known[static_cast<size_t>(dev)]) {
+            int sms = 0, per_sm = 0, coop = 0;
+            PMSZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            PMSZ_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+            if (!coop) return set_error(PMSZ_ERR_CUDA, "device does not support cooperative launches");
+            PMSZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSweepBlock, 0));
+            if (per_sm < 1) return set_error(PMSZ_ERR_CUDA, "sweep kernel does not fit on an SM");
+            known[static_cast<size_t>(dev)] = static_cast<unsigned>(per_sm * sms);
+        }
+        blocks = known[static_cast<size_t>(dev)];
+    }
+    const size_t groups = (words + kGroupWords - 1) / kGroupWords, want = (groups + kSweepWarps - 1) / kSweepWarps;
     const unsigned grid = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(want, blocks)));
-    void *args[] = {&a};
-    PMSZ_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_sweeps<T>), dim3(grid), dim3(kSweepBlock),
-                                          args, 0, s));
+    void *ptr[] = {const_cast<void *>(static_cast<const void *>(&args))...};
+    PMSZ_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(kSweepBlock), ptr, 0, s));
     return PMSZ_OK;
 }
 
@@ -413,27 +406,18 @@ int first_pass_ingest(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes
     return PMSZ_OK;
 }
 
-// Sweeps pipelined behind the host copy, and the fractions of the slabs after which they
-// advance: every piece of a sweep costs two compaction kernels and five more
-// launches whatever its size, so the early waves are large and the late
-// ones, whose remainder is all that is left once the copy ends, small (a
-// wave per slab piled these fixed costs up behind the copy).
-constexpr int kWaveSweeps = 6;
-// in sixteenths of the slabs; fp32 slabs cross the link in half the time of
-// fp64 slabs of as many voxels, while the sweeps cost about the same
-constexpr int kWaveAt8[] = {4, 8, 12, 14, 16};
-constexpr int kWaveAt4[] = {4, 8, 12, 16};
-
-// One-thread bookkeeping between the pieces of the wavefront (a kernel rather
-// than a small memset, which may queue behind the host copies on the copy
-// engine).
-static __global__ void k_wave_clear_spills(LoopState *ls) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) ls->lc[2] = 0;
-}
+// The fractions of the slabs after which the sweeps behind the host copy
+// (kWaveSweeps of them) advance, in sixteenths.  A wave costs its launch and two
+// barriers a sweep whatever its size, and dense sweeps are less efficient in
+// pieces, so the first ones are large; the last ones, all that is left once the
+// copy ends, are small.  256x320x288 and 512^3 fp64: 2521 us and 11.46 ms; at
+// 4, 8, 12, 14, 16: 2538 and 11.64; at 12, 15, 16: 2626 and 11.51; without waves
+// 2718 and 13.02.  (As voxel lists, seven launches a piece: 3347 us and 11.80.)
+constexpr int kWaveAt[] = {8, 12, 14, 15, 16};
 
 // The host-buffer wavefront.  The copy of slab j releases the first pass
 // of slab j (sweep 0's detection, complete below plane Z = (j + 1) * slab
-// depth, or nz after the last slab); after the slabs of kWaveAt8 / kWaveAt4
+// depth, or nz after the last slab); after the slabs of kWaveAt
 // follows a wave: on the planes already final, the pieces of sweeps 0 .. K that those
 // planes allow:
 //   sweep k's detection covers planes below D_k, its edits planes below A_k,
@@ -448,57 +432,47 @@ static __global__ void k_wave_clear_spills(LoopState *ls) {
 // crossing the host link leave little to do after it.  Counters go straight
 // to slots[k]; k_wave_gate then sets the loop state as after sweep K.
 template <typename T>
-static int first_pass_waves(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes, uint8_t *cnt, uint32_t *hp,
-                            uint32_t *req, uint32_t *const act[2], SweepSlot *slots, LoopState *ls, const Geom &g,
-                            const FirstMaps &maps, uint32_t *list, uint32_t *slist, uint32_t *bcnt,
-                            const FastDiv &div_nx, T eps, T delta, int q, int K, cudaStream_t s, int64_t *launches) {
-    if (in.df != f || !in.copies || in.copies->zc != g.zc)
+static int first_pass_waves(const HostIngest<T> &in, const SweepArgs<T> &a, const FirstMaps &maps, int K, cudaStream_t s,
+                            int64_t *launches) {
+    const Geom &g = a.g;
+    if (in.df != a.f || !in.copies || in.copies->zc != g.zc)
         return set_error(PMSZ_ERR_ARG, "ingest copies do not match the field");
     const IngestCopies &r = *in.copies;
     const int cps = r.cps, nchunks = r.nchunks, nslabs = r.nslabs;
-    const unsigned lb = 152 * 8;
+    const uint32_t plane_words = static_cast<uint32_t>(static_cast<size_t>(g.wpr) * g.ny);  // (nwords < 2^32)
     int rc;
-    std::vector<int> Dp(static_cast<size_t>(K) + 1, 0), Ap(static_cast<size_t>(K) + 1, 0);  // fronts so far
+    WaveFronts f{};
+    f.sweeps = K;
+    std::vector<int> Dp(static_cast<size_t>(K) + 1, 0), Ap(static_cast<size_t>(K) + 1, 0);  // fronts so far, in planes
     std::vector<char> wave_after(static_cast<size_t>(nslabs), 0);
-    auto mark = [&](int e) { wave_after[static_cast<size_t>(std::max(1, (nslabs * e + 15) / 16) - 1)] = 1; };
-    if (sizeof(T) == 8)
-        for (int e : kWaveAt8) mark(e);
-    else
-        for (int e : kWaveAt4) mark(e);
+    for (int e : kWaveAt) wave_after[static_cast<size_t>(std::max(1, (nslabs * e + 15) / 16) - 1)] = 1;
     for (int j = 0; j < nslabs; ++j) {
         const bool last = j == nslabs - 1;
         PMSZ_CUDA(cudaStreamWaitEvent(s, r.ev[j], 0));
         dim3 grid = tiled_grid(g);
         grid.z = static_cast<unsigned>(std::min(cps, nchunks - j * cps));
-        if ((rc = launch_first_pass<T>(maps, grid, s, f, fh, codes, hp, req, act[1], &slots[0], g, j * cps, &ls->lc[3],
-                             &ls->err))) return rc;
+        if ((rc = launch_first_pass<T>(maps, grid, s, a.f, a.fh, const_cast<uint8_t *>(a.codes), a.hp, a.req, a.act1,
+                                       &a.slots[0], g, j * cps, &a.ls->lc[3], &a.ls->err, a.freq, a.f1)))
+            return rc;
         ++*launches;
         if (!wave_after[static_cast<size_t>(j)]) continue;
-        PMSZ_CUDA(cudaGetLastError());
         PMSZ_CUDA(cudaStreamWaitEvent(s, r.evp[j], 0));  // fhat's pre-correction copy of slabs 0 .. j
         const int Z = last ? g.nz : std::min(g.nz, (j + 1) * cps * g.zc);
+        f.seen = static_cast<unsigned long long>(g.nx) * g.ny * Z;
+        size_t widest = 0;
         for (int k = 0; k <= K; ++k) {
-            const int D = k == 0 ? Z : (last ? g.nz : std::max(0, Ap[k - 1] - 1));
-            uint32_t *a_next = act[(k + 1) & 1];
-            if (k > 0 && D > Dp[k]) {
-                compact_bitmap_planes(act[k & 1], g, Dp[k], D, bcnt, list, &ls->lc[0], s);
-                k_detect_list<T><<<lb, 256, 0, s>>>(list, &ls->lc[0], fh, hp, codes, req, a_next, slist, &ls->lc[2],
-                                                    &slots[k], g, div_nx);
-                k_detect_exact<T><<<lb, 256, 0, s>>>(slist, &ls->lc[2], fh, codes, req, a_next, &slots[k], g, div_nx);
-                k_wave_clear_spills<<<1, 32, 0, s>>>(ls);
-                *launches += 5;
-            }
-            Dp[k] = std::max(Dp[k], D);
-            const int A = last ? g.nz : std::max(0, D - 1);
-            if (A > Ap[k]) {
-                compact_bitmap_planes(req, g, Ap[k], A, bcnt, list, &ls->lc[1], s);
-                k_apply_list<T><<<lb, 256, 0, s>>>(list, &ls->lc[1], f, fh, cnt, hp, a_next, &slots[k], g, div_nx, eps,
-                                                   delta, q);
-                *launches += 3;
-                Ap[k] = A;
-            }
-            PMSZ_CUDA(cudaGetLastError());
+            const int D = last ? g.nz : std::max(Dp[k], k == 0 ? Z : Ap[k - 1] - 1);
+            f.det0[k] = plane_words * static_cast<uint32_t>(Dp[k]);
+            f.det1[k] = plane_words * static_cast<uint32_t>(D);
+            Dp[k] = D;
+            const int A = last ? g.nz : std::max(Ap[k], D - 1);
+            f.edit0[k] = plane_words * static_cast<uint32_t>(Ap[k]);
+            f.edit1[k] = plane_words * static_cast<uint32_t>(A);
+            Ap[k] = A;
+            widest = std::max<size_t>(widest, std::max(f.det1[k] - f.det0[k], f.edit1[k] - f.edit0[k]));
         }
+        if ((rc = launch_cooperative<T>(k_sweep_wave<T>, widest, s, a, f))) return rc;
+        ++*launches;
     }
     return PMSZ_OK;
 }
@@ -545,13 +519,10 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
     const size_t o_codes = ws.reserve<uint8_t>(g.n);
     const size_t o_hp = ws.reserve<uint32_t>(g.n);
     // host-buffer calls of several slabs run sweeps 1 .. K behind the copy
-    // (first_pass_waves; K below max_sweeps) on voxel lists
+    // (first_pass_waves; K below max_sweeps)
     const int wave_k = static_cast<int>(std::min<int64_t>(kWaveSweeps, max_sweeps - 1));
-    const bool waves = ingest && !full && g.n < (static_cast<size_t>(1) << 32) && wave_k >= 1 && ingest->copies &&
+    const bool waves = ingest && !full && wave_k >= 1 && ingest->copies &&
                        ingest->copies->nslabs >= 2;
-    const size_t o_list = ws.reserve<uint32_t>(waves ? g.n : 0);
-    const size_t o_xlist = ws.reserve<uint32_t>(waves ? g.n : 0);
-    const size_t o_bcnt = ws.reserve<uint32_t>(waves ? kCompactBlocks : 0);
     if ((rc = ws.commit())) return rc;
     LoopState *ls = ws.at<LoopState>(o_ls);
     SweepSlot *slots = ws.at<SweepSlot>(o_slots);
@@ -598,16 +569,10 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         SweepArgs<T> a{f,  fh,         codes, cnt, hp,  req,   act[0], act[1], freq, fact[0], fact[1], slots,
                        ls, max_sweeps, 1,     g,   eps, delta, q};
         if (waves) {
-            if ((rc = first_pass_waves<T>(*ingest, f, fh, codes, cnt, hp, req, act, slots, ls, g, maps,
-                                          ws.at<uint32_t>(o_list), ws.at<uint32_t>(o_xlist), ws.at<uint32_t>(o_bcnt),
-                                          make_fastdiv(static_cast<uint32_t>(g.nx)), eps, delta, q, wave_k, s,
-                                          &launches)))
-                return rc;
+            if ((rc = first_pass_waves<T>(*ingest, a, maps, wave_k, s, &launches))) return rc;
             k_wave_gate<<<1, 32, 0, s>>>(ls, slots, wave_k, max_sweeps);
-            k_build_flags<<<static_cast<unsigned>(std::min<size_t>((groups + 7) / 8, 152 * 16)), 256, 0, s>>>(
-                act[0], act[1], g, fact[0], fact[1], &ls->k);
             PMSZ_CUDA(cudaGetLastError());
-            launches += 2;
+            ++launches;
             a.from_edits = 0;
         } else if (ingest) {
             if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, act[1], &slots[0], g, s, &launches,
@@ -620,7 +585,7 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
             ++launches;
         }
         if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[1], s));
-        if ((rc = launch_sweeps<T>(a, s))) return rc;
+        if ((rc = launch_cooperative<T>(k_sweeps<T>, g.nwords, s, a))) return rc;
         ++launches;
         if (timing) PMSZ_CUDA(cudaEventRecord(lt.ev[2], s));
         PMSZ_CUDA(cudaEventRecord(et.ev[0], s));  // end of the correction's device window

@@ -1,6 +1,6 @@
 // march.cuh -- full-field passes: the fused labelling + first detection, the
-// full detection sweeps and the direction codes, included by list.cuh after
-// tiled.cuh.
+// full detection sweeps and the direction codes, and the two-field pass of the
+// verification; included after tiled.cuh.
 //
 // One block of 32 x 4 threads owns a 32 x 8 column of the field (two voxels
 // per thread and plane, one above the other in y) and marches it through g.zc

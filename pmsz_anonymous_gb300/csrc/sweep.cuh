@@ -1,5 +1,5 @@
 // sweep.cuh -- the correction loop's sweeps in one cooperative launch, included
-// by correct.cu after list.cuh.
+// by correct.cu and sweep_multi.cuh.
 //
 // The launch takes over behind the fused first pass: the edits of sweep 0, then
 // detection and edits sweep after sweep until the stop rule holds, with a grid
@@ -41,7 +41,7 @@
 //   256^3 fp32, 27 dense sweeps     4727 -> 4467 -> 3744 us (on full keys)
 //   160^3 fp64, 40 dense sweeps     2308 -> 2320 -> 2046 us
 #pragma once
-#include "list.cuh"
+#include "march.cuh"
 
 namespace pmsz {
 
@@ -136,19 +136,31 @@ __device__ __forceinline__ void mark_stencils(uint32_t *act, uint8_t *flag, cons
     }
 }
 
-// Flags of a plain bitmap: act0 (f0) or act1 (f1), the one of sweep *k_at.
-static __global__ void __launch_bounds__(256) k_build_flags(const uint32_t *act0, const uint32_t *act1, Geom g, uint8_t *f0,
-                                                     uint8_t *f1, const long long *k_at) {
-    const bool odd = (*k_at & 1) != 0;
-    const uint32_t *bm = odd ? act1 : act0;
-    uint8_t *flag = odd ? f1 : f0;
-    // one thread per word; the lanes of a group vote
-    const size_t n = group_count(g) * kGroupWords, step = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (size_t w = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; w - (threadIdx.x & 31) < n; w += step) {
-        const uint32_t any = __ballot_sync(0xFFFFFFFFu, w < g.nwords && bm[w] != 0);
-        const uint32_t first = (threadIdx.x & 31) & ~(kGroupWords - 1);
-        if (w < n && w % kGroupWords == 0) flag[w / kGroupWords] = (any >> first) & ((1u << kGroupWords) - 1u) ? 1 : 0;
+// State of the sweep loop, ahead of the sweep slots in memory so that one copy
+// brings both to the host.
+struct LoopState {
+    long long k;          // the sweep k_sweeps starts with (the wavefront ran the ones before)
+    long long done;       // sweeps in all, once it ends
+    int go;               // that sweep runs
+    uint32_t lc[4];       // [3]: first-pass decisions on full keys
+    uint32_t deferred[2]; // voxels of a sweep decided on full keys, by the sweep's parity (fp32)
+    uint32_t err;         // set by the first pass when a tensor copy did not arrive
+};
+
+// Lanes whose voxels share a bitmap word carry the same key; in a list in
+// voxel order they are consecutive lanes.  ORs the changed bits cb over each
+// group (a suffix OR within the group) and returns true on the group's lowest
+// lane when the merged bits are non-zero: that lane marks the word's closed
+// stencil once for the whole group.
+__device__ __forceinline__ bool warp_merge_word(uint32_t key, uint32_t &cb) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t grp = __match_any_sync(0xFFFFFFFFu, key);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_down_sync(0xFFFFFFFFu, cb, o);
+        if (lane + o < 32 && ((grp >> (lane + o)) & 1u)) cb |= u;
     }
+    return cb && lane == static_cast<uint32_t>(__ffs(grp) - 1);
 }
 
 template <typename T>
@@ -493,15 +505,25 @@ __device__ __forceinline__ uint32_t list_words(SweepSmem &sm, const Geom &g, uin
 // thread, fewer in small fields.  The flagged groups of a block's chunks are
 // listed in order (blocks then move through the field together, and share its
 // cache lines), and its warps take them from the list as they come free.
-template <class Visit>
+// RANGE: only the words [lo, hi); a group that reaches beyond them stays flagged.
+template <bool RANGE, class Visit>
 __device__ __forceinline__ void for_each_group(SweepSmem &sm, uint32_t *bm, uint8_t *flag, const Geom &g, uint32_t chunk,
-                                               Visit &&visit) {
+                                               uint64_t lo, uint64_t hi, Visit &&visit) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t ng = group_count(g), nc = (ng + chunk - 1) / chunk;
+    // groups g0 (a multiple of the chunk) .. ng - 1
+    const uint64_t g0 = RANGE ? (lo / kGroupWords) & ~7ull : 0, ng = RANGE ? (hi + kGroupWords - 1) / kGroupWords : group_count(g);
+    const uint64_t nc = (ng - g0 + chunk - 1) / chunk;
     for (uint64_t base = 0; base < nc; base += static_cast<uint64_t>(kSweepBlock) * gridDim.x) {
-        const uint64_t mine = (base + static_cast<uint64_t>(threadIdx.x) * gridDim.x + blockIdx.x) * chunk;  // this thread's chunk
+        const uint64_t mine = g0 + (base + static_cast<uint64_t>(threadIdx.x) * gridDim.x + blockIdx.x) * chunk;  // this thread's chunk
         uint32_t fm = 0;
-        if (mine < ng) {  // (the flags are padded to 256 bytes and start at a multiple of the chunk)
+        if (RANGE) {
+            for (uint32_t j = 0; j < chunk && mine + j < ng; ++j) {
+                const uint64_t w0 = (mine + j) * kGroupWords;
+                if (w0 + kGroupWords <= lo || !flag[mine + j]) continue;
+                if (w0 >= lo && w0 + kGroupWords <= hi) flag[mine + j] = 0;
+                fm |= 1u << j;
+            }
+        } else if (mine < ng) {  // (the flags are padded to 256 bytes and start at a multiple of the chunk)
             if (chunk == 8) {
                 const uint2 v = *reinterpret_cast<const uint2 *>(flag + mine);
                 if (v.x | v.y) *reinterpret_cast<uint2 *>(flag + mine) = make_uint2(0u, 0u);
@@ -543,10 +565,10 @@ __device__ __forceinline__ void for_each_group(SweepSmem &sm, uint32_t *bm, uint
             const uint32_t i = lane >> 3;
             if (i < take && t + i < groups) {
                 const uint32_t e = sm.group[t + i];
-                w = ((base + static_cast<uint64_t>(e >> 3) * gridDim.x + blockIdx.x) * chunk + (e & 7u)) *
+                w = (g0 + (base + static_cast<uint64_t>(e >> 3) * gridDim.x + blockIdx.x) * chunk + (e & 7u)) *
                         kGroupWords + (lane & 7);
             }
-            return w < g.nwords ? bm[w] : 0u;
+            return (RANGE ? w >= lo && w < hi : w < g.nwords) ? bm[w] : 0u;
         };
         uint64_t w;
         uint32_t word = next_words(w);
@@ -595,7 +617,7 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps(const __grid_constant
             if (sweep_stops(p->fmax, p->fmin, p->fdir, p->progressed, k, a.max_sweeps) || (k == 1 && p->bad)) break;
             uint32_t c[4] = {0u, 0u, 0u, 0u}, ndefer = 0, ndeferred = 0;
             if (threadIdx.x == 0) sm.deferred = 0;
-            for_each_group(sm, cur, fcur, g, chunk, [&](uint32_t total, uint32_t w, bool last) {
+            for_each_group<false>(sm, cur, fcur, g, chunk, 0, 0, [&](uint32_t total, uint32_t w, bool last) {
                 detect_words<T>(sm, a, sm.step, nxt, fnxt, total, w, keys, last, c, ndefer, ndeferred);
             });
             const uint32_t v[8] = {c[0], c[1], c[2], 0u, 0u, 0u, c[3], 0u};
@@ -614,7 +636,7 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps(const __grid_constant
         edits_only = false;
         {
             uint32_t c[4] = {0u, 0u, 0u, 0u};
-            for_each_group(sm, a.req, a.freq, g, chunk,
+            for_each_group<false>(sm, a.req, a.freq, g, chunk, 0, 0,
                            [&](uint32_t total, uint32_t, bool) { edit_words<T>(sm, a, nxt, fnxt, total, c); });
             const uint32_t v[8] = {0u, 0u, 0u, c[0], c[1], c[2], 0u, 0u};
             block_flush_slot(a.slots + k, v);
@@ -623,6 +645,75 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps(const __grid_constant
         ++k;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) a.ls->done = k;
+}
+
+// The sweeps behind the host copy (first_pass_waves): in one launch, on the
+// planes that are final so far, the pieces of sweeps 0 .. K that these planes
+// allow: of sweep k the detection of words [det0, det1) and then the edits of
+// words [edit0, edit1), every piece behind a grid barrier.  The counters add up
+// in the sweeps' slots over the launches.
+constexpr int kWaveSweeps = 6;
+struct WaveFronts {  // words: the fronts of the launch before and of this one
+    uint32_t det0[kWaveSweeps + 1], det1[kWaveSweeps + 1], edit0[kWaveSweeps + 1], edit1[kWaveSweeps + 1];
+    int sweeps;             // K
+    unsigned long long seen;  // voxels of the first passes so far
+};
+template <typename T>
+__global__ void __launch_bounds__(kSweepBlock, 3) k_sweep_wave(const __grid_constant__ SweepArgs<T> a,
+                                                               const __grid_constant__ WaveFronts f) {
+    __shared__ SweepSmem sm;
+    cg::grid_group grid = cg::this_grid();
+    const Geom &g = a.g;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 0) fill_steps(sm.step, g, lane);
+    clear_bits(sm.bits[warp]);
+    __syncthreads();
+    const bool keys = sizeof(T) == 4 && 10ull * a.ls->lc[3] > f.seen;
+    auto chunk_of = [&](uint32_t words) {
+        uint32_t chunk = 8;
+        while (chunk > 1 && words / kGroupWords < static_cast<uint64_t>(chunk) * gridDim.x * kSweepWarps) chunk >>= 1;
+        return chunk;
+    };
+    for (int k = 0; k <= f.sweeps; ++k) {
+        uint32_t *cur = (k & 1) ? a.act1 : a.act0, *nxt = (k & 1) ? a.act0 : a.act1;
+        uint8_t *fcur = (k & 1) ? a.f1 : a.f0, *fnxt = (k & 1) ? a.f0 : a.f1;
+        if (k > 0 && f.det1[k] > f.det0[k]) {  // (of sweep 0 the first pass is the detection)
+            uint32_t c[4] = {0u, 0u, 0u, 0u}, ndefer = 0, ndeferred = 0;
+            for_each_group<true>(sm, cur, fcur, g, chunk_of(f.det1[k] - f.det0[k]), f.det0[k], f.det1[k],
+                                 [&](uint32_t total, uint32_t w, bool last) {
+                                     detect_words<T>(sm, a, sm.step, nxt, fnxt, total, w, keys, last, c, ndefer, ndeferred);
+                                 });
+            const uint32_t v[8] = {c[0], c[1], c[2], 0u, 0u, 0u, c[3], 0u};
+            block_flush_slot(a.slots + k, v);
+            grid.sync();
+        }
+        if (f.edit1[k] > f.edit0[k]) {
+            uint32_t c[4] = {0u, 0u, 0u, 0u};
+            for_each_group<true>(sm, a.req, a.freq, g, chunk_of(f.edit1[k] - f.edit0[k]), f.edit0[k], f.edit1[k],
+                                 [&](uint32_t total, uint32_t, bool) { edit_words<T>(sm, a, nxt, fnxt, total, c); });
+            const uint32_t v[8] = {0u, 0u, 0u, c[0], c[1], c[2], 0u, 0u};
+            block_flush_slot(a.slots + k, v);
+            grid.sync();
+        }
+    }
+}
+
+// After the wavefront has run sweeps 0 .. K to the end: the state after sweep
+// K, or after the first of those sweeps that stops the loop (the sweeps after a
+// stopping one changed nothing: they found an empty active set, or repeated a
+// sweep whose edits changed no value and no counter, or follow a NaN input
+// whose call fails).
+static __global__ void k_wave_gate(LoopState *ls, const SweepSlot *slots, long long K, long long max_sweeps) {
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    long long k = 0;
+    bool stop = false;
+    for (; k <= K; ++k) {
+        const SweepSlot c = slots[k];
+        stop = (k == 0 && c.bad) || sweep_stops(c.fmax, c.fmin, c.fdir, c.progressed, k + 1, max_sweeps);
+        if (stop) break;
+    }
+    ls->k = stop ? k + 1 : K + 1;
+    ls->go = stop ? 0 : 1;
 }
 
 }  // namespace pmsz

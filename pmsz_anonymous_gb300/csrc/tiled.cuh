@@ -292,17 +292,6 @@ struct ApplyFlush {
     }
 };
 
-__device__ __forceinline__ void flush_apply_counts(SweepSlot *slot, uint32_t nreq, uint32_t nchg, uint32_t nprog) {
-    nreq = warp_sum_u32(nreq);
-    nchg = warp_sum_u32(nchg);
-    nprog = warp_sum_u32(nprog);
-    if ((threadIdx.x & 31) == 0) {
-        if (nreq) atomicAdd(&slot->requested, (unsigned long long)nreq);
-        if (nchg) atomicAdd(&slot->changed, (unsigned long long)nchg);
-        if (nprog) atomicAdd(&slot->progressed, (unsigned long long)nprog);
-    }
-}
-
 template <typename T>
 __device__ __forceinline__ void apply_body(ListSmem &sm, const T *__restrict__ f, T *__restrict__ fh,
                                            uint8_t *__restrict__ cnt, uint32_t *__restrict__ hp,
