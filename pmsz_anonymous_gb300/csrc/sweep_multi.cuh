@@ -169,17 +169,8 @@ __device__ __forceinline__ void multi_phase(MultiSmem &ms, const FieldMasks &m, 
             if (mask_bit(mask, fi)) {
                 const Inst<T> &J = t.inst[fi];
                 uint8_t *flag = (PHASE == 1 ? J.freq : ((J.k + it) & 1) ? J.f1 : J.f0) + local;
-                if (chunk == 8) {
-                    const uint2 b = *reinterpret_cast<const uint2 *>(flag);
-                    if (b.x | b.y) *reinterpret_cast<uint2 *>(flag) = make_uint2(0u, 0u);
-                    fm = (((b.x * 0x01020408u) >> 24) & 0xFu) | (((b.y * 0x01020408u) >> 20) & 0xF0u);
-                } else {
-                    for (uint32_t j = 0; j < chunk; ++j)  // (the flags are padded to whole chunks of eight)
-                        if (flag[j]) {
-                            flag[j] = 0;
-                            fm |= 1u << j;
-                        }
-                }
+                fm = chunk_flags(flag, chunk);  // (padded to whole chunks of eight)
+                if (fm) clear_chunk_flags(flag, chunk);
             }
         }
         const uint32_t cnt = static_cast<uint32_t>(__popc(fm));
