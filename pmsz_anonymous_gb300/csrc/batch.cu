@@ -247,6 +247,7 @@ static int run_batch(MultiRun<float> *r32, MultiRun<double> *r64, std::vector<Ba
     if (r32) a.t32 = r32->table();
     if (r64) a.t64 = r64->table();
     a.ctl = r32 ? r32->ctl : r64->ctl;
+    PMSZ_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(SweepCtl), s));
     if ((rc = launch_multi_sweeps(a, s))) return rc;
     // the sweep count and, up to 256 KB a type, the first rows in pinned memory
     auto ahead = [](int n, int64_t max_sweeps) {
@@ -261,6 +262,7 @@ static int run_batch(MultiRun<float> *r32, MultiRun<double> *r64, std::vector<Ba
     if (b32) PMSZ_CUDA(cudaMemcpyAsync(hb + 256, r32->slots, b32, cudaMemcpyDeviceToHost, s));
     if (b64) PMSZ_CUDA(cudaMemcpyAsync(hb + 256 + b32, r64->slots, b64, cudaMemcpyDeviceToHost, s));
     PMSZ_CUDA(cudaStreamSynchronize(s));
+    if (reinterpret_cast<const SweepCtl *>(hb)->err) return set_error(PMSZ_ERR_CUDA, kBarrierMissing);
     const int64_t total = reinterpret_cast<const SweepCtl *>(hb)->iters;  // sweeps 0 .. total - 1
     auto collect = [&](auto *run, const unsigned char *head, int64_t have, std::vector<BatchOutcome> &out) -> int {
         if (!run) return PMSZ_OK;

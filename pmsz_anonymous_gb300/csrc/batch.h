@@ -110,9 +110,10 @@ struct SweepTable {
     uint32_t chunks = 0;             // their total
     SweepReport *report = nullptr;   // n
 };
-struct SweepCtl {
+struct SweepCtl {  // zero before the launch
     long long iters;  // sweeps run by the launch
     int yield[2];
+    uint32_t bar, err;  // the grid barrier's arrivals; kErrBarrier
 };
 struct MultiSweeps {
     SweepTable<float> t32;

@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cstring>
 #include <chrono>
+#include <iterator>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -414,6 +415,7 @@ int first_pass_ingest(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes
 // 4, 8, 12, 14, 16: 2538 and 11.64; at 12, 15, 16: 2626 and 11.51; without waves
 // 2718 and 13.02.  (As voxel lists, seven launches a piece: 3347 us and 11.80.)
 constexpr int kWaveAt[] = {8, 12, 14, 15, 16};
+static_assert(std::size(kWaveAt) < std::size(LoopState{}.bar), "a barrier counter for each");
 
 // The host-buffer wavefront.  The copy of slab j releases the first pass
 // of slab j (sweep 0's detection, complete below plane Z = (j + 1) * slab
@@ -471,6 +473,7 @@ static int first_pass_waves(const HostIngest<T> &in, const SweepArgs<T> &a, cons
             Ap[k] = A;
             widest = std::max<size_t>(widest, std::max(f.det1[k] - f.det0[k], f.edit1[k] - f.edit0[k]));
         }
+        ++f.launch;
         if ((rc = launch_cooperative<T>(k_sweep_wave<T>, widest, s, a, f))) return rc;
         ++*launches;
     }
@@ -596,7 +599,7 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
             if ((rc = ingest->after->fn(s))) return rc;
         }
         PMSZ_CUDA(cudaStreamSynchronize(s));
-        if (hls->err) return set_error(PMSZ_ERR_CUDA, kCopyMissing);
+        if (hls->err) return set_error(PMSZ_ERR_CUDA, hls->err & kErrCopy ? kCopyMissing : kBarrierMissing);
         const int64_t done = hls->done;  // sweeps 0 .. done-1
         if (timing) {  // sweep 0's edits run inside the launch and count as detection time
             float x = 0, y = 0;

@@ -91,6 +91,8 @@ struct EventTimer {
 // per slot (0: the correction's read-back, 1: the edit output's totals).
 void *host_pinned(size_t bytes, int slot = 0);
 
+constexpr char kBarrierMissing[] = "sweeps: a grid barrier did not complete within the bounded wait";
+
 // Implementations behind the C entry points (explicitly instantiated for
 // float and double in their translation units).
 int check_geom(size_t nx, size_t ny, size_t nz);

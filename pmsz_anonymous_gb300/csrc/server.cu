@@ -289,9 +289,11 @@ private:
         a.ctl = reinterpret_cast<SweepCtl *>(buf_.drep);
         a.yield = dyield_;
         a.until_stop = 1;
+        PMSZ_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(SweepCtl), s_));
         if ((rc = launch_multi_sweeps(a, s_))) return rc;
         PMSZ_CUDA(cudaMemcpyAsync(buf_.rep, buf_.drep, rep, cudaMemcpyDeviceToHost, s_));
         PMSZ_CUDA(cudaStreamSynchronize(s_));
+        if (reinterpret_cast<const SweepCtl *>(buf_.rep)->err) return set_error(PMSZ_ERR_CUDA, kBarrierMissing);
         read(g32);
         read(g64);
         return PMSZ_OK;

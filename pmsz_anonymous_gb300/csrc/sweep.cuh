@@ -144,8 +144,38 @@ struct LoopState {
     int go;               // that sweep runs
     uint32_t lc[4];       // [3]: first-pass decisions on full keys
     uint32_t deferred[2]; // voxels of a sweep decided on full keys, by the sweep's parity (fp32)
-    uint32_t err;         // set by the first pass when a tensor copy did not arrive
+    uint32_t err;         // kErrCopy, kErrBarrier
+    uint32_t bar[8];      // arrivals at the grid barriers of k_sweeps, and of the wavefront's launches
 };
+constexpr uint32_t kErrCopy = 1;     // set by the first pass: a tensor copy did not arrive
+constexpr uint32_t kErrBarrier = 2;  // set by a sweep kernel: a grid barrier did not complete
+
+// Grid barrier of a cooperative launch: `target` counts the arrivals that
+// complete the next one (a counter of the launch's own, zero before it).  The
+// arrival returns nothing, so a block polls right behind it; cooperative
+// groups' barrier waits for its arrival's answer first (a batch of 32 fields
+// 5803 us with that, 5681 with this; a burst of jobs 3998 and 3831).  Bounded:
+// all blocks are resident, but if one did not arrive, *err is set and the block
+// leaves (the result says so: the caller returns), as every other one then does.
+constexpr int kBarrierTries = 1 << 22;  // seconds
+__device__ __forceinline__ bool sweep_barrier(uint32_t *bar, uint32_t &target, uint32_t *err) {
+    target += gridDim.x;
+    __syncthreads();
+    int failed = 0;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        int tries = 0;
+        uint32_t seen;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+        } while (static_cast<int32_t>(seen - target) < 0 && ++tries < kBarrierTries);
+        if (tries == kBarrierTries) {
+            atomicOr(err, kErrBarrier);
+            failed = 1;
+        }
+    }
+    return __syncthreads_or(failed) == 0;
+}
 
 // Lanes whose voxels share a bitmap word carry the same key; in a list in
 // voxel order they are consecutive lanes.  ORs the changed bits cb over each
@@ -602,7 +632,7 @@ __device__ __forceinline__ void for_each_group(SweepSmem &sm, uint32_t *bm, uint
 template <typename T>
 __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps(const __grid_constant__ SweepArgs<T> a) {
     __shared__ SweepSmem sm;
-    cg::grid_group grid = cg::this_grid();
+    uint32_t target = 0;  // of the grid barrier
     const Geom &g = a.g;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t chunk = 8;
@@ -640,7 +670,7 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps(const __grid_constant
                 __syncthreads();
                 if (threadIdx.x == 0 && sm.deferred) atomicAdd(&a.ls->deferred[k & 1], sm.deferred);
             }
-            grid.sync();
+            if (!sweep_barrier(&a.ls->bar[0], target, &a.ls->err)) return;
             if (sizeof(T) == 4) {
                 keys = keys || 10ull * a.ls->deferred[k & 1] > a.slots[k].active;
                 if (blockIdx.x == 0 && threadIdx.x == 0) a.ls->deferred[(k + 1) & 1] = 0;
@@ -654,7 +684,7 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps(const __grid_constant
             const uint32_t v[8] = {0u, 0u, 0u, c[0], c[1], c[2], 0u, 0u};
             block_flush_slot(a.slots + k, v);
         }
-        grid.sync();
+        if (!sweep_barrier(&a.ls->bar[0], target, &a.ls->err)) return;
         ++k;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) a.ls->done = k;
@@ -669,13 +699,14 @@ constexpr int kWaveSweeps = 6;
 struct WaveFronts {  // words: the fronts of the launch before and of this one
     uint32_t det0[kWaveSweeps + 1], det1[kWaveSweeps + 1], edit0[kWaveSweeps + 1], edit1[kWaveSweeps + 1];
     int sweeps;             // K
+    int launch;             // its barrier counter, 1 ..
     unsigned long long seen;  // voxels of the first passes so far
 };
 template <typename T>
 __global__ void __launch_bounds__(kSweepBlock, 3) k_sweep_wave(const __grid_constant__ SweepArgs<T> a,
                                                                const __grid_constant__ WaveFronts f) {
     __shared__ SweepSmem sm;
-    cg::grid_group grid = cg::this_grid();
+    uint32_t target = 0;  // of the grid barrier
     const Geom &g = a.g;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp == 0) fill_steps(sm.step, g, lane);
@@ -698,7 +729,7 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweep_wave(const __grid_cons
                                  });
             const uint32_t v[8] = {c[0], c[1], c[2], 0u, 0u, 0u, c[3], 0u};
             block_flush_slot(a.slots + k, v);
-            grid.sync();
+            if (!sweep_barrier(&a.ls->bar[f.launch], target, &a.ls->err)) return;
         }
         if (f.edit1[k] > f.edit0[k]) {
             uint32_t c[4] = {0u, 0u, 0u, 0u};
@@ -706,7 +737,7 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweep_wave(const __grid_cons
                                  [&](uint32_t total, uint32_t, bool) { edit_words<T>(sm, a, nxt, fnxt, total, c); });
             const uint32_t v[8] = {0u, 0u, 0u, c[0], c[1], c[2], 0u, 0u};
             block_flush_slot(a.slots + k, v);
-            grid.sync();
+            if (!sweep_barrier(&a.ls->bar[f.launch], target, &a.ls->err)) return;
         }
     }
 }

@@ -289,7 +289,7 @@ __device__ __forceinline__ void write_reports(const FieldMasks &m, const SweepTa
 // every block sees the same value, through ctl->yield).
 __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps_multi(const __grid_constant__ MultiSweeps a) {
     __shared__ MultiSmem ms;
-    cg::grid_group grid = cg::this_grid();
+    uint32_t target = 0;  // of the grid barrier
     const bool first = blockIdx.x == 0;
     auto chunk_for = [&](uint64_t chunks) -> uint32_t {  // as in k_sweeps
         uint32_t c = 8;
@@ -314,12 +314,12 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps_multi(const __grid_co
         if (a.yield && first && threadIdx.x == 0) want = *a.yield;  // read while the sweep runs
         multi_phase<float, 0>(ms, ms.m32, a.t32, c32, it, home32, local32);
         multi_phase<double, 0>(ms, ms.m64, a.t64, c64, it, home64, local64);
-        grid.sync();
+        if (!sweep_barrier(&a.ctl->bar, target, &a.ctl->err)) return;
         if (first) next_deferred(ms.m32, a.t32, it);
         multi_phase<float, 1>(ms, ms.m32, a.t32, c32, it, home32, local32);
         multi_phase<double, 1>(ms, ms.m64, a.t64, c64, it, home64, local64);
         if (a.yield && first && threadIdx.x == 0) a.ctl->yield[it & 1] = want;
-        grid.sync();
+        if (!sweep_barrier(&a.ctl->bar, target, &a.ctl->err)) return;
         ++it;
     }
     if (first) {
