@@ -26,20 +26,23 @@
 //  * Failed certificates wait in a per-warp buffer and are decided on full keys
 //    32 at a time; fp32 fields with many (plateaus) detect on full keys
 //    throughout.
-//  * Dense visits collect their result bits in shared memory (SweepBits).
+//  * Result bits collect in shared memory, one word of them per bitmap word
+//    (SweepBits), and go out once per four groups: one atomic per word instead
+//    of one per voxel, and the closed stencils of all 32 words' changes marked
+//    side by side instead of word after word.
 //
 // Bound by the latency of the gathers (issue slots 40 % used) and, in small
 // fields and late sweeps, of the two grid barriers a sweep takes (about 2 us
-// each).  Three blocks per SM: four (64 registers) are 0-10 % slower.  The code
-// is kept small and with one site per decision: with dense and sparse visits as
-// two copies the same work took 15-25 % longer.
+// each).  Three blocks per SM: four (64 registers) are up to 8 % slower.  The
+// code is kept small and with one site per decision: with dense and sparse
+// visits as two copies the same work took 15-25 % longer.
 // Whole corrections: list kernels in a conditional CUDA graph -> warps on their
 // own chunks, every bit an atomic -> this:
-//   64^3 fp32, 8 sweeps              358 -> 181 -> 172 us
-//   173x141x203 fp32, 12 sweeps      560 -> 353 -> 335 us
-//   512^3 fp64, 16 sparse sweeps    3852 -> 3355 -> 3248 us
-//   256^3 fp32, 27 dense sweeps     4727 -> 4467 -> 3744 us (on full keys)
-//   160^3 fp64, 40 dense sweeps     2308 -> 2320 -> 2046 us
+//   64^3 fp32, 8 sweeps              358 -> 181 -> 163 us
+//   173x141x203 fp32, 12 sweeps      560 -> 353 -> 299 us
+//   512^3 fp64, 16 sparse sweeps    3852 -> 3355 -> 3211 us
+//   256^3 fp32, 27 dense sweeps     4727 -> 4467 -> 3111 us (on full keys)
+//   160^3 fp64, 40 dense sweeps     2308 -> 2320 -> 1664 us
 #pragma once
 #include "march.cuh"
 
@@ -78,61 +81,46 @@ __device__ __forceinline__ void fill_steps(SweepStep *t, const Geom &g, int lane
 
 // A warp's result bits for the 32 words it visits at a time: the words' own
 // (mismatches, changes) and the requests into their seven rows.  Collected
-// here they go out as one atomic per word instead of up to three per voxel
-// (L2 takes one atomic of an address at a time: 160^3 fp64, 40 dense sweeps,
-// 2393 us without, 2012 us with).
+// here they go out as one atomic per word instead of up to three per voxel (L2
+// takes one atomic of an address at a time: 160^3 fp64, 40 dense sweeps, 2393 ->
+// 2012 us with detection's, -> 1664 us with the edits' and their marks).
 struct SweepBits {
     uint32_t own[32], row[kSweepRows][32];  // zero between visits
 };
 
-__device__ __forceinline__ void or_word_f(uint32_t *act, uint8_t *flag, const Geom &g, int wx, int y, int z, uint32_t m) {
-    if (!m || wx < 0 || wx >= g.wpr || y < 0 || y >= g.ny || z < 0 || z >= g.nz) return;
-    m &= row_tail_mask(g, wx);
-    if (!m) return;
-    const size_t w = static_cast<size_t>(wx) + static_cast<size_t>(g.wpr) * (static_cast<size_t>(y) + static_cast<size_t>(g.ny) * z);
-    atomicOr(act + w, m);
-    flag[w / kGroupWords] = 1;
-}
-__device__ __forceinline__ void mark_stencil_f(uint32_t *act, uint8_t *flag, const Geom &g, int wx, int y, int z,
-                                               uint32_t c) {
-    const uint32_t lo = (c & 1u) << 31, hi = c >> 31;
-    or_word_f(act, flag, g, wx, y, z, c | (c << 1) | (c >> 1));
-    or_word_f(act, flag, g, wx - 1, y, z, lo);
-    or_word_f(act, flag, g, wx + 1, y, z, hi);
-    const uint32_t m = c | (c >> 1), p = c | (c << 1);
-    or_word_f(act, flag, g, wx, y + 1, z, m);     or_word_f(act, flag, g, wx - 1, y + 1, z, lo);
-    or_word_f(act, flag, g, wx, y, z + 1, m);     or_word_f(act, flag, g, wx - 1, y, z + 1, lo);
-    or_word_f(act, flag, g, wx, y + 1, z + 1, m); or_word_f(act, flag, g, wx - 1, y + 1, z + 1, lo);
-    or_word_f(act, flag, g, wx, y - 1, z, p);     or_word_f(act, flag, g, wx + 1, y - 1, z, hi);
-    or_word_f(act, flag, g, wx, y, z - 1, p);     or_word_f(act, flag, g, wx + 1, y, z - 1, hi);
-    or_word_f(act, flag, g, wx, y - 1, z - 1, p); or_word_f(act, flag, g, wx + 1, y - 1, z - 1, hi);
-}
-
-// Marks the closed stencils of the changed bits c of the lanes' words (every
-// lane calls it).  Many words: each lane's own marks one after the other, 350
-// instructions for up to 32 words.  Few -- runs of changed voxels, as in dense
-// sweeps: one word after the other, its marks on 15 lanes, 40 instructions each.
-__device__ __forceinline__ void mark_stencils(uint32_t *act, uint8_t *flag, const Geom &g, int wx, int y, int z, uint32_t c) {
-    uint32_t m = __ballot_sync(0xFFFFFFFFu, c != 0);
-    if (__popc(m) > 4) {
-        if (c) mark_stencil_f(act, flag, g, wx, y, z, c);
-        return;
+// Marks the closed stencil of the changed bits c of word w (x word wx, row y,
+// plane z): the word itself and its six rows' by constant steps from w, the
+// neighbouring words only where c reaches them.
+__device__ __forceinline__ void mark_words(uint32_t *act, uint8_t *flag, const Geom &g, uint32_t w, int wx, int y, int z,
+                                           uint32_t c) {
+    const uint32_t tail = wx + 1 == g.wpr ? row_tail_mask(g, wx) : 0xFFFFFFFFu;
+    const uint32_t sy = static_cast<uint32_t>(g.wpr), sz = sy * static_cast<uint32_t>(g.ny);
+    const bool yp = y + 1 < g.ny, yn = y > 0, zp = z + 1 < g.nz, zn = z > 0;
+    auto put = [&](uint32_t at, uint32_t m) {
+        atomicOr(act + at, m);
+        flag[at / kGroupWords] = 1;
+    };
+    const uint32_t p = c | (c >> 1), n = (c | (c << 1)) & tail;  // the rows ahead hold dx = 0, 1, the rows behind -1, 0
+    put(w, p | n);
+    if (yp) put(w + sy, p);
+    if (zp) put(w + sz, p);
+    if (yp && zp) put(w + sy + sz, p);
+    if (yn) put(w - sy, n);
+    if (zn) put(w - sz, n);
+    if (yn && zn) put(w - sy - sz, n);
+    if ((c & 1u) && wx > 0) {
+        const uint32_t l = w - 1, m = 1u << 31;
+        put(l, m);
+        if (yp) put(l + sy, m);
+        if (zp) put(l + sz, m);
+        if (yp && zp) put(l + sy + sz, m);
     }
-    // lane l < 14: row l / 2, and its own word (even) or the neighbouring one
-    // that the row's shifted bits reach (odd); row 0's second one is lane 14's
-    const int lane = threadIdx.x & 31, row = lane == 14 ? 0 : lane >> 1;
-    const int dy = row_dy(row), dz = row_dz(row);
-    const bool left = row <= 3 && lane != 14, right = row == 0 || row >= 4;
-    for (; m; m &= m - 1) {
-        const int src = __ffs(m) - 1;
-        const uint32_t cb = __shfl_sync(0xFFFFFFFFu, c, src);
-        const int bx = __shfl_sync(0xFFFFFFFFu, wx, src), by = __shfl_sync(0xFFFFFFFFu, y, src),
-                  bz = __shfl_sync(0xFFFFFFFFu, z, src);
-        if (lane < 15) {
-            const bool side = lane == 14 || (lane & 1);
-            const uint32_t bits = side ? (left ? cb << 31 : cb >> 31) : cb | (left ? cb >> 1 : 0u) | (right ? cb << 1 : 0u);
-            or_word_f(act, flag, g, bx + (side ? (left ? -1 : 1) : 0), by + dy, bz + dz, bits);
-        }
+    if ((c >> 31) && wx + 1 < g.wpr) {
+        const uint32_t r = w + 1;
+        put(r, 1u);
+        if (yn) put(r - sy, 1u);
+        if (zn) put(r - sz, 1u);
+        if (yn && zn) put(r - sy - sz, 1u);
     }
 }
 
@@ -175,22 +163,6 @@ __device__ __forceinline__ bool sweep_barrier(uint32_t *bar, uint32_t &target, u
         }
     }
     return __syncthreads_or(failed) == 0;
-}
-
-// Lanes whose voxels share a bitmap word carry the same key; in a list in
-// voxel order they are consecutive lanes.  ORs the changed bits cb over each
-// group (a suffix OR within the group) and returns true on the group's lowest
-// lane when the merged bits are non-zero: that lane marks the word's closed
-// stencil once for the whole group.
-__device__ __forceinline__ bool warp_merge_word(uint32_t key, uint32_t &cb) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t grp = __match_any_sync(0xFFFFFFFFu, key);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_down_sync(0xFFFFFFFFu, cb, o);
-        if (lane + o < 32 && ((grp >> (lane + o)) & 1u)) cb |= u;
-    }
-    return cb && lane == static_cast<uint32_t>(__ffs(grp) - 1);
 }
 
 template <typename T>
@@ -390,12 +362,6 @@ __device__ __forceinline__ SweepVoxel sweep_voxel(const SweepSmem &sm, uint32_t 
     return v;
 }
 
-// Four groups with this many set bits (of 1024) collect their result bits in
-// shared memory: below, sending the few that are left out one by one costs less
-// than the eight words per lane (from 64 on 160^3 fp64 takes 1949 us, from 192
-// on 2027 us; sparse fields are the same).
-constexpr uint32_t kSweepDense = 64;
-
 // Detection of the `total` listed voxels of a warp's 32 words (lane l holds
 // word w): on the proxies, failed certificates into the warp's buffer (ndefer
 // entries), or (keys) on full keys throughout.  The buffer is decided on full
@@ -407,7 +373,6 @@ __device__ __forceinline__ void detect_words(SweepSmem &sm, const A &a, const Sw
                                              uint32_t &ndefer, uint32_t &ndeferred) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     SweepBits &bits = sm.bits[warp];
-    const bool dense = total >= kSweepDense;
     v[3] += lane == 0 ? total : 0u;
     for (uint32_t j = 0;;) {
         const bool buffered = ndefer >= 32 || (finish && ndefer && j >= total);
@@ -423,7 +388,7 @@ __device__ __forceinline__ void detect_words(SweepSmem &sm, const A &a, const Sw
                 const Ext e = all_inside ? sweep_proxies(a, i) : sweep_proxies_face(a, i, p.x, p.y, p.z);
                 open = !e.exact;
                 if (!open)
-                    sweep_outcome(a, steps, bits, dense, nxt, fnxt, p.entry, p.w, e.asc, e.desc, c, v[0], v[1], v[2]);
+                    sweep_outcome(a, steps, bits, true, nxt, fnxt, p.entry, p.w, e.asc, e.desc, c, v[0], v[1], v[2]);
             }
             const uint32_t md = __ballot_sync(0xFFFFFFFFu, open);
             if (md) {
@@ -458,11 +423,10 @@ __device__ __forceinline__ void detect_words(SweepSmem &sm, const A &a, const Sw
             const size_t i = flat(a.g, p.x, p.y, p.z);
             int asc, desc;
             sweep_keys<T>(a, i, p.x, p.y, p.z, inside, asc, desc);
-            sweep_outcome(a, steps, bits, dense && !buffered, nxt, fnxt, p.entry, p.w, asc, desc, __ldg(a.codes + i), v[0],
+            sweep_outcome(a, steps, bits, !buffered, nxt, fnxt, p.entry, p.w, asc, desc, __ldg(a.codes + i), v[0],
                           v[1], v[2]);
         }
     }
-    if (!dense) return;
     __syncwarp();
     const uint32_t own = bits.own[lane];
     if (own) {
@@ -492,8 +456,14 @@ __device__ __forceinline__ void edit_words(SweepSmem &sm, const A &a, uint32_t *
         const SweepVoxel p = sweep_voxel(sm, j, total);
         uint32_t cb = 0;
         if (p.on && sweep_edit<T>(a, flat(a.g, p.x, p.y, p.z), v[0], v[1], v[2])) cb = 1u << (p.entry & 31u);
-        const bool lead = warp_merge_word(p.on ? p.w : 0xFFFFFFFFu, cb);
-        mark_stencils(nxt, fnxt, a.g, p.x >> 5, p.y, p.z, lead ? cb : 0u);
+        if (cb) atomicOr(&sm.bits[warp].own[p.entry >> 5], cb);
+    }
+    __syncwarp();
+    const uint32_t c = sm.bits[warp].own[lane];
+    if (c) {
+        sm.bits[warp].own[lane] = 0;
+        const int4 at = sm.at[warp][lane];
+        mark_words(nxt, fnxt, a.g, static_cast<uint32_t>(at.w), at.x >> 5, at.y, at.z, c);
     }
 }
 
