@@ -174,13 +174,18 @@ constexpr int kZChunkDefault = 32;  // zc when no tuned value is recorded for th
 constexpr int kTX = 32, kMY = 8;
 constexpr int kMarchMaxDepth = 64;  // deeper columns run as this (the passes keep bitmaps of a column)
 inline int march_depth(int zc) { return zc < kMarchMaxDepth ? zc : kMarchMaxDepth; }
-// Depth without a tuned value: the default, halved while the launch has fewer
-// columns than six blocks per SM (152 SMs hold six), down to 4 -- a 64^3 field
+// Depth without a tuned value.  152 SMs hold six columns each.  64 planes where
+// that leaves four rounds of columns (512^3 fp64: first pass 1204 -> 1178 us
+// against 32, and the two halo planes of a column are read half as often; with
+// two rounds, 256^3, the last one is too empty: 485 -> 587 us), else 32, halved
+// while a launch has fewer columns than the SMs hold, down to 4 -- a 64^3 field
 // has 16 columns of 32 x 8, and 32 planes deep they leave most SMs idle and
 // every block a long serial march (first pass 75 us at depth 32, 19 us at 4);
 // below 4 the two halo planes of a column cost more than the extra blocks gain.
-inline int default_depth(uint64_t columns_planes, int zc = kZChunkDefault) {  // sum over fields of columns * nz
-    while (zc > 4 && columns_planes / static_cast<uint64_t>(zc) < 152u * 6u) zc /= 2;
+inline int default_depth(uint64_t columns_planes) {  // sum over fields of columns * nz
+    int zc = kMarchMaxDepth;
+    if (columns_planes / static_cast<uint64_t>(zc) < 152u * 6u * 4u) zc /= 2;
+    while (zc <= 32 && zc > 4 && columns_planes / static_cast<uint64_t>(zc) < 152u * 6u) zc /= 2;
     return zc;
 }
 inline uint64_t column_planes(size_t nx, size_t ny, size_t nz) {

@@ -345,7 +345,9 @@ int enqueue_ingest(const T *hf, const T *hfh, T *df, T *dfh, T *dprev, size_t nx
     int rc = check_geom(nx, ny, nz);
     if (rc) return rc;
     Geom g = make_geom(nx, ny, nz);
-    g.zc = first_depth(nx, ny, nz, sizeof(T));  // the tile depth correct_impl will use
+    // the tile depth correct_impl will use; slabs are whole columns, and the last
+    // one is what is left when the copy ends, so at most 32 planes
+    g.zc = std::min(first_depth(nx, ny, nz, sizeof(T)), 32);
     const IngestSlabs sl = ingest_slabs(g, sizeof(T));
     c.cps = sl.cps;
     c.nchunks = sl.nchunks;
@@ -500,7 +502,7 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         (rc = autotune_impl<T>(f, fh, nx, ny, nz, nullptr, s)))
         return rc;
     Geom g = make_geom(nx, ny, nz);
-    g.zc = first_depth(nx, ny, nz, sizeof(T));
+    g.zc = ingest && ingest->copies ? ingest->copies->zc : first_depth(nx, ny, nz, sizeof(T));
     const T eps = static_cast<T>(eb);
     const T delta = static_cast<T>(eb / static_cast<double>(q));  // pMSz.cu:2814
 
