@@ -47,9 +47,9 @@
 // fp32 first pass took 754 us, then 626; with the
 // values compared directly on ties 485).
 //
-// Measured at 512^3, issue-bound throughout: first pass fp64 1.50 -> 1.19 ms
-// (350 -> 220 warp instructions per 32 voxels), fp32 1.07 ms; codes alone
-// 0.61 ms fp64, 0.54 ms fp32.  One voxel per thread, 256-thread blocks, the two
+// Measured at 512^3, issue-bound throughout: first pass fp64 1.50 -> 1.18 ms
+// (350 -> 220 warp instructions per 32 voxels), fp32 1.05 ms; codes alone
+// 0.58 ms fp64, 0.54 ms fp32.  One voxel per thread, 256-thread blocks, the two
 // fields on different warps and 15 gathers per lane in the exact queue were all
 // slower.
 #pragma once
