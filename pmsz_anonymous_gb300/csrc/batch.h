@@ -20,7 +20,6 @@ struct Inst {
     uint8_t *codes, *cnt;
     uint32_t *hp, *req, *act0, *act1;
     uint8_t *freq, *f0, *f1;  // group flags of req, act0, act1, padded to whole chunks of eight groups
-    uint32_t *def;      // voxels decided on full keys: the first pass, even and odd sweeps; [3]: full keys for good
     SweepSlot *slots;   // this field's slot of sweep k is slots[k * stride]
     int64_t stride;
     Geom g;
@@ -48,11 +47,10 @@ struct BatchOutcome {
 };
 
 // Scratch of one field, at 256-byte offsets: first what starts at zero
-// (counters, bitmaps and their group flags, the full-key counts), then codes
-// and proxies.  The sweep slots are the caller's.
+// (counters, bitmaps and their group flags), then codes and, fp64, proxies.  The sweep slots are the caller's.
 struct FieldScratch {
-    size_t cnt, req, act0, act1, freq, f0, f1, def, zero, codes, hp, total;
-    explicit FieldScratch(const Geom &g) {
+    size_t cnt, req, act0, act1, freq, f0, f1, zero, codes, hp, total;
+    FieldScratch(const Geom &g, size_t elem) {
         size_t at = 0;
         auto take = [&](size_t bytes) {
             const size_t off = at;
@@ -67,10 +65,9 @@ struct FieldScratch {
         freq = take(groups);
         f0 = take(groups);
         f1 = take(groups);
-        def = take(4 * sizeof(uint32_t));
         zero = at;
         codes = take(g.n);
-        hp = take(4 * g.n);
+        hp = take(elem == 8 ? 4 * g.n : 0);
         total = at;
     }
     // The table row's scratch pointers: zeroed part at z, the rest at r
@@ -84,9 +81,8 @@ struct FieldScratch {
         I.freq = z + freq;
         I.f0 = z + f0;
         I.f1 = z + f1;
-        I.def = reinterpret_cast<uint32_t *>(z + def);
         I.codes = r + codes;
-        I.hp = reinterpret_cast<uint32_t *>(r + hp);
+        I.hp = sizeof(T) == 8 ? reinterpret_cast<uint32_t *>(r + hp) : nullptr;
     }
 };
 // Chunks of eight groups (kGroupWords words each) of a field.

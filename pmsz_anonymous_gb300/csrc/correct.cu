@@ -31,6 +31,8 @@
 #include <iterator>
 #include <mutex>
 #include <string>
+#include <tuple>
+#include <utility>
 #include <vector>
 
 namespace pmsz {
@@ -252,12 +254,12 @@ constexpr char kCopyMissing[] = "first pass: a tile plane's tensor copy did not 
 
 // The fused first pass over the z-chunks bz0 .. bz0+grid.z-1: TMA-fed when the
 // maps exist; *err is set if a plane's copy did not arrive within the bounded
-// wait, *xc += the voxels decided on full keys.
+// wait.
 template <typename T>
 static int launch_first_pass(const FirstMaps &m, dim3 grid, cudaStream_t s, const T *f, T *fh, uint8_t *codes,
                              uint32_t *hp, uint32_t *req, uint32_t *act, SweepSlot *slot, const Geom &g, int bz0,
-                             uint32_t *xc, uint32_t *err, uint8_t *freq = nullptr, uint8_t *fact = nullptr) {
-    const MarchArgs<T> a{f, fh, codes, hp, req, nullptr, act, slot, xc, freq, fact};
+                             uint32_t *err, uint8_t *freq = nullptr, uint8_t *fact = nullptr) {
+    const MarchArgs<T> a{f, fh, codes, hp, req, nullptr, act, slot, freq, fact};
     if (m.ok) {
         PMSZ_CUDA(allow_smem(k_pair_tma<T, kFirst>, sizeof(TmaMarch<T>)));
         k_pair_tma<T, kFirst><<<grid, dim3(kTX, kThreads / kTX, 1), sizeof(TmaMarch<T>), s>>>(m.f, m.fh, a, g, bz0, err);
@@ -268,32 +270,37 @@ static int launch_first_pass(const FirstMaps &m, dim3 grid, cudaStream_t s, cons
     return PMSZ_OK;
 }
 
-// A sweep kernel over all resident blocks of the current device (three per SM:
-// queried once per device, since the queries cost more than a small field's
-// sweep), or as many as `words` bitmap words keep busy.
+// A sweep kernel over all resident blocks of the current device (queried once
+// per device, since the queries cost more than a small field's sweep), or as
+// many as `words` bitmap words keep busy.
 template <typename T, class Kernel, class... Args>
 static int launch_cooperative(Kernel kernel, size_t words, cudaStream_t s, const Args &...args) {
     static std::mutex mu;
-    static std::vector<unsigned> known;
-    unsigned blocks = 0;
+    static std::vector<std::pair<unsigned, unsigned>> known;  // resident blocks; three per SM
+    unsigned blocks = 0, three = 0;
     {
         int dev = 0;
         PMSZ_CUDA(cudaGetDevice(&dev));
         std::lock_guard<std::mutex> lk(mu);
-        if (static_cast<size_t>(dev) >= known.size()) known.resize(static_cast<size_t>(dev) + 1, 0u);
-        if (!known[static_cast<size_t>(dev)]) {
+        if (static_cast<size_t>(dev) >= known.size()) known.resize(static_cast<size_t>(dev) + 1, {0u, 0u});
+        if (!known[static_cast<size_t>(dev)].first) {
             int sms = 0, per_sm = 0, coop = 0;
             PMSZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             PMSZ_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
             if (!coop) return set_error(PMSZ_ERR_CUDA, "device does not support cooperative launches");
             PMSZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSweepBlock, 0));
             if (per_sm < 1) return set_error(PMSZ_ERR_CUDA, "sweep kernel does not fit on an SM");
-            known[static_cast<size_t>(dev)] = static_cast<unsigned>(per_sm * sms);
+            known[static_cast<size_t>(dev)] = {static_cast<unsigned>(per_sm * sms), static_cast<unsigned>(3 * sms)};
         }
-        blocks = known[static_cast<size_t>(dev)];
+        std::tie(blocks, three) = known[static_cast<size_t>(dev)];
     }
     const size_t groups = (words + kGroupWords - 1) / kGroupWords, want = (groups + kSweepWarps - 1) / kSweepWarps;
-    const unsigned grid = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(want, blocks)));
+    // fp32 fits four blocks per SM: they pay where every warp has eight groups
+    // (512^3 1966 us with three, 1871 with four; 256^3 2844 and 2662), fields
+    // below wait for their gathers less than for the larger barrier (128^3 383
+    // and 400, 120x130x128 931 and 990)
+    const unsigned most = groups >= 8u * kSweepWarps * static_cast<size_t>(blocks) ? blocks : std::min(blocks, three);
+    const unsigned grid = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(want, most)));
     void *ptr[] = {const_cast<void *>(static_cast<const void *>(&args))...};
     PMSZ_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(kSweepBlock), ptr, 0, s));
     return PMSZ_OK;
@@ -391,7 +398,7 @@ int enqueue_ingest(const T *hf, const T *hfh, T *df, T *dfh, T *dprev, size_t nx
 template <typename T>
 int first_pass_ingest(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes, uint32_t *hp, uint32_t *req,
                       uint32_t *a_next, SweepSlot *slot, const Geom &g, cudaStream_t s, int64_t *launches,
-                      uint32_t *xcount, const FirstMaps &maps, uint32_t *err, uint8_t *freq, uint8_t *fact) {
+                      const FirstMaps &maps, uint32_t *err, uint8_t *freq, uint8_t *fact) {
     if (in.df != f || !in.copies || in.copies->zc != g.zc)
         return set_error(PMSZ_ERR_ARG, "ingest copies do not match the field");
     const IngestCopies &r = *in.copies;
@@ -401,7 +408,7 @@ int first_pass_ingest(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes
         PMSZ_CUDA(cudaStreamWaitEvent(s, r.ev[j], 0));
         dim3 grid = tiled_grid(g);
         grid.z = static_cast<unsigned>(std::min(cps, nchunks - j * cps));
-        if ((rc = launch_first_pass<T>(maps, grid, s, f, fh, codes, hp, req, a_next, slot, g, j * cps, xcount, err, freq, fact))) return rc;
+        if ((rc = launch_first_pass<T>(maps, grid, s, f, fh, codes, hp, req, a_next, slot, g, j * cps, err, freq, fact))) return rc;
         PMSZ_CUDA(cudaGetLastError());
         ++*launches;
     }
@@ -456,13 +463,12 @@ static int first_pass_waves(const HostIngest<T> &in, const SweepArgs<T> &a, cons
         dim3 grid = tiled_grid(g);
         grid.z = static_cast<unsigned>(std::min(cps, nchunks - j * cps));
         if ((rc = launch_first_pass<T>(maps, grid, s, a.f, a.fh, const_cast<uint8_t *>(a.codes), a.hp, a.req, a.act1,
-                                       &a.slots[0], g, j * cps, &a.ls->lc[3], &a.ls->err, a.freq, a.f1)))
+                                       &a.slots[0], g, j * cps, &a.ls->err, a.freq, a.f1)))
             return rc;
         ++*launches;
         if (!wave_after[static_cast<size_t>(j)]) continue;
         PMSZ_CUDA(cudaStreamWaitEvent(s, r.evp[j], 0));  // fhat's pre-correction copy of slabs 0 .. j
         const int Z = last ? g.nz : std::min(g.nz, (j + 1) * cps * g.zc);
-        f.seen = static_cast<unsigned long long>(g.nx) * g.ny * Z;
         size_t widest = 0;
         for (int k = 0; k <= K; ++k) {
             const int D = last ? g.nz : std::max(Dp[k], k == 0 ? Z : Ap[k - 1] - 1);
@@ -522,7 +528,8 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
     const size_t o_fr = ws.reserve<uint8_t>(groups), o_f0 = ws.reserve<uint8_t>(groups), o_f1 = ws.reserve<uint8_t>(groups);
     const size_t zero_bytes = ws.reserve<uint8_t>(0);
     const size_t o_codes = ws.reserve<uint8_t>(g.n);
-    const size_t o_hp = ws.reserve<uint32_t>(g.n);
+    const bool proxies = sizeof(T) == 8 || full;  // (fp32 sweeps compare the values themselves)
+    const size_t o_hp = ws.reserve<uint32_t>(proxies ? g.n : 0);
     // host-buffer calls of several slabs run sweeps 1 .. K behind the copy
     // (first_pass_waves; K below max_sweeps)
     const int wave_k = static_cast<int>(std::min<int64_t>(kWaveSweeps, max_sweeps - 1));
@@ -536,7 +543,7 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
     uint32_t *act[2] = {ws.at<uint32_t>(o_a0), ws.at<uint32_t>(o_a1)};
     uint8_t *freq = ws.at<uint8_t>(o_fr), *fact[2] = {ws.at<uint8_t>(o_f0), ws.at<uint8_t>(o_f1)};
     uint8_t *codes = ws.at<uint8_t>(o_codes);
-    uint32_t *hp = ws.at<uint32_t>(o_hp);
+    uint32_t *hp = proxies ? ws.at<uint32_t>(o_hp) : nullptr;
     const FirstMaps maps = first_maps<T>(f, fh, g);
     EventTimer et;
     if ((rc = et.init())) return rc;
@@ -581,11 +588,11 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
             a.from_edits = 0;
         } else if (ingest) {
             if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, act[1], &slots[0], g, s, &launches,
-                                           &ls->lc[3], maps, &ls->err, freq, fact[1])))
+                                           maps, &ls->err, freq, fact[1])))
                 return rc;
         } else {
             if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, act[1], &slots[0], g, 0,
-                                           &ls->lc[3], &ls->err, freq, fact[1])))
+                                           &ls->err, freq, fact[1])))
                 return rc;
             ++launches;
         }
@@ -634,17 +641,17 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
         uint32_t *a_next = act[(sweeps + 1) & 1];
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[0], s));
         if (sweeps == 0 && ingest) {
-            if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, a_next, slot, g, s, &launches, nullptr, maps,
+            if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, a_next, slot, g, s, &launches, maps,
                                            &ls->err, nullptr, nullptr)))
                 return rc;
         } else if (sweeps == 0) {
-            if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, a_next, slot, g, 0, nullptr,
+            if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, a_next, slot, g, 0,
                                            &ls->err)))
                 return rc;
             ++launches;
         } else {
             PMSZ_CUDA((launch_march<T, kDetect>(
-                tiled_grid(g), s, MarchArgs<T>{nullptr, fh, codes, hp, req, nullptr, a_next, slot, nullptr}, g, 0)));
+                tiled_grid(g), s, MarchArgs<T>{nullptr, fh, codes, hp, req, nullptr, a_next, slot}, g, 0)));
             ++launches;
         }
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[1], s));
@@ -711,7 +718,7 @@ int codes_impl(const T *v, size_t nx, size_t ny, size_t nz, uint8_t *codes, cuda
     Geom g = make_geom(nx, ny, nz);
     g.zc = first_depth(nx, ny, nz, sizeof(T));
     PMSZ_CUDA((launch_march<T, kCodes>(
-        tiled_grid(g), s, MarchArgs<T>{v, nullptr, codes, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr}, g, 0)));
+        tiled_grid(g), s, MarchArgs<T>{v, nullptr, codes, nullptr, nullptr, nullptr, nullptr, nullptr}, g, 0)));
     PMSZ_CUDA(cudaGetLastError());
     return PMSZ_OK;
 }
@@ -723,7 +730,7 @@ int pair_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, T eps, u
               unsigned long long *counts, uint32_t *err, cudaStream_t s) {
     Geom g = make_geom(nx, ny, nz);
     g.zc = first_depth(nx, ny, nz, sizeof(T));
-    MarchArgs<T> a{f, fp, c0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    MarchArgs<T> a{f, fp, c0, nullptr, nullptr, nullptr, nullptr, nullptr};
     a.codes_h = c1;
     a.eps = eps;
     a.sure = sure;
@@ -752,13 +759,14 @@ int time_first_pass(const T *f, const T *fh, size_t nx, size_t ny, size_t nz, ui
                     float *ms, cudaStream_t s) {
     Geom g = make_geom(nx, ny, nz);
     Workspace ws(s);
-    const size_t o_hp = ws.reserve<uint32_t>(g.n), o_req = ws.reserve<uint32_t>(g.nwords),
+    const size_t o_hp = ws.reserve<uint32_t>(sizeof(T) == 8 ? g.n : 0), o_req = ws.reserve<uint32_t>(g.nwords),
                  o_act = ws.reserve<uint32_t>(g.nwords), o_slot = ws.reserve<SweepSlot>(1),
                  o_err = ws.reserve<uint32_t>(1);
     int rc = ws.commit();
     if (rc) return rc;
     const FirstMaps maps = first_maps<T>(f, fh, g);
-    uint32_t *hp = ws.at<uint32_t>(o_hp), *req = ws.at<uint32_t>(o_req), *act = ws.at<uint32_t>(o_act);
+    uint32_t *hp = sizeof(T) == 8 ? ws.at<uint32_t>(o_hp) : nullptr;  // as a correction runs it
+    uint32_t *req = ws.at<uint32_t>(o_req), *act = ws.at<uint32_t>(o_act);
     uint32_t *err = ws.at<uint32_t>(o_err);
     SweepSlot *slot = ws.at<SweepSlot>(o_slot);
     PMSZ_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), s));
@@ -773,7 +781,8 @@ int time_first_pass(const T *f, const T *fh, size_t nx, size_t ny, size_t nz, ui
             PMSZ_CUDA(cudaMemsetAsync(slot, 0, sizeof(SweepSlot), s));
             PMSZ_CUDA(cudaEventRecord(et.ev[0], s));
             if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, const_cast<T *>(fh), codes, hp, req, act, slot, g, 0,
-                                 nullptr, err))) return rc;
+                                               err)))
+                return rc;
             PMSZ_CUDA(cudaGetLastError());
             PMSZ_CUDA(cudaEventRecord(et.ev[1], s));
             PMSZ_CUDA(cudaEventSynchronize(et.ev[1]));

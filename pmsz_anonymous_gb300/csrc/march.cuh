@@ -159,7 +159,7 @@ __device__ __forceinline__ void exact_ranks(const T *__restrict__ v, size_t i, c
 }
 
 // What a march reads and writes.  kFirst: f and fhat in, codes, the proxies
-// hp, requests and mismatch bits out.  kDetect: the proxies hp (fhat for the
+// hp (fp32: or null), requests and mismatch bits out.  kDetect: the proxies hp (fhat for the
 // exact decisions) and the codes in; act_cur (or null: every voxel) is the
 // active set, consumed.  kCodes: f in, codes out.  kPair: f and fh in, both
 // codes out and their differences counted, the values compared with a bound:
@@ -171,7 +171,6 @@ struct MarchArgs {
     uint8_t *codes;
     uint32_t *hp, *req, *act_cur, *act_next;
     SweepSlot *slot;
-    uint32_t *xcount;  // += voxels decided on full keys (kFirst; may be null)
     uint8_t *freq = nullptr, *fact = nullptr;  // or null: the group flags of req / act_next
     // kPair: fh's codes; the bound and its magnitude bits (0 unless positive and
     // finite); counters += voxels whose codes differ, of those the ones whose
@@ -208,7 +207,7 @@ struct MarchSmem {
     uint32_t xq[kQueueCap], rq[kQueueCap];
     uint32_t qn;                           // queue lengths: rules, exact << 16
     uint32_t cnt[3];                       // fmax, fmin, fdir
-    uint32_t active, bad, deferred;
+    uint32_t active, bad;
     uint32_t pair[6];                      // kPair's counters
     // requests of planes zb-1 .. ze, rows y0-1 .. y0+8: a word of the columns
     // x0 .. x0+31, and two bits for the columns x0-1 and x0+32; mismatch bits
@@ -314,7 +313,6 @@ __device__ __noinline__ void march_queues(MarchSmemOf<T, MODE> &sm) {
         const uint32_t t = warp_sum_u32(v[c]);
         if (threadIdx.x == 0 && t) atomicAdd(&sm.cnt[c], t);
     }
-    if (tid == 0) sm.deferred += nx;
 }
 
 __device__ __forceinline__ uint32_t march_proxy(double v) { return proxy_of(v); }
@@ -411,7 +409,7 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
     if (tid == 0) {
         sm.qn = 0;
         sm.cnt[0] = sm.cnt[1] = sm.cnt[2] = 0;
-        sm.active = sm.bad = sm.deferred = 0;
+        sm.active = sm.bad = 0;
         if (MODE == kPair)
             for (int c = 0; c < 6; ++c) sm.pair[c] = 0;
         sm.a = a;
@@ -505,7 +503,7 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
             for (int r = 0; r < 2; ++r) {
                 const bool vin = r ? vin1 : vin0;
                 const size_t ir = i + (r ? static_cast<size_t>(g.nx) : 0);
-                if (MODE == kFirst && vin)  // fhat's proxies
+                if (MODE == kFirst && vin && (sizeof(T) == 8 || a.hp))  // fhat's proxies
                     a.hp[ir] = sm.p[last][NF - 1][ctr + (r ? (FACE ? rc : kHX) : 0)] & ~15u;
                 const uint32_t cert0 = (S[0][0][r].hi ^ S[0][1][r].hi) & (S[0][0][r].lo ^ S[0][1][r].lo);
                 uint32_t cert = cert0;
@@ -628,7 +626,6 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
     if (tid < 3 && sm.cnt[tid]) atomicAdd(reinterpret_cast<unsigned long long *>(a.slot) + tid, static_cast<unsigned long long>(sm.cnt[tid]));
     if (tid == 3 && sm.active) atomicAdd(&a.slot->active, static_cast<unsigned long long>(sm.active));
     if (tid == 4 && sm.bad) atomicAdd(&a.slot->bad, static_cast<unsigned long long>(sm.bad));
-    if (tid == 5 && a.xcount && sm.deferred) atomicAdd(a.xcount, sm.deferred);
 }
 
 __device__ __forceinline__ bool march_inside(const Geom &g, int bx, int by, int bz) {

@@ -64,7 +64,7 @@ template <typename T>
 static Inst<T> make_inst(const Job &j, int q, int64_t max_sweeps) {
     Inst<T> I{};
     const Geom &g = j.g;
-    const FieldScratch fs(g);
+    const FieldScratch fs(g, sizeof(T));
     fs.point(I, j.scratch, j.scratch + slot_bytes(max_sweeps));
     I.slots = reinterpret_cast<SweepSlot *>(j.scratch + fs.zero);
     I.f = static_cast<const T *>(j.fd.f);
@@ -118,7 +118,7 @@ public:
         j->fd = fd;
         j->g = make_geom(fd.nx, fd.ny, fd.nz);
         j->g.zc = first_depth(fd.nx, fd.ny, fd.nz, fd.elem_size);
-        j->scratch_bytes = FieldScratch(j->g).total + slot_bytes(cfg_.max_sweeps);
+        j->scratch_bytes = FieldScratch(j->g, fd.elem_size).total + slot_bytes(cfg_.max_sweeps);
         // its fields, its scratch, and 16 bytes a voxel for what the running
         // set shares (a charge that budgets are sized by: more than is held now)
         j->bytes = field_scratch_bytes(j->g, cfg_.max_sweeps) + 2 * j->g.n * fd.elem_size + 2 * sizeof(uint64_t) * j->g.n;
@@ -346,7 +346,7 @@ private:
             for (Job *j : admitted) {
                 j->t_start = Clock::now();
                 if (cudaMallocAsync(reinterpret_cast<void **>(&j->scratch), j->scratch_bytes, s_) != cudaSuccess ||
-                    cudaMemsetAsync(j->scratch, 0, FieldScratch(j->g).zero + slot_bytes(cfg_.max_sweeps), s_) != cudaSuccess) {
+                    cudaMemsetAsync(j->scratch, 0, FieldScratch(j->g, j->fd.elem_size).zero + slot_bytes(cfg_.max_sweeps), s_) != cudaSuccess) {
                     cudaGetLastError();
                     j->status = PMSZ_ERR_OOM;
                     j->over = true;

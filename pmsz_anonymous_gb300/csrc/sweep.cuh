@@ -23,9 +23,12 @@
 //    neighbours and written (detection reads proxies and codes and writes
 //    bitmaps, the edits touch their own voxel's values only), so the 15 gathers
 //    of neighbouring voxels share L1 lines.
-//  * Failed certificates wait in a per-warp buffer and are decided on full keys
-//    32 at a time; fp32 fields with many (plateaus) detect on full keys
-//    throughout.
+//  * fp64 detects on the 32-bit proxies; failed certificates wait in a per-warp
+//    buffer and are decided on full keys 32 at a time.  fp32 compares the values
+//    themselves (the same gathers; 15 values by max and min, then their ranks,
+//    cost what the proxies' four chains cost, and nothing is left open), and
+//    keeps no proxies: 256^3 dense 3104 -> 2656 us, 120x130x128 983 -> 912, 512^3
+//    sparse 2081 -> 1883 against proxies with a switch where many tied.
 //  * Result bits collect in shared memory, one word of them per bitmap word
 //    (SweepBits), and go out once per four groups: one atomic per word instead
 //    of one per voxel, and the closed stencils of all 32 words' changes marked
@@ -33,15 +36,15 @@
 //
 // Bound by the latency of the gathers (issue slots 40 % used) and, in small
 // fields and late sweeps, of the two grid barriers a sweep takes (about 2 us
-// each).  Three blocks per SM: four (64 registers) are up to 8 % slower.  The
-// code is kept small and with one site per decision: with dense and sparse
+// each).  Three blocks per SM; fp32 (64 registers) four in large fields, fp64
+// with four is up to 8 % slower.  The code is kept small and with one site per decision: with dense and sparse
 // visits as two copies the same work took 15-25 % longer.
 // Whole corrections: list kernels in a conditional CUDA graph -> warps on their
 // own chunks, every bit an atomic -> this:
-//   64^3 fp32, 8 sweeps              358 -> 181 -> 163 us
-//   173x141x203 fp32, 12 sweeps      560 -> 353 -> 299 us
+//   64^3 fp32, 8 sweeps              358 -> 181 -> 160 us
+//   173x141x203 fp32, 12 sweeps      560 -> 353 -> 282 us
 //   512^3 fp64, 16 sparse sweeps    3852 -> 3355 -> 3211 us
-//   256^3 fp32, 27 dense sweeps     4727 -> 4467 -> 3111 us (on full keys)
+//   256^3 fp32, 27 dense sweeps     4727 -> 4467 -> 2656 us
 //   160^3 fp64, 40 dense sweeps     2308 -> 2320 -> 1664 us
 #pragma once
 #include "march.cuh"
@@ -130,8 +133,6 @@ struct LoopState {
     long long k;          // the sweep k_sweeps starts with (the wavefront ran the ones before)
     long long done;       // sweeps in all, once it ends
     int go;               // that sweep runs
-    uint32_t lc[4];       // [3]: first-pass decisions on full keys
-    uint32_t deferred[2]; // voxels of a sweep decided on full keys, by the sweep's parity (fp32)
     uint32_t err;         // kErrCopy, kErrBarrier
     uint32_t bar[8];      // arrivals at the grid barriers of k_sweeps, and of the wavefront's launches
 };
@@ -189,7 +190,6 @@ struct SweepSmem {
     int4 at[kSweepWarps][32];             // x of bit 0, y, z of their words, and the word
     SweepBits bits[kSweepWarps];
     uint2 defer[kSweepWarps][64];         // word, bit
-    uint32_t deferred;
     SweepStep step[15];
 };
 
@@ -338,7 +338,7 @@ __device__ __forceinline__ bool sweep_edit(const A &a, size_t v, uint32_t &nreq,
     nprog += (chg || nc != oc) ? 1u : 0u;
     if (chg) {
         ++nchg;
-        a.hp[v] = proxy_of(nv);
+        if constexpr (sizeof(T) == 8) a.hp[v] = proxy_of(nv);
     }
     return chg;
 }
@@ -363,19 +363,18 @@ __device__ __forceinline__ SweepVoxel sweep_voxel(const SweepSmem &sm, uint32_t 
 }
 
 // Detection of the `total` listed voxels of a warp's 32 words (lane l holds
-// word w): on the proxies, failed certificates into the warp's buffer (ndefer
-// entries), or (keys) on full keys throughout.  The buffer is decided on full
-// keys 32 at a time, in the same place; `finish`: to the end.  v: fmax, fmin,
-// fdir, active; ndeferred += this lane's failed certificates.
+// word w).  fp64: on the proxies, failed certificates into the warp's buffer
+// (ndefer entries), which is decided on full keys 32 at a time; `finish`: to
+// the end.  fp32: on the values.  v: fmax, fmin, fdir, active.
 template <typename T, class A>
 __device__ __forceinline__ void detect_words(SweepSmem &sm, const A &a, const SweepStep *steps, uint32_t *nxt, uint8_t *fnxt,
-                                             uint32_t total, uint32_t w, bool keys, bool finish, uint32_t (&v)[4],
-                                             uint32_t &ndefer, uint32_t &ndeferred) {
+                                             uint32_t total, uint32_t w, bool finish, uint32_t (&v)[4], uint32_t &ndefer) {
+    constexpr bool keys = sizeof(T) == 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     SweepBits &bits = sm.bits[warp];
     v[3] += lane == 0 ? total : 0u;
     for (uint32_t j = 0;;) {
-        const bool buffered = ndefer >= 32 || (finish && ndefer && j >= total);
+        const bool buffered = !keys && (ndefer >= 32 || (finish && ndefer && j >= total));
         if (!buffered && j >= total) break;
         if (!buffered && !keys) {
             const SweepVoxel p = sweep_voxel(sm, j, total);
@@ -396,7 +395,6 @@ __device__ __forceinline__ void detect_words(SweepSmem &sm, const A &a, const Sw
                     sm.defer[warp][ndefer + static_cast<uint32_t>(__popc(md & ((1u << lane) - 1u)))] =
                         make_uint2(p.w, p.entry & 31u);
                 ndefer += static_cast<uint32_t>(__popc(md));
-                ndeferred += open;
             }
             j += 32;
             continue;
@@ -619,32 +617,19 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps(const __grid_constant
             return;
         }
     }
-    // fp32: exact keys when the first pass decided more than a tenth of the
-    // voxels on keys, or a sweep did (for good)
-    bool keys = sizeof(T) == 4 && 10ull * a.ls->lc[3] > static_cast<unsigned long long>(g.n);
     while (true) {
         uint32_t *cur = (k & 1) ? a.act1 : a.act0, *nxt = (k & 1) ? a.act0 : a.act1;
         uint8_t *fcur = (k & 1) ? a.f1 : a.f0, *fnxt = (k & 1) ? a.f0 : a.f1;
         if (!edits_only) {
             const SweepSlot *p = a.slots + (k - 1);
             if (sweep_stops(p->fmax, p->fmin, p->fdir, p->progressed, k, a.max_sweeps) || (k == 1 && p->bad)) break;
-            uint32_t c[4] = {0u, 0u, 0u, 0u}, ndefer = 0, ndeferred = 0;
-            if (threadIdx.x == 0) sm.deferred = 0;
+            uint32_t c[4] = {0u, 0u, 0u, 0u}, ndefer = 0;
             for_each_group<false>(sm, cur, fcur, g, chunk, 0, 0, [&](uint32_t total, uint32_t w, bool last) {
-                detect_words<T>(sm, a, sm.step, nxt, fnxt, total, w, keys, last, c, ndefer, ndeferred);
+                detect_words<T>(sm, a, sm.step, nxt, fnxt, total, w, last, c, ndefer);
             });
             const uint32_t v[8] = {c[0], c[1], c[2], 0u, 0u, 0u, c[3], 0u};
-            block_flush_slot(a.slots + k, v);  // (contains a barrier: sm.deferred is zero before)
-            if (sizeof(T) == 4) {
-                if (ndeferred) atomicAdd(&sm.deferred, ndeferred);
-                __syncthreads();
-                if (threadIdx.x == 0 && sm.deferred) atomicAdd(&a.ls->deferred[k & 1], sm.deferred);
-            }
+            block_flush_slot(a.slots + k, v);
             if (!sweep_barrier(&a.ls->bar[0], target, &a.ls->err)) return;
-            if (sizeof(T) == 4) {
-                keys = keys || 10ull * a.ls->deferred[k & 1] > a.slots[k].active;
-                if (blockIdx.x == 0 && threadIdx.x == 0) a.ls->deferred[(k + 1) & 1] = 0;
-            }
         }
         edits_only = false;
         {
@@ -670,7 +655,6 @@ struct WaveFronts {  // words: the fronts of the launch before and of this one
     uint32_t det0[kWaveSweeps + 1], det1[kWaveSweeps + 1], edit0[kWaveSweeps + 1], edit1[kWaveSweeps + 1];
     int sweeps;             // K
     int launch;             // its barrier counter, 1 ..
-    unsigned long long seen;  // voxels of the first passes so far
 };
 template <typename T>
 __global__ void __launch_bounds__(kSweepBlock, 3) k_sweep_wave(const __grid_constant__ SweepArgs<T> a,
@@ -682,7 +666,6 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweep_wave(const __grid_cons
     if (warp == 0) fill_steps(sm.step, g, lane);
     clear_bits(sm.bits[warp]);
     __syncthreads();
-    const bool keys = sizeof(T) == 4 && 10ull * a.ls->lc[3] > f.seen;
     auto chunk_of = [&](uint32_t words) {
         uint32_t chunk = 8;
         while (chunk > 1 && words / kGroupWords < static_cast<uint64_t>(chunk) * gridDim.x * kSweepWarps) chunk >>= 1;
@@ -692,10 +675,10 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweep_wave(const __grid_cons
         uint32_t *cur = (k & 1) ? a.act1 : a.act0, *nxt = (k & 1) ? a.act0 : a.act1;
         uint8_t *fcur = (k & 1) ? a.f1 : a.f0, *fnxt = (k & 1) ? a.f0 : a.f1;
         if (k > 0 && f.det1[k] > f.det0[k]) {  // (of sweep 0 the first pass is the detection)
-            uint32_t c[4] = {0u, 0u, 0u, 0u}, ndefer = 0, ndeferred = 0;
+            uint32_t c[4] = {0u, 0u, 0u, 0u}, ndefer = 0;
             for_each_group<true>(sm, cur, fcur, g, chunk_of(f.det1[k] - f.det0[k]), f.det0[k], f.det1[k],
                                  [&](uint32_t total, uint32_t w, bool last) {
-                                     detect_words<T>(sm, a, sm.step, nxt, fnxt, total, w, keys, last, c, ndefer, ndeferred);
+                                     detect_words<T>(sm, a, sm.step, nxt, fnxt, total, w, last, c, ndefer);
                                  });
             const uint32_t v[8] = {c[0], c[1], c[2], 0u, 0u, 0u, c[3], 0u};
             block_flush_slot(a.slots + k, v);

@@ -41,7 +41,6 @@ __device__ __forceinline__ int find_seg(const uint32_t *__restrict__ pre, int n,
 struct FieldMasks {
     uint32_t edits[kMaxBatch / 32];   // fields that run this iteration
     uint32_t detect[kMaxBatch / 32];  // of those, not in their first
-    uint32_t keys[kMaxBatch / 32];    // fp32 fields that detect on full keys
 };
 struct MultiSmem {
     SweepSmem s;
@@ -85,7 +84,7 @@ __device__ __forceinline__ bool field_masks(FieldMasks &m, const SweepTable<T> &
     for (int w = warp; w < (t.n + 31) / 32; w += kSweepWarps) {
         const int i = w * 32 + lane;
         const bool was = it == 0 ? i < t.n && t.inst[i].active : mask_bit(m.edits, i);
-        bool run = was, fresh = false, keys = it > 0 && sizeof(T) == 4 && mask_bit(m.keys, i);
+        bool run = was, fresh = false;
         if (was) {
             const Inst<T> &I = t.inst[i];
             const int64_t s = I.k + it;
@@ -93,36 +92,18 @@ __device__ __forceinline__ bool field_masks(FieldMasks &m, const SweepTable<T> &
             if (!fresh) {
                 const SweepSlot *p = slot_of(I, s - 1);
                 run = !sweep_stops(p->fmax, p->fmin, p->fdir, p->progressed, s, I.max_sweeps) && !(s == 1 && p->bad);
-                // exact keys for good once the first pass or a sweep decided more than a tenth on keys
-                if (sizeof(T) == 4)
-                    keys = keys || I.def[3] || 10ull * I.def[0] > static_cast<unsigned long long>(I.g.n) ||
-                           (s >= 2 && 10ull * I.def[1 + ((s - 1) & 1)] > p->active);
             }
         }
-        const uint32_t e = __ballot_sync(0xFFFFFFFFu, run), d = __ballot_sync(0xFFFFFFFFu, run && !fresh),
-                       x = __ballot_sync(0xFFFFFFFFu, keys), b = __ballot_sync(0xFFFFFFFFu, was);
+        const uint32_t e = __ballot_sync(0xFFFFFFFFu, run), d = __ballot_sync(0xFFFFFFFFu, run && !fresh), b = __ballot_sync(0xFFFFFFFFu, was);
         if (lane == 0) {
             m.edits[w] = e;
             m.detect[w] = d;
-            m.keys[w] = x;
         }
         any |= e;
         stop |= b & ~e;
     }
     stopped = stop != 0;
     return any != 0;
-}
-
-// After the grid barrier behind the detection of iteration `it`: the count of
-// the next sweep's failed certificates starts at zero, the switch to full keys
-// is kept for a later launch.  One block.
-__device__ __forceinline__ void next_deferred(const FieldMasks &m, const SweepTable<float> &t, int64_t it) {
-    for (int i = threadIdx.x; i < t.n; i += kSweepBlock) {
-        if (!mask_bit(m.edits, i)) continue;
-        const Inst<float> &I = t.inst[i];
-        I.def[1 + ((I.k + it + 1) & 1)] = 0;
-        if (mask_bit(m.keys, i)) I.def[3] = 1;
-    }
 }
 
 // One phase (0: detection, 1: edits) of iteration `it` over a table.  home,
@@ -135,18 +116,13 @@ __device__ __forceinline__ void multi_phase(MultiSmem &ms, const FieldMasks &m, 
     const uint32_t *mask = PHASE == 0 ? m.detect : m.edits;
     const uint64_t nc = static_cast<uint64_t>(t.chunks) * (8u / chunk);
     int cf = -1;  // the field whose counters are in v
-    uint32_t v[4] = {0u, 0u, 0u, 0u}, ndefer = 0, ndeferred = 0;
+    uint32_t v[4] = {0u, 0u, 0u, 0u}, ndefer = 0;
 
     const Inst<T> &I = *reinterpret_cast<const Inst<T> *>(ms.row[warp]);  // of field cf
 
     auto leave = [&] {  // the warp is done with field cf
         const int64_t s = I.k + it;
         if (PHASE == 0) {
-            if (sizeof(T) == 4) {
-                const uint32_t d = warp_sum_u32(ndeferred);
-                if (lane == 0 && d) atomicAdd(I.def + 1 + (s & 1), d);
-            }
-            ndeferred = 0;
             SweepSlot *slot = slot_of(I, s);
             if (lane == 0 && v[3]) atomicAdd(&slot->active, static_cast<unsigned long long>(v[3]));
             v[3] = 0;
@@ -243,7 +219,7 @@ __device__ __forceinline__ void multi_phase(MultiSmem &ms, const FieldMasks &m, 
             const uint32_t total = list_words(sm, g, w, word);
             if (PHASE == 0)
                 detect_words<T>(sm, I, ms.step[warp], nxt, fnxt, total, static_cast<uint32_t>(w),
-                                sizeof(T) == 4 && mask_bit(m.keys, f), f_next != f, v, ndefer, ndeferred);
+                                f_next != f, v, ndefer);
             else
                 edit_words<T>(sm, I, nxt, fnxt, total, v);
             __syncwarp();  // list and at are rewritten by the next groups
@@ -315,7 +291,6 @@ __global__ void __launch_bounds__(kSweepBlock, 3) k_sweeps_multi(const __grid_co
         multi_phase<float, 0>(ms, ms.m32, a.t32, c32, it, home32, local32);
         multi_phase<double, 0>(ms, ms.m64, a.t64, c64, it, home64, local64);
         if (!sweep_barrier(&a.ctl->bar, target, &a.ctl->err)) return;
-        if (first) next_deferred(ms.m32, a.t32, it);
         multi_phase<float, 1>(ms, ms.m32, a.t32, c32, it, home32, local32);
         multi_phase<double, 1>(ms, ms.m64, a.t64, c64, it, home64, local64);
         if (a.yield && first && threadIdx.x == 0) a.ctl->yield[it & 1] = want;
