@@ -44,8 +44,8 @@
 // Bitmaps of a column.  A word of the request and mismatch bitmaps is one row
 // of one plane of the column: collected in shared memory and written once, with
 // the group flags that k_sweeps reads (atomics per voxel before: a dense 256^3
-// fp32 first pass took 754 us, then 626; with the
-// values compared directly on ties 485).
+// fp32 first pass took 754 us, then 626; with the values compared directly on
+// ties 485).
 //
 // Measured at 512^3, issue-bound throughout: first pass fp64 1.50 -> 1.18 ms
 // (350 -> 220 warp instructions per 32 voxels), fp32 1.05 ms; codes alone

@@ -18,7 +18,7 @@
 //
 // A generation used to be one sweep, with up to nine launches, two copies and a
 // read-back for each type: a burst of 24 mixed jobs (18 million voxels) took
-// 8.6 ms, now 3.7.  What is left is the depth of the longest job's sweeps and a
+// 8.6 ms, now 3.6.  What is left is the depth of the longest job's sweeps and a
 // generation's fixed costs for every job that ends.
 #include "batch.h"
 

@@ -37,8 +37,9 @@
 // Bound by the latency of the gathers (issue slots 40 % used) and, in small
 // fields and late sweeps, of the two grid barriers a sweep takes (about 2 us
 // each).  Three blocks per SM; fp32 (64 registers) four in large fields, fp64
-// with four is up to 8 % slower.  The code is kept small and with one site per decision: with dense and sparse
-// visits as two copies the same work took 15-25 % longer.
+// with four is up to 8 % slower.  The code is kept small and with one site per
+// decision: with dense and sparse visits as two copies the same work took
+// 15-25 % longer.
 // Whole corrections: list kernels in a conditional CUDA graph -> warps on their
 // own chunks, every bit an atomic -> this:
 //   64^3 fp32, 8 sweeps              358 -> 181 -> 160 us

@@ -16,10 +16,10 @@
 // in registers until the warp's next field (a block's list is in field order:
 // once per field and phase at most).
 //
-// Measured: 32 fp32 fields (116 million voxels) 8.7 -> 5.5 ms end to end, from
+// Measured: 32 fp32 fields (116 million voxels) 8.7 -> 5.1 ms end to end, from
 // compacted lists in a conditional CUDA graph and a cooperative tail (4.9 ms of
-// kernels, and the gaps between them) to one launch of 3.7 ms; a burst of 24
-// mixed jobs through the server 8.6 -> 3.7 ms.
+// kernels, and the gaps between them) to one launch of 3.4 ms; a burst of 24
+// mixed jobs through the server 8.6 -> 3.6 ms.
 #pragma once
 #include "batch.h"
 #include "sweep.cuh"
