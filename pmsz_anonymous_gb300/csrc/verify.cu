@@ -39,8 +39,12 @@ __global__ void __launch_bounds__(256) k_init_ptr(const uint8_t *__restrict__ co
     const size_t i = flat(g, x, y, z);
     const uint8_t c = codes[i];
     const int a = c & 15, d = c >> 4;
-    if (as) as[i] = static_cast<uint32_t>(flat(g, x + rank_dx(a), y + rank_dy(a), z + rank_dz(a)));
-    if (ds) ds[i] = static_cast<uint32_t>(flat(g, x + rank_dx(d), y + rank_dy(d), z + rank_dz(d)));
+    const uint32_t valid = valid_mask(x, y, z, g.nx, g.ny, g.nz);
+    auto target = [&](int r) {  // a step out of the domain (not the codes of a field) stays put
+        return static_cast<uint32_t>((valid >> r) & 1u ? flat(g, x + rank_dx(r), y + rank_dy(r), z + rank_dz(r)) : i);
+    };
+    if (as) as[i] = target(a);
+    if (ds) ds[i] = target(d);
 }
 
 __global__ void __launch_bounds__(256) k_jump(uint32_t *__restrict__ L, size_t n, unsigned int *changed,
@@ -110,9 +114,9 @@ struct TileRootsSmem {
 
 // One block of 16 warps per tile; warp w owns the row y = w of every plane (with
 // 8 warps and two rows each the chase has half the chains in flight: both
-// labels of 32 M voxels 545 us, now 494).  L[l][i] receives the label so far of nibble lo[l] (0: ascent, 4:
-// descent), exits[l] the tile's exits (global indices) and count[l] their
-// number.  *flag is set if a chain does not end within the tile's voxel count
+// labels of 32 M voxels 545 us, now 494); planes beyond the field are left out.
+// L[l][i] receives the label so far of nibble lo[l] (0: ascent, 4: descent),
+// exits[l] the tile's exits (global indices) and count[l] their number.  *flag is set if a chain does not end within the tile's voxel count
 // (a cycle: not the codes of a field).  Bound by shared-memory latency and
 // conflicts of the pointer chase (L1 78 % busy, issue 63 %): pointers are stored
 // as byte offsets, steps come from a shuffle, the in-tile test from rank masks,
@@ -153,12 +157,12 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
     const uint32_t v0 = static_cast<uint32_t>(lane + kLX * w);                       // row w of plane 0
     const uint32_t i0 = origin + static_cast<uint32_t>(lane) + sy * static_cast<uint32_t>(w);
 #pragma unroll 4
-    for (int z = 0; z < kLZ; ++z) {
+    for (int z = 0; z < ez; ++z) {
         const uint32_t zmask = kAllValid & ~(z == 0 ? kNegZ : 0u) & ~(z + 1 >= ez ? kPosZ : 0u);
 #pragma unroll
         for (int h = 0; h < H; ++h) {
             const uint32_t v = v0 + static_cast<uint32_t>(kLX * NW * h + kLX * kLY * z);
-            const uint32_t c = in_row[h] && z < ez ? codes[i0 + sy * static_cast<uint32_t>(NW * h) + sz * static_cast<uint32_t>(z)] : 0x77u;
+            const uint32_t c = in_row[h] ? codes[i0 + sy * static_cast<uint32_t>(NW * h) + sz * static_cast<uint32_t>(z)] : 0x77u;
             const uint32_t mask = ymask[h] & zmask;
 #pragma unroll
             for (int l = 0; l < NL; ++l) {
@@ -176,7 +180,7 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
 #pragma unroll 1
     for (int round = 0; round < 2; ++round) {
 #pragma unroll 8
-        for (int k = 0; k < H * kLZ; ++k) {
+        for (int k = 0; k < H * ez; ++k) {
             const uint32_t off = 2 * v0 + static_cast<uint32_t>(2 * kLX * NW * k);
 #pragma unroll
             for (int l = 0; l < NL; ++l) at(l, off) = at(l, at(l, at(l, off)));
@@ -185,10 +189,10 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
     }
     bool stuck = false;
 #pragma unroll 2
-    for (int k = 0; k < H * kLZ; ++k) {
+    for (int k = 0; k < H * ez; ++k) {
         const int z = k / H;
         const uint32_t off = 2 * v0 + static_cast<uint32_t>(2 * kLX * NW * k);
-        const bool in = in_row[k % H] && z < ez;
+        const bool in = in_row[k % H];
         const uint32_t i = i0 + sy * static_cast<uint32_t>(NW * (k % H)) + sz * static_cast<uint32_t>(z);
 #pragma unroll
         for (int l = 0; l < NL; ++l) {
@@ -297,8 +301,20 @@ struct LabelRun {
     static size_t list_words(const TileGrid &t) { return t.tiles() * (static_cast<size_t>(t.stride) + 1); }
     uint32_t *counts(int l) const { return lists + static_cast<size_t>(l) * list_words(t); }
     uint32_t *exits(int l) const { return counts(l) + t.tiles(); }
+    // Lines, and fields a few rows thick: a tile holds 32 to 96 voxels, and
+    // nearly every chain leaves its tile.  They go to the general jumping at once
+    // (2 M voxels in a line: codes and labels 694 us by tiles, 562 so; a plane of
+    // 2048 x 2000: 206 by tiles, 577 so).
+    static bool general(const Geom &g) { return std::min(g.ny, kLY) * std::min(g.nz, kLZ) < 4; }
     int roots(const uint8_t *codes, cudaStream_t s) {  // everything up to k_finish
         PMSZ_CUDA(cudaMemsetAsync(words, 0, 2 * sizeof(unsigned int), s));
+        if (general(g)) {
+            const dim3 grid(static_cast<unsigned>(g.wpr), static_cast<unsigned>((g.ny + 7) / 8), static_cast<unsigned>(g.nz));
+            k_init_ptr<<<grid, dim3(32, 8, 1), 0, s>>>(codes, lo[0] == 0 ? L[0] : nullptr, nl == 2 ? L[1] : lo[0] == 4 ? L[0] : nullptr, g);
+            PMSZ_CUDA(cudaGetLastError());
+            PMSZ_CUDA(cudaMemsetAsync(words, 1, 1, s));  // (little-endian int 1)
+            return PMSZ_OK;
+        }
         if (nl == 2)
             k_tile_roots<2><<<t.grid, kLThreads, 0, s>>>(codes, L[0], L[1], lo[0], lo[1], exits(0), exits(1), t.stride,
                                                          counts(0), counts(1), words, g);
@@ -510,8 +526,9 @@ int verify_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, double
         r.words = ws.at<unsigned int>(o_w) + 2 * (2 * kind + field);
         return r;
     };
+    const bool jump = LabelRun::general(g);
     for (int kind = 0; kind < 2; ++kind) {
-        if (!wanted[kind]) continue;
+        if (!wanted[kind] || jump) continue;
         for (int field = 0; field < 2; ++field)
             if ((rc = run_of(kind, field).roots(field ? c1 : c0, s))) return rc;
         k_count_diff<<<grid_for((g.n + 3) / 4), 256, 0, s>>>(ws.at<uint32_t>(o_l0), ws.at<uint32_t>(o_l1), g.n, 1,
@@ -519,7 +536,7 @@ int verify_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, double
         PMSZ_CUDA(cudaGetLastError());
     }
     unsigned int words[8] = {};
-    if (wanted[0] || wanted[1]) {
+    if ((wanted[0] || wanted[1]) && !jump) {
         unsigned int *hw = reinterpret_cast<unsigned int *>(h + 9);
         PMSZ_CUDA(cudaMemcpyAsync(h, cnt, kCounts, cudaMemcpyDeviceToHost, s));
         PMSZ_CUDA(cudaMemcpyAsync(hw, ws.at<unsigned int>(o_w), 8 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
@@ -528,7 +545,7 @@ int verify_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, double
         got[6] = h[6];
         got[7] = h[7];
     }
-    const bool open[2] = {wanted[0] && (words[0] | words[2]) != 0, wanted[1] && (words[4] | words[6]) != 0};
+    const bool open[2] = {wanted[0] && (jump || (words[0] | words[2]) != 0), wanted[1] && (jump || (words[4] | words[6]) != 0)};
     for (int kind = 0; kind < 2; ++kind) {
         // chains beyond the walks' bounds: that kind once more, jumped to the fixpoint
         if (!open[kind]) continue;
