@@ -319,9 +319,10 @@ __device__ __forceinline__ uint32_t march_proxy(double v) { return proxy_of(v); 
 __device__ __forceinline__ uint32_t march_proxy(float v) { return proxy_of(v); }
 __device__ __forceinline__ uint32_t march_proxy(uint32_t p) { return p; }  // a stored proxy
 // Proxies outside [lo, hi) may belong to a NaN or to the sentinel 1e30 (fp64).
+// A NaN of high word 0xFFF00000 has the proxy of -inf, which is thus outside.
 template <typename T> struct PlainRange;
 template <> struct PlainRange<double> {
-    static constexpr uint32_t lo = 0x00100000u, hi = (0x80000000u + 0x46293E59u) & ~15u;  // 1e30 = 0x46293E59...
+    static constexpr uint32_t lo = 0x00100010u, hi = (0x80000000u + 0x46293E59u) & ~15u;  // 1e30 = 0x46293E59...
 };
 template <> struct PlainRange<float> {
     static constexpr uint32_t lo = 0x00800000u, hi = 0xFF800000u;

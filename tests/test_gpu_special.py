@@ -40,3 +40,37 @@ def test_special(cuda, shape, dtype, kind):
         assert (r.status, r.sweeps) == (st, sw)
         np.testing.assert_array_equal(r.log[:, :5], recs)
         np.testing.assert_array_equal(d.cpu().numpy().view(np.uint8), ref.view(np.uint8))
+
+
+# NaNs of every kind of payload: quiet and signalling, either sign, the payload
+# in the high or (fp64) the low word only, where the high word is an infinity's
+NAN_BITS = {np.float64: [0x7FF8000000000000, 0xFFF8000000000000, 0x7FF0000000000001, 0xFFF0000000000001,
+                         0x7FF00000FFFFFFFF, 0xFFF00000FFFFFFFF, 0xFFFFFFFFFFFFFFFF],
+            np.float32: [0x7FC00000, 0xFFC00000, 0x7F800001, 0xFF800001, 0xFFFFFFFF]}
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("target", [0, 1], ids=["f", "fhat"])
+@pytest.mark.parametrize("shape,where", [((40, 17, 48), (20, 8, 23)), ((40, 17, 48), (0, 0, 0)),
+                                         ((19, 21, 37), (18, 20, 36))], ids=str)
+def test_nans_of_every_payload_are_refused(cuda, shape, where, target, dtype):
+    from pmsz_anonymous_gb300 import capi
+    A = api()
+    base = np.random.default_rng(6).random(shape).astype(dtype)
+    for bits in NAN_BITS[dtype]:
+        pair = [base.copy(), base.copy()]
+        pair[target].view(np.uint32 if dtype is np.float32 else np.uint64)[where] = bits
+        assert np.isnan(pair[target][where])
+        dev = [torch.from_numpy(a).to(cuda) for a in pair]
+        for full in (False, True):
+            with pytest.raises(capi.PmszError):
+                A.correct(dev[0], dev[1].clone(), 1e-3, max_sweeps=40, full_sweeps=full)
+        with pytest.raises(capi.PmszError):
+            A.correct_host(*[torch.from_numpy(a).pin_memory() for a in pair], 1e-3, max_sweeps=40)
+        good = torch.from_numpy(base).to(cuda)
+        got = A.correct_batch([(dev[0], dev[1].clone(), 1e-3), (good, good.clone(), 1e-3)], max_sweeps=40)
+        assert [r.status for r in got] == [capi.PMSZ_ERR_ARG, capi.PMSZ_OK], hex(bits)
+        work = dev[1].clone()
+        torch.cuda.synchronize()
+        with A.Server(max_sweeps=40) as srv:
+            assert srv.wait(srv.submit(dev[0], work, 1e-3))["status"] == capi.PMSZ_ERR_ARG, hex(bits)
