@@ -142,10 +142,13 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
     };
     if (threadIdx.x < NL) sm.n[threadIdx.x] = 0;
     __syncthreads();
-    // lane r: the step of rank r, in bytes; ranks whose target lies in the tile
+    // lane r: the step of rank r, in bytes; ranks whose target lies in the tile.
+    // A nibble of 15 (no rank, and not the code of a field) stays put, which is
+    // in the tile: only voxels of its shell are exits, at most kLShell.
+    constexpr uint32_t kStay = kAllValid | 1u << 15;
     const int r16 = lane & 15;
     const int step = r16 < 15 ? 2 * (rank_dx(r16) + kLX * rank_dy(r16) + kLX * kLY * rank_dz(r16)) : 0;
-    const uint32_t xmask = kAllValid & ~(lane == 0 ? kNegX : 0u) & ~(lane + 1 >= ex ? kPosX : 0u);
+    const uint32_t xmask = kStay & ~(lane == 0 ? kNegX : 0u) & ~(lane + 1 >= ex ? kPosX : 0u);
     uint32_t ymask[H];
     bool in_row[H];
 #pragma unroll
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
     const uint32_t i0 = origin + static_cast<uint32_t>(lane) + sy * static_cast<uint32_t>(w);
 #pragma unroll 4
     for (int z = 0; z < ez; ++z) {
-        const uint32_t zmask = kAllValid & ~(z == 0 ? kNegZ : 0u) & ~(z + 1 >= ez ? kPosZ : 0u);
+        const uint32_t zmask = kStay & ~(z == 0 ? kNegZ : 0u) & ~(z + 1 >= ez ? kPosZ : 0u);
 #pragma unroll
         for (int h = 0; h < H; ++h) {
             const uint32_t v = v0 + static_cast<uint32_t>(kLX * NW * h + kLX * kLY * z);
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
                 const int s = __shfl_sync(0xFFFFFFFFu, step, static_cast<int>(r));
                 const bool inside = ((mask >> r) & 1u) != 0u;
                 at(l, 2 * v) = static_cast<uint16_t>(static_cast<int>(2 * v) + (inside ? s : 0));
-                // a step out of the tile (or of the domain, or rank 15: found below)
+                // a step out of the tile (or of the domain: found below)
                 if (!inside) sm.exits[l][atomicAdd(&sm.n[l], 1u)] = static_cast<uint16_t>(v);
             }
         }
@@ -212,7 +215,7 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
     }
     if (stuck) atomicOr(flag, 1u);
     __syncthreads();  // the exits' labels come after the loop's
-    // dx + 1, dy + 1, dz + 1 of every rank, two bits each (rank 15 stays put)
+    // dx + 1, dy + 1, dz + 1 of every rank, two bits each (nibble 15 is no exit)
     constexpr auto steps = [](int axis) {
         uint32_t t = 1u << 30;
         for (int r = 0; r < 15; ++r)

@@ -101,3 +101,29 @@ def test_verify(cuda, shape, dtype, kind):
         want["bound_beyond_clamp"] = int((~((fp >= f - e) & (fp <= f + e))).sum())
         got = api().verify(_dev(f, cuda), _dev(fp, cuda), bound)
         assert got == want, (bound, got, want)
+
+
+# nibbles of 15 name no neighbour: such a voxel is its own label, in the tiles as
+# in the general jumping, however many of them a tile holds
+@pytest.mark.parametrize("shape", [(16, 16, 32), (17, 33, 65), (40, 48, 70), (1, 1, 5000), (2, 1, 300)], ids=str)
+@pytest.mark.parametrize("share", [1.0, 0.5, 0.01])
+def test_nibbles_beyond_the_ranks_stay_put(cuda, shape, share):
+    n = int(np.prod(shape))
+    rng = np.random.default_rng(17)
+    codes = api().codes(_dev(_field("ramp", shape), cuda)).cpu().numpy().ravel()
+    off = api().rank_offsets()
+    nx, ny = shape[2], shape[1]
+    flat = off[:, 0] + nx * (off[:, 1] + ny * off[:, 2])
+    nibbles = [codes & 15, codes >> 4]
+    want = []
+    for k in range(2):
+        hit = rng.random(n) < share
+        nibbles[k] = np.where(hit, 15, nibbles[k]).astype(np.uint8)
+        p = np.arange(n) + np.where(hit, 0, flat[np.minimum(nibbles[k], 14)])
+        while not np.array_equal(p, p[p]):
+            p = p[p]
+        want.append(p)
+    both = _dev((nibbles[0] | (nibbles[1] << 4)).astype(np.uint8).reshape(shape), cuda)
+    a, d = api().labels(both)
+    np.testing.assert_array_equal(a.cpu().numpy().ravel(), want[0])
+    np.testing.assert_array_equal(d.cpu().numpy().ravel(), want[1])
