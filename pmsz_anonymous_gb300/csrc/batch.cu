@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_first_multi(const Inst<T> *__re
     const uint32_t lt = blockIdx.x - __ldg(tpre + i);
     const uint32_t bx = lt % I.tiles_x, rest = lt / I.tiles_x;
     const uint32_t by = rest % I.tiles_y, bz = rest / I.tiles_y;
-    const MarchArgs<T> a{I.f, I.fh, I.codes, I.hp, I.req, nullptr, I.act1, I.slots, I.freq, I.f1};
+    const MarchArgs<T> a{I.f, I.fh, I.codes, I.hp, I.req, I.act1, I.slots, I.freq, I.f1};
     const int x = static_cast<int>(bx), y = static_cast<int>(by), z = static_cast<int>(bz);
     if (march_inside(I.g, x, y, z))
         march_copies<T, kFirst, false>(sm, a, I.g, x, y, z);

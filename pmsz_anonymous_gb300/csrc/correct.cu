@@ -167,23 +167,6 @@ __global__ void __launch_bounds__(256) k_apply(const T *__restrict__ f, T *__res
     }
 }
 
-// Codes only (pmsz_codes): the labelling half of the first pass.
-template <typename T>
-__global__ void __launch_bounds__(256) k_codes(const T *__restrict__ v, uint8_t *__restrict__ codes, Geom g) {
-    using K = typename KeyOf<T>::type;
-    const int x = blockIdx.x * 32 + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z = blockIdx.z;
-    if (x >= g.nx || y >= g.ny) return;
-    const size_t i = flat(g, x, y, z);
-    const uint32_t valid = valid_mask(x, y, z, g.nx, g.ny, g.nz);
-    K k[15];
-    load_keys(v, i, g, valid, k);
-    int a, d;
-    arg_ext(k, valid, a, d);
-    codes[i] = static_cast<uint8_t>(a | (d << 4));
-}
-
 }  // namespace pmsz
 
 #include "sweep.cuh"
@@ -259,7 +242,7 @@ template <typename T>
 static int launch_first_pass(const FirstMaps &m, dim3 grid, cudaStream_t s, const T *f, T *fh, uint8_t *codes,
                              uint32_t *hp, uint32_t *req, uint32_t *act, SweepSlot *slot, const Geom &g, int bz0,
                              uint32_t *err, uint8_t *freq = nullptr, uint8_t *fact = nullptr) {
-    const MarchArgs<T> a{f, fh, codes, hp, req, nullptr, act, slot, freq, fact};
+    const MarchArgs<T> a{f, fh, codes, hp, req, act, slot, freq, fact};
     if (m.ok) {
         PMSZ_CUDA(allow_smem(k_pair_tma<T, kFirst>, sizeof(TmaMarch<T>)));
         k_pair_tma<T, kFirst><<<grid, dim3(kTX, kThreads / kTX, 1), sizeof(TmaMarch<T>), s>>>(m.f, m.fh, a, g, bz0, err);
@@ -651,7 +634,7 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
             ++launches;
         } else {
             PMSZ_CUDA((launch_march<T, kDetect>(
-                tiled_grid(g), s, MarchArgs<T>{nullptr, fh, codes, hp, req, nullptr, a_next, slot}, g, 0)));
+                tiled_grid(g), s, MarchArgs<T>{nullptr, fh, codes, hp, req, a_next, slot}, g, 0)));
             ++launches;
         }
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[1], s));
@@ -718,7 +701,7 @@ int codes_impl(const T *v, size_t nx, size_t ny, size_t nz, uint8_t *codes, cuda
     Geom g = make_geom(nx, ny, nz);
     g.zc = first_depth(nx, ny, nz, sizeof(T));
     PMSZ_CUDA((launch_march<T, kCodes>(
-        tiled_grid(g), s, MarchArgs<T>{v, nullptr, codes, nullptr, nullptr, nullptr, nullptr, nullptr}, g, 0)));
+        tiled_grid(g), s, MarchArgs<T>{v, nullptr, codes, nullptr, nullptr, nullptr, nullptr}, g, 0)));
     PMSZ_CUDA(cudaGetLastError());
     return PMSZ_OK;
 }
@@ -730,7 +713,7 @@ int pair_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, T eps, u
               unsigned long long *counts, uint32_t *err, cudaStream_t s) {
     Geom g = make_geom(nx, ny, nz);
     g.zc = first_depth(nx, ny, nz, sizeof(T));
-    MarchArgs<T> a{f, fp, c0, nullptr, nullptr, nullptr, nullptr, nullptr};
+    MarchArgs<T> a{f, fp, c0, nullptr, nullptr, nullptr, nullptr};
     a.codes_h = c1;
     a.eps = eps;
     a.sure = sure;

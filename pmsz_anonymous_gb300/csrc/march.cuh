@@ -100,7 +100,6 @@ __device__ __forceinline__ Ext2 join(const Ext2 &a, const Ext2 &b, const Ext2 &c
 __device__ __forceinline__ Ext2 join(uint32_t a, uint32_t b, const Ext2 &c) {
     return Ext2{__vimax3_u32(a, b, c.hi), __vimin3_u32(a, b, c.lo)};
 }
-__device__ __forceinline__ Ext2 ext2_identity() { return Ext2{0u, 0xFFFFFFFFu}; }
 
 // Steepest ranks of one voxel on the full keys of v, gathered from global
 // memory five at a time (arg_ext's rule: ties by rank).  fp32 without NANS
@@ -160,8 +159,7 @@ __device__ __forceinline__ void exact_ranks(const T *__restrict__ v, size_t i, c
 
 // What a march reads and writes.  kFirst: f and fhat in, codes, the proxies
 // hp (fp32: or null), requests and mismatch bits out.  kDetect: the proxies hp (fhat for the
-// exact decisions) and the codes in; act_cur (or null: every voxel) is the
-// active set, consumed.  kCodes: f in, codes out.  kPair: f and fh in, both
+// exact decisions) and the codes in, of every voxel.  kCodes: f in, codes out.  kPair: f and fh in, both
 // codes out and their differences counted, the values compared with a bound:
 // 71.5 M voxels fp64 684 us, where the codes of either field and a pass that
 // compares them took 658 + 308.
@@ -169,7 +167,7 @@ template <typename T>
 struct MarchArgs {
     const T *f, *fh;
     uint8_t *codes;
-    uint32_t *hp, *req, *act_cur, *act_next;
+    uint32_t *hp, *req, *act_next;
     SweepSlot *slot;
     uint8_t *freq = nullptr, *fact = nullptr;  // or null: the group flags of req / act_next
     // kPair: fh's codes; the bound and its magnitude bits (0 unless positive and
@@ -346,7 +344,7 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
     const size_t plane = static_cast<size_t>(g.nx) * g.ny;
     const int nplanes = ze - zb + 2;  // zb-1 .. ze
 
-    // tags of this thread's cells (tid + 256 j of the 34 x 18 halo tile) in
+    // tags of this thread's cells (tid + 128 j of the 34 x 10 halo tile) in
     // plane zb-1, 4 bits each
     uint32_t ctags = 0;
     uint32_t mine = 0, beyond = 0, clamped = 0;  // kPair: cells of the tile itself; values beyond the bound, the clamp
@@ -433,7 +431,6 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
     __syncthreads();
 #pragma unroll 1
     for (int k = 0; k < 3; ++k) src.release(k, k);
-    uint32_t active = 0;
     size_t i = static_cast<size_t>(x) + static_cast<size_t>(y) * g.nx + static_cast<size_t>(zb) * plane;
     const uint32_t stag0 = stencil_tag(x, y, zb - 2);
     int k = 2;  // the next plane; it completes the voxels of plane k-1, z = zb + k - 2
@@ -467,13 +464,10 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
             const int last = 3 - slot - next;  // the slot of plane k-1, and of k+2's stage
             src.prefetch(k + 2, last);
             const int zrel = k - 2;
-            uint32_t word[2] = {0xFFFFFFFFu, 0xFFFFFFFFu}, was[2] = {0u, 0u};
+            uint32_t was[2] = {0u, 0u};
             if (MODE == kDetect) {
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    if (a.act_cur) word[r] = (!FACE || y + r < g.ny) ? a.act_cur[word_of(g, x0, y + r, zb + zrel)] : 0u;
-                    if ((r ? vin1 : vin0) && word[r]) was[r] = a.codes[i + (r ? g.nx : 0)];
-                }
+                if (vin0) was[0] = a.codes[i];
+                if (vin1) was[1] = a.codes[i + g.nx];
             }
             Ext2 S[NF][2][2];
             if (plane_in(k)) {
@@ -538,12 +532,8 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
                            ((((S[0][0][r].hi ^ S[NF - 1][0][r].hi) | (S[0][0][r].lo ^ S[NF - 1][0][r].lo)) & 15u) != 0u ||
                             (FACE && c0 == 0x77u));
                 } else {
-                    const bool on = vin && ((word[r] >> tx) & 1u);
-                    active += on ? 1u : 0u;
                     c = was[r];
-                    ex = ex && on;
-                    rule = on && ok && (c0 != c || (FACE && c == 0x77u));
-                    if (a.act_cur && word[r] && tx == 0) a.act_cur[word_of(g, x0, y + r, zb + zrel)] = 0;
+                    rule = vin && ok && (c0 != c || (FACE && c == 0x77u));
                 }
                 const uint32_t wq = __ballot_sync(0xFFFFFFFFu, rule || ex);
                 if (wq) {
@@ -619,8 +609,7 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
             a.act_next[w] = sm.mism[e];
             if (a.fact) a.fact[w / kGroupWords] = 1;
         }
-    if (MODE == kFirst) active = static_cast<uint32_t>(ze - zb) * ((vin0 ? 1u : 0u) + (vin1 ? 1u : 0u));
-    active = warp_sum_u32(active);
+    const uint32_t active = warp_sum_u32(static_cast<uint32_t>(ze - zb) * ((vin0 ? 1u : 0u) + (vin1 ? 1u : 0u)));
     if (tx == 0 && active) atomicAdd(&sm.active, active);
     __syncthreads();
     // one atomic per non-zero counter and block
@@ -635,7 +624,7 @@ __device__ __forceinline__ bool march_inside(const Geom &g, int bx, int by, int 
 }
 
 // ---------------------------------------------------------------------------
-// Plane sources.  cell(k, j, F): this thread's cell tid + 256 j of the halo
+// Plane sources.  cell(k, j, F): this thread's cell tid + 128 j of the halo
 // tile, of field F, in plane zb-1+k.
 //
 // CopySource: cp.async of single elements, any alignment and row length; every

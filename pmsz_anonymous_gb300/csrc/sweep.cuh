@@ -301,7 +301,7 @@ __device__ __forceinline__ Ext sweep_proxies(const A &a, size_t i) {
     uint32_t t[15];
 #pragma unroll
     for (int r = 0; r < 15; ++r) t[r] = c0[rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz];
-    return proxy_ext_interior<true>(t);
+    return proxy_ext_interior(t);
 }
 template <class A>
 __device__ __forceinline__ Ext sweep_proxies_face(const A &a, size_t i, int x, int y, int z) {
@@ -311,7 +311,7 @@ __device__ __forceinline__ Ext sweep_proxies_face(const A &a, size_t i, int x, i
     const uint32_t valid = valid_mask(x, y, z, a.g.nx, a.g.ny, a.g.nz);
 #pragma unroll
     for (int r = 0; r < 15; ++r) t[r] = ((valid >> r) & 1u) ? c0[rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz] : 0u;
-    return proxy_ext<true>(t);
+    return proxy_ext(t);
 }
 __device__ __forceinline__ bool sweep_interior(const Geom &g, int x, int y, int z) {
     return x >= 1 && x <= g.nx - 2 && y >= 1 && y <= g.ny - 2 && z >= 1 && z <= g.nz - 2;
