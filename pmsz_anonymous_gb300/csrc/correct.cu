@@ -511,7 +511,7 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
     const size_t o_fr = ws.reserve<uint8_t>(groups), o_f0 = ws.reserve<uint8_t>(groups), o_f1 = ws.reserve<uint8_t>(groups);
     const size_t zero_bytes = ws.reserve<uint8_t>(0);
     const size_t o_codes = ws.reserve<uint8_t>(g.n);
-    const bool proxies = sizeof(T) == 8 || full;  // (fp32 sweeps compare the values themselves)
+    constexpr bool proxies = sizeof(T) == 8;  // (fp32 sweeps compare the values themselves)
     const size_t o_hp = ws.reserve<uint32_t>(proxies ? g.n : 0);
     // host-buffer calls of several slabs run sweeps 1 .. K behind the copy
     // (first_pass_waves; K below max_sweeps)
@@ -621,24 +621,23 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
     // The reference's schedule: every sweep over the whole field, host-driven.
     while (full && sweeps < max_sweeps) {
         SweepSlot *slot = slots + sweeps;
-        uint32_t *a_next = act[(sweeps + 1) & 1];
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[0], s));
         if (sweeps == 0 && ingest) {
-            if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, a_next, slot, g, s, &launches, maps,
+            if ((rc = first_pass_ingest<T>(*ingest, f, fh, codes, hp, req, act[1], slot, g, s, &launches, maps,
                                            &ls->err, nullptr, nullptr)))
                 return rc;
         } else if (sweeps == 0) {
-            if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, a_next, slot, g, 0,
+            if ((rc = launch_first_pass<T>(maps, tiled_grid(g), s, f, fh, codes, hp, req, act[1], slot, g, 0,
                                            &ls->err)))
                 return rc;
             ++launches;
         } else {
             PMSZ_CUDA((launch_march<T, kDetect>(
-                tiled_grid(g), s, MarchArgs<T>{nullptr, fh, codes, hp, req, a_next, slot}, g, 0)));
+                tiled_grid(g), s, MarchArgs<T>{nullptr, fh, codes, nullptr, req, nullptr, slot}, g, 0)));
             ++launches;
         }
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[1], s));
-        k_apply_px<T><<<list_grid(g), kListBlock, 0, s>>>(f, fh, cnt, hp, req, a_next, slot, g, eps, delta, q);
+        k_apply_full<T><<<list_grid(g), kListBlock, 0, s>>>(f, fh, cnt, req, slot, g, eps, delta, q);
         ++launches;
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[2], s));
         PMSZ_CUDA(cudaGetLastError());

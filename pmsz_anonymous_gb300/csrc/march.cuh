@@ -39,7 +39,8 @@
 // warps instead of one lane per warp, no second kernel and no global list.
 // The same holds for voxels whose two codes differ and that need the rules,
 // and for values that may be NaN or the sentinel.  The queues are emptied when
-// one could overflow in the next plane, and at the end.
+// one could overflow in the next plane, and at the end.  Where most certificates
+// of one field fail, the rest of the column needs none (march_tied).
 //
 // Bitmaps of a column.  A word of the request and mismatch bitmaps is one row
 // of one plane of the column: collected in shared memory and written once, with
@@ -47,12 +48,15 @@
 // fp32 first pass took 754 us, then 626; with the values compared directly on
 // ties 485).
 //
-// Measured at 512^3, issue-bound throughout: first pass fp64 1.50 -> 1.18 ms
-// (350 -> 220 warp instructions per 32 voxels), fp32 1.05 ms; codes alone
-// 0.58 ms fp64, 0.54 ms fp32.  One voxel per thread, 256-thread blocks, the two
+// Measured at 512^3, issue-bound throughout: first pass fp64 1.50 -> 1.14 ms
+// (350 -> 220 warp instructions per 32 voxels), fp32 1.00 ms; codes alone
+// 0.56 ms fp64, 0.53 ms fp32.  One voxel per thread, 256-thread blocks, the two
 // fields on different warps and 15 gathers per lane in the exact queue were all
 // slower.
 #pragma once
+#include <limits>
+#include <type_traits>
+
 #include "tiled.cuh"
 
 namespace pmsz {
@@ -88,6 +92,15 @@ __device__ __forceinline__ uint8_t tag_pair_code(uint32_t d) {  // two tag diffe
     return static_cast<uint8_t>(((t >> (4 * (d & 15u))) & 15u) | (((t >> (4 * ((d >> 4) & 15u))) & 15u) << 4));
 }
 
+__device__ __forceinline__ uint32_t rank_pair_tags(uint32_t code) {  // and back
+    constexpr uint64_t t = [] {
+        uint64_t v = 0;
+        for (int r = 0; r < 15; ++r) v |= static_cast<uint64_t>(stencil_tag(rank_dx(r), rank_dy(r), rank_dz(r))) << (4 * r);
+        return v;
+    }();
+    return (static_cast<uint32_t>(t >> (4 * (code & 15u))) & 15u) | ((static_cast<uint32_t>(t >> (4 * (code >> 4))) & 15u) << 4);
+}
+
 // Maximum and minimum of a set of tagged values.
 struct Ext2 {
     uint32_t hi, lo;
@@ -101,65 +114,120 @@ __device__ __forceinline__ Ext2 join(uint32_t a, uint32_t b, const Ext2 &c) {
     return Ext2{__vimax3_u32(a, b, c.hi), __vimin3_u32(a, b, c.lo)};
 }
 
-// Steepest ranks of one voxel on the full keys of v, gathered from global
-// memory five at a time (arg_ext's rule: ties by rank).  fp32 without NANS
-// (a correction refuses them after its first pass, and only the direction codes
-// order them): the values themselves, all 15 at once -- their extremes by max
-// and min, NaN standing for a point outside the domain, then the last rank that
-// holds the maximum and the first that holds the minimum; -0 and +0 are equal
-// in both forms.  A first pass over plateaus (256^3 fp32) takes 485 us instead
-// of 626, 311 M fp32 voxels with many ties 2.98 ms instead of 3.29.
-template <typename T, bool NANS>
-__device__ __forceinline__ void exact_ranks(const T *__restrict__ v, size_t i, const Geom &g, uint32_t valid,
-                                            int &asc, int &desc) {
+// Order-preserving signed keys: the magnitude bits, negated where the sign is set
+// (-0 and +0 are both 0; the order of okey, NaN included).
+__device__ __forceinline__ int32_t signed_key(float v) {
+    const int32_t b = __float_as_int(v), m = b >> 31;
+    return ((b & 0x7FFFFFFF) ^ m) - m;
+}
+__device__ __forceinline__ int64_t signed_key(double v) {
+    const int64_t b = __double_as_longlong(v), m = b >> 63;
+    return ((b & 0x7FFFFFFFFFFFFFFFll) ^ m) - m;
+}
+
+// Steepest ranks of one voxel on the values load(r) of its valid stencil points
+// (arg_ext's rule: ties by rank).  fp32 takes all 15 at once: their extremes by
+// max and min, then the last rank that holds the maximum and the first that holds
+// the minimum; without NANS (a correction refuses them after its first pass, and
+// only the direction codes order them) on the values themselves, NaN standing
+// for a point outside the domain, -0 and +0 equal in both forms.  A first pass
+// over plateaus (256^3 fp32) takes 485 us so instead of 626 on keys one by one, 311 M
+// fp32 voxels with many ties 2.98 ms instead of 3.29.  fp64: LOADS keys at a time.
+template <typename T, bool NANS, int LOADS, class Load>
+__device__ __forceinline__ void scan_ranks(Load load, uint32_t valid, int &asc, int &desc) {
+    asc = desc = kSelf;
     if constexpr (sizeof(T) == 4 && !NANS) {
-        const ptrdiff_t sy = g.nx, sz = static_cast<ptrdiff_t>(g.nx) * g.ny;
         T t[15];
 #pragma unroll
-        for (int r = 0; r < 15; ++r)
-            t[r] = ((valid >> r) & 1u) ? __ldg(v + (static_cast<ptrdiff_t>(i) + rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz))
-                                       : __int_as_float(0x7FC00000);
+        for (int r = 0; r < 15; ++r) t[r] = ((valid >> r) & 1u) ? load(r) : __int_as_float(0x7FC00000);
         T hi = t[0], lo = t[0];
 #pragma unroll
         for (int r = 1; r < 15; r += 2) {
             hi = fmaxf(fmaxf(hi, t[r]), t[r + 1]);
             lo = fminf(fminf(lo, t[r]), t[r + 1]);
         }
-        asc = desc = kSelf;
 #pragma unroll
         for (int r = 0; r < 15; ++r) {
             if (t[r] == hi) asc = r;
             if (t[14 - r] == lo) desc = 14 - r;
         }
-        return;
-    }
-    using K = typename KeyOf<T>::type;
-    const ptrdiff_t sy = g.nx, sz = static_cast<ptrdiff_t>(g.nx) * g.ny;
-    K bmax = 0, bmin = ~K(0);
-    asc = desc = kSelf;
+    } else {
+        using K = std::conditional_t<sizeof(T) == 4, int32_t, int64_t>;
+        K hi = std::numeric_limits<K>::min(), lo = std::numeric_limits<K>::max();
 #pragma unroll
-    for (int r0 = 0; r0 < 15; r0 += 5) {
-        K k[5];
+        for (int r0 = 0; r0 < 15; r0 += LOADS) {
+            T t[LOADS];
 #pragma unroll
-        for (int j = 0; j < 5; ++j) {
-            const int r = r0 + j;
-            const ptrdiff_t off = rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz;
-            k[j] = ((valid >> r) & 1u) ? okey(__ldg(v + (static_cast<ptrdiff_t>(i) + off))) : K(0);
-        }
+            for (int j = 0; j < LOADS; ++j) t[j] = ((valid >> (r0 + j)) & 1u) ? load(r0 + j) : T(0);
 #pragma unroll
-        for (int j = 0; j < 5; ++j) {
-            const int r = r0 + j;
-            if ((valid >> r) & 1u) {
-                if (k[j] >= bmax) { bmax = k[j]; asc = r; }
-                if (k[j] < bmin) { bmin = k[j]; desc = r; }
+            for (int j = 0; j < LOADS; ++j) {
+                const K k = signed_key(t[j]);
+                if ((valid >> (r0 + j)) & 1u) {
+                    if (k >= hi) { hi = k; asc = r0 + j; }
+                    if (k < lo) { lo = k; desc = r0 + j; }
+                }
             }
         }
     }
 }
 
+// The same on values that lie in shared memory: all at once, as they are where no
+// sign is set (their bits are in order then), else as keys.
+template <typename T, class Load>
+__device__ __forceinline__ void scan_tile(Load load, uint32_t valid, int &asc, int &desc) {
+    using K = std::conditional_t<sizeof(T) == 4, int32_t, int64_t>;
+    constexpr K kLow = std::numeric_limits<K>::min(), kHigh = std::numeric_limits<K>::max();
+    K k[15], signs = 0;
+#pragma unroll
+    for (int r = 0; r < 15; ++r) {
+        const T t = ((valid >> r) & 1u) ? load(r) : T(0);
+        if constexpr (sizeof(T) == 4) k[r] = __float_as_int(t);
+        else k[r] = __double_as_longlong(t);
+        signs |= k[r];
+    }
+    if (signs < 0) {
+#pragma unroll
+        for (int r = 0; r < 15; ++r) {
+            const K m = k[r] >> (8 * sizeof(K) - 1);
+            k[r] = ((k[r] & kHigh) ^ m) - m;
+        }
+    }
+    asc = desc = kSelf;
+    K hi = kLow, lo = kHigh;  // (beyond the keys of all values)
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+        for (int r = 0; r < 15; ++r) {
+            const bool in = ((valid >> r) & 1u) != 0u;
+            hi = max(hi, in ? k[r] : kLow);
+            lo = min(lo, in ? k[r] : kHigh);
+        }
+#pragma unroll
+        for (int r = 0; r < 15; ++r) {
+            if (((valid >> r) & 1u) && k[r] == hi) asc = r;
+            if (((valid >> (14 - r)) & 1u) && k[14 - r] == lo) desc = 14 - r;
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 15; ++r) {
+            const bool in = ((valid >> r) & 1u) != 0u;
+            if (in && k[r] >= hi) { hi = k[r]; asc = r; }
+            if (in && k[r] < lo) { lo = k[r]; desc = r; }
+        }
+    }
+}
+
+// The same on the field in global memory.
+template <typename T, bool NANS>
+__device__ __forceinline__ void exact_ranks(const T *__restrict__ v, size_t i, const Geom &g, uint32_t valid,
+                                            int &asc, int &desc) {
+    const ptrdiff_t sy = g.nx, sz = static_cast<ptrdiff_t>(g.nx) * g.ny;
+    const T *c = v + i;
+    scan_ranks<T, NANS, 5>([&](int r) { return __ldg(c + (rank_dx(r) + rank_dy(r) * sy + rank_dz(r) * sz)); }, valid, asc, desc);
+}
+
 // What a march reads and writes.  kFirst: f and fhat in, codes, the proxies
-// hp (fp32: or null), requests and mismatch bits out.  kDetect: the proxies hp (fhat for the
-// exact decisions) and the codes in, of every voxel.  kCodes: f in, codes out.  kPair: f and fh in, both
+// hp (fp64), requests and mismatch bits out.  kDetect: fhat and the codes in,
+// requests out, of every voxel.  kCodes: f in, codes out.  kPair: f and fh in, both
 // codes out and their differences counted, the values compared with a bound:
 // 71.5 M voxels fp64 684 us, where the codes of either field and a pass that
 // compares them took 658 + 308.
@@ -188,13 +256,22 @@ __device__ __forceinline__ uint64_t bits_mag(float v) { return __float_as_uint(v
 constexpr int kMHY = kMY + 2;        // rows of a tile, and with the halo
 constexpr int kMCells = kHX * kMHY;            // cells of a tile's plane
 constexpr int kPerThread = (kMCells + kThreads - 1) / kThreads;
-// Raw stages of planes (k+1 and k+2 in flight while plane k is computed), and
-// planes of proxies (k-1, k, then k+1 over k-2): plane k is in slot k mod 3 of
-// both, and the plane loop carries the slot along.
+// Planes of proxies (k-1, k, then k+1 over k-2): plane k is in slot k mod 3,
+// and the plane loop carries the slot along.  Raw stages: the planes k+1 and k+2
+// are in flight while plane k is computed, and the passes over one field keep
+// the values of k-2, k-1 and k as well, for the decisions in place.
 constexpr int kRing = 3;
+constexpr int raw_stages(int fields) { return fields == 1 ? 5 : kRing; }
 static_assert(kMarchMaxDepth <= 128 && kMY <= 16, "queue entries hold 7 bits of depth and 4 of the row");
 constexpr uint32_t kQueueFlush = 256;          // a queue longer than this is emptied after the plane
 constexpr uint32_t kQueueCap = kQueueFlush + 2 * kThreads;
+// One field: as many failed certificates within this many planes (a quarter of
+// their voxels; three quarters of one plane's) take the rest of a column to
+// march_tied.  At 255 in four planes, fields of ties take up to 3 % longer, at 128
+// in two, fields with some 4 %.
+constexpr uint32_t kTiedFlush = 192;
+constexpr int kTiedPlanes = 3;
+static_assert(kTiedFlush <= kQueueFlush, "the queue holds what is appended before it is emptied");
 
 // Queue entries: tx | row << 5 | (z - zb) << 9 | b << 16 | c << 24 with c the
 // code byte of the original.  Rules: b = the current field's tag differences.
@@ -244,7 +321,7 @@ __device__ __noinline__ void march_queues(MarchSmemOf<T, MODE> &sm) {
         uint32_t tm = detect_rules(static_cast<int>(asc), static_cast<int>(desc), static_cast<int>(c & 15u),
                                    static_cast<int>(c >> 4), cmax, cmin, cdir);
         if (!tm) return;
-        atomicOr(&sm.mism[lz * kMY + ly], 1u << lx);
+        if (MODE == kFirst) atomicOr(&sm.mism[lz * kMY + ly], 1u << lx);
         for (; tm; tm &= tm - 1) {
             const uint32_t r2 = 2u * static_cast<uint32_t>(__ffs(tm) - 1);
             const int cx = lx + static_cast<int>((kStepX >> r2) & 3u) - 1;
@@ -313,9 +390,6 @@ __device__ __noinline__ void march_queues(MarchSmemOf<T, MODE> &sm) {
     }
 }
 
-__device__ __forceinline__ uint32_t march_proxy(double v) { return proxy_of(v); }
-__device__ __forceinline__ uint32_t march_proxy(float v) { return proxy_of(v); }
-__device__ __forceinline__ uint32_t march_proxy(uint32_t p) { return p; }  // a stored proxy
 // Proxies outside [lo, hi) may belong to a NaN or to the sentinel 1e30 (fp64).
 // A NaN of high word 0xFFF00000 has the proxy of -inf, which is thus outside.
 template <typename T> struct PlainRange;
@@ -330,12 +404,82 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The rest of a column of one field, from plane k on (the voxels of plane k-1), where
+// many certificates fail, as on plateaus: every voxel is decided on the values
+// of the raw stages, with no proxies, and no queue but for the rules.  Through
+// the queue such a voxel costs about as much as six certified ones: its gather from
+// global memory, and the state rebuilt each time the queue is emptied.
+// Direction codes, queue -> here: 32 M voxels quantised to a hundred values fp32
+// 724 -> 312 us, fp64 1046 -> 478 (unquantised 165 and 174); a ramp of 17 M, all
+// ties, 386 -> 222 and 580 -> 291.  Four detections of 256^3 fp64 plateaus, every
+// voxel asking for edits: 2.9 -> 2.2 ms with their edits.  Bound by the ALU pipe:
+// about 80 (fp32) or 160 (fp64) compares and selects per voxel on half-rate units;
+// decided row by row inside the certified loop, both rows at once or out of
+// line, that loop or this one took 5 to 20 % longer.
+template <typename T, int MODE, bool FACE, class SRC>
+__device__ __forceinline__ void march_tied(MarchSmemOf<T, MODE> &sm, SRC &src, const MarchArgs<T> &a, const Geom &g, int x,
+                                           int y, int zb, int ctr, bool vin0, bool vin1, int k, int nplanes, int stage,
+                                           size_t i) {
+    constexpr int kStages = raw_stages(1);
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const size_t plane = static_cast<size_t>(g.nx) * g.ny;
+    auto stage_of = [&](int ahead) { return stage + ahead < kStages ? stage + ahead : stage + ahead - kStages; };
+#pragma unroll 1
+    while (k < nplanes) {
+        src.prefetch(k + 2, stage_of(2));
+        const int zrel = k - 2;
+        const T *z0 = src.values(stage_of(3)) + ctr, *z1 = src.values(stage_of(4)) + ctr, *z2 = src.values(stage) + ctr;
+        bool over = false;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const bool vin = r ? vin1 : vin0;
+            const size_t ir = i + (r ? static_cast<size_t>(g.nx) : 0);
+            uint32_t c = 0, code = 0;
+            if (vin) {
+                if (MODE == kDetect) c = a.codes[ir];
+                int asc, desc;
+                scan_tile<T>([&](int q) {
+                    return (rank_dz(q) < 0 ? z0 : rank_dz(q) > 0 ? z2 : z1)[rank_dx(q) + (rank_dy(q) + r) * kHX];
+                }, FACE ? valid_mask(x, y + r, zb + zrel, g.nx, g.ny, g.nz) : kAllValid, asc, desc);
+                code = static_cast<uint32_t>(asc | (desc << 4));
+                if (MODE == kCodes) a.codes[ir] = static_cast<uint8_t>(code);
+            }
+            if constexpr (MODE == kDetect) {
+                const bool rule = vin && (code != c || (FACE && c == 0x77u));
+                const uint32_t wr = __ballot_sync(0xFFFFFFFFu, rule);
+                if (wr) {
+                    uint32_t base = 0;
+                    if (tx == 0) base = atomicAdd(&sm.qn, static_cast<uint32_t>(__popc(wr)));
+                    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                    if (rule)
+                        sm.rq[base + static_cast<uint32_t>(__popc(wr & ((1u << tx) - 1u)))] =
+                            static_cast<uint32_t>(tx) | (static_cast<uint32_t>(2 * ty + r) << 5) |
+                            (static_cast<uint32_t>(zrel) << 9) | (rank_pair_tags(code) << 16) | (c << 24);
+                    over |= base + static_cast<uint32_t>(__popc(wr)) > kQueueFlush;
+                }
+            }
+        }
+        i += plane;
+        if (k + 1 < nplanes) src.wait(0, 0u);
+        over = __syncthreads_or(over) != 0;
+        ++k;
+        stage = stage_of(1);
+        if (MODE == kDetect && over) {
+            march_queues<T, MODE>(sm);
+            __syncthreads();
+            if (threadIdx.x == 0 && ty == 0) sm.qn = 0;
+            __syncthreads();
+        }
+    }
+    if (MODE == kDetect) march_queues<T, MODE>(sm);
+}
+
 // FACE: a block on a domain face, or one whose tile crosses the domain's far
 // end; the other blocks' tile, halo and planes zb-1 .. ze lie inside.
 template <typename T, int MODE, bool FACE, class SRC>
 __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, const MarchArgs<T> &a,
                                            const Geom &g, int bx, int by, int bz) {
-    constexpr int NF = march_pair(MODE) ? 2 : 1;
+    constexpr int NF = march_pair(MODE) ? 2 : 1, kStages = raw_stages(NF);
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTX + tx;
     const int x0 = bx * kTX, y0 = by * kMY, zb = bz * g.zc;
     const int ze = FACE ? min(g.nz, zb + g.zc) : zb + g.zc;
@@ -358,8 +502,8 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
             mine |= 1u << j;
     }
     auto plane_in = [&](int k) { return !FACE || (zb - 1 + k >= 0 && zb - 1 + k < g.nz); };
-    auto convert = [&](int k, int slot, uint32_t parity) {
-        src.wait(slot, parity);
+    auto convert = [&](int k, int slot, int stage, uint32_t parity) {
+        src.wait(stage, parity);
         if (!plane_in(k)) return;
         uint32_t *dst = &sm.p[slot][0][tid];
         const uint32_t tags = ctags + 0x020202u * (static_cast<uint32_t>(k) & 7u);
@@ -368,14 +512,14 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
             if (j == kPerThread - 1 && tid + j * kThreads >= kMCells) break;
             const uint32_t tag = (tags >> (8 * j)) & 15u;
 #pragma unroll
-            for (int F = 0; F < NF; ++F) dst[F * kMCells + j * kThreads] = march_proxy(src.cell(slot, j, F)) | tag;
+            for (int F = 0; F < NF; ++F) dst[F * kMCells + j * kThreads] = proxy_of(src.cell(stage, j, F)) | tag;
             if constexpr (MODE == kPair) {
                 // One subtraction decides nearly all (GB300's fp64 pipe runs two
                 // operations per SM and cycle): fl(p - f) rounds monotonically
                 // and eps is representable, so |fl(p - f)| < eps means
                 // |p - f| < eps, and then p lies within [fl(f - eps), fl(f + eps)].
                 if (((mine >> j) & 1u) && k >= 1 && k < nplanes - 1) {
-                    const T fv = src.cell(slot, j, 0), pv = src.cell(slot, j, 1), d = pv - fv;
+                    const T fv = src.cell(stage, j, 0), pv = src.cell(stage, j, 1), d = pv - fv;
                     if (bits_mag(d) >= a.sure) {  // NaN included
                         beyond += !(fabs(d) <= a.eps);
                         clamped += !(pv >= fv - a.eps && pv <= fv + a.eps);
@@ -421,12 +565,13 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
     if (march_edits(MODE)) {
         for (int e = tid; e < nplanes * kMHY; e += kThreads) sm.req[e] = 0;
         for (int e = tid; e < (nplanes * kMHY + 15) / 16; e += kThreads) sm.edge[e] = 0;
-        for (int e = tid; e < (nplanes - 2) * kMY; e += kThreads) sm.mism[e] = 0;
+        if (MODE == kFirst)
+            for (int e = tid; e < (nplanes - 2) * kMY; e += kThreads) sm.mism[e] = 0;
     }
 #pragma unroll 1
     for (int k = 0; k < 3; ++k) {  // at least 3 planes
-        convert(k, k, 0u);
-        if (k == 0) src.prefetch(kRing, 0);
+        convert(k, k, k, 0u);
+        if (k == 0) src.prefetch(kRing, kRing % kStages);
     }
     __syncthreads();
 #pragma unroll 1
@@ -435,6 +580,9 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
     const uint32_t stag0 = stencil_tag(x, y, zb - 2);
     int k = 2;  // the next plane; it completes the voxels of plane k-1, z = zb + k - 2
     int slot = 2, next = 0;  // of planes k and k+1
+    int stage = 2;           // one field: of plane k (two fields: the slots)
+    int flushed = 2;         // the plane before which the queues were last empty
+    auto stage_of = [&](int ahead) { return stage + ahead < kStages ? stage + ahead : stage + ahead - kStages; };
     uint32_t parity = 1u;    // of plane k+1's stage
 #pragma unroll 1
     while (true) {
@@ -462,7 +610,7 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
 #pragma unroll 1
         while (!over && k < nplanes) {
             const int last = 3 - slot - next;  // the slot of plane k-1, and of k+2's stage
-            src.prefetch(k + 2, last);
+            src.prefetch(k + 2, NF == 1 ? stage_of(2) : last);
             const int zrel = k - 2;
             uint32_t was[2] = {0u, 0u};
             if (MODE == kDetect) {
@@ -498,7 +646,7 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
             for (int r = 0; r < 2; ++r) {
                 const bool vin = r ? vin1 : vin0;
                 const size_t ir = i + (r ? static_cast<size_t>(g.nx) : 0);
-                if (MODE == kFirst && vin && (sizeof(T) == 8 || a.hp))  // fhat's proxies
+                if (MODE == kFirst && sizeof(T) == 8 && vin)  // fhat's proxies
                     a.hp[ir] = sm.p[last][NF - 1][ctr + (r ? (FACE ? rc : kHX) : 0)] & ~15u;
                 const uint32_t cert0 = (S[0][0][r].hi ^ S[0][1][r].hi) & (S[0][0][r].lo ^ S[0][1][r].lo);
                 uint32_t cert = cert0;
@@ -553,25 +701,34 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
                         sm.rq[(base & 0xFFFFu) + static_cast<uint32_t>(__popc(wr & lower))] = here | (now << 16);
                     }
                     const uint32_t end = base + add;
-                    over |= (end & 0xFFFFu) > kQueueFlush || (end >> 16) > kQueueFlush;
+                    over |= (end & 0xFFFFu) > kQueueFlush || (end >> 16) > (NF == 1 ? kTiedFlush : kQueueFlush);
                 }
             }
             i += plane;
-            if (k + 1 < nplanes) convert(k + 1, next, parity);
+            if (k + 1 < nplanes) convert(k + 1, next, NF == 1 ? stage_of(1) : next, parity);
             // the barrier that ends the plane also tells whether a queue could
             // overflow in the next one (every appending warp knows its end)
             over = __syncthreads_or(over) != 0;
             src.release(k + 1, next);
             ++k;
+            if (NF == 1) stage = stage_of(1);
             slot = next;
             next = next == kRing - 1 ? 0 : next + 1;
             if (next == 0) parity ^= 1u;
         }
+        const uint32_t queued = sm.qn >> 16;
         march_queues<T, MODE>(sm);
         if (k >= nplanes) break;
         __syncthreads();
         if (tid == 0) sm.qn = 0;
         __syncthreads();
+        if constexpr (NF == 1) {
+            if (queued > kTiedFlush && k - flushed <= kTiedPlanes) {
+                march_tied<T, MODE, FACE>(sm, src, a, g, x, y, zb, ctr, vin0, vin1, k, nplanes, stage, i);
+                break;
+            }
+            flushed = k;
+        }
     }
     if (MODE == kCodes) return;
     if (MODE == kPair) {
@@ -603,7 +760,7 @@ __device__ __forceinline__ void march_body(MarchSmemOf<T, MODE> &sm, SRC &src, c
             }
         }
     }
-    for (int e = tid; e < (nplanes - 2) * kMY; e += kThreads)
+    for (int e = tid; MODE == kFirst && e < (nplanes - 2) * kMY; e += kThreads)
         if (sm.mism[e]) {
             const size_t w = word_of(g, x0, y0 + e % kMY, zb + e / kMY);
             a.act_next[w] = sm.mism[e];
@@ -629,12 +786,13 @@ __device__ __forceinline__ bool march_inside(const Geom &g, int bx, int by, int 
 //
 // CopySource: cp.async of single elements, any alignment and row length; every
 // thread copies and later converts its own cells, so a plane needs no barrier
-// between its arrival and its conversion.  prefetch(k) starts plane k into the
-// stage of plane k - 3, which this thread has converted.
+// between its arrival and its conversion.  prefetch(k) starts plane k into a
+// stage whose plane this thread has converted and, of one field, no thread reads
+// any more.  values(s): the tile in stage s, cell after cell.
 // ---------------------------------------------------------------------------
 template <typename R, int NF>
 struct CopyTile {
-    R raw[kRing][NF][kMCells];
+    R raw[raw_stages(NF)][NF][kMCells];
 };
 
 template <typename R, int NF, bool FACE>
@@ -685,38 +843,29 @@ struct CopySource {
     __device__ __forceinline__ R cell(int s, int j, int F) const {
         return ct->raw[s][F][threadIdx.y * kTX + threadIdx.x + j * kThreads];
     }
+    __device__ __forceinline__ const R *values(int s) const { return ct->raw[s][0]; }
     __device__ __forceinline__ void release(int, int) {}
 };
 
-// The element type a march streams: the field itself, or the stored proxies.
-template <typename T, int MODE> struct MarchRaw { using type = T; };
-template <typename T> struct MarchRaw<T, kDetect> { using type = uint32_t; };
-
 template <typename T, int MODE>
 struct CopyMarch {  // shared memory of a copy-fed march
-    CopyTile<typename MarchRaw<T, MODE>::type, march_pair(MODE) ? 2 : 1> raw;
+    CopyTile<T, march_pair(MODE) ? 2 : 1> raw;
     MarchSmemOf<T, MODE> m;
 };
 
 template <typename T, int MODE, bool FACE>
 __device__ __forceinline__ void march_copies(CopyMarch<T, MODE> &sm, const MarchArgs<T> &a, const Geom &g, int bx,
                                              int by, int bz) {
-    using R = typename MarchRaw<T, MODE>::type;
-    const R *v0, *v1 = nullptr;
-    if constexpr (MODE == kDetect) {
-        v0 = a.hp;
-    } else {
-        v0 = a.f;
-        v1 = a.fh;
-    }
-    CopySource<R, march_pair(MODE) ? 2 : 1, FACE> s(sm.raw, v0, v1, g, bx, by, bz);
+    CopySource<T, march_pair(MODE) ? 2 : 1, FACE> s(sm.raw, MODE == kDetect ? a.fh : a.f, a.fh, g, bx, by, bz);
     march_body<T, MODE, FACE>(sm.m, s, a, g, bx, by, bz);
 }
 
 // bz0: index of the first z-chunk the launch covers (a launch may cover a
 // z-range of chunks, e.g. the part of the field already copied in).
+// Six blocks per SM with one field (codes 512^3 fp64 611 -> 587 us, fp32 564 -> 552),
+// five with two, whose state does not fit 80 registers.
 template <typename T, int MODE>
-__global__ void __launch_bounds__(kThreads, 5) k_march(const __grid_constant__ MarchArgs<T> a,
+__global__ void __launch_bounds__(kThreads, march_pair(MODE) ? 5 : 6) k_march(const __grid_constant__ MarchArgs<T> a,
                                                        const __grid_constant__ Geom g, int bz0) {
     extern __shared__ __align__(128) unsigned char march_smem[];
     CopyMarch<T, MODE> &sm = *reinterpret_cast<CopyMarch<T, MODE> *>(march_smem);

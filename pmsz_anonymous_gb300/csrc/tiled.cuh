@@ -103,7 +103,6 @@ constexpr uint32_t kListCap = 8192;
 
 struct ListSmem {
     uint32_t list[kListCap];
-    uint32_t mask[kRoundWords];   // per-word result bits (mismatch / changed)
     uint32_t warp_tot[kListBlock / 32];
     uint32_t total;
 };
@@ -129,14 +128,12 @@ __device__ __forceinline__ bool load_round(const uint32_t *__restrict__ bm, size
     return __syncthreads_or(any != 0) != 0;
 }
 
-// Calls work(x, y, z, word_local) for every set bit of bitmap `bm` (clearing
-// the bitmap); a true result sets the voxel's bit in a per-word result mask,
-// and flush(w, mask) is then called once per word with a non-zero mask, by the
-// thread that owns the word.  Every thread of the block must call this.
+// Calls work(x, y, z) for every set bit of bitmap `bm` (clearing the bitmap).
+// Every thread of the block must call this.
 // One round (2048 words from `base`) of for_each_set_bit.
-template <class Work, class Flush>
+template <class Work>
 __device__ __forceinline__ void process_round(ListSmem &sm, uint32_t *__restrict__ bm, const Geom &g, size_t base,
-                                              Work &work, Flush &flush) {
+                                              Work &work) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     {
         uint32_t w8[kWordsPerThread];
@@ -146,7 +143,6 @@ __device__ __forceinline__ void process_round(ListSmem &sm, uint32_t *__restrict
 #pragma unroll
         for (int j = 0; j < kWordsPerThread; ++j) {
             if (w8[j]) bm[w0 + j] = 0;
-            sm.mask[t * kWordsPerThread + j] = 0;
             c += __popc(w8[j]);
         }
         uint32_t inc = c;
@@ -192,101 +188,53 @@ __device__ __forceinline__ void process_round(ListSmem &sm, uint32_t *__restrict
                 const int b = static_cast<int>(e & 31u);
                 int wx, y, z;
                 word_coords(g, base + wl, wx, y, z);
-                if (work(wx * 32 + b, y, z, wl)) atomicOr(&sm.mask[wl], 1u << b);
+                work(wx * 32 + b, y, z);
             }
             __syncthreads();
         }
-#pragma unroll
-        for (int j = 0; j < kWordsPerThread; ++j) {
-            const uint32_t m = sm.mask[t * kWordsPerThread + j];
-            if (w8[j] && m) flush(w0 + j, m);
-        }
-        __syncthreads();
     }
 }
 
-template <class Work, class Flush>
-__device__ __forceinline__ void for_each_set_bit(ListSmem &sm, uint32_t *__restrict__ bm, const Geom &g, Work &work,
-                                                 Flush &flush) {
+template <class Work>
+__device__ __forceinline__ void for_each_set_bit(ListSmem &sm, uint32_t *__restrict__ bm, const Geom &g, Work &work) {
     for (size_t base = static_cast<size_t>(blockIdx.x) * kRoundWords; base < g.nwords;
          base += static_cast<size_t>(gridDim.x) * kRoundWords)
-        process_round(sm, bm, g, base, work, flush);
+        process_round(sm, bm, g, base, work);
 }
 
 // ---------------------------------------------------------------------------
-// Apply with the proxy array: applyDeltaBuffer_local (pMSz.cu:623-645) on
+// The edits of a full sweep: applyDeltaBuffer_local (pMSz.cu:623-645) on
 // every requested vertex, in T:
 //   if |f - (fhat - delta)| <= eps && cnt < q-1 { fhat -= delta; cnt++ }
 //   else { cnt = q; fhat = f - eps }
-// the proxy of every changed value refreshed; ApplyFlush marks the closed
-// stencil of the changed vertices of a word in act_next (owner thread).
+// (The next full sweep looks at every voxel: no active set, no proxies.)
 // ---------------------------------------------------------------------------
 template <typename T>
 struct ApplyWork {
     const T *f;
     T *fh;
     uint8_t *cnt;
-    uint32_t *hp;
     Geom g;
     T eps, delta;
     int q;
-    uint32_t nreq = 0, nprog = 0;
-    __device__ __forceinline__ bool operator()(int x, int y, int z, uint32_t) {
-        const size_t v = flat(g, x, y, z);
-        const T old = __ldg(fh + v);
-        const uint8_t oc = __ldg(cnt + v);
-        const T fv = __ldg(f + v);
-        const T lowered = old - delta;
-        T nv;
-        uint8_t nc;
-        if (fabs(fv - lowered) <= eps && static_cast<int>(oc) < q - 1) {
-            nv = lowered;
-            nc = static_cast<uint8_t>(oc + 1);
-        } else {
-            nc = static_cast<uint8_t>(q);
-            nv = fv - eps;
-        }
-        fh[v] = nv;
-        cnt[v] = nc;
-        const bool chg = bits_of(old) != bits_of(nv);
-        if (chg) hp[v] = proxy_of(nv);
+    uint32_t nreq = 0, nchg = 0, nprog = 0;
+    __device__ __forceinline__ void operator()(int x, int y, int z) {
+        bool progressed;
+        nchg += apply_one(f, fh, cnt, flat(g, x, y, z), eps, delta, q, progressed);
         ++nreq;
-        nprog += (chg || nc != oc) ? 1u : 0u;
-        return chg;
-    }
-};
-
-struct ApplyFlush {
-    uint32_t *act_next;
-    Geom g;
-    uint32_t nchg = 0;
-    __device__ __forceinline__ void operator()(size_t w, uint32_t m) {
-        nchg += __popc(m);
-        int wx, y, z;
-        word_coords(g, w, wx, y, z);
-        mark_stencil(act_next, g, wx, y, z, m);
+        nprog += progressed ? 1u : 0u;
     }
 };
 
 template <typename T>
-__device__ __forceinline__ void apply_body(ListSmem &sm, const T *__restrict__ f, T *__restrict__ fh,
-                                           uint8_t *__restrict__ cnt, uint32_t *__restrict__ hp,
-                                           uint32_t *__restrict__ req, uint32_t *__restrict__ act_next, SweepSlot *slot,
-                                           const Geom &g, T eps, T delta, int q) {
-    ApplyWork<T> work{f, fh, cnt, hp, g, eps, delta, q};
-    ApplyFlush flush{act_next, g};
-    for_each_set_bit(sm, req, g, work, flush);
-    const uint32_t v[8] = {0u, 0u, 0u, work.nreq, flush.nchg, work.nprog, 0u, 0u};
-    block_flush_slot(slot, v);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kListBlock) k_apply_px(const T *__restrict__ f, T *__restrict__ fh,
-                                                         uint8_t *__restrict__ cnt, uint32_t *__restrict__ hp,
-                                                         uint32_t *__restrict__ req, uint32_t *__restrict__ act_next,
-                                                         SweepSlot *slot, Geom g, T eps, T delta, int q) {
+__global__ void __launch_bounds__(kListBlock) k_apply_full(const T *__restrict__ f, T *__restrict__ fh,
+                                                           uint8_t *__restrict__ cnt, uint32_t *__restrict__ req,
+                                                           SweepSlot *slot, Geom g, T eps, T delta, int q) {
     __shared__ ListSmem sm;
-    apply_body(sm, f, fh, cnt, hp, req, act_next, slot, g, eps, delta, q);
+    ApplyWork<T> work{f, fh, cnt, g, eps, delta, q};
+    for_each_set_bit(sm, req, g, work);
+    const uint32_t v[8] = {0u, 0u, 0u, work.nreq, work.nchg, work.nprog, 0u, 0u};
+    block_flush_slot(slot, v);
 }
 
 // Stop rule of the correction loop after a sweep (the slot of that sweep):
