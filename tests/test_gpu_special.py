@@ -74,3 +74,31 @@ def test_nans_of_every_payload_are_refused(cuda, shape, where, target, dtype):
         torch.cuda.synchronize()
         with A.Server(max_sweeps=40) as srv:
             assert srv.wait(srv.submit(dev[0], work, 1e-3))["status"] == capi.PMSZ_ERR_ARG, hex(bits)
+
+
+# beyond the sentinel (1e30) and down to the lowest values nothing is special: such
+# fields take the ordinary path, and a NaN or a sentinel among them is found
+@pytest.mark.parametrize("shape", [(34, 10, 34), (5, 9, 33), (37, 25, 100)], ids=str)
+@pytest.mark.parametrize("dtype,scale", [(np.float64, s) for s in (1e30, 1e35, -1e35, 1e308, -1e308)] +
+                         [(np.float32, s) for s in (1e35, -1e35, 3e38, -3e38)], ids=str)
+def test_huge_values(cuda, shape, dtype, scale):
+    from pmsz_anonymous_gb300 import capi
+    rng = np.random.default_rng(shape[0])
+    f = (rng.random(shape) * 0.5 + 0.25) * scale  # (|scale| itself does not occur)
+    eb = abs(scale) * 1e-2 if abs(scale) < 1e300 else 9e299
+    f = f.astype(dtype)
+    fh = (f + rng.uniform(-1, 1, shape) * eb * 0.9).astype(dtype)
+    ref, _, st, sw, recs = O.correct(f, fh, eb, max_sweeps=40)
+    for full in (False, True):
+        d = torch.from_numpy(fh).to(cuda)
+        r = api().correct(torch.from_numpy(f).to(cuda), d, eb, max_sweeps=40, full_sweeps=full)
+        assert (r.status, r.sweeps) == (st, sw)
+        np.testing.assert_array_equal(r.log[:, :5], recs)
+        np.testing.assert_array_equal(d.cpu().numpy().view(np.uint8), ref.view(np.uint8))
+    at = tuple(s // 2 for s in shape)
+    for bad in [np.nan, -np.nan] + ([1e30] if dtype is np.float64 else []):
+        for k in range(2):
+            pair = [f.copy(), fh.copy()]
+            pair[k][at] = bad
+            with pytest.raises(capi.PmszError):
+                api().correct(*[torch.from_numpy(a).to(cuda) for a in pair], eb, max_sweeps=40)
