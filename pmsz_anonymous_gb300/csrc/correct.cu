@@ -632,8 +632,7 @@ int correct_impl(const T *f, T *fh, size_t nx, size_t ny, size_t nz, double eb, 
                 return rc;
             ++launches;
         } else {
-            PMSZ_CUDA((launch_march<T, kDetect>(
-                tiled_grid(g), s, MarchArgs<T>{nullptr, fh, codes, nullptr, req, nullptr, slot}, g, 0)));
+            PMSZ_CUDA((launch_field<T, kDetect>(s, MarchArgs<T>{nullptr, fh, codes, nullptr, req, nullptr, slot}, g)));
             ++launches;
         }
         if (timing) PMSZ_CUDA(cudaEventRecord(et.ev[1], s));
@@ -699,8 +698,7 @@ int codes_impl(const T *v, size_t nx, size_t ny, size_t nz, uint8_t *codes, cuda
     if (rc) return rc;
     Geom g = make_geom(nx, ny, nz);
     g.zc = first_depth(nx, ny, nz, sizeof(T));
-    PMSZ_CUDA((launch_march<T, kCodes>(
-        tiled_grid(g), s, MarchArgs<T>{v, nullptr, codes, nullptr, nullptr, nullptr, nullptr}, g, 0)));
+    PMSZ_CUDA((launch_field<T, kCodes>(s, MarchArgs<T>{v, nullptr, codes, nullptr, nullptr, nullptr, nullptr}, g)));
     PMSZ_CUDA(cudaGetLastError());
     return PMSZ_OK;
 }

@@ -54,6 +54,7 @@
 // fields on different warps and 15 gathers per lane in the exact queue were all
 // slower.
 #pragma once
+#include <algorithm>
 #include <limits>
 #include <type_traits>
 
@@ -890,6 +891,46 @@ __global__ void __launch_bounds__(kThreads, march_pair(MODE) ? 5 : 6) k_march(co
 }
 
 // ---------------------------------------------------------------------------
+// Thin fields, kCodes and kDetect: one voxel per thread in storage order, its 15
+// values gathered.  A march works on 32 x 8 planes whatever part of them the field
+// fills, and of a field of one plane on three: a line of 2 M voxels is 62 500
+// blocks of 32 voxels.  The gathers win below a third of the cells in use (codes
+// of 2 M fp32 voxels, march and here: 1/8, a line, 180 and 38 us; 1/4, four planes two
+// voxels high, 65 and 44; 3/8, 300 planes three high, 53 and 45, but fp64 55 and
+// 60), in a single plane up to a half (four rows: 64 and 42, fp64 68 and 49; eight:
+// 45 and 41, 47 and 51).
+// ---------------------------------------------------------------------------
+inline bool march_thin(const Geom &g) {
+    const uint64_t used = static_cast<uint64_t>(g.nx) * static_cast<uint64_t>(g.ny),
+                   cells = column_planes(static_cast<size_t>(g.nx), static_cast<size_t>(g.ny), 1) * kTX * kMY;
+    return g.n < (static_cast<size_t>(1) << 32) && (3 * used < cells || (g.nz == 1 && 2 * used <= cells));
+}
+
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256) k_flat(const __grid_constant__ MarchArgs<T> a, const __grid_constant__ Geom g) {
+    uint32_t cmax = 0, cmin = 0, cdir = 0, active = 0;
+    const uint32_t n = static_cast<uint32_t>(g.n), step = gridDim.x * 256u;
+    for (uint64_t at = blockIdx.x * 256u + threadIdx.x; at < n; at += step) {
+        const uint32_t i = static_cast<uint32_t>(at), row = fdiv(i, g.div_nx), zz = fdiv(row, g.div_ny);
+        const int x = static_cast<int>(i - row * static_cast<uint32_t>(g.nx)),
+                  y = static_cast<int>(row - zz * static_cast<uint32_t>(g.ny)), z = static_cast<int>(zz);
+        int asc, desc;
+        exact_ranks<T, MODE == kCodes>(MODE == kCodes ? a.f : a.fh, i, g, valid_mask(x, y, z, g.nx, g.ny, g.nz), asc, desc);
+        if (MODE == kCodes) {
+            a.codes[i] = static_cast<uint8_t>(asc | (desc << 4));
+        } else {
+            const uint8_t c = a.codes[i];
+            request_targets(a.req, g, x, y, z, detect_rules(asc, desc, c & 15, c >> 4, cmax, cmin, cdir));
+            ++active;
+        }
+    }
+    if (MODE == kDetect) {
+        const uint32_t v[8] = {cmax, cmin, cdir, 0u, 0u, 0u, active, 0u};
+        block_flush_slot(a.slot, v);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // TmaSource (two fields): one thread issues, per plane, a
 // cp.async.bulk.tensor box of f and one of fhat (the tile with its one-voxel
 // halo, widened in x so that the box starts on a 16-byte boundary) into the
@@ -1039,6 +1080,14 @@ inline cudaError_t launch_march(dim3 grid, cudaStream_t s, const MarchArgs<T> &a
     const cudaError_t e = allow_smem(k_march<T, MODE>, sizeof(CopyMarch<T, MODE>));
     if (e != cudaSuccess) return e;
     k_march<T, MODE><<<grid, dim3(kTX, kThreads / kTX, 1), sizeof(CopyMarch<T, MODE>), s>>>(a, g, bz0);
+    return cudaGetLastError();
+}
+
+// kCodes or kDetect of a whole field.
+template <typename T, int MODE>
+inline cudaError_t launch_field(cudaStream_t s, const MarchArgs<T> &a, const Geom &g) {
+    if (!march_thin(g)) return launch_march<T, MODE>(tiled_grid(g), s, a, g, 0);
+    k_flat<T, MODE><<<static_cast<unsigned>(std::min<size_t>((g.n + 255) / 256, 152 * 16)), 256, 0, s>>>(a, g);
     return cudaGetLastError();
 }
 

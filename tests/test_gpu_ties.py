@@ -2,7 +2,7 @@
 proxies (csrc/march.cuh), where a row of 32 voxels is decided in place or voxel
 by voxel through the queue: rows with any number of tied voxels, infinities and
 NaN of every sign (codes order them by their keys), ragged tiles, shallow and
-deep columns.  Codes, fields and counters are whole numbers and bits: equal, no
+deep columns, and thin fields.  Codes, fields and counters are whole numbers and bits: equal, no
 tolerance."""
 import numpy as np
 import pytest
@@ -61,6 +61,8 @@ def _codes(f):
 
 
 SHAPES = [(1, 1, 40), (1, 2, 33), (9, 10, 34), (5, 17, 65), (12, 40, 100), (70, 40, 70)]
+# thin fields, whose voxels are decided one by one, and the first that are not
+THIN = [(1, 1, 1), (1, 1, 5000), (2, 1, 300), (700, 1, 33), (5, 900, 1), (3, 2, 65), (1, 4, 32), (1, 5, 32), (4, 3, 32), (1, 500, 17)]
 
 
 @pytest.fixture(params=[None, 7, 64], ids=["depth-by-size", "depth-7", "depth-64"])
@@ -70,7 +72,7 @@ def depth(request):
     api().tune_clear()
 
 
-@pytest.mark.parametrize("shape", SHAPES, ids=str)
+@pytest.mark.parametrize("shape", SHAPES + THIN, ids=str)
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("kind", ["ints", "ramp", "rows", "special"])
 def test_codes(cuda, shape, dtype, kind, depth):
@@ -81,7 +83,7 @@ def test_codes(cuda, shape, dtype, kind, depth):
     np.testing.assert_array_equal(got, _codes(f))
 
 
-@pytest.mark.parametrize("shape", SHAPES, ids=str)
+@pytest.mark.parametrize("shape", SHAPES + THIN, ids=str)
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("kind", ["ints", "ramp", "rows"])
 def test_full_sweeps(cuda, shape, dtype, kind, depth):
