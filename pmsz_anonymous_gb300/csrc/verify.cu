@@ -14,10 +14,11 @@
 // voxel, which its tile shares; the walks start from the few percent of voxels
 // that are exits.  Whole-field three-hop jumping (k_jump) needed five launches
 // over all voxels and a host read after each: 32.4 M voxels, codes and both label
-// kinds as int64, 1850 -> 722 us; verification of 71.5 M fp64 voxels 7.58 -> 2.8
-// ms.  It remains as the general form for chains
-// beyond the bounds of the tile and exit walks: a flag tells the host, the labels
+// kinds as int64, 1850 -> 722 us.  It remains as the general form, for fields a few
+// voxels thick and for what the walks leave: a flag tells the host, the labels
 // so far are valid ancestors, and jumping goes on from them to the fixpoint.
+// Chains beyond one walk's bound are walked on first, where the labels are not
+// yet finished.
 //
 // Verification replaces the reference's disabled check_consistency block
 // (pMSz.cu:3038-3126) and count_false_cases (pMSz.cu:1852-1870).
@@ -73,12 +74,22 @@ static inline unsigned grid_for(size_t n) {
     return static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 152 * 16)));
 }
 
-static int jump_to_roots(uint32_t *L, size_t n, unsigned int *d_flag, cudaStream_t s, int rounds) {
+// The labels of `kinds` arrays to their roots: together, with one read-back a round,
+// where they share the 129 MB L2, else one after the other (17 M voxels, both kinds
+// of a ramp: 564 us, together 595; 20 000 voxels 150 and 120).
+static int jump_to_roots(uint32_t *const *L, int kinds, size_t n, unsigned int *d_flag, cudaStream_t s, int rounds) {
+    if (kinds > 1 && kinds * n * sizeof(uint32_t) > (static_cast<size_t>(64) << 20)) {
+        for (int l = 0; l < kinds; ++l) {
+            const int rc = jump_to_roots(L + l, 1, n, d_flag, s, rounds);
+            if (rc) return rc;
+        }
+        return PMSZ_OK;
+    }
     unsigned int *h = static_cast<unsigned int *>(host_pinned(sizeof(unsigned int)));
     if (!h) return set_error(PMSZ_ERR_OOM, "pinned host allocation failed");
     for (int launch = 0; launch < 64; ++launch) {
         PMSZ_CUDA(cudaMemsetAsync(d_flag, 0, sizeof(unsigned int), s));
-        k_jump<<<grid_for(n), 256, 0, s>>>(L, n, d_flag, rounds);
+        for (int l = 0; l < kinds; ++l) k_jump<<<grid_for(n), 256, 0, s>>>(L[l], n, d_flag, rounds);
         PMSZ_CUDA(cudaGetLastError());
         PMSZ_CUDA(cudaMemcpyAsync(h, d_flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
         PMSZ_CUDA(cudaStreamSynchronize(s));
@@ -91,6 +102,8 @@ constexpr int kLX = 32, kLY = 16, kLZ = 16, kLTile = kLX * kLY * kLZ;
 constexpr int kLWarps = 16, kLThreads = 32 * kLWarps;
 constexpr uint32_t kLShell = kLTile - (kLX - 2) * (kLY - 2) * (kLZ - 2);  // most exits a tile can have
 constexpr int kWalkHops = 64;  // hops of an exit per launch (two per tile crossed)
+constexpr int kWalks = 8;      // launches: each goes on from where the last one's chains ended
+constexpr unsigned int kOpen = 1, kCycle = 2;  // flags: a walk ran out of hops; a chain in a tile does not end
 
 struct TileGrid {
     dim3 grid;         // tiles
@@ -117,7 +130,8 @@ struct TileRootsSmem {
 // labels of 32 M voxels 545 us, now 494); planes beyond the field are left out.
 // L[l][i] receives the label so far of nibble lo[l] (0: ascent, 4: descent),
 // exits[l] the tile's exits (global indices) and count[l] their number.  *flag is set if a chain does not end within the tile's voxel count
-// (a cycle: not the codes of a field).  Bound by shared-memory latency and
+// (a cycle: not the codes of a field).  gate (or null): nothing is done where it is
+// set.  Bound by shared-memory latency and
 // conflicts of the pointer chase (L1 78 % busy, issue 63 %): pointers are stored
 // as byte offsets, steps come from a shuffle, the in-tile test from rank masks,
 // and exits are handled by full warps behind the loop.  71.5 M voxels, one kind, with 8
@@ -128,7 +142,9 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
                                                           uint32_t *__restrict__ l1, int lo0, int lo1,
                                                           uint32_t *__restrict__ exits0, uint32_t *__restrict__ exits1,
                                                           uint32_t stride, uint32_t *__restrict__ count0,
-                                                          uint32_t *__restrict__ count1, unsigned int *flag, Geom g) {
+                                                          uint32_t *__restrict__ count1, unsigned int *flag,
+                                                          const unsigned int *gate, Geom g) {
+    if (gate && *gate) return;
     constexpr int NW = kLWarps, H = kLY / NW;  // rows of a plane per thread
     __shared__ TileRootsSmem<NL> sm;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -213,7 +229,7 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
             if (in) (l == 0 ? l0 : l1)[i] = origin + ((p >> 1) & 31u) + sy * ((p >> 6) & 15u) + sz * (p >> 10);
         }
     }
-    if (stuck) atomicOr(flag, 1u);
+    if (stuck) atomicOr(flag, kCycle);
     __syncthreads();  // the exits' labels come after the loop's
     // dx + 1, dy + 1, dz + 1 of every rank, two bits each (nibble 15 is no exit)
     constexpr auto steps = [](int axis) {
@@ -254,7 +270,9 @@ __global__ void __launch_bounds__(kLThreads) k_tile_roots(const uint8_t *__restr
 __global__ void __launch_bounds__(512) k_exit_walk(uint32_t *l0, uint32_t *l1, const uint32_t *__restrict__ exits0,
                                                    const uint32_t *__restrict__ exits1, uint32_t stride,
                                                    const uint32_t *__restrict__ count0,
-                                                   const uint32_t *__restrict__ count1, unsigned int *flag) {
+                                                   const uint32_t *__restrict__ count1, unsigned int *flag,
+                                                   const unsigned int *gate) {
+    if (gate && *gate) return;
     uint32_t *L = blockIdx.y ? l1 : l0;
     const uint32_t m = (blockIdx.y ? count1 : count0)[blockIdx.x];
     const uint32_t *list = (blockIdx.y ? exits1 : exits0) + static_cast<size_t>(blockIdx.x) * stride;
@@ -271,7 +289,7 @@ __global__ void __launch_bounds__(512) k_exit_walk(uint32_t *l0, uint32_t *l1, c
         L[e] = l;
         open |= hop == kWalkHops;
     }
-    if (__any_sync(0xFFFFFFFFu, open) && (threadIdx.x & 31) == 0) atomicOr(flag, 1u);
+    if (__any_sync(0xFFFFFFFFu, open) && (threadIdx.x & 31) == 0) atomicOr(flag, kOpen);
 }
 
 // Every voxel's label: that of its local root (roots and exits already hold
@@ -300,34 +318,46 @@ struct LabelRun {
     int lo[2] = {0, 4};
     int nl = 0;
     uint32_t *lists = nullptr;      // per label kind: the tiles' counts, then their exits
-    unsigned int *words = nullptr;  // the flag, and the jumping's
+    unsigned int *flag = nullptr, *jump = nullptr;  // chains beyond the bounds; the jumping's
     static size_t list_words(const TileGrid &t) { return t.tiles() * (static_cast<size_t>(t.stride) + 1); }
     uint32_t *counts(int l) const { return lists + static_cast<size_t>(l) * list_words(t); }
     uint32_t *exits(int l) const { return counts(l) + t.tiles(); }
-    // Lines, and fields a few rows thick: a tile holds 32 to 96 voxels, and
+    // Lines, and fields a few rows thick: a tile holds 16 to 96 voxels, and
     // nearly every chain leaves its tile.  They go to the general jumping at once
-    // (2 M voxels in a line: codes and labels 694 us by tiles, 562 so; a plane of
-    // 2048 x 2000: 206 by tiles, 577 so).
-    static bool general(const Geom &g) { return std::min(g.ny, kLY) * std::min(g.nz, kLZ) < 4; }
-    int roots(const uint8_t *codes, cudaStream_t s) {  // everything up to k_finish
-        PMSZ_CUDA(cudaMemsetAsync(words, 0, 2 * sizeof(unsigned int), s));
-        if (general(g)) {
-            const dim3 grid(static_cast<unsigned>(g.wpr), static_cast<unsigned>((g.ny + 7) / 8), static_cast<unsigned>(g.nz));
-            k_init_ptr<<<grid, dim3(32, 8, 1), 0, s>>>(codes, lo[0] == 0 ? L[0] : nullptr, nl == 2 ? L[1] : lo[0] == 4 ? L[0] : nullptr, g);
-            PMSZ_CUDA(cudaGetLastError());
-            PMSZ_CUDA(cudaMemsetAsync(words, 1, 1, s));  // (little-endian int 1)
-            return PMSZ_OK;
-        }
+    // (2 M voxels in a line: codes and labels 694 us by tiles, 562 so; 500 000 along
+    // y verified, 986 and 720; a plane of 2048 x 2000: 206 by tiles, 577 so).
+    static bool general(const Geom &g) {
+        const int rows = std::min(g.ny, kLY) * std::min(g.nz, kLZ);
+        return rows < 4 || rows * std::min(g.nx, kLX) <= 16;
+    }
+    int init(const uint8_t *codes, cudaStream_t s) {  // every voxel's neighbour
+        const dim3 grid(static_cast<unsigned>(g.wpr), static_cast<unsigned>((g.ny + 7) / 8), static_cast<unsigned>(g.nz));
+        k_init_ptr<<<grid, dim3(32, 8, 1), 0, s>>>(codes, lo[0] == 0 ? L[0] : nullptr, nl == 2 ? L[1] : lo[0] == 4 ? L[0] : nullptr, g);
+        PMSZ_CUDA(cudaGetLastError());
+        return PMSZ_OK;
+    }
+    int tile_roots(const uint8_t *codes, const unsigned int *gate, cudaStream_t s) {  // *flag |= 1 where chains go on
         if (nl == 2)
             k_tile_roots<2><<<t.grid, kLThreads, 0, s>>>(codes, L[0], L[1], lo[0], lo[1], exits(0), exits(1), t.stride,
-                                                         counts(0), counts(1), words, g);
+                                                         counts(0), counts(1), flag, gate, g);
         else
             k_tile_roots<1><<<t.grid, kLThreads, 0, s>>>(codes, L[0], nullptr, lo[0], 0, exits(0), nullptr, t.stride,
-                                                         counts(0), nullptr, words, g);
+                                                         counts(0), nullptr, flag, gate, g);
+        return walk(flag, gate, s);
+    }
+    int walk(unsigned int *f, const unsigned int *gate, cudaStream_t s) {  // one more walk of the exits
         const int last = nl - 1;
         k_exit_walk<<<dim3(static_cast<unsigned>(t.tiles()), static_cast<unsigned>(nl)), 512, 0, s>>>(
-            L[0], L[last], exits(0), exits(last), t.stride, counts(0), counts(last), words);
+            L[0], L[last], exits(0), exits(last), t.stride, counts(0), counts(last), f, gate);
         PMSZ_CUDA(cudaGetLastError());
+        return PMSZ_OK;
+    }
+    int roots(const uint8_t *codes, cudaStream_t s) {  // everything up to k_finish
+        PMSZ_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned int), s));
+        if (!general(g)) return tile_roots(codes, nullptr, s);
+        const int rc = init(codes, s);
+        if (rc) return rc;
+        PMSZ_CUDA(cudaMemsetAsync(flag, 1, 1, s));  // (little-endian int 1)
         return PMSZ_OK;
     }
     template <typename OUT>
@@ -336,14 +366,28 @@ struct LabelRun {
         PMSZ_CUDA(cudaGetLastError());
         return PMSZ_OK;
     }
-    // Chains beyond the bounds: the general jumping, from the labels so far.
-    int complete(cudaStream_t s, int rounds) {
-        for (int l = 0; l < nl; ++l) {
-            const int rc = jump_to_roots(L[l], g.n, words + 1, s, rounds);
-            if (rc) return rc;
+    // Chains beyond the walks' bounds, of `m` runs that have not been finished: more
+    // walks of their exits, each from the last one's ends (so 64 times as far), until
+    // none is open (*left 0) or, as on a cycle, for kWalks launches.  The other
+    // voxels need none: 8 M voxels in a ramp 4 x 4 wide, verified, 1850 us by jumping,
+    // 1488 so; 17 M of 64 planes 1502 and 1256.
+    static int walk_on(LabelRun *r, int m, unsigned int *left, cudaStream_t s) {
+        unsigned int *h = static_cast<unsigned int *>(host_pinned(sizeof(unsigned int)));
+        if (!h) return set_error(PMSZ_ERR_OOM, "pinned host allocation failed");
+        for (int launch = 0; launch < kWalks; ++launch) {
+            int rc;
+            PMSZ_CUDA(cudaMemsetAsync(r->jump, 0, sizeof(unsigned int), s));
+            for (int k = 0; k < m; ++k)
+                if ((rc = r[k].walk(r->jump, nullptr, s))) return rc;
+            PMSZ_CUDA(cudaMemcpyAsync(h, r->jump, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+            PMSZ_CUDA(cudaStreamSynchronize(s));
+            *left = *h;
+            if (!*left) break;
         }
         return PMSZ_OK;
     }
+    // The general jumping, from the labels so far.
+    int complete(cudaStream_t s, int rounds) { return jump_to_roots(L, nl, g.n, jump, s, rounds); }
 };
 
 template <typename OUT>
@@ -364,19 +408,21 @@ static int labels_run(const uint8_t *codes, size_t nx, size_t ny, size_t nz, OUT
     const size_t o_w = ws.reserve<unsigned int>(2), o_e = ws.reserve<uint32_t>(LabelRun::list_words(r.t) * r.nl);
     const size_t o_l = ws.reserve<uint32_t>(kInPlace ? 0 : r.g.n * r.nl);
     if ((rc = ws.commit())) return rc;
-    r.words = ws.at<unsigned int>(o_w);
+    r.flag = ws.at<unsigned int>(o_w);
+    r.jump = r.flag + 1;
     r.lists = ws.at<uint32_t>(o_e);
     for (int l = 0; l < r.nl; ++l)
         r.L[l] = kInPlace ? reinterpret_cast<uint32_t *>(out[l]) : ws.at<uint32_t>(o_l) + static_cast<size_t>(l) * r.g.n;
     unsigned int *h = static_cast<unsigned int *>(host_pinned(sizeof(unsigned int)));
     if (!h) return set_error(PMSZ_ERR_OOM, "pinned host allocation failed");
     if ((rc = r.roots(codes, s))) return rc;
-    PMSZ_CUDA(cudaMemcpyAsync(h, r.words, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+    PMSZ_CUDA(cudaMemcpyAsync(h, r.flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
     for (int l = 0; l < r.nl; ++l)
         if ((rc = r.finish<OUT>(l, out[l], s))) return rc;
     PMSZ_CUDA(cudaStreamSynchronize(s));
-    if (*h) {
-        if ((rc = r.complete(s, tuned_jump_rounds(nx, ny, nz)))) return rc;
+    if (unsigned int left = *h) {
+        if (!kInPlace && !LabelRun::general(r.g) && left == kOpen && (rc = LabelRun::walk_on(&r, 1, &left, s))) return rc;
+        if (left && (rc = r.complete(s, tuned_jump_rounds(nx, ny, nz)))) return rc;
         for (int l = 0; l < r.nl && !kInPlace; ++l)
             if ((rc = r.finish<OUT>(l, out[l], s))) return rc;
     }
@@ -396,7 +442,8 @@ static LabelRun both_kinds(size_t nx, size_t ny, size_t nz, uint32_t *as, uint32
     r.L[1] = ds;
     r.nl = 2;
     r.lists = lists;
-    r.words = words;
+    r.flag = words;
+    r.jump = words + 1;
     return r;
 }
 size_t label_list_words(size_t nx, size_t ny, size_t nz) {
@@ -433,7 +480,7 @@ int time_jump_rounds(const uint8_t *codes, size_t nx, size_t ny, size_t nz, cons
         for (int rep = 0; rep < 3; ++rep) {  // the first run of each candidate is a warm-up
             k_init_ptr<<<grid, dim3(32, 8, 1), 0, s>>>(codes, L, nullptr, g);
             PMSZ_CUDA(cudaEventRecord(et.ev[0], s));
-            if ((rc = jump_to_roots(L, g.n, ws.at<unsigned int>(o_flag), s, rounds[k]))) return rc;
+            if ((rc = jump_to_roots(&L, 1, g.n, ws.at<unsigned int>(o_flag), s, rounds[k]))) return rc;
             PMSZ_CUDA(cudaEventRecord(et.ev[1], s));
             PMSZ_CUDA(cudaEventSynchronize(et.ev[1]));
             float t = 0.f;
@@ -446,9 +493,11 @@ int time_jump_rounds(const uint8_t *codes, size_t nx, size_t ny, size_t nz, cons
 }
 
 // Voxels whose labels differ, the labels of both fields finished on the way
-// (hop: L holds local roots as before k_finish; else the labels themselves).
+// (hop: L holds local roots as before k_finish; else the labels themselves);
+// nothing where *gate is set.
 __global__ void __launch_bounds__(256) k_count_diff(const uint32_t *__restrict__ a, const uint32_t *__restrict__ b,
-                                                    size_t n, int hop, unsigned long long *out) {
+                                                    size_t n, int hop, const unsigned int *gate, unsigned long long *out) {
+    if (gate && *gate) return;
     constexpr int kPer = 8;
     uint32_t c = 0;
     const size_t step = static_cast<size_t>(gridDim.x) * blockDim.x;
@@ -486,13 +535,13 @@ int verify_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, double
     Workspace ws(s);
     const size_t o_c0 = ws.reserve<uint8_t>(g.n), o_c1 = ws.reserve<uint8_t>(g.n);
     const size_t o_l0 = ws.reserve<uint32_t>(with_labels ? g.n : 0), o_l1 = ws.reserve<uint32_t>(with_labels ? g.n : 0);
-    const size_t o_e = ws.reserve<uint32_t>(with_labels ? LabelRun::list_words(tiles) : 0), o_w = ws.reserve<unsigned int>(8);
+    const size_t o_e = ws.reserve<uint32_t>(with_labels ? 2 * LabelRun::list_words(tiles) : 0), o_w = ws.reserve<unsigned int>(3);
     const size_t o_cnt = ws.reserve<unsigned long long>(9);
     if ((rc = ws.commit())) return rc;
     uint8_t *c0 = ws.at<uint8_t>(o_c0), *c1 = ws.at<uint8_t>(o_c1);
     unsigned long long *cnt = ws.at<unsigned long long>(o_cnt);
     constexpr size_t kCounts = 9 * sizeof(unsigned long long);
-    unsigned long long *h = static_cast<unsigned long long *>(host_pinned(kCounts + 8 * sizeof(unsigned int)));
+    unsigned long long *h = static_cast<unsigned long long *>(host_pinned(kCounts + 2 * sizeof(unsigned int)));
     if (!h) return set_error(PMSZ_ERR_OOM, "pinned host allocation failed");
     PMSZ_CUDA(cudaMemsetAsync(cnt, 0, kCounts, s));
     const T eps = static_cast<T>(eb);
@@ -516,54 +565,71 @@ int verify_impl(const T *f, const T *fp, size_t nx, size_t ny, size_t nz, double
     // 1017 us, and 727 with both codes and the comparison in one pass); reading
     // that back first costs the others 15 us.
     const bool wanted[2] = {with_labels && got[4] != 0, with_labels && got[5] != 0};
-    // AS, then DS labels of both fields in the same two arrays; the flags of
-    // the runs are read once, at the end
+    // AS, then DS labels of both fields in the same two arrays
+    uint32_t *const L[2] = {ws.at<uint32_t>(o_l0), ws.at<uint32_t>(o_l1)};
+    unsigned int *flags = ws.at<unsigned int>(o_w);  // per kind: chains go on beyond the walks' bounds; then the jumping's
     auto run_of = [&](int kind, int field) {
         LabelRun r;
         r.g = g;
         r.nl = 1;
         r.lo[0] = 4 * kind;
-        r.L[0] = ws.at<uint32_t>(field ? o_l1 : o_l0);
+        r.L[0] = L[field];
         r.t = tiles;
-        r.lists = ws.at<uint32_t>(o_e);
-        r.words = ws.at<unsigned int>(o_w) + 2 * (2 * kind + field);
+        r.lists = ws.at<uint32_t>(o_e) + static_cast<size_t>(field) * LabelRun::list_words(tiles);
+        r.flag = flags + kind;
+        r.jump = flags + 2;
         return r;
     };
-    const bool jump = LabelRun::general(g);
-    for (int kind = 0; kind < 2; ++kind) {
-        if (!wanted[kind] || jump) continue;
-        for (int field = 0; field < 2; ++field)
-            if ((rc = run_of(kind, field).roots(field ? c1 : c0, s))) return rc;
-        k_count_diff<<<grid_for((g.n + 3) / 4), 256, 0, s>>>(ws.at<uint32_t>(o_l0), ws.at<uint32_t>(o_l1), g.n, 1,
-                                                             cnt + 6 + kind);
+    auto count = [&](int kind, int hop, const unsigned int *gate) -> int {
+        k_count_diff<<<grid_for((g.n + 3) / 4), 256, 0, s>>>(L[0], L[1], g.n, hop, gate, cnt + 6 + kind);
         PMSZ_CUDA(cudaGetLastError());
-    }
-    unsigned int words[8] = {};
-    if ((wanted[0] || wanted[1]) && !jump) {
+        return PMSZ_OK;
+    };
+    auto walk = [&](int kind, const unsigned int *gate) -> int {
+        for (int field = 0; field < 2; ++field)
+            if ((rc = run_of(kind, field).tile_roots(field ? c1 : c0, gate, s))) return rc;
+        return count(kind, 1, gate);
+    };
+    auto go_on = [&](int kind, bool tiled) -> int {  // from the labels so far to the end
+        unsigned int left = kOpen;
+        LabelRun r[2] = {run_of(kind, 0), run_of(kind, 1)};
+        if (tiled && (rc = LabelRun::walk_on(r, 2, &left, s))) return rc;
+        if (left && (rc = jump_to_roots(L, 2, g.n, flags + 2, s, tuned_jump_rounds(nx, ny, nz)))) return rc;
+        PMSZ_CUDA(cudaMemsetAsync(cnt + 6 + kind, 0, sizeof(unsigned long long), s));
+        return count(kind, left ? 0 : 1, nullptr);
+    };
+    unsigned int open[2] = {0, 0};
+    auto read_counts = [&]() -> int {
         unsigned int *hw = reinterpret_cast<unsigned int *>(h + 9);
         PMSZ_CUDA(cudaMemcpyAsync(h, cnt, kCounts, cudaMemcpyDeviceToHost, s));
-        PMSZ_CUDA(cudaMemcpyAsync(hw, ws.at<unsigned int>(o_w), 8 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+        PMSZ_CUDA(cudaMemcpyAsync(hw, flags, sizeof(open), cudaMemcpyDeviceToHost, s));
         PMSZ_CUDA(cudaStreamSynchronize(s));
-        std::memcpy(words, hw, sizeof(words));
+        std::memcpy(open, hw, sizeof(open));
         got[6] = h[6];
         got[7] = h[7];
-    }
-    const bool open[2] = {wanted[0] && (jump || (words[0] | words[2]) != 0), wanted[1] && (jump || (words[4] | words[6]) != 0)};
-    for (int kind = 0; kind < 2; ++kind) {
-        // chains beyond the walks' bounds: that kind once more, jumped to the fixpoint
-        if (!open[kind]) continue;
-        const int rounds = tuned_jump_rounds(nx, ny, nz);
-        for (int field = 0; field < 2; ++field) {
-            LabelRun r = run_of(kind, field);
-            if ((rc = r.roots(field ? c1 : c0, s)) || (rc = r.complete(s, rounds))) return rc;
+        return PMSZ_OK;
+    };
+    if (wanted[0] || wanted[1]) {
+        PMSZ_CUDA(cudaMemsetAsync(flags, 0, sizeof(open), s));
+        if (LabelRun::general(g)) {
+            for (int kind = 0; kind < 2; ++kind) {
+                if (!wanted[kind]) continue;
+                for (int field = 0; field < 2; ++field)
+                    if ((rc = run_of(kind, field).init(field ? c1 : c0, s))) return rc;
+                if ((rc = go_on(kind, false))) return rc;
+            }
+            if ((rc = read_counts())) return rc;
+        } else {
+            // both kinds, the second only where the first is done; else the arrays
+            // keep the first one's labels so far, and the walks go on from them
+            if (wanted[0] && (rc = walk(0, nullptr))) return rc;
+            if (wanted[1] && (rc = walk(1, wanted[0] ? flags : nullptr))) return rc;
+            if ((rc = read_counts())) return rc;
+            if (open[0]) {
+                if ((rc = go_on(0, true)) || (wanted[1] && (rc = walk(1, nullptr))) || (rc = read_counts())) return rc;
+            }
+            if (open[1] && ((rc = go_on(1, true)) || (rc = read_counts()))) return rc;
         }
-        PMSZ_CUDA(cudaMemsetAsync(cnt + 6 + kind, 0, sizeof(unsigned long long), s));
-        k_count_diff<<<grid_for((g.n + 3) / 4), 256, 0, s>>>(ws.at<uint32_t>(o_l0), ws.at<uint32_t>(o_l1), g.n, 0,
-                                                             cnt + 6 + kind);
-        PMSZ_CUDA(cudaGetLastError());
-        PMSZ_CUDA(cudaMemcpyAsync(h, cnt + 6 + kind, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-        PMSZ_CUDA(cudaStreamSynchronize(s));
-        got[6 + kind] = h[0];
     }
     out->dir_mismatch = got[0];
     out->ext_mismatch = got[1];

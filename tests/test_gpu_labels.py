@@ -127,3 +127,31 @@ def test_nibbles_beyond_the_ranks_stay_put(cuda, shape, share):
     a, d = api().labels(both)
     np.testing.assert_array_equal(a.cpu().numpy().ravel(), want[0])
     np.testing.assert_array_equal(d.cpu().numpy().ravel(), want[1])
+
+
+def _ridge(shape, sign):
+    """A line of voxels that rises (falls) along x for longer than the exit walks
+    go, in a field whose other chains are short: long chains of one kind only."""
+    rng = np.random.default_rng(21)
+    f = rng.random(shape)
+    f[shape[0] // 2, shape[1] // 2, :] = 10 + np.arange(shape[2]) * 0.01
+    return sign * f
+
+
+@pytest.mark.parametrize("shape", [(8, 9, 3000), (20, 33, 1500), (2, 3, 4000)], ids=str)
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("kind", ["up", "down", "ramp", "noise"])
+def test_verify_of_long_chains(cuda, shape, dtype, kind):
+    f = {"up": lambda: _ridge(shape, 1), "down": lambda: _ridge(shape, -1), "ramp": lambda: _field("ramp", shape),
+         "noise": lambda: np.random.default_rng(5).random(shape)}[kind]().astype(dtype)
+    rng = np.random.default_rng(9)
+    for change in ("some", "ridge"):
+        fp = f.copy()
+        if change == "some":
+            fp += (rng.random(shape) < 0.01) * dtype(0.5)
+        else:  # only the line itself: every chain that follows it is cut
+            fp[shape[0] // 2, shape[1] // 2, shape[2] // 3] += dtype(3 if kind != "down" else -3)
+        want = O.verify(f, fp, 0.25)
+        want["bound_strict"] = want.pop("bound_violations")
+        want["bound_beyond_clamp"] = int((~((fp >= f - dtype(0.25)) & (fp <= f + dtype(0.25)))).sum())
+        assert api().verify(_dev(f, cuda), _dev(fp, cuda), 0.25) == want
