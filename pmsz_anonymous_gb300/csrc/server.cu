@@ -127,6 +127,7 @@ public:
         j->t_submit = Clock::now();
         std::lock_guard<std::mutex> lk(mu_);
         if (stopping_) return set_error(PMSZ_ERR_ARG, "server is shutting down");
+        if (broken_) return set_error(PMSZ_ERR_CUDA, "the server's worker could not start");
         j->id = ++next_id_;
         *id = j->id;
         pending_.push_back(j.get());
@@ -299,14 +300,44 @@ private:
         return PMSZ_OK;
     }
 
-    void fail_all(int rc) {
-        std::lock_guard<std::mutex> lk(mu_);
-        for (Job *j : running_) {
-            j->status = rc;
-            j->done = true;
-            j->t_done = Clock::now();
+    // After a generation that failed: the running jobs end with `rc`, once nothing
+    // that it enqueued runs any more, and give back their budget and scratch.
+    void fail_running(int rc) {
+        cudaStreamSynchronize(s_);
+        cudaGetLastError();  // the failed call's: later launches are checked by it
+        std::vector<unsigned char *> scratch;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            for (Job *j : running_) {
+                if (!j->over) j->status = rc;
+                if (j->scratch) scratch.push_back(j->scratch);
+                j->scratch = nullptr;
+                used_ -= j->bytes;
+                j->t_done = Clock::now();
+                j->done = true;
+            }
+            running_.clear();
         }
-        running_.clear();
+        cv_done_.notify_all();
+        for (unsigned char *p : scratch) cudaFreeAsync(p, s_);
+    }
+
+    // Where the worker cannot start: nothing will run the jobs.
+    void fail_setup(int *flag) {
+        cudaGetLastError();
+        if (flag) cudaFreeHost(flag);
+        if (s_) cudaStreamDestroy(s_);
+        s_ = nullptr;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            broken_ = true;
+            for (Job *j : pending_) {
+                j->status = PMSZ_ERR_CUDA;
+                j->t_start = j->t_done = Clock::now();
+                j->done = true;
+            }
+            pending_.clear();
+        }
         cv_done_.notify_all();
     }
 
@@ -316,7 +347,7 @@ private:
         if (cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking) != cudaSuccess ||
             cudaHostAlloc(reinterpret_cast<void **>(&flag), sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
             cudaHostGetDevicePointer(reinterpret_cast<void **>(&dflag), flag, 0) != cudaSuccess) {
-            fail_all(PMSZ_ERR_CUDA);
+            fail_setup(flag);
             return;
         }
         *flag = 0;
@@ -361,7 +392,7 @@ private:
             for (Job *j : running_)
                 if (!j->over) (j->fd.elem_size == 4 ? (std::vector<Job *> &)g32.jobs : g64.jobs).push_back(j);
             if (step(g32, g64) != PMSZ_OK) {
-                fail_all(PMSZ_ERR_CUDA);
+                fail_running(PMSZ_ERR_CUDA);
                 continue;
             }
             // retire finished jobs (a waiter may release its job as soon as the lock is free)
@@ -414,6 +445,7 @@ private:
     uint64_t next_id_ = 0;
     size_t used_ = 0;
     bool stopping_ = false;
+    bool broken_ = false;  // the worker could not start
 };
 
 }  // namespace pmsz
