@@ -359,13 +359,17 @@ int pmsz_standin_f64(const double *f, double *fhat, size_t n, double eb, int kin
  * of each axis, and the element size for the tile depth) and kept in a
  * process-wide table that every entry point reads:
  *   zchunk      planes per tile column of the fused first pass and the other
- *               tiled passes (tile 32 x 8 x zchunk); candidates 8, 16, 32, 64;
- *               default 32.
- *   jump_rounds pointer-jumping rounds per launch of the label passes
- *               (pmsz_labels, pmsz_verify_*, the naive strategy): each launch
- *               lets every voxel take that many three-hop jumps before the
- *               host reads the convergence flag; candidates 1, 2, 4, 8;
- *               default 1.
+ *               full-field passes (tile 32 x 8 x zchunk); candidates 8, 16, 32,
+ *               64; more than 64 run as 64.  Without an entry the depth goes by
+ *               the number of columns, 4 to 64 planes; the tuner times that
+ *               depth, too, and where it is the fastest the class goes on
+ *               running by size (the entry reports the fastest candidate).
+ *   jump_rounds pointer-jumping rounds per launch of the general label passes,
+ *               which label fields a few voxels thick and chains beyond the
+ *               bounds of the tile passes (pmsz_labels, pmsz_verify_*, the naive
+ *               strategy): each launch lets every voxel take that many
+ *               three-hop jumps before the host reads the convergence flag;
+ *               candidates 1, 2, 4, 8; default 1.
  * pmsz_autotune_{f32,f64} times every candidate on the given device field pair
  * (the first pass on f / fhat, then the AS labels of f's codes) on `stream`,
  * records the fastest in the table and returns the measurements.  Results of
@@ -383,7 +387,7 @@ int pmsz_autotune_f32(const float *f, const float *fhat, size_t nx, size_t ny, s
 int pmsz_autotune_f64(const double *f, const double *fhat, size_t nx, size_t ny, size_t nz, pmsz_tune *out,
                       void *stream);
 /* Table entry of a shape class: returns 1 and fills *out if one is recorded,
- * else 0 and the defaults (negative: bad arguments). */
+ * else 0 with zchunk 32 and jump_rounds 1 (negative: bad arguments). */
 int pmsz_tune_get(size_t nx, size_t ny, size_t nz, size_t elem_size, pmsz_tune *out);
 /* The tile depth recorded for a batch's size class (ceil log2 of its total
  * voxels, ceil log2 of its field count, the element size): pmsz_correct_batch

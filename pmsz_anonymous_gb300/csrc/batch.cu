@@ -98,8 +98,7 @@ int MultiRun<T>::setup(const std::vector<FieldSpec<T>> &specs, int64_t max_sweep
         voxels += sp.nx * sp.ny * sp.nz;
         columns += column_planes(sp.nx, sp.ny, sp.nz);
     }
-    const int zc = batch_tune_known(voxels, n, sizeof(T)) ? march_depth(tuned_batch_zchunk(voxels, n, sizeof(T)))
-                                                          : default_depth(columns);  // one first-pass launch covers the batch
+    const int zc = batch_depth(voxels, n, sizeof(T), columns);  // one first-pass launch covers the batch
     for (int i = 0; i < n; ++i) {
         Geom g = make_geom(specs[i].nx, specs[i].ny, specs[i].nz);
         g.zc = zc;
@@ -198,19 +197,20 @@ int MultiRun<T>::set_zchunk(int zc) {
 
 template <typename T>
 int MultiRun<T>::tune_zchunk() {
-    int m = 0;
+    int m = 0, maxnz = 1;
     const int *cands = zchunk_candidates(&m);
-    int maxnz = 1;
-    for (const Inst<T> &I : host) maxnz = std::max(maxnz, I.g.nz);
+    uint64_t columns = 0;
+    for (const Inst<T> &I : host) {
+        maxnz = std::max(maxnz, I.g.nz);
+        columns += column_planes(static_cast<size_t>(I.g.nx), static_cast<size_t>(I.g.ny), static_cast<size_t>(I.g.nz));
+    }
     EventTimer et;
     int rc = et.init();
     if (rc) return rc;
-    int best = cands[0];
-    float best_ms = 0.f;
-    for (int c = 0; c < m; ++c) {
-        if ((rc = set_zchunk(cands[c])) || (rc = upload())) return rc;
-        float t_best = 0.f;
-        for (int rep = 0; rep < 3; ++rep) {  // the first run of each candidate is a warm-up
+    auto time = [&](int zc, float &t_best) -> int {  // best of two after a warm-up
+        if ((rc = set_zchunk(zc)) || (rc = upload())) return rc;
+        t_best = 0.f;
+        for (int rep = 0; rep < 3; ++rep) {
             PMSZ_CUDA(cudaMemsetAsync(zero_base, 0, zero_total, s));
             PMSZ_CUDA(cudaEventRecord(et.ev[0], s));
             if ((rc = launch_first_multi<T>(dinst, dtpre, n, tpre[n], s))) return rc;
@@ -220,13 +220,27 @@ int MultiRun<T>::tune_zchunk() {
             PMSZ_CUDA(cudaEventElapsedTime(&t, et.ev[0], et.ev[1]));
             if (rep > 0 && (t_best == 0.f || t < t_best)) t_best = t;
         }
-        if (c == 0 || t_best < best_ms) {
-            best_ms = t_best;
+        return PMSZ_OK;
+    };
+    int best = cands[0];
+    float best_ms = 0.f, t = 0.f;
+    for (int c = 0; c < m; ++c) {
+        if ((rc = time(cands[c], t))) return rc;
+        if (c == 0 || t < best_ms) {
+            best_ms = t;
             best = cands[c];
         }
         if (cands[c] >= maxnz) break;  // deeper columns are one chunk for every field
     }
-    record_batch_zchunk(voxels, n, sizeof(T), best);
+    // and the depth by size, where it is none of them (as autotune_impl)
+    const int own = default_depth(columns);
+    bool by_size = false;
+    if (own < cands[0]) {
+        if ((rc = time(own, t))) return rc;
+        by_size = t <= best_ms;
+    }
+    record_batch_zchunk(voxels, n, sizeof(T), best, by_size);
+    if (by_size) best = own;
     if ((rc = set_zchunk(best))) return rc;
     PMSZ_CUDA(cudaMemsetAsync(zero_base, 0, zero_total, s));
     return PMSZ_OK;

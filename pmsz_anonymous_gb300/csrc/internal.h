@@ -176,7 +176,9 @@ bool tune_known(size_t nx, size_t ny, size_t nz, size_t elem);
 // size), tuned over the whole table; and the candidate depths.
 int tuned_batch_zchunk(size_t voxels, int nfields, size_t elem);
 bool batch_tune_known(size_t voxels, int nfields, size_t elem);
-void record_batch_zchunk(size_t voxels, int nfields, size_t elem, int zc);
+// The depth a batch's first pass runs at, as first_depth.
+int batch_depth(size_t voxels, int nfields, size_t elem, uint64_t columns_planes);
+void record_batch_zchunk(size_t voxels, int nfields, size_t elem, int zc, bool by_size);
 const int *zchunk_candidates(int *count);
 template <typename T>
 int autotune_impl(const T *f, const T *fh, size_t nx, size_t ny, size_t nz, pmsz_tune *out, cudaStream_t s);

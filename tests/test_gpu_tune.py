@@ -136,3 +136,32 @@ def test_batch_results_do_not_depend_on_batch_tile_depth(cuda, tmp_path, zchunk)
         assert r.status == 0
     for (_, dfh, _), ref in zip(items, refs):
         np.testing.assert_array_equal(dfh.cpu().numpy().view(np.uint8), ref.view(np.uint8))
+
+
+def _first_pass_us(f, fh):
+    w, best = fh.clone(), []
+    for _ in range(25):
+        w.copy_(fh)
+        best.append(api().correct(f, w, 1e-3, timing=True).ms_first_pass * 1e3)
+    return min(best)
+
+
+# small fields run fastest at fewer planes than the tuner's candidates have: a
+# tuned call is no slower than an untuned one (27 us; at the shallowest
+# candidate 37), also from a saved table and in a batch
+def test_tuning_keeps_the_depth_by_size_where_it_wins(cuda, tmp_path):
+    f, fh = (_dev(a, cuda) for a in _case((64, 64, 64), np.float64, "sz3", 1e-3, 2))
+    untuned = _first_pass_us(f, fh)
+    t = api().autotune(f, fh)
+    assert api().tune_get(f.shape, f.dtype) == (True, {"zchunk": t["zchunk"], "jump_rounds": t["jump_rounds"]})
+    tuned = _first_pass_us(f, fh)
+    path = str(tmp_path / "table.txt")
+    api().tune_save(path)
+    api().tune_clear()
+    api().tune_load(path)
+    assert api().tune_get(f.shape, f.dtype) == (True, {"zchunk": t["zchunk"], "jump_rounds": t["jump_rounds"]})
+    loaded = _first_pass_us(f, fh)
+    assert max(tuned, loaded) < 1.2 * untuned, (untuned, tuned, loaded)
+    # an explicit depth is a depth again
+    api().tune_set(f.shape, f.dtype, 32, 1)
+    assert _first_pass_us(f, fh) > 1.5 * untuned

@@ -226,3 +226,24 @@ def test_python_api_rejects_host_tensors_without_gpu():
         api.reconstruct(f, d, torch.zeros(0, dtype=torch.float64), 1e-3)
     with pytest.raises(TypeError):
         api.correct(f, f.clone(), 1e-3)
+
+
+def test_tuning_table_of_classes_that_run_by_size(lib, tmp_path):
+    # an 's' behind an entry; anything else there is refused, and setting a depth ends it
+    a, b = str(tmp_path / "a.txt"), str(tmp_path / "b.txt")
+    lib.pmsz_tune_clear()
+    try:
+        open(a, "w").write("pmsz-tune 1\n4 6 6 6 8 2 s\n8 6 6 6 16 2\nb 4 20 3 8 s\nb 8 20 3 16\n")
+        assert lib.pmsz_tune_load(a.encode()) == capi.PMSZ_OK
+        assert lib.pmsz_tune_save(b.encode()) == capi.PMSZ_OK
+        assert sorted(open(b).read().splitlines()) == sorted(open(a).read().splitlines())
+        found, t = _tune(lib, (64, 64, 64), 4)
+        assert found == 1 and (t.zchunk, t.jump_rounds) == (8, 2)
+        assert lib.pmsz_tune_set(64, 64, 64, 4, ctypes.byref(capi.Tune(8, 2))) == capi.PMSZ_OK
+        assert lib.pmsz_tune_save(b.encode()) == capi.PMSZ_OK
+        assert "4 6 6 6 8 2" in open(b).read().splitlines()
+        for bad in ("4 6 6 6 8 2 t", "4 6 6 6 8 2 s s", "b 4 20 3 8 x", "b 4 20 3 8 s 1"):
+            open(a, "w").write(f"pmsz-tune 1\n{bad}\n")
+            assert lib.pmsz_tune_load(a.encode()) == capi.PMSZ_ERR_IO, bad
+    finally:
+        lib.pmsz_tune_clear()
