@@ -134,7 +134,6 @@ int MultiRun<T>::setup(const std::vector<FieldSpec<T>> &specs, int64_t max_sweep
     const size_t o_inst = ws.reserve<Inst<T>>(n);
     const size_t o_pre = ws.reserve<uint32_t>(2 * (n + 1));
     const size_t o_ctl = ws.reserve<SweepCtl>(1);
-    const size_t o_rep = ws.reserve<SweepReport>(n);
     const int rc = ws.commit();
     if (rc) return rc;
     zero_base = ws.at<unsigned char>(o_z);
@@ -148,7 +147,6 @@ int MultiRun<T>::setup(const std::vector<FieldSpec<T>> &specs, int64_t max_sweep
     dtpre = ws.at<uint32_t>(o_pre);
     dcpre = dtpre + (n + 1);
     ctl = ws.at<SweepCtl>(o_ctl);
-    report = ws.at<SweepReport>(o_rep);
     PMSZ_CUDA(cudaMemsetAsync(zero_base, 0, zero_total, s));
     return PMSZ_OK;
 }
@@ -176,7 +174,6 @@ SweepTable<T> MultiRun<T>::table() const {
     t.cpre = dcpre;
     t.n = n;
     t.chunks = cpre[n];
-    t.report = report;
     return t;
 }
 

@@ -104,7 +104,7 @@ struct SweepTable {
     const uint32_t *cpre = nullptr;  // n + 1 prefixes of sweep_chunks
     int n = 0;
     uint32_t chunks = 0;             // their total
-    SweepReport *report = nullptr;   // n
+    SweepReport *report = nullptr;   // n, or null: none wanted (a batch reads the slots)
 };
 struct SweepCtl {  // zero before the launch
     long long iters;  // sweeps run by the launch
@@ -153,7 +153,6 @@ struct MultiRun {
     Inst<T> *dinst = nullptr;
     uint32_t *dtpre = nullptr, *dcpre = nullptr;
     SweepCtl *ctl = nullptr;
-    SweepReport *report = nullptr;
     SweepSlot *slots = nullptr;
     unsigned char *zero_base = nullptr;  // the scratch that starts zeroed (counters, bitmaps, slots)
     size_t zero_total = 0;

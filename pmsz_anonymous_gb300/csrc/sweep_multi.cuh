@@ -242,10 +242,10 @@ __device__ __forceinline__ void first_chunk(const SweepTable<T> &t, uint32_t chu
     }
 }
 
-// What the host reads of each field once the launch has ended.
+// What the server reads of each field once the launch has ended.
 template <typename T>
 __device__ __forceinline__ void write_reports(const FieldMasks &m, const SweepTable<T> &t, int64_t it) {
-    for (int i = threadIdx.x; i < t.n; i += kSweepBlock) {
+    for (int i = threadIdx.x; t.report && i < t.n; i += kSweepBlock) {
         const Inst<T> &I = t.inst[i];
         if (!I.active) continue;
         SweepReport r{};
