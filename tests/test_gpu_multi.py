@@ -1,8 +1,7 @@
 """The sweeps of many fields in one launch (csrc/sweep_multi.cuh) where they can
 go wrong, against the CPU oracle: tables of one type and of both, fields of one
 voxel and of several chunks side by side, fields that stop at different sweeps,
-plateaus next to smooth fields (full keys per field), more log rows than one
-read brings back, jobs that join a running server.  Whole numbers and bits:
+plateaus next to smooth fields, more log rows than one read brings back, jobs that join a running server.  Whole numbers and bits:
 equal, no tolerance."""
 import numpy as np
 import pytest

@@ -1,7 +1,7 @@
 """The sweeps in one cooperative launch (csrc/sweep.cuh) where they can go
 wrong, against the CPU oracle: one group of words and several, sparse and dense
-sweeps, failed certificates beyond the buffer, the switch to full keys, limits
-on the sweeps, logs longer than what one read brings back.  Fields and
+sweeps, failed certificates beyond the buffer, limits on the sweeps, logs longer
+than what one read brings back.  Fields and
 counters are bits and whole numbers: equal, no tolerance."""
 import numpy as np
 import pytest
@@ -64,8 +64,8 @@ def test_limits(cuda, dtype, limit):
     _check(cuda, f, fh, eb, q=40, max_sweeps=limit)
 
 
-# chunks of 2, 4 and 8 groups (and more than one round of them per warp are
-# beyond any field that fits): the full-field sweeps are the reference here
+# chunks of 2, 4 and 8 groups (several rounds of them: test_gpu_rounds.py): the
+# full-field sweeps are the reference here
 @pytest.mark.parametrize("shape", [(120, 250, 500), (250, 256, 500), (401, 400, 410)], ids=str)
 def test_chunks(cuda, shape):
     A = api()

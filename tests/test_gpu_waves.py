@@ -1,7 +1,6 @@
 """The sweeps behind the host copy (k_sweep_wave in csrc/sweep.cuh): fields of
 several copy slabs whose planes begin inside a group of bitmap words, sparse and
-dense, with ties (full keys), and limits on the sweeps below and above the
-wavefront's, against the correction of the same field on the device.  Bits and
+dense, with ties, and limits on the sweeps below and above the wavefront's, against the correction of the same field on the device.  Bits and
 whole numbers: equal, no tolerance."""
 import numpy as np
 import pytest
