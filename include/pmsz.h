@@ -209,16 +209,15 @@ typedef struct pmsz_field {
 /*
  * pmsz_correct_batch: corrects `count` (1..4096) independent fields together --
  * the batched form of the c_loops call (pMSz.cu:1872-2074), which the
- * reference runs one field per program.  One fused first pass covers the tiles
- * of every field, multi-field sweeps follow while the fields' active sets are
- * large, and a single cooperative persistent launch finishes the light tail
- * with a per-field stop decision on the device.  Every field keeps its own
+ * reference runs one field per program.  One fused first pass per type covers
+ * the tiles of every field, and one cooperative launch runs the sweeps of all of
+ * them, of both types, with a per-field stop decision on the device (types one
+ * after the other where their scratch does not fit at once).  Every field keeps its own
  * scratch, sweep index and stop state, so fields[i].fhat ends bit-identical to
  * what pmsz_correct_* produces for that field alone, and results[i] /
  * statuses[i] (either may be NULL) are what that call would report (timing
- * fields 0).  Fields of both types may be mixed; they run as one batch per
- * type.  Returns PMSZ_OK if every field converged, else the first non-OK
- * status.
+ * fields 0).  Fields of both types may be mixed.  Returns PMSZ_OK if every
+ * field converged, else the first non-OK status.
  */
 int pmsz_correct_batch(const pmsz_field *fields, int count, const pmsz_opts *opts, pmsz_result *results,
                        int *statuses, void *stream);

@@ -59,7 +59,7 @@ __host__ __device__ __forceinline__ size_t group_count(const Geom &g) {
 }
 
 // The stencil's seven rows (dy, dz): (0,0) (1,0) (0,1) (1,1) (-1,0) (0,-1)
-// (-1,-1).  Row 0 holds dx = -1, 0, 1; rows 1-3 dx = 0, 1; rows 4-6 dx = -1, 0.
+// (-1,-1).  Row 0 holds dx = -1, 0, 1; rows 1-3 dx = -1, 0; rows 4-6 dx = 0, 1.
 constexpr int kSweepRows = 7;
 __host__ __device__ constexpr int step_row(int dy, int dz) {
     return dy == 0 && dz == 0 ? 0 : (dy > 0 || dz > 0 ? 0 : 3) + (dy != 0 ? 1 : 0) + (dz != 0 ? 2 : 0);
@@ -104,7 +104,7 @@ __device__ __forceinline__ void mark_words(uint32_t *act, uint8_t *flag, const G
         atomicOr(act + at, m);
         flag[at / kGroupWords] = 1;
     };
-    const uint32_t p = c | (c >> 1), n = (c | (c << 1)) & tail;  // the rows ahead hold dx = 0, 1, the rows behind -1, 0
+    const uint32_t p = c | (c >> 1), n = (c | (c << 1)) & tail;  // the rows ahead hold dx = -1, 0, the rows behind 0, 1
     put(w, p | n);
     if (yp) put(w + sy, p);
     if (zp) put(w + sz, p);

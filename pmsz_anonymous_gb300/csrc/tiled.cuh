@@ -1,10 +1,10 @@
-// tiled.cuh -- proxy-based sweep kernels, included by correct.cu after its
-// shared device helpers.
+// tiled.cuh -- the proxies that the stencil kernels compare (march.cuh and
+// sweep.cuh include this file), and the edits of full sweeps.
 //
 // GB300 executes integer compare / min / max (and FP32 min / max) on one
 // 64-lane-per-clock pipe per SM, so a 15-point argmax / argmin on 64-bit keys
-// (about five instructions per candidate) is what bounds the sweep, not HBM.
-// These kernels compare 32-bit PROXIES instead:
+// (about five instructions per candidate) would bound the sweeps, not HBM.
+// They compare 32-bit PROXIES instead:
 //
 //   proxy(v) = the high 28 bits of an order-preserving key, low 4 bits clear
 //
@@ -15,7 +15,8 @@
 // unique.  A second chain with the ranks reversed (15 - r) picks the LOWEST
 // rank among tied proxies; both chains agree exactly when the winner is
 // unique -- the exactness certificate.  Where they disagree (ties in the
-// truncated proxy) the voxel takes the exact path on full keys.
+// truncated proxy) the voxel takes the exact path on full keys.  (march.cuh packs
+// tags of the coordinates instead of ranks.)
 //
 // Out-of-domain stencil cells hold proxy 0: as `0 + r` they lose every max
 // chain (real proxies are >= 16), and the min chains add -16 (or -1) so that
