@@ -406,8 +406,8 @@ int first_pass_ingest(const HostIngest<T> &in, const T *f, T *fh, uint8_t *codes
 // copy ends, are small.  256x320x288 and 512^3 fp64: 2521 us and 11.46 ms; at
 // 4, 8, 12, 14, 16: 2538 and 11.64; at 12, 15, 16: 2626 and 11.51; without waves
 // 2718 and 13.02.  (As voxel lists, seven launches a piece: 3347 us and 11.80.)
-// With what the sweeps have gained since, 2410 us and 11.36 ms, up to 2680 us from box
-// to box.
+// With what the sweeps have gained since, 2410 us (up to 2680 from run to run) and
+// 11.35 ms.
 constexpr int kWaveAt[] = {8, 12, 14, 15, 16};
 static_assert(std::size(kWaveAt) < std::size(LoopState{}.bar), "a barrier counter for each");
 

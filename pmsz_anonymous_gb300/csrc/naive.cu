@@ -17,7 +17,7 @@
 // the changed voxels only; labels are compared as local roots, one hop short of
 // finished; extrema sweeps are enqueued a few at a time.  160x144x176 fp64, 32
 // passes: 3.7 ms with one voxel per thread, whole-field codes after each pass,
-// finished labels and a wait per pass, now 2.0 to 2.2 from box to box; the labels of
+// finished labels and a wait per pass, now 2.0 to 2.2 from run to run; the labels of
 // the 14 checks and repairs are half of that.
 //
 // Semantics per pass are the snapshot ones of the pMSz loop: an extrema sweep
